@@ -131,17 +131,18 @@ SW2D_HD double sw2d_scale_down(double x, int k) {
     const uint64_t r = q + ((rem > halfw || (rem == halfw && (q & 1))) ? 1 : 0);
     return sw2d_f64_from_bits(sign | r);
 }
-/* x/2 and x/4 as used by the step.  On the device the whole warp takes the
- * exponent decrement when every lane's operand is a normal number whose
- * result stays normal, and the binary64 product otherwise (both exact); the
- * host evaluates the product. */
+/* x/2 and x/4 as used by the step.  On the device an exponent decrement
+ * when the result stays normal, x itself when it is zero, and the binary64
+ * product for the rest (all exact); the host evaluates the product.  Each
+ * lane decides for itself: a zero among normal operands (dry or still cells)
+ * costs no binary64 operation. */
 #if defined(__CUDACC__)
 __device__ __forceinline__ double sw2d_pow2_down(double x, int k, double m) { /* m = 2^-k, k >= 1 */
 #if defined(__CUDA_ARCH__)
-    const uint64_t b = sw2d_f64_bits(x);
-    const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
-    if (__all_sync(__activemask(), e > (uint32_t)k && e != 0x7ffu))
-        return sw2d_f64_from_bits(b - ((uint64_t)k << 52));
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    const uint32_t e = hi & 0x7ff00000u, kk = (uint32_t)k << 20;
+    if (e - (kk + 0x00100000u) < 0x7fe00000u - kk) return __hiloint2double((int)(hi - kk), (int)lo);
+    if (((hi << 1) | lo) == 0u) return x;
 #endif
     return x * m;
 }
@@ -214,6 +215,31 @@ SW2D_HD double sw2d_div_const(double a, double d, double rd) {
     double q = a * rd;
     double e = sw2d_fma(-q, d, a);
     return sw2d_fma(e, rd, q);
+}
+
+/* The same quotient on the integer pipes (the sequence above is three
+ * binary64 operations, each 71 issue cycles of a GB300 warp): with md the
+ * 53-bit significand of d, ed its biased exponent and rc = floor(2^115 / md),
+ * the high half of (ma 2^11) rc is ma 2^62 / md less at most 2, so its top 56
+ * bits are the 55 or 56 quotient bits or one less; the exact remainder
+ * completes them and rounds.  Operands or quotients that are not normal take
+ * the sequence above. */
+typedef struct {
+    double d, rd;
+    uint64_t md, rc;
+    uint32_t ed;
+} sw2d_divisor;
+
+static inline sw2d_divisor sw2d_divisor_of(double d) { /* d > 0, on the host */
+    sw2d_divisor c;
+    const uint64_t u = sw2d_f64_bits(d);
+    c.d = d;
+    c.rd = 1.0 / d;
+    c.ed = (uint32_t)(u >> 52) & 0x7ffu;
+    c.md = (u & ((1ull << 52) - 1ull)) | (1ull << 52);
+    c.rc = (uint64_t)(((unsigned __int128)1 << 115) / c.md);
+    if (c.ed == 0u || c.ed == 0x7ffu) c.ed = 0u; /* not normal: always the plain sequence */
+    return c;
 }
 
 /* binary32 seed r ~ x^(-1/3) (relative error ~1e-7): exponent-halving bit
@@ -325,22 +351,28 @@ SW2D_HD double sw2d_rpow_manning(double x) {
  * a / b correctly rounded (round to nearest even) with integer and binary32
  * operations only, for the GB300's FP64 pipe, which runs at 1/64 of the
  * binary32 rate: a binary64 division there costs about as much as fifteen
- * binary64 multiplies, while this schoolbook long division in base 2^22
- * runs on the integer and binary32 pipes beside the step's other binary64
- * work.  For a and b normal and a normal quotient (every other case returns
- * the hardware a / b), with ma, mb the 53-bit significands scaled so that
- * ma / mb is in [1, 2):
- *   - quotient digits of 22, 22 and 10 bits, each estimated from the
- *     leading 32 bits of the running remainder times a binary32 reciprocal
- *     of mb (relative error ~2^-21, so the estimate is within a few units
- *     of the digit), then made exact by the integer remainder
- *     R' = R 2^k - d mb (computed modulo 2^64; the true value is below
- *     4 mb < 2^56) and corrected by whole steps of mb until 0 <= R' < mb;
- *   - the 55-bit quotient floor(ma 2^54 / mb) and the sticky bit R != 0
- *     give the 53-bit significand rounded to nearest even.
- * Being the correctly rounded quotient, the result is bit-identical to the
- * IEEE division on any machine (the CPU tests compare it with the host's
- * division over every class of operands). */
+ * binary64 multiplies, while this long division runs on the integer and
+ * binary32 pipes beside the step's other binary64 work.  For a and b normal
+ * and a normal quotient (a zero dividend returns the signed zero, every other
+ * case the hardware a / b), with ma, mb the 53-bit significands:
+ *   - the digits of (ma - mb) 2^55 / mb in steps of 22, 22 and 11 bits, each
+ *     estimated from the leading 32 bits of the signed running remainder
+ *     times a binary32 reciprocal of mb and subtracted exactly (the remainder
+ *     modulo 2^64).  Nothing corrects a digit but the next one: digits and
+ *     remainders carry signs, so an estimate that is off leaves a remainder
+ *     a few mb larger that the next digit takes up.  With the reciprocal off
+ *     by up to 2^-19 (the tests force 2^-20) the first digit is within 10 of
+ *     its value, the second within 100, the third within 0.3, |R| < 2^60;
+ *   - the third digit is biased by 0.35 and rounded down, so it is at most
+ *     the true one and less than 2 below it: one conditional subtraction
+ *     makes Q = floor(ma 2^55 / mb), 55 or 56 bits, and the sticky bit
+ *     R != 0 completes the rounding to 53 bits.
+ * The signed digits leave no data-dependent loop: on a GB300 one warp issues
+ * it in 127 cycles against 492 for a form that corrected every digit by
+ * steps of mb, and its latency is a fifth.  Being the correctly rounded
+ * quotient, the result is bit-identical to the IEEE division on any machine
+ * (the CPU tests compare it with the host's division over every class of
+ * operands). */
 SW2D_HD float sw2d_rcp_est(float x) {
 #if defined(__CUDA_ARCH__)
     float r;
@@ -355,65 +387,6 @@ SW2D_HD float sw2d_rcp_est(float x) {
 #endif
 }
 
-/* one base-2^k digit of R 2^k / mb: returns the digit, R becomes the new
- * remainder; rfk = 2^(k-8) / (mb >> 29) estimated in binary32 */
-SW2D_HD uint32_t sw2d_div_digit(uint64_t* R, uint64_t mb, int k, float rfk) {
-    const uint64_t r = *R;
-    uint32_t d = (uint32_t)((float)(uint32_t)(r >> 21) * rfk); /* truncating conversion */
-    int64_t rn = (int64_t)((r << k) - (uint64_t)d * mb);        /* exact: |true value| < 2^56 */
-    while (rn < 0) {
-        d--;
-        rn += (int64_t)mb;
-    }
-    while (rn >= (int64_t)mb) {
-        d++;
-        rn -= (int64_t)mb;
-    }
-    *R = (uint64_t)rn;
-    return d;
-}
-
-SW2D_HD double sw2d_div_rn(double a, double b) {
-    const uint64_t ua = sw2d_f64_bits(a), ub = sw2d_f64_bits(b);
-    const uint32_t ea = (uint32_t)(ua >> 52) & 0x7ffu, eb = (uint32_t)(ub >> 52) & 0x7ffu;
-    if (ea - 1u >= 0x7feu || eb - 1u >= 0x7feu) return a / b; /* zero, subnormal, inf, NaN */
-    const uint64_t M = (1ull << 52) - 1ull, H = 1ull << 52;
-    uint64_t ma = (ua & M) | H;
-    const uint64_t mb = (ub & M) | H;
-    int e = (int)ea - (int)eb + 1023;
-    if (ma < mb) {
-        ma <<= 1;
-        e -= 1;
-    }
-    if ((uint32_t)(e - 1) >= 0x7feu) return a / b; /* subnormal or overflowing quotient */
-    const float rf = sw2d_rcp_est((float)(uint32_t)(mb >> 29));
-    uint64_t R = ma - mb; /* the leading quotient bit is 1 */
-    const uint64_t d1 = sw2d_div_digit(&R, mb, 22, rf * 16384.0f);
-    const uint64_t d2 = sw2d_div_digit(&R, mb, 22, rf * 16384.0f);
-    const uint64_t d3 = sw2d_div_digit(&R, mb, 10, rf * 4.0f);
-    const uint64_t Q = H << 2 | d1 << 32 | d2 << 10 | d3; /* floor(ma 2^54 / mb), 55 bits */
-    uint64_t m = Q >> 2;
-    const uint64_t g = (Q >> 1) & 1ull, st = (Q & 1ull) | (R != 0 ? 1ull : 0ull);
-    m += g & (st | (m & 1ull));
-    /* the significand's leading bit carries into the exponent field; a
-     * significand rounded up to 2^53 carries once more */
-    return sw2d_f64_from_bits(((ua ^ ub) & (1ull << 63)) + ((uint64_t)(e - 1) << 52) + m);
-}
-
-/* ------------------------------------------------------------------------
- * sqrt(x) correctly rounded with integer and binary32 operations only (the
- * companion of sw2d_div_rn), for x positive and normal (every other x
- * returns the hardware sqrt).  With x = m 2^E, E even, m in [2^52, 2^54):
- *   - an estimate S0 of S = floor(sqrt(m 2^56)) (55 bits) from sqrt(f),
- *     f = m / 2^52, in a pair of binary32 numbers: a binary32 square root
- *     and one Newton correction (error ~2^-46, S0 within a few hundred units);
- *   - one correction by the exact 128-bit remainder N - S0^2 over 2 S0
- *     (binary32 estimate, S1 within a couple of units), then whole steps on
- *     the exact 64-bit remainder until 0 <= N - S^2 <= 2 S;
- *   - S and the sticky bit N - S^2 != 0 give the 53-bit significand rounded
- *     to nearest even (a square root is never exactly halfway).
- * Bit-identical to the IEEE square root (the CPU tests compare it with the
- * host's sqrt). */
 SW2D_HD uint64_t sw2d_umulhi(uint64_t a, uint64_t b) {
 #if defined(__CUDA_ARCH__)
     return __umul64hi(a, b);
@@ -422,6 +395,83 @@ SW2D_HD uint64_t sw2d_umulhi(uint64_t a, uint64_t b) {
 #endif
 }
 
+/* floor(x) as an integer, |x| < 2^31 */
+SW2D_HD int32_t sw2d_i32_floor_f32(float x) {
+#if defined(__CUDA_ARCH__)
+    return __float2int_rd(x);
+#else
+    return (int32_t)floorf(x);
+#endif
+}
+
+/* the significand q 2^-(2+n) of a result whose leading bit sits at 2^(54+n),
+ * rounded to 53 bits (nearest even; the sticky bit already or-ed into bit 0),
+ * with the biased exponent e of the case n = 0 */
+SW2D_HD double sw2d_round_pack(uint64_t q, uint32_t n, uint32_t e, uint64_t sign) {
+    const uint32_t sh = 2u + n;
+    const uint32_t rc = (2u << n) - 1u + ((uint32_t)(q >> sh) & 1u);
+    /* the significand's leading bit carries into the exponent field; a
+     * significand rounded up to 2^53 carries once more */
+    return sw2d_f64_from_bits(sign + ((uint64_t)(e + n - 1u) << 52) + ((q + rc) >> sh));
+}
+
+SW2D_HD double sw2d_div_by(double a, const sw2d_divisor* c) {
+    const uint64_t ua = sw2d_f64_bits(a);
+    const uint32_t ea = (uint32_t)(ua >> 52) & 0x7ffu;
+    const uint32_t e = ea - c->ed + 1022u;
+    if (ea - 1u >= 0x7feu || c->ed == 0u || e - 1u >= 0x7fdu) return sw2d_div_const(a, c->d, c->rd);
+    const uint64_t ma = (ua & ((1ull << 52) - 1ull)) | (1ull << 52);
+    uint64_t Q = sw2d_umulhi(ma << 11, c->rc) >> 7;
+    uint64_t R = (ma << 55) - Q * c->md;
+    if (R >= c->md) {
+        R -= c->md;
+        Q += 1ull;
+    }
+    return sw2d_round_pack(Q | (R != 0 ? 1ull : 0ull), (uint32_t)(Q >> 55), e, ua & (1ull << 63));
+}
+
+SW2D_HD double sw2d_div_rn(double a, double b) {
+    const uint64_t ua = sw2d_f64_bits(a), ub = sw2d_f64_bits(b);
+    const uint32_t ea = (uint32_t)(ua >> 52) & 0x7ffu, eb = (uint32_t)(ub >> 52) & 0x7ffu;
+    const uint64_t sign = (ua ^ ub) & (1ull << 63);
+    const uint32_t e = ea - eb + 1022u; /* biased exponent of a quotient below 1 (ma < mb) */
+    if (ea - 1u >= 0x7feu || eb - 1u >= 0x7feu || e - 1u >= 0x7fdu) {
+        if ((ua << 1) == 0 && eb - 1u < 0x7feu) return sw2d_f64_from_bits(sign); /* 0 / b */
+        return a / b; /* subnormal, inf, NaN; a quotient that is or may be subnormal or overflow */
+    }
+    const uint64_t M = (1ull << 52) - 1ull, H = 1ull << 52;
+    const uint64_t ma = (ua & M) | H, mb = (ub & M) | H;
+    const float rf = sw2d_rcp_est((float)(int32_t)(mb >> 29)); /* 2^29 / mb */
+    int64_t R = (int64_t)(ma - mb);
+    const int32_t d1 = (int32_t)((float)(int32_t)(R >> 22) * (rf * 32768.0f));
+    R = (int64_t)(((uint64_t)R << 22) - (uint64_t)(int64_t)d1 * mb);
+    const int32_t d2 = (int32_t)((float)(int32_t)(R >> 26) * (rf * 524288.0f));
+    R = (int64_t)(((uint64_t)R << 22) - (uint64_t)(int64_t)d2 * mb);
+    const int32_t d3 = sw2d_i32_floor_f32(sw2d_fmaf((float)(int32_t)(R >> 29), rf * 2048.0f, -0.35f));
+    R = (int64_t)(((uint64_t)R << 11) - (uint64_t)(int64_t)d3 * mb);
+    uint64_t Q = (1ull << 55) + ((uint64_t)(int64_t)d1 << 33) + ((uint64_t)(int64_t)d2 << 11) + (uint64_t)(int64_t)d3;
+    if (R >= (int64_t)mb) {
+        R -= (int64_t)mb;
+        Q += 1ull;
+    }
+    return sw2d_round_pack(Q | (R != 0 ? 1ull : 0ull), (uint32_t)(Q >> 55), e, sign);
+}
+
+/* ------------------------------------------------------------------------
+ * sqrt(x) correctly rounded with integer and binary32 operations only (the
+ * companion of sw2d_div_rn), for x positive and normal (every other x
+ * returns the hardware sqrt).  With x = m 2^E, E even, m in [2^52, 2^54),
+ * S = floor(sqrt(m 2^54)) (54 bits) is built from its leading 24 bits, a
+ * binary32 square root, and two signed digits of 15 bits, each the exact
+ * remainder over twice the root so far, estimated with a binary32
+ * reciprocal; the next digit takes up what an estimate is off by, the last
+ * one is biased by 0.2 and rounded down, so one comparison with the exact
+ * remainder completes it.  A 54-bit S decides the rounding by itself: its
+ * last bit is the half bit, and m 2^54 is never an odd square.
+ * Issue 72 cycles a warp on a GB300 against 185 for a form that corrected a
+ * 46-bit estimate on its 128-bit remainder by single steps.
+ * Bit-identical to the IEEE square root (the CPU tests compare it with the
+ * host's sqrt). */
 SW2D_HD float sw2d_sqrt_est(float x) {
 #if defined(__CUDA_ARCH__)
     float r;
@@ -441,62 +491,24 @@ SW2D_HD double sw2d_sqrt_rn(double x) {
     const uint32_t ex = (uint32_t)(ux >> 52);
     if (ex - 1u >= 0x7feu) return sqrt(x); /* negative, zero, subnormal, inf, NaN */
     const uint64_t H = 1ull << 52;
-    uint64_t m = (ux & (H - 1ull)) | H;
-    int E = (int)ex - 1075; /* x = m 2^E */
-    if (E & 1) {
-        m <<= 1;
-        E -= 1;
-    }
-    /* f = m / 2^52 in [1, 4) as fh + fl: fh its leading 24 bits (exact) */
-    const int big = (int)(m >> 53); /* f >= 2 */
-    const uint64_t mt = m >> (29 + big), ml = m & ((1ull << (29 + big)) - 1ull);
-    const float fh = sw2d_f32_from_bits(((uint32_t)(127 + big) << 23) | ((uint32_t)mt & 0x7fffffu));
-    const float fl = (float)(uint32_t)ml * sw2d_f32_from_bits((uint32_t)(127 - 52) << 23);
-    const float sh = sw2d_sqrt_est(fh);
-    const float d = sw2d_fmaf(-sh, sh, fh) + fl;      /* f - sh^2 */
-    const float corr = d * (0.5f * sw2d_rcp_est(sh)); /* Newton: sqrt(f) ~ sh + d / (2 sh) */
-    /* S0 = (sh + corr) 2^54: sh has 24 significant bits, so sh 2^54 is an
-     * integer; corr 2^54 (|corr| < 2^-16 for any seed within 2^-17 of
-     * sqrt(fh)) is taken to the nearest integer as 2^16 hi + lo, both in 32
-     * bits */
-    const uint32_t sb = sw2d_f32_bits(sh);
-    const int se = (int)(sb >> 23) - 127; /* sh in [1, 2): se = 0 (or 1 when sh rounds to 2) */
-    const uint64_t s_int = ((uint64_t)((sb & 0x7fffffu) | 0x800000u)) << (31 + se);
-    const float c = corr * 18014398509481984.0f; /* corr 2^54, |c| < 2^38 */
-    const int32_t chi = sw2d_i32_near_f32(c * 1.52587890625e-05f);
-    const int32_t clo = sw2d_i32_near_f32(sw2d_fmaf((float)chi, -65536.0f, c));
-    uint64_t S = s_int + (uint64_t)((int64_t)chi * 65536 + clo);
-    /* exact remainder N - S^2 in 128 bits, N = m 2^56 */
-    const uint64_t nh = m >> 8, nl = m << 56;
-    const uint64_t sl = S * S, sh2 = sw2d_umulhi(S, S);
-    const uint64_t rl = nl - sl;
-    const uint64_t rh = nh - sh2 - (nl < sl ? 1ull : 0ull);
-    /* r / 2^16 fits in a signed 64-bit number (|r| < 2^79: S0 within 2^22
-     * units); its estimate in binary32 from its two 32-bit halves, and
-     * 1 / (2 S) from S's top 32 bits (S < 2^56); the correction
-     * dl = r / (2 S) is below 2^22 */
-    const int64_t r16 = (int64_t)((rh << 48) | (rl >> 16));
-    const uint64_t ar = r16 < 0 ? (uint64_t)0 - (uint64_t)r16 : (uint64_t)r16;
-    const float rf = sw2d_fmaf(sw2d_f32_est_of_u32((uint32_t)(ar >> 32)), 4294967296.0f,
-                               sw2d_f32_est_of_u32((uint32_t)ar));
-    const float sf = sw2d_f32_est_of_u32((uint32_t)(S >> 24)) * 16777216.0f;
-    const float dl = rf * 65536.0f * (0.5f * sw2d_rcp_est(sf));
-    const int64_t di = (int64_t)sw2d_i32_near_f32(dl);
-    S += (uint64_t)(r16 < 0 ? -di : di);
-    int64_t r = (int64_t)((m << 56) - S * S); /* exact: |N - S^2| < 2^60 now */
-    while (r < 0) {
-        S--;
-        r += (int64_t)(2 * S + 1);
-    }
-    while (r > (int64_t)(2 * S)) {
-        r -= (int64_t)(2 * S + 1);
-        S++;
-    }
-    uint64_t q = S >> 2;
-    const uint64_t g = (S >> 1) & 1ull, st = (S & 1ull) | (r != 0 ? 1ull : 0ull);
-    q += g & (st | (q & 1ull));
-    const int eb = (E + 52) / 2 + 1023;
-    return sw2d_f64_from_bits(((uint64_t)(eb - 1) << 52) + q);
+    const uint32_t odd = (ex + 1u) & 1u; /* E = ex - 1075 odd */
+    const uint64_t m = ((ux & (H - 1ull)) | H) << odd;
+    /* f = m / 2^52 in [1, 4) truncated to 23 bits, its root in [1, 2) */
+    const float f = (float)(int32_t)(m >> 30) * 2.384185791015625e-07f;
+    const float sh = sw2d_sqrt_est(f);
+    const float rs = sw2d_rcp_est(sh) * 5.9604644775390625e-08f; /* 1 / (2 s0), s0 = sh 2^23 */
+    const int32_t s0 = (int32_t)(sh * 8388608.0f);
+    int64_t R = (int64_t)(m - ((uint64_t)s0 * (uint64_t)s0 << 6)); /* m - (s0 2^3)^2 */
+    /* S1 = s0 2^15 + c1, remainder m 2^24 - S1^2 */
+    const int32_t c1 = (int32_t)((float)(int32_t)(R >> 6) * (rs * 32768.0f));
+    const uint64_t S1 = ((uint64_t)s0 << 15) + (uint64_t)(int64_t)c1;
+    R = (int64_t)(((uint64_t)R << 24) - (uint64_t)(int64_t)c1 * (((uint64_t)s0 << 16) + (uint64_t)(int64_t)c1));
+    /* S = S1 2^15 + c2, remainder m 2^54 - S^2 */
+    const int32_t c2 = sw2d_i32_floor_f32(sw2d_fmaf((float)(int32_t)(R >> 15), rs * 32768.0f, -0.2f));
+    uint64_t S = (S1 << 15) + (uint64_t)(int64_t)c2;
+    R = (int64_t)(((uint64_t)R << 30) - (uint64_t)(int64_t)c2 * ((S1 << 16) + (uint64_t)(int64_t)c2));
+    if (R > (int64_t)(2 * S)) S++;
+    return sw2d_f64_from_bits(((uint64_t)((ex - odd + 1021u) >> 1) << 52) + ((S + 1ull) >> 1));
 }
 
 #endif /* SW2D_MATH_H */
