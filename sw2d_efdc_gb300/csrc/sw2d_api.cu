@@ -76,7 +76,7 @@ struct sw2d_handle {
     double* evap = nullptr;
     double* srcq = nullptr;
     double* partials = nullptr;
-    double* partials_f = nullptr;
+    Flight64* flight = nullptr;
     double* outlet = nullptr;
     DevClock* clk = nullptr;
     double* scratch = nullptr; /* 4 * rows * cols doubles, lazily */
@@ -129,8 +129,6 @@ struct sw2d_handle {
         p.nrain = nrain;
         p.nevap = nevap;
         p.nq = nq;
-        p.nblocks_cells = ((C + SW2D_BX - 1) / SW2D_BX) * ((R + SW2D_BY - 1) / SW2D_BY);
-        p.nblocks_faces = ((C + 1 + SW2D_BX - 1) / SW2D_BX) * ((R + 1 + SW2D_BY - 1) / SW2D_BY);
         p.outlet_cap = outlet_cap;
         p.pct_lake = 1.00 - cfg.frac_lwl;                  /* SW2D-EFDC.cu:627 */
         p.pct_land = 1.00 - (cfg.frac_int + cfg.frac_inf); /* SW2D-EFDC.cu:631 */
@@ -166,6 +164,8 @@ struct sw2d_handle {
         };
         p.kdx = pow2_exp(cfg.dx);
         p.kdy = pow2_exp(cfg.dy);
+        p.ddx = sw2d_divisor_of(cfg.dx);
+        p.ddy = sw2d_divisor_of(cfg.dy);
         p.rainw = rainw;
         p.src_idx = src_idx;
         p.rain = rain;
@@ -179,7 +179,7 @@ struct sw2d_handle {
         p.uu1 = uu1;
         p.vv1 = vv1;
         p.partials = partials;
-        p.partials_f = partials_f;
+        p.flight = flight;
         p.outlet = outlet;
         p.clk = clk;
         return p;
@@ -401,6 +401,7 @@ int launch_iterations(sw2d_handle* h, long long n) {
             }
             h->prof_iters++;
         }
+        fp64_launch_settle(p, h->stream);
         return sync_check(h);
     }
     int rc = build_graph(h);
@@ -409,6 +410,7 @@ int launch_iterations(sw2d_handle* h, long long n) {
     for (long long k = 0; k < full; k++) CK(cudaGraphLaunch(h->graph, h->stream));
     StepParams p = h->params();
     for (long long k = 0; k < rem; k++) fp64_launch_iteration(p, (int)(k & 1), h->stream, nullptr);
+    fp64_launch_settle(p, h->stream);
     CK(cudaGetLastError());
     return SW2D_OK;
 }
@@ -690,8 +692,8 @@ int sw2d_create(const sw2d_config* cfg, sw2d_handle** out) {
     }
     TRY(dalloc(&h->uu1, h->ncell));
     TRY(dalloc(&h->vv1, h->ncell));
-    TRY(dalloc(&h->partials, (size_t)h->params().nblocks_cells * 4 + 8));
-    TRY(dalloc(&h->partials_f, (size_t)h->params().nblocks_faces * 2 + 8));
+    TRY(dalloc(&h->partials, fp64_partials(h->R, h->C)));
+    TRY(dalloc(&h->flight, 1));
     TRY(dalloc(&h->clk, 1));
     TRY(dalloc(&h->rain, 4));
     TRY(dalloc(&h->srcq, 4));
@@ -745,7 +747,7 @@ int sw2d_destroy(sw2d_handle* h) {
     dfree(h->evap);
     dfree(h->srcq);
     dfree(h->partials);
-    dfree(h->partials_f);
+    dfree(h->flight);
     dfree(h->outlet);
     dfree(h->clk);
     dfree(h->scratch);

@@ -2,22 +2,29 @@
  * reference's own kernels (SW2D-EFDC.cu:97-725).
  *
  * GB300's FP64 pipe runs at ~1/64 of the FP32 rate, so this path is bound by
- * FP64 instructions, not HBM.  The step is therefore split so that nothing
- * FP64 is computed twice, in two kernels per iteration:
+ * FP64 instructions, not HBM: one takes a warp 71 issue cycles of its SM
+ * quarter whether one lane or 32 take part.  The step is therefore split so
+ * that nothing FP64 is computed twice and what is computed runs on full
+ * warps, in two kernels per iteration:
  *   k64_flux   : new x/y face discharges of every face (flux, :97-353) from the
  *                stored face velocities uu1/vv1 of the previous iteration
- *                (the block's momentum faces packed into a list so that
- *                their binary64 update runs on full warps), and the CFL
- *                face-speed maxima of the entering state
- *   k64_update : per tile, the provisional depth (continuity at t,
- *                :602-664) -> "active and h* < th" flags in shared memory;
+ *                (momentum faces, weir and dry-bed faces and edge terms each
+ *                packed into a list per block), and the CFL face-speed
+ *                maxima of the entering state
+ *   k64_update : per tile, "active and h* < th" flags of the provisional depth
+ *                (continuity at t, :602-664) in shared memory, decided in
+ *                binary32 wherever its error allows;
  *                treat_error (:695-725, restated per face) and the final
  *                depth at t+dt; the closed faces written back and the face
  *                velocities uu1 = qx/hm, vv1 = qy/hn of the new state
- *                (hm_hn, uu1_vv1, :362-452); FP64 volume / rain / clamp /
- *                outlet sums by block reduction; the last block reduces the
- *                per-block partials in a fixed order and prepares the next
- *                iteration's length and forcing on the device.
+ *                (hm_hn, uu1_vv1, :362-452); partials of the ledger sums.  One
+ *                extra block adds up the previous iteration's partials in a
+ *                fixed order and prepares the next iteration's length and
+ *                forcing beside the tiles.
+ * At 4096 x 4096 (pond break, 120 s in) an iteration takes 2.44 ms against
+ * 5.17 ms with part-empty warps and a binary64 provisional depth; at 256 x
+ * 256 26 us against 62 us, most of it the clock's work at the end of the last
+ * tile's block before.
  * forward (:670-693) is a buffer swap for the depth (h[cur] -> h[nxt]); the
  * discharges keep fixed roles: qx[0]/qy[0] hold the state, k64_flux writes
  * its new faces into qx[1]/qy[1], and k64_update writes every face, closed
@@ -30,59 +37,54 @@
 #include "sw2d_internal.h"
 #include "sw2d_math.h"
 
+#include <algorithm>
+
 namespace sw2d {
 
 #define H SW2D_HALO
 
+/* the entry in force at `time`: sw2d_series_index with the division on the integer pipes */
+__device__ __forceinline__ int series_index(double time, double dts, int n) {
+    const double f = sw2d_div_rn(time, dts);
+    return f >= (double)n ? n : (int)f;
+}
+
 __device__ __forceinline__ double series_at(const double* v, int n, double dts, double time, int mode) {
-    double r;
-    int it;
-    if (mode == 0) { /* SW2D-EFDC.cu:546-551 */
-        if (time <= 1.00) {
-            r = v[0] * time;
-        } else {
-            it = sw2d_series_index(time, dts, n);
-            r = v[it] + (v[it + 1] - v[it]) / (dts * (time - dts * (it)));
-        }
-    } else if (mode == 1) {
-        it = sw2d_series_index(time, dts, n);
-        r = v[it] + (v[it + 1] - v[it]) * ((time - dts * (it)) / dts);
-    } else {
-        it = sw2d_series_index(time, dts, n);
-        r = v[it];
-    }
-    return r;
+    if (mode == 0 && time <= 1.00) return v[0] * time; /* SW2D-EFDC.cu:546-551 */
+    const int it = series_index(time, dts, n);
+    const double a = v[it];
+    if (mode == 2) return a;
+    const double b = v[it + 1], d = time - dts * (it);
+    return mode == 0 ? a + sw2d_div_rn(b - a, dts * d) : a + (b - a) * sw2d_div_rn(d, dts);
 }
 
 __device__ __forceinline__ double source_at(const StepParams& p, int i, double time) {
     double q;
     const double* Q = p.srcq;
     const int ns = p.nsrc;
-    if (p.series_mode == 0) { /* stream_flow SW2D-EFDC.cu:531-538 */
-        if (time <= 1.00) {
-            q = Q[i] * time;
-        } else {
-            const int it = sw2d_series_index(time, p.dtoq, p.nq);
-            q = Q[(size_t)it * ns + i] + (Q[(size_t)(it + 1) * ns + i] - Q[(size_t)it * ns + i]) /
-                                             (p.dtoq * (time - p.dtoq * (it)));
-        }
+    if (p.series_mode == 0 && time <= 1.00) { /* stream_flow SW2D-EFDC.cu:531-538 */
+        q = Q[i] * time;
     } else {
-        const int it = sw2d_series_index(time, p.dtoq, p.nq);
-        double a = Q[(size_t)it * ns + i];
-        if (p.series_mode == 1) {
-            double b = Q[(size_t)(it + 1) * ns + i];
-            q = a + (b - a) * ((time - p.dtoq * (it)) / p.dtoq);
-        } else {
-            q = a;
+        const int it = series_index(time, p.dtoq, p.nq);
+        const double a = Q[(size_t)it * ns + i];
+        q = a;
+        if (p.series_mode != 2) {
+            const double b = Q[(size_t)(it + 1) * ns + i], d = time - p.dtoq * (it);
+            q = p.series_mode == 0 ? a + sw2d_div_rn(b - a, p.dtoq * d) : a + (b - a) * sw2d_div_rn(d, p.dtoq);
         }
     }
-    return q / (p.dx * p.dy);
+    return sw2d_div_rn(q, p.dx * p.dy);
 }
 
-/* Length and forcing of the iteration that starts at time t (run by one
- * thread).  FIXED: the reference's loop (:4798, :4838, :4876).  CFL:
- * min(dt_max, cfl/s), shortened to end exactly at t_end. */
-__device__ void prepare_slot(const StepParams& p, Slot* s, double t, double smax, double t_end) {
+/* Length and forcing of the iteration that starts at time t, by one whole
+ * warp.  FIXED: the reference's loop (:4798, :4838, :4876).  CFL:
+ * min(dt_max, cfl/s), shortened to end exactly at t_end.  Every lane computes
+ * the length; the quotients and series values that follow from it are
+ * independent, so lane k computes the k-th of them (a binary64 operation
+ * costs a warp 71 cycles however many lanes take part, and a chain of nine
+ * divisions by one thread took longer than a small raster's tiles). */
+__device__ __forceinline__ void prepare_slot(const StepParams& p, Slot* s, double t, double smax, double t_end) {
+    const int lane = threadIdx.x & 31;
     double dt2, tm, tn;
     int active;
     if (p.dt_mode == 0) {
@@ -93,29 +95,31 @@ __device__ void prepare_slot(const StepParams& p, Slot* s, double t, double smax
         tn = tm + dt;
     } else {
         active = (t < t_end);
-        dt2 = smax > 0 ? fmin(p.dt_max, p.cfl / smax) : p.dt_max;
+        dt2 = smax > 0 ? fmin(p.dt_max, sw2d_div_rn(p.cfl, smax)) : p.dt_max;
         if (t + dt2 > t_end) dt2 = t_end - t;
         tm = t + 0.5 * dt2;
         tn = t + dt2;
     }
-    s->t = t;
-    s->t_mid = tm;
-    s->t_next = tn;
-    s->dt2 = dt2;
-    s->dt2dx = dt2 / p.dx;
-    s->dt2dy = dt2 / p.dy;
-    s->active = active;
-    s->rr1 = series_at(p.rain, p.nrain, p.dtrain, t, p.series_mode) / (p.dtrain * 1000.0);
-    s->rr2 = series_at(p.rain, p.nrain, p.dtrain, tm, p.series_mode) / (p.dtrain * 1000.0);
-    if (p.evap) {
-        s->ev1 = series_at(p.evap, p.nevap, p.dtrain, t, p.series_mode) / (p.dtrain * 1000.0);
-        s->ev2 = series_at(p.evap, p.nevap, p.dtrain, tm, p.series_mode) / (p.dtrain * 1000.0);
-    } else {
-        s->ev1 = s->ev2 = 0.0;
+    if (lane == 0) {
+        s->t = t;
+        s->t_mid = tm;
+        s->t_next = tn;
+        s->dt2 = dt2;
+        s->active = active;
     }
-    for (int k = 0; k < p.nsrc; k++) {
-        s->ql1[k] = source_at(p, k, t);
-        s->ql2[k] = source_at(p, k, tm);
+    if (lane < 2) (lane ? &s->dt2dy : &s->dt2dx)[0] = sw2d_div_rn(dt2, lane ? p.dy : p.dx);
+    if (lane < 4) { /* rain at t and tm, then evaporation */
+        const bool ev = lane >= 2;
+        const double* v = ev ? p.evap : p.rain;
+        double r = 0.0;
+        if (v)
+            r = sw2d_div_rn(series_at(v, ev ? p.nevap : p.nrain, p.dtrain, (lane & 1) ? tm : t, p.series_mode),
+                            p.dtrain * 1000.0);
+        (ev ? ((lane & 1) ? &s->ev2 : &s->ev1) : ((lane & 1) ? &s->rr2 : &s->rr1))[0] = r;
+    }
+    for (int k = lane; k < 2 * p.nsrc; k += 32) {
+        const int i = k >> 1;
+        ((k & 1) ? s->ql2 : s->ql1)[i] = source_at(p, i, (k & 1) ? tm : t);
     }
 }
 
@@ -144,11 +148,17 @@ __device__ __forceinline__ double friction(const StepParams& p, double coef, dou
 }
 
 /* a / dx for the continuity: exact scaling when dx is a power of two (the
- * constant-division sequence returns the same bits), else sw2d_div_const */
-__device__ __forceinline__ double div_spacing(double a, double d, double rd, int k) {
-    if (k < 0) return sw2d_div_const(a, d, rd);
+ * constant division returns the same bits), else sw2d_div_by */
+__device__ __forceinline__ double div_spacing(double a, const sw2d_divisor& d, int k) {
     if (sw2d_is0(a)) return 0.0;
-    return k == 0 ? a : sw2d_pow2_down(a, k, rd);
+    if (k < 0) return sw2d_div_by(a, &d);
+    return k == 0 ? a : sw2d_pow2_down(a, k, d.rd);
+}
+
+/* x is zero, or of a magnitude in [2^-400, 2^400] */
+__device__ __forceinline__ bool mid_range(double x) {
+    const uint32_t hi = (uint32_t)__double2hiint(x);
+    return ((hi & 0x7ff00000u) - (623u << 20) <= (800u << 20)) || ((hi << 1) | (uint32_t)__double2loint(x)) == 0u;
 }
 
 /* Upwind donor-cell transport across the edge between two neighbouring
@@ -158,10 +168,14 @@ __device__ __forceinline__ double div_spacing(double a, double d, double rd, int
  * with q0 the discharge of the face the edge is read from first.  The
  * reference evaluates every edge twice, once from each face beside it, with
  * the same operands in the same order (+ commutes exactly), so one
- * evaluation per edge gives bit-identical fluxes. */
+ * evaluation per edge gives bit-identical fluxes.  Halvings are exact while
+ * nothing is subnormal, so with operands in the middle of the exponent range
+ * the three of them are one quartering of the sum at the end. */
 __device__ __forceinline__ double edge_term(double w1, double w0, double q0, double q1) {
-    const double a = sw2d_half(w1 + w0);
-    return sw2d_half(a * (q1 + q0)) + sw2d_half(fabs(a) * (q0 - q1));
+    const double w = w1 + w0, qs = q1 + q0, qd = q0 - q1;
+    if (mid_range(w) && mid_range(qs) && mid_range(qd)) return sw2d_quarter(w * qs + fabs(w) * qd);
+    const double a = sw2d_half(w);
+    return sw2d_half(a * qs) + sw2d_half(fabs(a) * qd);
 }
 
 /* Kind of a face (SW2D-EFDC.cu:115-165, same tests in the same order):
@@ -169,62 +183,43 @@ __device__ __forceinline__ double edge_term(double w1, double w0, double q0, dou
  *   1 momentum (gravity, convection, friction)
  *   2 weir from side a, 3 weir from side b (a side's surface below the
  *     other side's bed), 4 dry-bed front (exactly one side above th).
- * Side a is the north (x faces) / west (y faces) cell.  The product
- * (hb - th) (ha - th) < 0 of the reference is decided from the two
- * comparisons with th (the differences keep the comparisons' signs and
- * their product of depths cannot underflow). */
-struct FaceK {
-    int kind;
-    bool wa, wb;
-    double ha, hb, za, zb, hha, hhb;
-};
-__device__ __forceinline__ FaceK classify(bool act, double ha, double hb, const double* __restrict__ z, size_t ia,
-                                          size_t ib, double th) {
-    FaceK f;
-    f.kind = 0;
-    f.ha = ha;
-    f.hb = hb;
-    f.wa = sw2d_gt_pos(ha, th);
-    f.wb = sw2d_gt_pos(hb, th);
-    f.za = f.zb = f.hha = f.hhb = 0.0;
-    if (!act || !(f.wa || f.wb)) return f;
-    f.za = z[ia];
-    f.zb = z[ib];
-    f.hhb = hb + f.zb;
-    f.hha = ha + f.za;
-    if (sw2d_lt(f.hhb, f.za)) f.kind = 2;
-    else if (sw2d_lt(f.hha, f.zb)) f.kind = 3;
-    else if ((f.wb && sw2d_lt_pos(ha, th)) || (f.wa && sw2d_lt_pos(hb, th))) f.kind = 4;
-    else f.kind = 1;
-    return f;
+ * Side a is the north (x faces) / west (y faces) cell, e = h + z its surface.
+ * The product (hb - th) (ha - th) < 0 of the reference is decided from the
+ * two comparisons with th (the differences keep the comparisons' signs and
+ * their product of depths cannot underflow).  A weir from a side at or below
+ * th carries nothing: closed. */
+__device__ __forceinline__ int classify(bool act, double ha, double hb, double ea, double eb, double za, double zb,
+                                        double th) {
+    const bool wa = sw2d_gt_pos(ha, th), wb = sw2d_gt_pos(hb, th);
+    if (!act || !(wa || wb)) return 0;
+    if (sw2d_lt(eb, za)) return wa ? 2 : 0;
+    if (sw2d_lt(ea, zb)) return wb ? 3 : 0;
+    return ((wb && sw2d_lt_pos(ha, th)) || (wa && sw2d_lt_pos(hb, th))) ? 4 : 1;
 }
 
-/* discharge of a non-momentum face */
-__device__ __forceinline__ double face_special(const FaceK& f, double th, double gg) {
-    switch (f.kind) {
-    case 2: return f.wa ? 0.5440 * f.ha * sw2d_sqrt_rn(gg * f.ha) : 0.0;
-    case 3: return f.wb ? -0.544 * f.hb * sw2d_sqrt_rn(gg * f.hb) : 0.0;
-    case 4:
-        if (sw2d_gt0(f.hb) || sw2d_gt0(f.ha)) {
-            const double hhan = (f.hb - th) - (f.ha - th);
-            const double sgnm = copysign(1.0, hhan);
-            const double hh3 = fmax(f.hhb, f.hha) - fmax(f.zb, f.za);
-            return -sgnm * 0.350 * hh3 * sw2d_sqrt_rn(2.00 * gg * hh3);
-        }
-        return 0.0;
-    default: return 0.0;
-    }
+__device__ __forceinline__ double max_ord(double a, double b) { return sw2d_gt(a, b) ? a : b; }
+
+/* Discharge of a weir or dry-bed face, (c d) sqrt(G d): d the depth on the
+ * weir's side, or the higher surface above the higher bed (:125-157). */
+__device__ __forceinline__ double face_special(bool from_a, double ha, double hb, double ea, double eb, double za,
+                                               double zb, double th, double gg) {
+    const bool k2 = from_a || sw2d_lt(eb, za), k3 = !k2 && sw2d_lt(ea, zb);
+    const bool wb = sw2d_gt_pos(hb, th);
+    double d = k2 ? ha : hb;
+    if (!(k2 || k3)) d = max_ord(eb, ea) - max_ord(zb, za);
+    const double c = k2 ? 0.5440 : k3 ? -0.544 : wb ? -0.350 : 0.350; /* -sign((hb - th) - (ha - th)) 0.350 */
+    return c * d * sw2d_sqrt_rn(((k2 || k3) ? gg : 2.00 * gg) * d);
 }
 
 /* momentum update of a face (SW2D-EFDC.cu:165-202 x, :282-319 y): along /
  * across are the face's two edge differences, already scaled. */
-__device__ __forceinline__ double face_momentum(const StepParams& p, const FaceK& f, double hm, double q0,
-                                                double u0, double vt, double along, double across,
-                                                double dt2, double dt2n, size_t ia, size_t ib) {
+__device__ __forceinline__ double face_momentum(const StepParams& p, double coef, double ha, double za, double eb,
+                                                double hm, double q0, double u0, double vt, double along,
+                                                double across, double dt2, double dt2n) {
     const double gg = p.g;
-    const double g13 = gg * hm * dt2n * (f.hhb - f.ha - f.za);
+    const double g13 = gg * hm * dt2n * (eb - ha - za);
     const double sq = sw2d_sqrt_rn(u0 * u0 + vt * vt); /* on the integer pipes, correctly rounded */
-    const double ram = friction(p, friction_coef(p, ib, ia), sq, hm);
+    const double ram = friction(p, coef, sq, hm);
     const double a = sw2d_half(dt2 * ram);
     /* the division on the integer pipes, correctly rounded (sw2d_div_rn) */
     return sw2d_div_rn((1.00 - a) * q0 + (-along - across - g13), 1.00 + a);
@@ -307,163 +302,196 @@ __device__ __forceinline__ void block_face_speed_max2(bool okx, double vx, doubl
     *sy = by;
 }
 
-__global__ void __launch_bounds__(SW2D_BX * SW2D_BY, 3) k64_flux(StepParams p, int cur) {
-    __shared__ float smf[2 * SW2D_BX * SW2D_BY / 32];
-    __shared__ unsigned long long smu[2 * SW2D_BX * SW2D_BY / 32];
-    /* momentum faces of the block, then the edges of the block's cells and of
-     * the row above / column left of it */
-    __shared__ unsigned char regx[SW2D_BY][SW2D_BX], regy[SW2D_BY][SW2D_BX];
-    __shared__ double sea[SW2D_BY + 1][SW2D_BX], sec[SW2D_BY + 1][SW2D_BX];
-    __shared__ double seb[SW2D_BY][SW2D_BX + 1], sed[SW2D_BY][SW2D_BX + 1];
-    /* the block's momentum faces, packed (thread << 1 | axis), so that the
-     * binary64 momentum update runs on full warps whatever the mix of face
-     * kinds (weir and dry-bed faces sit among momentum faces on steep thin
-     * films); hhb = hb + zb of each momentum face, kept from the
-     * classification */
-    __shared__ unsigned short mlist[2 * SW2D_BX * SW2D_BY];
-    __shared__ double mhhb[2 * SW2D_BX * SW2D_BY];
-    __shared__ int mwarp[SW2D_BX * SW2D_BY / 32 + 1];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int c = blockIdx.x * SW2D_BX + tx;
-    const int r = blockIdx.y * SW2D_BY + ty;
+/* raise a running maximum of non-negative doubles kept as bit patterns */
+__device__ __forceinline__ void raise_max(unsigned long long* at, double v) {
+    atomicMax(at, (unsigned long long)__double_as_longlong(v));
+}
+
+/* mean depth of a face >= th, exactly: decided from the two depths unless
+ * th lies between them, then in binary32, in binary64 only within its error */
+__device__ __forceinline__ bool mean_ge(double ha, double hb, float est, double th, float thf) {
+    const bool a = sw2d_ge_pos(ha, th), b = sw2d_ge_pos(hb, th);
+    if (a == b) return a;
+    if (fabsf(est - thf) > 1e-5f * thf) return est > thf;
+    return sw2d_ge_pos(sw2d_half(ha + hb), th);
+}
+
+/* The new discharges of the faces of a 32 x BY block of cells (north and
+ * west face of each), four block barriers:
+ *   1  the block and a ring around it staged in shared memory; the surface
+ *      h + z once per cell;
+ *   2  every thread classifies its two faces; momentum faces are listed from
+ *      the front of a list, weir and dry-bed faces from its back; closed faces
+ *      are written at once;
+ *   3  the edge terms some listed face reads are listed (from the rows'
+ *      bit masks), and the weir and dry-bed faces computed;
+ *   4  the edge terms, then the momentum faces, computed from their lists.
+ * What bounds it: a binary64 instruction takes a warp 71 cycles on a GB300
+ * whether one lane or all take part (measured), so the point of the lists is
+ * that every binary64 instruction runs on full warps and that x and y faces,
+ * the four kinds of edges and the three kinds of weir share one instruction
+ * stream each (they differ in shared-memory offsets and selected operands).
+ * CFL: face speeds estimated in binary32; a warp whose best estimate does
+ * not reach the running maximum is done, else its lanes within 1e-5 of the
+ * best are evaluated in binary64 and raise the maximum: the result is the
+ * exact maximum in any order. */
+template <int BY>
+__global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 4 : 16) k64_flux(StepParams p, int cur) {
+    constexpr int BX = SW2D_BX, NT = BX * BY, SW = BX + 2, NV = (BY + 2) * SW, NH = (BY + 1) * SW;
+    static_assert(BX == 32, "one row per warp: its ballot is the row's bit mask");
+    __shared__ double sh[NH], sz[NH], se[NH];         /* depth, bed, surface: rows -1 .. BY-1 */
+    constexpr int U = 0, V = NV, QX = 2 * NV, QY = 3 * NV;
+    __shared__ double sf[4 * NV];                     /* face velocities and discharges: rows -1 .. BY */
+    __shared__ double sedge[4 * NH];
+    __shared__ uint8_t sact[NH];
+    __shared__ unsigned short flist[2 * NT], elist[4 * NT + 2 * BX + 2 * BY];
+    __shared__ unsigned rowx[BY + 1], rowy[BY + 1];
+    __shared__ int cnt[3];
+    const int tx = threadIdx.x, ty = threadIdx.y, t = ty * BX + tx;
+    const int c0 = blockIdx.x * BX, r0 = blockIdx.y * BY;
+    const int c = c0 + tx, r = r0 + ty;
     const Slot& s = p.clk->slot[cur];
-    const bool in = (r <= p.R && c <= p.C);
-    const int P = p.P;
+    if (!s.active) return;
+    const double dt2 = s.dt2, dt2dx = s.dt2dx, dt2dy = s.dt2dy;
+    const int P = p.P, R = p.R, C = p.C;
     const size_t i = (size_t)(r + H) * P + (c + H);
-    const double* __restrict__ h = p.h[cur];
-    const double* __restrict__ umo = p.qx[0]; /* the state's discharges */
-    const double* __restrict__ vno = p.qy[0];
-    const double* __restrict__ uu1 = p.uu1;
-    const double* __restrict__ vv1 = p.vv1;
     const double th = p.th;
-    /* 1: classify the thread's x face (north of the cell) and y face (west) */
-    FaceK fx, fy;
-    fx.kind = fy.kind = 0;
-    const bool doX = in && s.active && c < p.C, doY = in && s.active && r < p.R;
-    const bool edgeS = doX && r == p.R && p.outflow_south;
-    if (doX && !edgeS) {
-        const uint8_t fe = p.flags[i], fw = p.flags[i - P];
-        fx = classify((fe & fw & SW2D_F_ACTIVE) != 0, h[i - P], h[i], p.z, i - P, i, th);
-    }
-    if (doY) {
-        const uint8_t fn = p.flags[i], fs = p.flags[i - 1];
-        fy = classify((fn & fs & SW2D_F_ACTIVE) != 0, h[i - 1], h[i], p.z, i - 1, i, th);
-    }
-    regx[ty][tx] = (unsigned char)(fx.kind == 1);
-    regy[ty][tx] = (unsigned char)(fy.kind == 1);
-    const int t = ty * SW2D_BX + tx, lane = t & 31, warp = t >> 5;
-    if (fx.kind == 1) mhhb[2 * t] = fx.hhb;
-    if (fy.kind == 1) mhhb[2 * t + 1] = fy.hhb;
-    const unsigned bx = __ballot_sync(0xffffffffu, fx.kind == 1), by = __ballot_sync(0xffffffffu, fy.kind == 1);
-    if (lane == 0) mwarp[warp] = __popc(bx) + __popc(by);
-    __syncthreads();
-    /* 2: each edge once, where a momentum face of the block reads it */
     {
-        const bool rx = regx[ty][tx], ry = regy[ty][tx];
-        const bool rxS = ty + 1 < SW2D_BY && regx[ty + 1][tx], ryS = ty + 1 < SW2D_BY && regy[ty + 1][tx];
-        const bool rxE = tx + 1 < SW2D_BX && regx[ty][tx + 1], ryE = tx + 1 < SW2D_BX && regy[ty][tx + 1];
-        sea[ty + 1][tx] = (rx || rxS) ? edge_term(uu1[i + P], uu1[i], umo[i], umo[i + P]) : 0.0;
-        seb[ty][tx + 1] = (rx || rxE) ? edge_term(vv1[i + 1], vv1[i - P + 1], umo[i], umo[i + 1]) : 0.0;
-        sec[ty + 1][tx] = (ry || ryS) ? edge_term(uu1[i + P], uu1[i + P - 1], vno[i], vno[i + P]) : 0.0;
-        sed[ty][tx + 1] = (ry || ryE) ? edge_term(vv1[i + 1], vv1[i], vno[i], vno[i + 1]) : 0.0;
-        if (ty == 0) { /* warp 0: the row above, read by the first row's faces */
-            const size_t u = i - P;
-            sea[0][tx] = rx ? edge_term(uu1[u + P], uu1[u], umo[u], umo[u + P]) : 0.0;
-            sec[0][tx] = ry ? edge_term(uu1[u + P], uu1[u + P - 1], vno[u], vno[u + P]) : 0.0;
-        } else if (ty == 1 && tx < SW2D_BY) { /* warp 1, eight lanes: the column left */
-            const size_t l = (size_t)(blockIdx.y * SW2D_BY + tx + H) * P + (blockIdx.x * SW2D_BX - 1 + H);
-            seb[tx][0] = regx[tx][0] ? edge_term(vv1[l + 1], vv1[l - P + 1], umo[l], umo[l + 1]) : 0.0;
-            sed[tx][0] = regy[tx][0] ? edge_term(vv1[l + 1], vv1[l], vno[l], vno[l + 1]) : 0.0;
+        const double* __restrict__ h = p.h[cur];
+        const double* __restrict__ z = p.z;
+        const double* __restrict__ qx = p.qx[0]; /* the state's discharges */
+        const double* __restrict__ qy = p.qy[0];
+        const double* __restrict__ u = p.uu1;
+        const double* __restrict__ v = p.vv1;
+        const uint8_t* __restrict__ flags = p.flags;
+        if (t < 3) cnt[t] = 0;
+        if (t == 3) rowx[BY] = rowy[BY] = 0u;
+        for (int k = t; k < NV; k += NT) {
+            const int rr = k / SW, cc = k - rr * SW;
+            const int gr = r0 - 1 + rr, gc = c0 - 1 + cc;
+            const bool in = gr <= R + 1 && gc <= C + 1; /* the padded raster */
+            const size_t g = (size_t)(gr + H) * P + (gc + H);
+            sf[U + k] = in ? u[g] : 0.0;
+            sf[V + k] = in ? v[g] : 0.0;
+            sf[QX + k] = in ? qx[g] : 0.0;
+            sf[QY + k] = in ? qy[g] : 0.0;
+            if (k < NH) {
+                const double hh = in ? h[g] : 0.0, zz = in ? z[g] : 0.0;
+                sh[k] = hh;
+                sz[k] = zz;
+                se[k] = hh + zz;
+                sact[k] = in ? (flags[g] & SW2D_F_ACTIVE) : 0;
+            }
         }
     }
+    __syncthreads();
+    const int s0 = (ty + 1) * SW + tx + 1;
+    const bool doX = r <= R && c < C, doY = r < R && c <= C;
     {
+        const double hc = sh[s0], ec = se[s0], zc = sz[s0];
+        const int an = sact[s0 - SW], aw = sact[s0 - 1], ac = sact[s0];
+        int kx = 0, ky = 0;
+        if (doX) {
+            if (r == R && p.outflow_south) /* south edge: free overfall when open */
+                kx = (an && sw2d_gt_pos(sh[s0 - SW], th)) ? 2 : 0;
+            else
+                kx = classify(an & ac, sh[s0 - SW], hc, se[s0 - SW], ec, sz[s0 - SW], zc, th);
+        }
+        if (doY) ky = classify(aw & ac, sh[s0 - 1], hc, se[s0 - 1], ec, sz[s0 - 1], zc, th);
+        if (doX && kx == 0) p.qx[1][i] = 0.0;
+        if (doY && ky == 0) p.qy[1][i] = 0.0;
+        const unsigned all = 0xffffffffu, lt = (1u << tx) - 1u;
+        const unsigned mx = __ballot_sync(all, kx == 1), my = __ballot_sync(all, ky == 1);
+        const unsigned px = __ballot_sync(all, kx > 1), py = __ballot_sync(all, ky > 1);
         int base = 0;
-        for (int w = 0; w < warp; w++) base += mwarp[w];
-        const unsigned lt = (1u << lane) - 1u;
-        const int off = base + __popc(bx & lt) + __popc(by & lt);
-        if (fx.kind == 1) mlist[off] = (unsigned short)(2 * t);
-        if (fy.kind == 1) mlist[off + (fx.kind == 1 ? 1 : 0)] = (unsigned short)(2 * t + 1);
+        if (tx == 0) {
+            rowx[ty] = mx;
+            rowy[ty] = my;
+            base = atomicAdd(&cnt[0], __popc(mx) + __popc(my));
+        } else if (tx == 1) {
+            base = atomicAdd(&cnt[1], __popc(px) + __popc(py));
+        }
+        int mb = __shfl_sync(all, base, 0) + __popc(mx & lt);
+        int pb = 2 * NT - 1 - (__shfl_sync(all, base, 1) + __popc(px & lt));
+        if (kx == 1) flist[mb] = (unsigned short)(2 * t);
+        if (kx > 1) flist[pb] = (unsigned short)(2 * t);
+        mb = mb - __popc(mx & lt) + __popc(mx) + __popc(my & lt);
+        pb = pb + __popc(px & lt) - __popc(px) - __popc(py & lt);
+        if (ky == 1) flist[mb] = (unsigned short)(2 * t + 1);
+        if (ky > 1) flist[pb] = (unsigned short)(2 * t + 1);
+        if (p.dt_mode == 1) {
+            const float thf = sw2d_f32_est_of_f64(th), gf = sw2d_f32_est_of_f64(p.g);
+            const float hf = sw2d_f32_est_of_f64(hc);
+            const float hx = 0.5f * (hf + sw2d_f32_est_of_f64(sh[s0 - SW]));
+            const float hy = 0.5f * (hf + sw2d_f32_est_of_f64(sh[s0 - 1]));
+            const bool okx = doX && r > 0 && r < R && (an & ac) && mean_ge(sh[s0 - SW], hc, hx, th, thf);
+            const bool oky = doY && c > 0 && c < C && (aw & ac) && mean_ge(sh[s0 - 1], hc, hy, th, thf);
+            const float ex = okx ? fmaxf((fabsf(sw2d_f32_est_of_f64(sf[U + s0])) + sqrtf(gf * hx)) * sw2d_f32_est_of_f64(p.rdx), 0.f) : 0.f;
+            const float ey = oky ? fmaxf((fabsf(sw2d_f32_est_of_f64(sf[V + s0])) + sqrtf(gf * hy)) * sw2d_f32_est_of_f64(p.rdy), 0.f) : 0.f;
+            unsigned long long* best = p.flight->smax[cur];
+            const float cx = sw2d_f32_est_of_f64(__longlong_as_double((long long)__ldcg(best)));
+            const float cy = sw2d_f32_est_of_f64(__longlong_as_double((long long)__ldcg(best + 1)));
+            const float wx = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ex))), cx) * 0.99999f;
+            const float wy = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ey))), cy) * 0.99999f;
+            if (okx && ex >= wx) raise_max(best, face_speed(sf[U + s0], sw2d_half(hc + sh[s0 - SW]), p.g, p.rdx));
+            if (oky && ey >= wy) raise_max(best + 1, face_speed(sf[V + s0], sw2d_half(hc + sh[s0 - 1]), p.g, p.rdy));
+        }
     }
     __syncthreads();
-    /* 3: face discharges: the non-momentum faces by their own thread, then
-     * the momentum faces from the packed list */
-    bool okx = false, oky = false;
-    double hmx = 0, hmy = 0, vx = 0, vy = 0;
-    if (in) {
-        if (s.active) {
-            const double gg = p.g;
-            /* mean depths of the two faces: the momentum update and the CFL speed */
-            const double hmX = (doX && r > 0) ? sw2d_half(h[i] + h[i - P]) : 0.0;
-            const double hmY = (doY && c > 0) ? sw2d_half(h[i] + h[i - 1]) : 0.0;
-            if (doX) {
-                double F;
-                if (edgeS) { /* south edge: free overfall when open */
-                    const double hw = h[i - P];
-                    F = ((p.flags[i - P] & SW2D_F_ACTIVE) && sw2d_gt_pos(hw, th)) ? 0.5440 * hw * sw2d_sqrt_rn(gg * hw)
-                                                                                     : 0.0;
-                } else {
-                    F = face_special(fx, th, gg);
-                }
-                if (fx.kind != 1) p.qx[1][i] = F;
-            }
-            if (doY) {
-                if (fy.kind != 1) p.qy[1][i] = face_special(fy, th, gg);
-            }
-            if (p.dt_mode == 1) {
-                const uint8_t fc = p.flags[i];
-                if (c < p.C && r > 0 && r < p.R && (fc & p.flags[i - P] & SW2D_F_ACTIVE)) {
-                    hmx = hmX;
-                    okx = sw2d_ge_pos(hmx, th);
-                    vx = uu1[i];
-                }
-                if (r < p.R && c > 0 && c < p.C && (fc & p.flags[i - 1] & SW2D_F_ACTIVE)) {
-                    hmy = hmY;
-                    oky = sw2d_ge_pos(hmy, th);
-                    vy = vv1[i];
-                }
-            }
-        }
+    {
+        /* edges of the row: south of its cells for x and y faces (types 0,
+         * 2), east of them and west of the first (1, 3); warp 0 also the
+         * edges north of the block */
+        const unsigned X = rowx[ty], Y = rowy[ty], m0 = X | rowx[ty + 1], m2 = Y | rowy[ty + 1];
+        const unsigned m1 = X | (X >> 1), m3 = Y | (Y >> 1);
+        const unsigned u0 = ty == 0 ? X : 0u, u2 = ty == 0 ? Y : 0u;
+        const unsigned w1 = X & 1u, w3 = Y & 1u;
+        const int n0 = __popc(m0), n1 = n0 + __popc(m1), n2 = n1 + __popc(m2), n3 = n2 + __popc(m3);
+        const int n4 = n3 + __popc(u0), n5 = n4 + __popc(u2), n6 = n5 + (int)w1;
+        int base = 0;
+        if (tx == 0) base = atomicAdd(&cnt[2], n6 + (int)w3);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const unsigned lt = (1u << tx) - 1u, bit = 1u << tx;
+        if (m0 & bit) elist[base + __popc(m0 & lt)] = (unsigned short)(s0 << 2);
+        if (m1 & bit) elist[base + n0 + __popc(m1 & lt)] = (unsigned short)(s0 << 2 | 1);
+        if (m2 & bit) elist[base + n1 + __popc(m2 & lt)] = (unsigned short)(s0 << 2 | 2);
+        if (m3 & bit) elist[base + n2 + __popc(m3 & lt)] = (unsigned short)(s0 << 2 | 3);
+        if (u0 & bit) elist[base + n3 + __popc(u0 & lt)] = (unsigned short)((s0 - SW) << 2);
+        if (u2 & bit) elist[base + n4 + __popc(u2 & lt)] = (unsigned short)((s0 - SW) << 2 | 2);
+        if (tx == 0 && w1) elist[base + n5] = (unsigned short)((s0 - 1) << 2 | 1);
+        if (tx == 0 && w3) elist[base + n6] = (unsigned short)((s0 - 1) << 2 | 3);
     }
-    /* the momentum faces, packed: face k of the list is a face of cell
-     * (ry, rx) of the block, x (north) or y (west) by its low bit */
-    if (s.active) {
-        int M = 0;
-        for (int w = 0; w < SW2D_BX * SW2D_BY / 32; w++) M += mwarp[w];
-        const double dt2 = s.dt2, dt2dx = s.dt2dx, dt2dy = s.dt2dy;
-        for (int k = t; k < M; k += SW2D_BX * SW2D_BY) {
-            const int id = mlist[k], ft = id >> 1, lx = ft % SW2D_BX, ly = ft / SW2D_BX;
-            const int cc = blockIdx.x * SW2D_BX + lx, rr = blockIdx.y * SW2D_BY + ly;
-            const size_t j = (size_t)(rr + H) * P + (cc + H);
-            FaceK f;
-            f.kind = 1;
-            f.hhb = mhhb[id];
-            if ((id & 1) == 0) { /* x face north of cell j */
-                f.ha = h[j - P];
-                f.za = p.z[j - P];
-                const double hm = sw2d_half(h[j] + h[j - P]);
-                const double u11 = dt2dx * (sea[ly + 1][lx] - sea[ly][lx]);
-                const double u12 = (cc == 0) ? 0.0 : dt2dy * (seb[ly][lx + 1] - seb[ly][lx]);
-                const double vt = sw2d_quarter(vv1[j] + vv1[j + 1] + vv1[j - P] + vv1[j - P + 1]);
-                p.qx[1][j] = face_momentum(p, f, hm, umo[j], uu1[j], vt, u11, u12, dt2, dt2dx, j - P, j);
-            } else { /* y face west of cell j */
-                f.ha = h[j - 1];
-                f.za = p.z[j - 1];
-                const double hm = sw2d_half(h[j] + h[j - 1]);
-                const double v11 = (rr == 0) ? 0.0 : dt2dx * (sec[ly + 1][lx] - sec[ly][lx]);
-                const double v12 = dt2dy * (sed[ly][lx + 1] - sed[ly][lx]);
-                const double ut = sw2d_quarter(uu1[j] + uu1[j + P] + uu1[j - 1] + uu1[j + P - 1]);
-                p.qy[1][j] = face_momentum(p, f, hm, vno[j], vv1[j], ut, v11, v12, dt2, dt2dy, j - 1, j);
-            }
-        }
+    for (int k = t; k < cnt[1]; k += NT) {
+        const int id = flist[2 * NT - 1 - k], ft = id >> 1, ly = ft / BX, lx = ft % BX;
+        const int sj = (ly + 1) * SW + lx + 1, sa = (id & 1) ? sj - 1 : sj - SW;
+        const bool edge = !(id & 1) && r0 + ly == R; /* the open south edge: a weir from the last row */
+        const double F = face_special(edge, sh[sa], sh[sj], se[sa], se[sj], sz[sa], sz[sj], th, p.g);
+        ((id & 1) ? p.qy[1] : p.qx[1])[(size_t)(r0 + ly + H) * P + (c0 + lx + H)] = F;
     }
-    if (p.dt_mode == 1) {
-        unsigned long long sx, sy;
-        block_face_speed_max2(okx, vx, hmx, p.rdx, oky, vy, hmy, p.rdy, p.g, smf, smu, &sx, &sy);
-        if (threadIdx.x == 0 && threadIdx.y == 0) {
-            const int b = blockIdx.y * gridDim.x + blockIdx.x;
-            p.partials_f[2 * b] = __longlong_as_double((long long)sx);
-            p.partials_f[2 * b + 1] = __longlong_as_double((long long)sy);
-        }
+    __syncthreads();
+    for (int k = t; k < cnt[2]; k += NT) {
+        const int id = elist[k], e = id >> 2;
+        const int w = ((id & 1) ? V : U) + e, q = ((id & 2) ? QY : QX) + e, step = (id & 1) ? 1 : SW;
+        const int back = (id & 3) == 1 ? 1 - SW : (id & 3) == 2 ? SW - 1 : 0;
+        sedge[(id & 3) * NH + e] = edge_term(sf[w + step], sf[w + back], sf[q], sf[q + step]);
+    }
+    __syncthreads();
+    for (int k = t; k < cnt[0]; k += NT) {
+        const int id = flist[k], ft = id >> 1, ly = ft / BX, lx = ft % BX;
+        const bool y = (id & 1) != 0; /* the y face west of cell j, else the x face north of it */
+        const int sj = (ly + 1) * SW + lx + 1, da = y ? 1 : SW, so = y ? SW : 1;
+        const size_t j = (size_t)(r0 + ly + H) * P + (c0 + lx + H);
+        const int ea = (y ? 2 * NH : 0) + sj, eb = ea + NH;
+        double along = dt2dx * (sedge[ea] - sedge[ea - SW]), across = dt2dy * (sedge[eb] - sedge[eb - 1]);
+        if (y && r0 + ly == 0) along = 0.0;    /* the reference's edge rules (:280-284, :184-186) */
+        if (!y && c0 + lx == 0) across = 0.0;
+        const double hm = sw2d_half(sh[sj] + sh[sj - da]);
+        const int T = (y ? U : V) + sj; /* the other direction's face velocities */
+        const double vt = sw2d_quarter(sf[T] + sf[T + so] + sf[T - da] + sf[T - da + so]);
+        const double F = face_momentum(p, friction_coef(p, j, j - (y ? 1 : P)), sh[sj - da], sz[sj - da], se[sj], hm,
+                                       sf[(y ? QY : QX) + sj], sf[(y ? V : U) + sj], vt, along, across, dt2,
+                                       y ? dt2dy : dt2dx);
+        (y ? p.qy[1] : p.qx[1])[j] = F;
     }
 }
 
@@ -485,7 +513,7 @@ __device__ __forceinline__ double continuity(const StepParams& p, size_t i, uint
     const double rcell = p.rainw ? rr * sw2d_f64_of_f32(p.rainw[i]) : rr; /* exact, off the FP64 pipe */
     /* (((dqx/dx + dqy/dy) - q_src) - r pct) + e; subtracting a zero source
      * and adding a zero evaporation change no value, so they are skipped */
-    double sum = div_spacing(divx, p.dx, p.rdx, p.kdx) + div_spacing(divy, p.dy, p.rdy, p.kdy);
+    double sum = div_spacing(divx, p.ddx, p.kdx) + div_spacing(divy, p.ddy, p.kdy);
     if (f & SW2D_F_SOURCE) {
         double qli = 0.0;
         for (int k = 0; k < p.nsrc; k++)
@@ -507,7 +535,7 @@ __device__ __forceinline__ double continuity(const StepParams& p, size_t i, uint
 
 
 __device__ __forceinline__ double block_sum(double v, double* sm) {
-    const int lane = tid_linear() & 31, warp = tid_linear() >> 5;
+    const int lane = tid_linear() & 31, warp = tid_linear() >> 5, nw = (int)(blockDim.x * blockDim.y) >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     __syncthreads();
@@ -515,7 +543,7 @@ __device__ __forceinline__ double block_sum(double v, double* sm) {
     __syncthreads();
     double t = 0.0;
     if (warp == 0) {
-        t = lane < NWARP ? sm[lane] : 0.0;
+        t = lane < nw ? sm[lane] : 0.0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
     }
@@ -544,107 +572,146 @@ __device__ unsigned long long block_max_u64(unsigned long long v, unsigned long 
     return t; /* valid in thread 0 */
 }
 
-#define NPART 4 /* rain, evap, qout, s_max bits */
+#define NPART 4 /* prime: volume, CFL bits x, y; update: weighted rain, lake cells, land cells, outlet */
 
-/* Final reduction over the per-block partials by the last block to finish,
- * then the iteration's ledger update and the next slot. */
-__device__ void finish_iteration(const StepParams& p, int cur, int nblocks) {
-    __shared__ bool last;
+/* Adds the ledger sums of the iteration whose slot is `par` (its tiles'
+ * partials were written by the previous k64_update) and its outlet record;
+ * by one whole block.  last_row: the tile row that holds the raster's last row. */
+__device__ void settle_ledger(const StepParams& p, int par, int gx, int gy, int last_row) {
     __shared__ double smd[NWARP];
-    __shared__ unsigned long long smu[NWARP];
-    __threadfence();
-    const int tid = tid_linear();
-    if (tid == 0) {
-        unsigned int ticket = atomicAdd(&p.clk->counter, 1u);
-        last = (ticket == (unsigned)nblocks - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double vr = 0.0, ve = 0.0, vq = 0.0;
-    for (int b = tid; b < nblocks; b += SW2D_BX * SW2D_BY) {
-        const volatile double* pb = p.partials + (size_t)b * NPART;
-        vr += pb[0];
-        ve += pb[1];
-        vq += pb[2];
-    }
+    const int nt = blockDim.x, tid = threadIdx.x, tiles = gx * gy;
+    const double* part = p.partials + (size_t)par * tiles * NPART;
+    double vr = 0.0, ve = 0.0, vd = 0.0, vq = 0.0;
     if (p.ledger_cells) {
-        vr = block_sum(vr, smd);
-        ve = block_sum(ve, smd);
-    }
-    if (p.outflow_south) vq = block_sum(vq, smd);
-    /* CFL speed of the state this iteration started from, from k64_flux */
-    unsigned long long ux = 0ull, uy = 0ull;
-    if (p.dt_mode == 1) {
-        for (int b = tid; b < p.nblocks_faces; b += SW2D_BX * SW2D_BY) {
-            const volatile double* pb = p.partials_f + (size_t)b * 2;
-            unsigned long long a = (unsigned long long)__double_as_longlong(pb[0]);
-            unsigned long long c = (unsigned long long)__double_as_longlong(pb[1]);
-            ux = a > ux ? a : ux;
-            uy = c > uy ? c : uy;
+        for (int b = tid; b < tiles; b += nt) {
+            const double* pb = part + (size_t)b * NPART;
+            if (p.rainw) vr += __ldcg(pb);
+            ve += __ldcg(pb + 1);
+            if (!p.rainw) vd += __ldcg(pb + 2);
         }
-        ux = block_max_u64(ux, smu);
-        uy = block_max_u64(uy, smu);
+        if (p.rainw) vr = block_sum(vr, smd);
+        ve = block_sum(ve, smd);
+        if (!p.rainw) vd = block_sum(vd, smd);
+    }
+    if (p.outflow_south) { /* the tiles that hold the last row */
+        for (int b = tid; b < gx; b += nt) vq += __ldcg(part + (size_t)(last_row * gx + b) * NPART + 3);
+        vq = block_sum(vq, smd);
     }
     if (tid == 0) {
         DevClock* clk = p.clk;
-        const Slot& s = clk->slot[cur];
-        if (s.active) {
-            const double dt2 = s.dt2;
-            const double smax = __longlong_as_double((long long)ux) + __longlong_as_double((long long)uy);
-            double src = 0.0;
-            for (int k = 0; k < p.nsrc; k++) /* a source overridden on its cell adds nothing */
-                if (p.src_idx[k] >= 0) src += s.ql2[k];
-            const double rain = p.ledger_cells ? vr : s.rr2 * p.rain_static;
-            clk->led[LED_RAIN] += dt2 * rain * p.area;
-            clk->led[LED_EVAP] += dt2 * ve * p.area;
-            clk->led[LED_SOURCE] += dt2 * src * p.area;
-            clk->led[LED_QOUT] = vq * p.dy;
-            clk->led[LED_OUTFLOW] += dt2 * clk->led[LED_QOUT];
-            clk->led[LED_DTLAST] = dt2;
-            clk->led[LED_SMAX] = smax;
-            if (!isfinite(smax) || !isfinite(vq)) clk->status |= 1;
-            clk->t = s.t_next;
-            clk->s_max = smax;
-            clk->iters += 1;
-            if (p.outlet) {
-                long long k = clk->outlet_n % p.outlet_cap;
-                p.outlet[2 * k] = s.t_next;
-                p.outlet[2 * k + 1] = clk->led[LED_QOUT];
-                clk->outlet_n += 1;
-            }
-            /* past the iteration limit the next slot is inactive: t_end = t */
-            prepare_slot(p, &clk->slot[cur ^ 1], clk->t, clk->s_max,
-                         clk->iters < clk->iter_end ? clk->t_end : clk->t);
-        } else {
-            clk->slot[cur ^ 1] = s;
+        const Slot& s = clk->slot[par];
+        const double dt2 = s.dt2, area = p.area, rr2 = s.rr2, ev2 = s.ev2, tn = s.t_next;
+        const double l0 = clk->led[LED_RAIN], l1 = clk->led[LED_EVAP], l2 = clk->led[LED_SOURCE], l3 = clk->led[LED_OUTFLOW];
+        double src = 0.0;
+        for (int k = 0; k < p.nsrc; k++) /* a source overridden on its cell adds nothing */
+            if (p.src_idx[k] >= 0) src += s.ql2[k];
+        const double rain = !p.ledger_cells ? rr2 * p.rain_static
+                            : p.rainw       ? vr
+                                            : ve * (rr2 * p.pct_lake) + vd * (rr2 * p.pct_land);
+        const double qo = vq * p.dy;
+        clk->led[LED_RAIN] = l0 + dt2 * rain * area;
+        clk->led[LED_EVAP] = l1 + dt2 * (ve * ev2) * area;
+        clk->led[LED_SOURCE] = l2 + dt2 * src * area;
+        clk->led[LED_QOUT] = qo;
+        clk->led[LED_OUTFLOW] = l3 + dt2 * qo;
+        if (!isfinite(vq)) clk->status |= 1;
+        if (p.outlet) {
+            const long long n = clk->outlet_n, k = n % p.outlet_cap;
+            p.outlet[2 * k] = tn;
+            p.outlet[2 * k + 1] = qo;
+            clk->outlet_n = n + 1;
         }
-        clk->counter = 0;
     }
+}
+
+/* The clock of the iteration in slot `cur`, by the extra block of its
+ * k64_update, beside the tiles: the previous iteration's ledger sums, then
+ * the CFL speed k64_flux found and the next iteration's length and forcing. */
+__device__ void advance_clock(const StepParams& p, int cur, int gx, int gy, int last_row) {
+    DevClock* clk = p.clk;
+    Flight64* fl = p.flight;
+    const int pending = __ldcg(&fl->pending);
+    if (pending) settle_ledger(p, pending - 1, gx, gy, last_row);
+    __syncthreads(); /* slot cur^1 is read above and overwritten below */
+    if (threadIdx.x >= 32) return;
+    const Slot& s = clk->slot[cur];
+    if (!s.active) {
+        const unsigned long long* from = reinterpret_cast<const unsigned long long*>(&s);
+        unsigned long long* to = reinterpret_cast<unsigned long long*>(&clk->slot[cur ^ 1]);
+        for (int k = threadIdx.x; k < (int)(sizeof(Slot) / 8); k += 32) to[k] = from[k];
+        if (threadIdx.x == 0) fl->pending = 0;
+        return;
+    }
+    /* of the state this iteration started from */
+    const double smax = __longlong_as_double((long long)__ldcg(&fl->smax[cur][0])) +
+                        __longlong_as_double((long long)__ldcg(&fl->smax[cur][1]));
+    const double t = s.t_next, t_end = clk->t_end;
+    const long long iters = clk->iters + 1, lim = clk->iter_end;
+    __syncwarp();
+    if (threadIdx.x == 0) {
+        fl->smax[cur][0] = fl->smax[cur][1] = 0ull;
+        fl->pending = cur + 1;
+        clk->led[LED_DTLAST] = s.dt2;
+        clk->led[LED_SMAX] = smax;
+        if (!isfinite(smax)) clk->status |= 1;
+        clk->t = t;
+        clk->s_max = smax;
+        clk->iters = iters;
+    }
+    /* past the iteration limit the next slot is inactive: t_end = t */
+    prepare_slot(p, &clk->slot[cur ^ 1], t, smax, iters < lim ? t_end : t);
 }
 
 /* ------------------------------------------------------------------------ */
 /* continuity at t, treat_error, continuity at t+dt, hm_hn + uu1_vv1:         */
 /* SW2D-EFDC.cu:602-664, :695-725, :362-452 in one pass                       */
 
-/* Tile of the update kernel: UT_W x UT_H cells (and their north and west
- * faces) per CTA.  The provisional depths ("dry" flags) are evaluated on the
- * tile plus two rows north and west and one row south and east, the new
- * depths on the tile plus the row north and the column west: the faces of
- * the tile read both; the halo is recomputed, not exchanged. */
-#define UT_W 64
-#define UT_H 16
-#define UT_DW (UT_W + 3)
-#define UT_DH (UT_H + 3)
-#define UT_NW (UT_W + 1)
-#define UT_NH (UT_H + 1)
+/* "active and provisional depth < th" of a cell: decided from a binary32
+ * estimate of the depth, by the exact binary64 continuity only where th lies
+ * within the estimate's error (2^-19 of the magnitudes that enter it; the
+ * estimate's own rounding stays below 2^-20 of them). */
+struct DryEst {
+    float th, ewl, dt2, rdx, rdy, pl, pd, ev;
+};
+__device__ __forceinline__ bool provisional_dry(const StepParams& p, const Slot& s, const DryEst& q, size_t i,
+                                                uint8_t f, double ho, double fN, double fS, double fW, double fE) {
+    const float h = sw2d_f32_est_of_f64(ho), n = sw2d_f32_est_of_f64(fN), so = sw2d_f32_est_of_f64(fS),
+                w = sw2d_f32_est_of_f64(fW), e = sw2d_f32_est_of_f64(fE);
+    const bool lake = sw2d_gt(ho, p.ev_wl_min);
+    float rain = lake ? q.pl : q.pd;
+    if (p.rainw) rain *= p.rainw[i];
+    const float ev = lake ? q.ev : 0.f;
+    const float hs = h - q.dt2 * (((so - n) * q.rdx + (e - w) * q.rdy - rain) + ev);
+    const float mag = fabsf(h) + q.dt2 * ((fabsf(so) + fabsf(n)) * q.rdx + (fabsf(e) + fabsf(w)) * q.rdy + fabsf(rain) +
+                                          fabsf(ev));
+    const float d = hs - q.th;
+    if (!(f & SW2D_F_SOURCE) && fabsf(d) > 1.9073486e-6f * (mag + q.th) + 1e-35f) return d < 0.f;
+    double raw, rt;
+    return sw2d_lt_pos(continuity(p, i, f, ho, fS - fN, fE - fW, s.dt2, s.rr1, s.ev1, s.ql1, &raw, &rt), p.th);
+}
 
-__global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_update(StepParams p, int cur) {
-    __shared__ uint8_t sdry[UT_DH][UT_DW];   /* rows r0-2 .. r0+UT_H, cols c0-2 .. c0+UT_W */
-    __shared__ double shn[UT_NH][UT_NW];     /* rows r0-1 .. r0+UT_H-1, cols c0-1 .. c0+UT_W-1 */
+/* Tile of the update kernel: TW x TH cells (and their north and west faces)
+ * per block.  The dry flags are evaluated on the tile plus two rows north
+ * and west and one row south and east, the new depths on the tile plus the
+ * row north and the column west: the faces of the tile read both; the halo
+ * is recomputed, not exchanged.  Block 0 keeps the clock meanwhile (what it
+ * does is a chain of dependent reads and divisions; at the end of the last
+ * tile it would be the longest part of a small raster's iteration).
+ * Bounded by the binary64 additions and products of the final depth and of
+ * the face means (71 issue cycles a warp each): the flags take none. */
+template <int TW, int TH, int NT>
+__global__ void __launch_bounds__(NT) k64_update(StepParams p, int cur, int gx, int gy) {
+    constexpr int DW = TW + 3, DH = TH + 3, NW = TW + 1, NH = TH + 1;
+    if (blockIdx.x == 0) {
+        advance_clock(p, cur, gx, gy, (p.R - 1) / TH);
+        return;
+    }
+    __shared__ uint8_t sdry[DH][DW];   /* rows r0-2 .. r0+TH, cols c0-2 .. c0+TW */
+    __shared__ double shn[NH][NW];     /* rows r0-1 .. r0+TH-1, cols c0-1 .. c0+TW-1 */
     __shared__ double smd[NWARP];
     const int tid = threadIdx.x;
-    const int c0 = blockIdx.x * UT_W, r0 = blockIdx.y * UT_H;
+    const int tile = blockIdx.x - 1, tyi = tile / gx;
+    const int c0 = (tile - tyi * gx) * TW, r0 = tyi * TH;
     const int nxt = cur ^ 1;
     const Slot& s = p.clk->slot[cur];
     const int P = p.P, R = p.R, C = p.C;
@@ -652,122 +719,157 @@ __global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_update(StepParams p, in
     const double* __restrict__ fx = p.qx[1]; /* k64_flux's new discharges, read only */
     const double* __restrict__ fy = p.qy[1];
     const double* __restrict__ hc = p.h[cur];
-    double vr = 0.0, ve = 0.0, vq = 0.0;
     if (!s.active) {
         /* the loop condition failed: the iteration copies the depth */
-        for (int k = tid; k < UT_W * UT_H; k += SW2D_BX * SW2D_BY) {
-            const int r = r0 + k / UT_W, c = c0 + k % UT_W;
+        for (int k = tid; k < TW * TH; k += NT) {
+            const int r = r0 + k / TW, c = c0 + k % TW;
             if (r < R && c < C) {
                 const size_t i = (size_t)(r + H) * P + (c + H);
                 p.h[nxt][i] = hc[i];
             }
         }
-    } else {
+        return;
+    }
+    const double dt2 = s.dt2, rr2 = s.rr2, ev2 = s.ev2;
+    {
         /* 1: provisional depth at t -> "active and h* < th" (0 outside the raster) */
-        for (int k = tid; k < UT_DH * UT_DW; k += SW2D_BX * SW2D_BY) {
-            const int rr = k / UT_DW, cc = k - rr * UT_DW;
+        DryEst q;
+        q.th = sw2d_f32_est_of_f64(th);
+        q.dt2 = sw2d_f32_est_of_f64(dt2);
+        q.rdx = sw2d_f32_est_of_f64(p.rdx);
+        q.rdy = sw2d_f32_est_of_f64(p.rdy);
+        const float rr1 = sw2d_f32_est_of_f64(s.rr1);
+        q.pl = rr1 * sw2d_f32_est_of_f64(p.pct_lake);
+        q.pd = rr1 * sw2d_f32_est_of_f64(p.pct_land);
+        q.ev = sw2d_f32_est_of_f64(s.ev1);
+        for (int k = tid; k < DH * DW; k += NT) {
+            const int rr = k / DW, cc = k - rr * DW;
             const int r = r0 - 2 + rr, c = c0 - 2 + cc;
             uint8_t dflag = 0;
             if (r >= 0 && r < R && c >= 0 && c < C) {
                 const size_t i = (size_t)(r + H) * P + (c + H);
                 const uint8_t f = p.flags[i];
-                double raw, rt;
-                const double hs = continuity(p, i, f, hc[i], fx[i + P] - fx[i], fy[i + 1] - fy[i], s.dt2, s.rr1,
-                                             s.ev1, s.ql1, &raw, &rt);
-                dflag = (uint8_t)((f & SW2D_F_ACTIVE) && sw2d_lt_pos(hs, th));
+                if (f & SW2D_F_ACTIVE) dflag = provisional_dry(p, s, q, i, f, hc[i], fx[i], fx[i + P], fy[i], fy[i + 1]);
             }
             sdry[rr][cc] = dflag;
         }
-        __syncthreads();
-        /* 2: treat_error per face (a face carrying water out of a cell whose
-         * provisional depth fell below th is closed, :704-719), final depth
-         * at t+dt; written for the tile's own cells, kept in shared memory
-         * for the faces */
-        for (int k = tid; k < UT_NH * UT_NW; k += SW2D_BX * SW2D_BY) {
-            const int rr = k / UT_NW, cc = k - rr * UT_NW;
-            const int r = r0 - 1 + rr, c = c0 - 1 + cc;
-            double hn = 0.0;
-            if (r >= 0 && r < R && c >= 0 && c < C) {
-                const size_t i = (size_t)(r + H) * P + (c + H);
-                const uint8_t f = p.flags[i];
-                const int dr = rr + 1, dc = cc + 1;
-                const uint8_t dC = sdry[dr][dc];
-                double fN = fx[i], fS = fx[i + P], fW = fy[i], fE = fy[i + 1];
-                if ((sw2d_gt0(fN) && sdry[dr - 1][dc]) || (sw2d_lt0(fN) && dC)) fN = 0;
-                if ((sw2d_gt0(fS) && dC) || (sw2d_lt0(fS) && sdry[dr + 1][dc])) fS = 0;
-                if ((sw2d_gt0(fW) && sdry[dr][dc - 1]) || (sw2d_lt0(fW) && dC)) fW = 0;
-                if ((sw2d_gt0(fE) && dC) || (sw2d_lt0(fE) && sdry[dr][dc + 1])) fE = 0;
-                const double ho = hc[i];
-                double raw, rt;
-                hn = continuity(p, i, f, ho, fS - fN, fE - fW, s.dt2, s.rr2, s.ev2, s.ql2, &raw, &rt);
-                if (rr >= 1 && cc >= 1) { /* the tile's own cell */
-                    p.h[nxt][i] = hn;
-                    if (f & SW2D_F_ACTIVE) {
-                        if (sw2d_lt0(raw)) atomicAdd(&p.clk->led[LED_CLAMP], -raw * p.area); /* max(h, 0) gain */
-                        if (p.ledger_cells) {
-                            vr += rt;
-                            ve += sw2d_gt(ho, p.ev_wl_min) ? s.ev2 : 0.0;
-                        }
-                        if (r == R - 1) vq += fS;
+    }
+    __syncthreads();
+    /* 2: treat_error per face (a face carrying water out of a cell whose
+     * provisional depth fell below th is closed, :704-719), final depth
+     * at t+dt; written for the tile's own cells, kept in shared memory
+     * for the faces */
+    double vr = 0.0, vq = 0.0;
+    int nlake = 0, nland = 0;
+    for (int k = tid; k < NH * NW; k += NT) {
+        const int rr = k / NW, cc = k - rr * NW;
+        const int r = r0 - 1 + rr, c = c0 - 1 + cc;
+        double hn = 0.0;
+        if (r >= 0 && r < R && c >= 0 && c < C) {
+            const size_t i = (size_t)(r + H) * P + (c + H);
+            const uint8_t f = p.flags[i];
+            const int dr = rr + 1, dc = cc + 1;
+            const uint8_t dC = sdry[dr][dc];
+            double fN = fx[i], fS = fx[i + P], fW = fy[i], fE = fy[i + 1];
+            if ((sw2d_gt0(fN) && sdry[dr - 1][dc]) || (sw2d_lt0(fN) && dC)) fN = 0;
+            if ((sw2d_gt0(fS) && dC) || (sw2d_lt0(fS) && sdry[dr + 1][dc])) fS = 0;
+            if ((sw2d_gt0(fW) && sdry[dr][dc - 1]) || (sw2d_lt0(fW) && dC)) fW = 0;
+            if ((sw2d_gt0(fE) && dC) || (sw2d_lt0(fE) && sdry[dr][dc + 1])) fE = 0;
+            const double ho = hc[i];
+            double raw, rt;
+            hn = continuity(p, i, f, ho, fS - fN, fE - fW, dt2, rr2, ev2, s.ql2, &raw, &rt);
+            if (rr >= 1 && cc >= 1) { /* the tile's own cell */
+                p.h[nxt][i] = hn;
+                if (f & SW2D_F_ACTIVE) {
+                    if (sw2d_lt0(raw)) atomicAdd(&p.clk->led[LED_CLAMP], -raw * p.area); /* max(h, 0) gain */
+                    if (p.ledger_cells) {
+                        if (p.rainw) vr += rt;
+                        if (sw2d_gt(ho, p.ev_wl_min)) nlake++;
+                        else nland++;
                     }
+                    if (r == R - 1 && p.outflow_south) vq += fS;
                 }
             }
-            shn[rr][cc] = hn;
+        }
+        shn[rr][cc] = hn;
+    }
+    __syncthreads();
+    /* 3: the closed faces written back and the face velocities of the new
+     * state, uu1 = qx/hm and vv1 = qy/hn (hm_hn, uu1_vv1), for the
+     * tile's north and west faces (the raster's south and east edge
+     * faces in the last tile row / column) */
+    for (int k = tid; k < TH * TW; k += NT) {
+        const int rr = k / TW, cc = k - rr * TW;
+        const int r = r0 + rr, c = c0 + cc;
+        if (r > R || c > C) continue;
+        const size_t i = (size_t)(r + H) * P + (c + H);
+        const int dr = rr + 2, dc = cc + 2, nr = rr + 1, nc = cc + 1;
+        if (c < C) {
+            double F = fx[i];
+            if ((sw2d_gt0(F) && sdry[dr - 1][dc]) || (sw2d_lt0(F) && sdry[dr][dc])) F = 0;
+            p.qx[0][i] = F;
+            double hm;
+            if (r == 0) hm = shn[nr][nc];
+            else if (r == R) hm = shn[nr - 1][nc];
+            else hm = sw2d_half(shn[nr][nc] + shn[nr - 1][nc]);
+            p.uu1[i] = sw2d_ge_pos(hm, th) ? sw2d_div_rn(F, hm) : 0.00;
+        }
+        if (r < R) {
+            double F = fy[i];
+            if ((sw2d_gt0(F) && sdry[dr][dc - 1]) || (sw2d_lt0(F) && sdry[dr][dc])) F = 0;
+            p.qy[0][i] = F;
+            double hn;
+            if (c == 0) hn = shn[nr][nc];
+            else if (c == C) hn = shn[nr][nc - 1];
+            else hn = sw2d_half(shn[nr][nc] + shn[nr][nc - 1]);
+            p.vv1[i] = sw2d_ge_pos(hn, th) ? sw2d_div_rn(F, hn) : 0.0;
+        }
+    }
+    /* ledger sums of the tile, added up by the next iteration's block 0 */
+    double* pb = p.partials + ((size_t)cur * gx * gy + tile) * NPART;
+    if (p.ledger_cells) {
+        if (p.rainw) vr = block_sum(vr, smd);
+        /* counts as binary32-exact integers: at most TW * TH */
+        nlake = __reduce_add_sync(0xffffffffu, nlake);
+        nland = __reduce_add_sync(0xffffffffu, nland);
+        __shared__ int sc[2];
+        if (tid < 2) sc[tid] = 0;
+        __syncthreads();
+        if ((tid & 31) == 0) {
+            atomicAdd(&sc[0], nlake);
+            atomicAdd(&sc[1], nland);
         }
         __syncthreads();
-        /* 3: the closed faces written back and the face velocities of the new
-         * state, uu1 = qx/hm and vv1 = qy/hn (hm_hn, uu1_vv1), for the
-         * tile's north and west faces (the raster's south and east edge
-         * faces in the last tile row / column) */
-        for (int k = tid; k < UT_H * UT_W; k += SW2D_BX * SW2D_BY) {
-            const int rr = k / UT_W, cc = k - rr * UT_W;
-            const int r = r0 + rr, c = c0 + cc;
-            if (r > R || c > C) continue;
-            const size_t i = (size_t)(r + H) * P + (c + H);
-            const int dr = rr + 2, dc = cc + 2, nr = rr + 1, nc = cc + 1;
-            if (c < C) {
-                double F = fx[i];
-                if ((sw2d_gt0(F) && sdry[dr - 1][dc]) || (sw2d_lt0(F) && sdry[dr][dc])) F = 0;
-                p.qx[0][i] = F;
-                double hm;
-                if (r == 0) hm = shn[nr][nc];
-                else if (r == R) hm = shn[nr - 1][nc];
-                else hm = sw2d_half(shn[nr][nc] + shn[nr - 1][nc]);
-                p.uu1[i] = sw2d_ge_pos(hm, th) ? (sw2d_is0(F) ? F : sw2d_div_rn(F, hm)) : 0.00; /* 0/hm is 0 of F's sign */
-            }
-            if (r < R) {
-                double F = fy[i];
-                if ((sw2d_gt0(F) && sdry[dr][dc - 1]) || (sw2d_lt0(F) && sdry[dr][dc])) F = 0;
-                p.qy[0][i] = F;
-                double hn;
-                if (c == 0) hn = shn[nr][nc];
-                else if (c == C) hn = shn[nr][nc - 1];
-                else hn = sw2d_half(shn[nr][nc] + shn[nr][nc - 1]);
-                p.vv1[i] = sw2d_ge_pos(hn, th) ? (sw2d_is0(F) ? F : sw2d_div_rn(F, hn)) : 0.0;
-            }
+        if (tid == 0) {
+            pb[0] = vr;
+            pb[1] = (double)sc[0];
+            pb[2] = (double)sc[1];
         }
     }
-    /* ledger partials of the tile, then the last block's reduction */
-    double pr = 0.0, pe = 0.0, pq = 0.0;
-    if (p.ledger_cells) {
-        pr = block_sum(vr, smd);
-        pe = block_sum(ve, smd);
+    if (p.outflow_south && r0 <= R - 1 && R - 1 < r0 + TH) {
+        vq = block_sum(vq, smd);
+        if (tid == 0) pb[3] = vq;
     }
-    if (p.outflow_south) pq = block_sum(vq, smd);
-    const int b = blockIdx.y * gridDim.x + blockIdx.x;
-    if (tid == 0) {
-        double* pb = p.partials + (size_t)b * NPART;
-        pb[0] = pr;
-        pb[1] = pe;
-        pb[2] = pq;
-    }
-    finish_iteration(p, cur, gridDim.x * gridDim.y);
+}
+
+__global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_settle(StepParams p, int gx, int gy,
+                                                                     int last_row) {
+    const int pending = __ldcg(&p.flight->pending);
+    if (!pending) return;
+    settle_ledger(p, pending - 1, gx, gy, last_row);
+    if (threadIdx.x == 0) p.flight->pending = 0;
 }
 
 /* Volume (sum of h over active cells) and, with full, the CFL speed of the
  * current state (face rule of k64_flux); the last block stores them and
  * prepares the next slot. */
 __global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_prime(StepParams p, int cur, int full) {
+    if (!full) { /* one block: the next slot only */
+        DevClock* clk = p.clk;
+        if (tid_linear() < 32)
+            prepare_slot(p, &clk->slot[cur], clk->t, clk->s_max, clk->iters < clk->iter_end ? clk->t_end : clk->t);
+        return;
+    }
     __shared__ double smd[NWARP];
     __shared__ float smf[2 * NWARP];
     __shared__ unsigned long long smu[2 * NWARP];
@@ -777,7 +879,7 @@ __global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_prime(StepParams p, int
     double vol = 0.0;
     bool okx = false, oky = false;
     double hmx = 0, hmy = 0, vx = 0, vy = 0;
-    if (full && r < p.R && c < p.C) {
+    if (r < p.R && c < p.C) {
         const int P = p.P;
         const size_t i = (size_t)(r + H) * P + (c + H);
         const double* h = p.h[cur];
@@ -825,19 +927,24 @@ __global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_prime(StepParams p, int
     v = block_sum(v, smd);
     ux = block_max_u64(ux, smu);
     uy = block_max_u64(uy, smu);
-    if (tid == 0) {
+    if (tid < 32) {
         DevClock* clk = p.clk;
         /* full: 1 = volume only (the clock is left alone), 2 = initial state
-         * (volume origin, CFL speed and the first slot), 0 = slot only */
-        if (full) clk->led[LED_VOLUME] = v * p.area;
-        if (full == 2) {
-            clk->s_max = __longlong_as_double((long long)ux) + __longlong_as_double((long long)uy);
-            clk->led[LED_SMAX] = clk->s_max;
-            clk->led[LED_VOLUME0] = clk->led[LED_VOLUME];
+         * (volume origin, CFL speed and the first slot) */
+        const double vol = __shfl_sync(0xffffffffu, v, 0) * p.area;
+        const double smax = __longlong_as_double((long long)__shfl_sync(0xffffffffu, ux, 0)) +
+                            __longlong_as_double((long long)__shfl_sync(0xffffffffu, uy, 0));
+        if (tid == 0) {
+            clk->led[LED_VOLUME] = vol;
+            if (full == 2) {
+                clk->s_max = smax;
+                clk->led[LED_SMAX] = smax;
+                clk->led[LED_VOLUME0] = vol;
+            }
+            clk->counter = 0;
         }
-        if (full != 1)
-            prepare_slot(p, &clk->slot[cur], clk->t, clk->s_max, clk->iters < clk->iter_end ? clk->t_end : clk->t);
-        clk->counter = 0;
+        if (full == 2)
+            prepare_slot(p, &clk->slot[cur], clk->t, smax, clk->iters < clk->iter_end ? clk->t_end : clk->t);
     }
 }
 
@@ -860,7 +967,7 @@ __global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_facevel(StepParams p, i
         if (r == 0) hm = h[i];
         else if (r == p.R) hm = h[i - P];
         else hm = sw2d_half(h[i] + h[i - P]);
-        p.uu1[i] = sw2d_ge_pos(hm, th) ? (sw2d_is0(F) ? F : sw2d_div_rn(F, hm)) : 0.00; /* 0/hm is 0 of F's sign */
+        p.uu1[i] = sw2d_ge_pos(hm, th) ? sw2d_div_rn(F, hm) : 0.00;
     }
     if (r < p.R) {
         const double F = p.qy[0][i];
@@ -868,7 +975,7 @@ __global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_facevel(StepParams p, i
         if (c == 0) hn = h[i];
         else if (c == p.C) hn = h[i - 1];
         else hn = sw2d_half(h[i] + h[i - 1]);
-        p.vv1[i] = sw2d_ge_pos(hn, th) ? (sw2d_is0(F) ? F : sw2d_div_rn(F, hn)) : 0.0;
+        p.vv1[i] = sw2d_ge_pos(hn, th) ? sw2d_div_rn(F, hn) : 0.0;
     }
 }
 
@@ -942,18 +1049,51 @@ static dim3 grid_cells(const StepParams& p) {
 
 int fp64_kernels_per_iteration() { return 2; }
 
+/* How a raster is cut into the update kernel's tiles and the flux kernel's blocks. */
+struct Cut64 {
+    int kind, tw, th, gx, gy;
+    dim3 flux;
+    int by;
+};
+static Cut64 cut_of(int R, int C) {
+    Cut64 k;
+    const long long cells = (long long)(R + 1) * (C + 1);
+    k.kind = cells >= 64LL * 16 * 152 * 4 ? 0 : cells >= 32LL * 8 * 152 ? 1 : 2;
+    k.tw = k.kind == 0 ? 64 : 32;
+    k.th = k.kind == 0 ? 16 : k.kind == 1 ? 8 : 4;
+    k.gx = (C + 1 + k.tw - 1) / k.tw;
+    k.gy = (R + 1 + k.th - 1) / k.th;
+    k.by = cells >= 32LL * 8 * 152 * 2 ? 8 : 2;
+    k.flux = dim3((C + 1 + SW2D_BX - 1) / SW2D_BX, (R + 1 + k.by - 1) / k.by);
+    return k;
+}
+
+size_t fp64_partials(int rows, int cols) {
+    const Cut64 k = cut_of(rows, cols);
+    const size_t prime = (size_t)((cols + SW2D_BX - 1) / SW2D_BX) * ((rows + SW2D_BY - 1) / SW2D_BY);
+    return NPART * std::max(prime, (size_t)2 * k.gx * k.gy);
+}
+
 void fp64_launch_iteration(const StepParams& p, int cur, cudaStream_t s, cudaEvent_t* ev) {
-    const dim3 blk(SW2D_BX, SW2D_BY);
+    const Cut64 k = cut_of(p.R, p.C);
     if (ev) cudaEventRecord(ev[0], s);
-    k64_flux<<<grid_faces(p), blk, 0, s>>>(p, cur);
+    if (k.by == 8) k64_flux<8><<<k.flux, dim3(SW2D_BX, 8), 0, s>>>(p, cur);
+    else k64_flux<2><<<k.flux, dim3(SW2D_BX, 2), 0, s>>>(p, cur);
     if (ev) cudaEventRecord(ev[1], s);
-    const dim3 gu((p.C + 1 + UT_W - 1) / UT_W, (p.R + 1 + UT_H - 1) / UT_H);
-    k64_update<<<gu, SW2D_BX * SW2D_BY, 0, s>>>(p, cur);
+    const int n = k.gx * k.gy + 1;
+    if (k.kind == 0) k64_update<64, 16, 256><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
+    else if (k.kind == 1) k64_update<32, 8, 256><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
+    else k64_update<32, 4, 128><<<n, 128, 0, s>>>(p, cur, k.gx, k.gy);
     if (ev) cudaEventRecord(ev[2], s);
 }
 
+void fp64_launch_settle(const StepParams& p, cudaStream_t s) {
+    const Cut64 k = cut_of(p.R, p.C);
+    k64_settle<<<1, SW2D_BX * SW2D_BY, 0, s>>>(p, k.gx, k.gy, (p.R - 1) / k.th);
+}
+
 void fp64_launch_prime(const StepParams& p, int cur, int full, cudaStream_t s) {
-    k64_prime<<<grid_cells(p), dim3(SW2D_BX, SW2D_BY), 0, s>>>(p, cur, full);
+    k64_prime<<<full ? grid_cells(p) : dim3(1, 1), dim3(SW2D_BX, SW2D_BY), 0, s>>>(p, cur, full);
 }
 
 void fp64_launch_face_velocity(const StepParams& p, int cur, cudaStream_t s) {

@@ -20,6 +20,8 @@
 #include <stdint.h>
 #include <cuda_runtime.h>
 
+#include "sw2d_math.h"
+
 #define SW2D_HALO 2
 #define SW2D_MAX_SRC 64
 #define SW2D_BX 32
@@ -59,10 +61,18 @@ struct DevClock {
     double s_max;      /* CFL speed of the current state */
     long long iters;
     double led[LED_N];
-    unsigned int counter; /* last-block ticket of the reduction kernels */
+    unsigned int counter; /* last-block ticket of k64_prime */
     int status;           /* bit 0: non-finite volume seen */
     long long outlet_n;
     long long iter_end;   /* the slot after iteration iter_end is inactive (a state copy) */
+};
+
+/* Running state between the kernels of consecutive iterations (not part of a
+ * snapshot: all zero whenever no iteration is in flight). */
+struct Flight64 {
+    unsigned long long smax[2][2]; /* per iteration parity: CFL face-speed maxima (bit patterns), x and y faces */
+    int pending;                   /* 1 + parity of the iteration whose ledger sums are not added yet, 0 none */
+    int pad;
 };
 
 /* Everything a step kernel needs, passed by value. */
@@ -71,7 +81,6 @@ struct StepParams {
     int outflow_south;
     int dt_mode, series_mode;
     int nsrc, nrain, nevap, nq;
-    int nblocks_cells;     /* blocks of the cell-grid reduction kernels */
     int outlet_cap;
     int ledger_cells;      /* 1: rain/evaporation volumes need a per-cell sum */
     double rain_static;    /* else: sum over active cells of weight * runoff fraction */
@@ -86,6 +95,7 @@ struct StepParams {
     int ncls;
     double gnn_uni;        /* (g n) n of the uniform n */
     int kdx, kdy;          /* dx = 2^kdx (dy = 2^kdy) when a power of two >= 1, else -1 */
+    sw2d_divisor ddx, ddy;
     const float* rainw;    /* rain weight per cell or NULL */
     const int* src_idx;    /* padded cell index per source */
     const double* rain;    /* nrain + 2 */
@@ -96,15 +106,17 @@ struct StepParams {
     double* qy[2];
     double* uu1;
     double* vv1;
-    double* partials;      /* nblocks_cells * 4: rain, evaporation, outlet sums */
-    double* partials_f;    /* nblocks_faces * 2: CFL face-speed maxima (bit patterns) */
-    int nblocks_faces;
+    double* partials;      /* fp64_partials(): per tile and iteration parity rain, evaporation, outlet sums */
+    Flight64* flight;
     double* outlet;        /* outlet_cap * 2 or NULL */
     DevClock* clk;
 };
 
 /* FP64 step kernels (sw2d_fp64.cu) */
+size_t fp64_partials(int rows, int cols); /* doubles the partials of a raster of this size take */
 void fp64_launch_iteration(const StepParams& p, int cur, cudaStream_t s, cudaEvent_t* ev);
+/* after the last iteration of a run: its ledger sums */
+void fp64_launch_settle(const StepParams& p, cudaStream_t s);
 void fp64_launch_prime(const StepParams& p, int cur, int full, cudaStream_t s);
 void fp64_launch_face_velocity(const StepParams& p, int cur, cudaStream_t s);
 void fp64_launch_cell_velocity(const StepParams& p, int cur, double* uu, double* vv, double* uua,
