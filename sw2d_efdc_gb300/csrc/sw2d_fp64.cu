@@ -21,10 +21,10 @@
  *                extra block adds up the previous iteration's partials in a
  *                fixed order and prepares the next iteration's length and
  *                forcing beside the tiles.
- * At 4096 x 4096 (pond break, 120 s in) an iteration takes 2.44 ms against
- * 5.17 ms with part-empty warps and a binary64 provisional depth; at 256 x
- * 256 26 us against 62 us, most of it the clock's work at the end of the last
- * tile's block before.
+ * At 4096 x 4096 (pond break) an iteration takes 1.92 ms against 5.17 ms
+ * with part-empty warps, a binary64 provisional depth and conversions and
+ * sums predicated off beside the path taken; at 256 x 256 24 us against 62 us,
+ * most of it the clock's work at the end of the last tile's block before.
  * forward (:670-693) is a buffer swap for the depth (h[cur] -> h[nxt]); the
  * discharges keep fixed roles: qx[0]/qy[0] hold the state, k64_flux writes
  * its new faces into qx[1]/qy[1], and k64_update writes every face, closed
@@ -42,6 +42,15 @@
 namespace sw2d {
 
 #define H SW2D_HALO
+
+/* a + b that stays inside the branch it is written in: the compiler otherwise
+ * computes it ahead for every lane and selects, 71 cycles a warp for a branch
+ * that is rarely or never taken */
+__device__ __forceinline__ double add_here(double a, double b) {
+    double r;
+    asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+}
 
 /* the entry in force at `time`: sw2d_series_index with the division on the integer pipes */
 __device__ __forceinline__ int series_index(double time, double dts, int n) {
@@ -171,11 +180,14 @@ __device__ __forceinline__ bool mid_range(double x) {
  * evaluation per edge gives bit-identical fluxes.  Halvings are exact while
  * nothing is subnormal, so with operands in the middle of the exponent range
  * the three of them are one quartering of the sum at the end. */
+__device__ __noinline__ double edge_term_wide(double w, double qs, double qd) {
+    const double a = sw2d_half(w);
+    return sw2d_half(a * qs) + sw2d_half(fabs(a) * qd);
+}
 __device__ __forceinline__ double edge_term(double w1, double w0, double q0, double q1) {
     const double w = w1 + w0, qs = q1 + q0, qd = q0 - q1;
     if (mid_range(w) && mid_range(qs) && mid_range(qd)) return sw2d_quarter(w * qs + fabs(w) * qd);
-    const double a = sw2d_half(w);
-    return sw2d_half(a * qs) + sw2d_half(fabs(a) * qd);
+    return edge_term_wide(w, qs, qd);
 }
 
 /* Kind of a face (SW2D-EFDC.cu:115-165, same tests in the same order):
@@ -313,7 +325,7 @@ __device__ __forceinline__ bool mean_ge(double ha, double hb, float est, double 
     const bool a = sw2d_ge_pos(ha, th), b = sw2d_ge_pos(hb, th);
     if (a == b) return a;
     if (fabsf(est - thf) > 1e-5f * thf) return est > thf;
-    return sw2d_ge_pos(sw2d_half(ha + hb), th);
+    return sw2d_ge_pos(sw2d_half(add_here(ha, hb)), th);
 }
 
 /* The new discharges of the faces of a 32 x BY block of cells (north and
@@ -336,7 +348,7 @@ __device__ __forceinline__ bool mean_ge(double ha, double hb, float est, double 
  * best are evaluated in binary64 and raise the maximum: the result is the
  * exact maximum in any order. */
 template <int BY>
-__global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 4 : 16) k64_flux(StepParams p, int cur) {
+__global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 5 : 16) k64_flux(StepParams p, int cur) {
     constexpr int BX = SW2D_BX, NT = BX * BY, SW = BX + 2, NV = (BY + 2) * SW, NH = (BY + 1) * SW;
     static_assert(BX == 32, "one row per warp: its ballot is the row's bit mask");
     __shared__ double sh[NH], sz[NH], se[NH];         /* depth, bed, surface: rows -1 .. BY-1 */
@@ -433,8 +445,8 @@ __global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 4 : 16) k64_flux(StepP
             const float cy = sw2d_f32_est_of_f64(__longlong_as_double((long long)__ldcg(best + 1)));
             const float wx = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ex))), cx) * 0.99999f;
             const float wy = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ey))), cy) * 0.99999f;
-            if (okx && ex >= wx) raise_max(best, face_speed(sf[U + s0], sw2d_half(hc + sh[s0 - SW]), p.g, p.rdx));
-            if (oky && ey >= wy) raise_max(best + 1, face_speed(sf[V + s0], sw2d_half(hc + sh[s0 - 1]), p.g, p.rdy));
+            if (okx && ex >= wx) raise_max(best, face_speed(sf[U + s0], sw2d_half(add_here(hc, sh[s0 - SW])), p.g, p.rdx));
+            if (oky && ey >= wy) raise_max(best + 1, face_speed(sf[V + s0], sw2d_half(add_here(hc, sh[s0 - 1])), p.g, p.rdy));
         }
     }
     __syncthreads();
@@ -518,10 +530,10 @@ __device__ __forceinline__ double continuity(const StepParams& p, size_t i, uint
         double qli = 0.0;
         for (int k = 0; k < p.nsrc; k++)
             if (p.src_idx[k] == (int)i) qli = ql[k];
-        sum = sum - qli;
+        sum = add_here(sum, -qli);
     }
     sum = sum - rcell * pct;
-    if (p.evap) sum = sum + evapo;
+    if (p.evap) sum = add_here(sum, evapo);
     double hn = ho - dt2 * sum;
     *raw = hn;
     *rain_term = rcell * pct;
@@ -670,6 +682,11 @@ __device__ void advance_clock(const StepParams& p, int cur, int gx, int gy, int 
  * estimate of the depth, by the exact binary64 continuity only where th lies
  * within the estimate's error (2^-19 of the magnitudes that enter it; the
  * estimate's own rounding stays below 2^-20 of them). */
+__device__ __noinline__ bool provisional_exact(const StepParams& p, const Slot& s, size_t i, uint8_t f, double ho,
+                                               double fN, double fS, double fW, double fE) {
+    double raw, rt;
+    return sw2d_lt_pos(continuity(p, i, f, ho, fS - fN, fE - fW, s.dt2, s.rr1, s.ev1, s.ql1, &raw, &rt), p.th);
+}
 struct DryEst {
     float th, ewl, dt2, rdx, rdy, pl, pd, ev;
 };
@@ -686,8 +703,7 @@ __device__ __forceinline__ bool provisional_dry(const StepParams& p, const Slot&
                                           fabsf(ev));
     const float d = hs - q.th;
     if (!(f & SW2D_F_SOURCE) && fabsf(d) > 1.9073486e-6f * (mag + q.th) + 1e-35f) return d < 0.f;
-    double raw, rt;
-    return sw2d_lt_pos(continuity(p, i, f, ho, fS - fN, fE - fW, s.dt2, s.rr1, s.ev1, s.ql1, &raw, &rt), p.th);
+    return provisional_exact(p, s, i, f, ho, fN, fS, fW, fE);
 }
 
 /* Tile of the update kernel: TW x TH cells (and their north and west faces)
@@ -698,9 +714,11 @@ __device__ __forceinline__ bool provisional_dry(const StepParams& p, const Slot&
  * does is a chain of dependent reads and divisions; at the end of the last
  * tile it would be the longest part of a small raster's iteration).
  * Bounded by the binary64 additions and products of the final depth and of
- * the face means (71 issue cycles a warp each): the flags take none. */
+ * the face means (71 issue cycles a warp each; the flags take none) and by
+ * the latencies between them: six blocks an SM (40 registers, 40 bytes of
+ * spills) against four measured 613 against 730 us at 4096 x 4096. */
 template <int TW, int TH, int NT>
-__global__ void __launch_bounds__(NT) k64_update(StepParams p, int cur, int gx, int gy) {
+__global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int gx, int gy) {
     constexpr int DW = TW + 3, DH = TH + 3, NW = TW + 1, NH = TH + 1;
     if (blockIdx.x == 0) {
         advance_clock(p, cur, gx, gy, (p.R - 1) / TH);
@@ -783,11 +801,11 @@ __global__ void __launch_bounds__(NT) k64_update(StepParams p, int cur, int gx, 
                 if (f & SW2D_F_ACTIVE) {
                     if (sw2d_lt0(raw)) atomicAdd(&p.clk->led[LED_CLAMP], -raw * p.area); /* max(h, 0) gain */
                     if (p.ledger_cells) {
-                        if (p.rainw) vr += rt;
+                        if (p.rainw) vr = add_here(vr, rt);
                         if (sw2d_gt(ho, p.ev_wl_min)) nlake++;
                         else nland++;
                     }
-                    if (r == R - 1 && p.outflow_south) vq += fS;
+                    if (r == R - 1 && p.outflow_south) vq = add_here(vq, fS);
                 }
             }
         }

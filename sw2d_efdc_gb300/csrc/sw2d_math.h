@@ -132,10 +132,10 @@ SW2D_HD double sw2d_scale_down(double x, int k) {
     return sw2d_f64_from_bits(sign | r);
 }
 /* x/2 and x/4 as used by the step.  On the device an exponent decrement
- * when the result stays normal, x itself when it is zero, and the binary64
- * product for the rest (all exact); the host evaluates the product.  Each
- * lane decides for itself: a zero among normal operands (dry or still cells)
- * costs no binary64 operation. */
+ * when the result stays normal, x itself when it is zero, and the shift of
+ * sw2d_scale_down for the rest (all exact; no binary64 instruction on any
+ * path: one that is predicated off still takes its 71 cycles); the host
+ * evaluates the product. */
 #if defined(__CUDACC__)
 __device__ __forceinline__ double sw2d_pow2_down(double x, int k, double m) { /* m = 2^-k, k >= 1 */
 #if defined(__CUDA_ARCH__)
@@ -143,8 +143,10 @@ __device__ __forceinline__ double sw2d_pow2_down(double x, int k, double m) { /*
     const uint32_t e = hi & 0x7ff00000u, kk = (uint32_t)k << 20;
     if (e - (kk + 0x00100000u) < 0x7fe00000u - kk) return __hiloint2double((int)(hi - kk), (int)lo);
     if (((hi << 1) | lo) == 0u) return x;
-#endif
+    return sw2d_scale_down(x, k);
+#else
     return x * m;
+#endif
 }
 __device__ __forceinline__ double sw2d_half(double x) { return sw2d_pow2_down(x, 1, 0.5); }
 __device__ __forceinline__ double sw2d_quarter(double x) { return sw2d_pow2_down(x, 2, 0.25); }
@@ -167,8 +169,8 @@ SW2D_HD float sw2d_fmaf(float a, float b, float c) { return fmaf(a, b, c); }
  * micro-benchmark: about one binary64 addition each).  These build the
  * result from the bit pattern instead. */
 
-/* (double)f, exact: normal and zero operands by integer operations (the
- * rest, subnormal, infinite or NaN, through the hardware conversion) */
+/* (double)f, exact, by integer operations and, for a subnormal, an exact
+ * binary32 scaling by 2^64 */
 SW2D_HD double sw2d_f64_of_f32(float f) {
     const uint32_t b = sw2d_f32_bits(f);
     const uint32_t e = (b >> 23) & 0xffu;
@@ -176,20 +178,24 @@ SW2D_HD double sw2d_f64_of_f32(float f) {
     if (e - 1u < 0xfeu)
         return sw2d_f64_from_bits(sign | ((uint64_t)(e + 896u) << 52) | ((uint64_t)(b & 0x7fffffu) << 29));
     if ((b & 0x7fffffffu) == 0u) return sw2d_f64_from_bits(sign);
-    return (double)f;
+    if (e == 0xffu) return sw2d_f64_from_bits(sign | 0x7ff0000000000000ULL | ((uint64_t)(b & 0x7fffffu) << 29));
+    const uint32_t n = sw2d_f32_bits(f * 18446744073709551616.0f);
+    return sw2d_f64_from_bits(sign | ((uint64_t)(((n >> 23) & 0xffu) + 832u) << 52) | ((uint64_t)(n & 0x7fffffu) << 29));
 }
 
 /* an estimate of (float)x for the binary32 prefilters: the significand
  * truncated to 24 bits (relative error below 2^-23); magnitudes below the
- * binary32 normal range give 0, above it the hardware conversion */
+ * binary32 normal range give 0, above it infinity.  No path holds a hardware
+ * conversion: predicated off, it would still take its 71 cycles of the FP64
+ * pipe. */
 SW2D_HD float sw2d_f32_est_of_f64(double x) {
     const uint64_t b = sw2d_f64_bits(x);
     const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
     const uint32_t e = (hi >> 20) & 0x7ffu;
-    if (e - 897u < 254u)
-        return sw2d_f32_from_bits((hi & 0x80000000u) | ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
-    if (e < 897u) return 0.0f;
-    return (float)x;
+    uint32_t r = (hi & 0x80000000u) | ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+    if (e < 897u) r = 0u;
+    if (e > 1150u) r = (hi & 0x80000000u) | ((b << 1) > 0xffe0000000000000ULL ? 0x7fc00000u : 0x7f800000u);
+    return sw2d_f32_from_bits(r);
 }
 
 /* an estimate of (float)v for a 32-bit unsigned v (relative error below
