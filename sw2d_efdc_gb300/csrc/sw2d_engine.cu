@@ -468,18 +468,19 @@ int Engine32::rebuild(std::string* err) {
     return SW2D_OK;
 }
 
-/* CTAs of class k's persistent launch over niter iterations: the CTAs per
- * SM in use (at most what the SM holds) on every SM, at most one per queue
- * ticket */
-int Engine32::grid_of(int k, int niter) const {
+/* CTAs of class k's persistent launch: the CTAs per SM in use (at most what
+ * the SM holds) on every SM, at most one per work item -- no more items than
+ * that can run at a time, and CTAs that hold later iterations' tickets poll
+ * the counters that the running ones release */
+int Engine32::grid_of(int k) const {
     const int per_sm = cps_ > 0 ? std::min(cps_, bps_[k]) : bps_[k];
-    return (int)std::max<long long>(1, std::min<long long>((long long)per_sm * nsm_, (long long)class_n_[k] * niter));
+    return std::max(1, std::min(per_sm * nsm_, class_n_[k]));
 }
 
 /* niter iterations: one persistent launch per feature class present */
 int Engine32::launch(int niter, std::string* err) {
     int grid[T32_NCLASS];
-    for (int k = 0; k < T32_NCLASS; k++) grid[k] = grid_of(k, niter);
+    for (int k = 0; k < T32_NCLASS; k++) grid[k] = grid_of(k);
     ECK(fp32_launch_chunk(d_scn_, (int)scn_.size(), d_work_, class_first_, class_n_, d_part_, d_ctl_, niter, grid,
                           stream_));
     return SW2D_OK;
@@ -490,7 +491,7 @@ int Engine32::build_graph(std::string* err) {
     cudaGraph_t g = nullptr;
     ECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     int grid[T32_NCLASS];
-    for (int k = 0; k < T32_NCLASS; k++) grid[k] = grid_of(k, kChunk);
+    for (int k = 0; k < T32_NCLASS; k++) grid[k] = grid_of(k);
     cudaError_t el = fp32_launch_chunk(d_scn_, (int)scn_.size(), d_work_, class_first_, class_n_, d_part_, d_ctl_, kChunk,
                                        grid, stream_);
     cudaError_t ec = cudaStreamEndCapture(stream_, &g);

@@ -148,7 +148,7 @@ class Engine32 {
      * the fastest, cached per size bucket (log2 of the work set's cells).
      * Advances at most `budget` iterations and returns how many. */
     int tune(long long budget, std::string* err, long long* advanced);
-    int grid_of(int k, int niter) const;
+    int grid_of(int k) const;
     int device_;
     int nsm_ = 0;
     int bps_[T32_NCLASS] = {};  /* CTAs per SM of each class's persistent kernel */

@@ -60,8 +60,8 @@ struct SmemM {
     unsigned long long bar[NS];
     float ntab[T32_MAXCLASS];
     float dband[M_MAXBANDS][3]; /* datums of the bands the item spans, strips west / own / east */
-    double red[NW][4];
-    float redf[NW][2];
+    double red[NW][4];          /* a scenario's reduction, warp by warp: clamp, outlet, rain, lake cells */
+    float redf[NW][6];          /* the same of an item, then the CFL face-speed maxima */
     int nls;                    /* point sources inside the work item's staged window */
     int srow[T32_MAXSRC], scol[T32_MAXSRC];
     float sq1[T32_MAXSRC], sq2[T32_MAXSRC];
@@ -312,6 +312,30 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
         }
         return true; /* tile skipped, status bit 2 */
     }
+    constexpr bool has_cls = CLS, has_rw = RW;
+    const unsigned blk_bytes = (unsigned)NF * RB * BW * 4u + (has_cls ? (unsigned)(M_CLSR * M_CLSW) : 0u) +
+                               (has_rw ? (unsigned)(M_RWR * BW * 4) : 0u);
+    /* block b holds rows Ls + b*RB .. +RB-1 of h, z, qx, qy, the Kahan
+     * compensation of the rows three above (the rows finished during b) and,
+     * when present, the class rows from two above and the rain weights from
+     * three above */
+    auto issue = [&](int b, int st) {
+        mbar_arrive_expect_tx(&S.bar[st], blk_bytes);
+        const int y = Ls + b * RB + M_H; /* padded row of the block's first row */
+        tma_load_2d(&S.stage[st][0][0][0], &P.tm_h[cur], c0, y, &S.bar[st]);
+        tma_load_2d(&S.stage[st][1][0][0], &P.tm_z, c0, y, &S.bar[st]);
+        tma_load_2d(&S.stage[st][2][0][0], &P.tm_qx[cur], c0, y, &S.bar[st]);
+        tma_load_2d(&S.stage[st][3][0][0], &P.tm_qy[cur], c0, y, &S.bar[st]);
+        tma_load_2d(&S.stage[st][4][0][0], &P.tm_kc, c0, y - 3, &S.bar[st]);
+        if (has_cls) tma_load_2d(&S.cls[st].v[0][0], &P.tm_cls, c0, y - 2, &S.bar[st]);
+        if (has_rw) tma_load_2d(&S.rw[st].v[0][0], &P.tm_rw, c0, y - 3, &S.bar[st]);
+    };
+    if (tid == 0 && !P.stall_staging) {
+        /* the staging buffers were last read by the generic proxy */
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        for (int b = 0; b < NS && b < nblk; b++) issue(b, (int)((gb + b) % NS));
+    }
+    /* while the first blocks are on their way */
     if (tid < T32_MAXCLASS) S.ntab[tid] = P.ntab[tid];
     if (SRC && warp == 0) {
         /* the point sources inside the staged window (rows rs-3 .. re+2,
@@ -347,29 +371,6 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
         S.dband[j][cr] = (nx >= 0 && nx < P.tiles_x && b0 + j < P.bands) ? P.datum[(b0 + j) * P.tiles_x + nx] : 0.f;
     }
     __syncthreads();
-    constexpr bool has_cls = CLS, has_rw = RW;
-    const unsigned blk_bytes = (unsigned)NF * RB * BW * 4u + (has_cls ? (unsigned)(M_CLSR * M_CLSW) : 0u) +
-                               (has_rw ? (unsigned)(M_RWR * BW * 4) : 0u);
-    /* block b holds rows Ls + b*RB .. +RB-1 of h, z, qx, qy, the Kahan
-     * compensation of the rows three above (the rows finished during b) and,
-     * when present, the class rows from two above and the rain weights from
-     * three above */
-    auto issue = [&](int b, int st) {
-        mbar_arrive_expect_tx(&S.bar[st], blk_bytes);
-        const int y = Ls + b * RB + M_H; /* padded row of the block's first row */
-        tma_load_2d(&S.stage[st][0][0][0], &P.tm_h[cur], c0, y, &S.bar[st]);
-        tma_load_2d(&S.stage[st][1][0][0], &P.tm_z, c0, y, &S.bar[st]);
-        tma_load_2d(&S.stage[st][2][0][0], &P.tm_qx[cur], c0, y, &S.bar[st]);
-        tma_load_2d(&S.stage[st][3][0][0], &P.tm_qy[cur], c0, y, &S.bar[st]);
-        tma_load_2d(&S.stage[st][4][0][0], &P.tm_kc, c0, y - 3, &S.bar[st]);
-        if (has_cls) tma_load_2d(&S.cls[st].v[0][0], &P.tm_cls, c0, y - 2, &S.bar[st]);
-        if (has_rw) tma_load_2d(&S.rw[st].v[0][0], &P.tm_rw, c0, y - 3, &S.bar[st]);
-    };
-    if (tid == 0 && !P.stall_staging) {
-        /* the staging buffers were last read by the generic proxy */
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        for (int b = 0; b < NS && b < nblk; b++) issue(b, (int)((gb + b) % NS));
-    }
 
     /* lane geometry: staged columns sc, sc+1; global columns cg, cg+1 */
     const int sc = warp * M_SW + 2 * lane;
@@ -690,73 +691,78 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
         evc += __shfl_xor_sync(0xffffffffu, evc, o);
     }
     if (lane == 0) {
-        S.red[warp][0] = clamp;
-        S.red[warp][1] = qout;
-        S.red[warp][2] = rainacc;
-        S.red[warp][3] = evc;
-        S.redf[warp][0] = sxm;
-        S.redf[warp][1] = sym;
+        float* f = S.redf[warp];
+        f[0] = clamp;
+        f[1] = qout;
+        f[2] = rainacc;
+        f[3] = evc;
+        f[4] = sxm;
+        f[5] = sym;
     }
     __syncthreads();
-    if (tid == 0) {
-        Part32 pr = {};
-        float mx = 0.f, my = 0.f;
-        for (int k = 0; k < NW; k++) {
-            pr.clamp += S.red[k][0];
-            pr.qout += S.red[k][1];
-            pr.rain += S.red[k][2];
-            pr.evap += S.red[k][3];
-            mx = fmaxf(mx, S.redf[k][0]);
-            my = fmaxf(my, S.redf[k][1]);
+    /* lane q of the first warp combines the q-th quantity (a binary64 addition
+     * takes 71 cycles whether one lane or six take part) */
+    if (tid < 6) {
+        Part32* o = part + w.w; /* the partials stay in scenario order whatever the launch order */
+        if (tid < 4) {
+            double v = 0.0;
+            for (int k = 0; k < NW; k++) v += sw2d_f64_of_f32(S.redf[k][tid]);
+            (tid == 0 ? &o->clamp : tid == 1 ? &o->qout : tid == 2 ? &o->rain : &o->evap)[0] = v;
+        } else {
+            float v = 0.f;
+            for (int k = 0; k < NW; k++) v = fmaxf(v, S.redf[k][tid]);
+            /* rdx > 0: the maximum commutes with the scaling */
+            (tid == 4 ? &o->sx : &o->sy)[0] = v * (tid == 4 ? rdxy.x : rdxy.y);
         }
-        pr.sx = mx * rdxy.x; /* rdx > 0: the maximum commutes with the scaling */
-        pr.sy = my * rdxy.y;
-        part[w.w] = pr; /* the partials stay in scenario order whatever the launch order */
     }
+    __syncwarp();
     return true;
 }
 
 /* ---------------- per-scenario finalize ---------------------------------- */
 
-__device__ double series_at32(const double* v, int n, double dts, double time, int mode) {
-    int it;
-    if (mode == 0) {
-        if (time <= 1.00) return v[0] * time;
-        it = sw2d_series_index(time, dts, n);
-        return v[it] + (v[it + 1] - v[it]) / (dts * (time - dts * (it)));
-    } else if (mode == 1) {
-        it = sw2d_series_index(time, dts, n);
-        return v[it] + (v[it + 1] - v[it]) * ((time - dts * (it)) / dts);
-    }
-    it = sw2d_series_index(time, dts, n);
-    return v[it];
+/* the entry in force at `time`: sw2d_series_index with the division on the integer pipes */
+__device__ __forceinline__ int series_index32(double time, double dts, int n) {
+    const double f = sw2d_div_rn(time, dts);
+    return f >= (double)n ? n : (int)f;
+}
+
+__device__ __forceinline__ double series_at32(const double* v, int n, double dts, double time, int mode) {
+    if (mode == 0 && time <= 1.00) return v[0] * time;
+    const int it = series_index32(time, dts, n);
+    const double a = v[it];
+    if (mode == 2) return a;
+    const double b = v[it + 1], d = time - dts * (it);
+    return mode == 0 ? a + sw2d_div_rn(b - a, dts * d) : a + (b - a) * sw2d_div_rn(d, dts);
 }
 
 /* point-source rate (m/s) of source i at time t: the reference's stream_flow
  * interpolation (SW2D-EFDC.cu:531-538) in REFERENCE mode, else LINEAR / STEP */
-__device__ float source_at32(const Scn32& P, int i, double time) {
+__device__ __forceinline__ float source_at32(const Scn32& P, int i, double time) {
     const double* Q = P.srcq;
     const int ns = P.nsrc;
     double q;
     if (P.series_mode == 0 && time <= 1.00) {
         q = Q[i] * time;
     } else {
-        const int it = sw2d_series_index(time, P.dtoq, P.nq);
-        const double a = Q[(size_t)it * ns + i], b = Q[(size_t)(it + 1) * ns + i];
+        const int it = series_index32(time, P.dtoq, P.nq);
+        const double a = Q[(size_t)it * ns + i], b = Q[(size_t)(it + 1) * ns + i], d = time - P.dtoq * (it);
         if (P.series_mode == 0)
-            q = a + (b - a) / (P.dtoq * (time - P.dtoq * (it)));
+            q = a + sw2d_div_rn(b - a, P.dtoq * d);
         else if (P.series_mode == 1)
-            q = a + (b - a) * ((time - P.dtoq * (it)) / P.dtoq);
+            q = a + (b - a) * sw2d_div_rn(d, P.dtoq);
         else
             q = a;
     }
-    return (float)(q / (P.dxd * P.dyd));
+    return (float)sw2d_div_rn(q, P.dxd * P.dyd);
 }
 
-/* Length and forcing of the iteration starting at time t.  The clock is
- * accessed as volatile: inside a persistent launch the CTA that reduces a
- * scenario's iteration may sit on another SM than the previous one's. */
-__device__ void prepare_slot32(const Scn32& P, volatile Clock32* clk, double t, double t_end, double s_max) {
+/* Length and forcing of the iteration starting at time t, by one whole warp:
+ * every lane computes the length, lane k the k-th of the quotients and series
+ * values that follow from it (independent chains of divisions and reads that
+ * one thread would walk one after another). */
+__device__ __forceinline__ void prepare_slot32(const Scn32& P, Clock32* clk, double t, double t_end, double s_max) {
+    const int lane = threadIdx.x & 31;
     double dt2, tm;
     int active;
     if (P.dt_mode == 0) {
@@ -768,108 +774,138 @@ __device__ void prepare_slot32(const Scn32& P, volatile Clock32* clk, double t, 
         tm = t + dt;
     } else {
         active = (t < t_end);
-        dt2 = s_max > 0 ? fmin(P.dt_max, P.cfl / s_max) : P.dt_max;
+        dt2 = s_max > 0 ? fmin(P.dt_max, sw2d_div_rn(P.cfl, s_max)) : P.dt_max;
         dt2 = (double)(float)dt2;
         if (t + dt2 > t_end) dt2 = t_end - t;
         tm = t + 0.5 * dt2;
     }
-    volatile Slot32& s = clk->slot;
-    s.active = active;
-    s.dt2 = (float)dt2;
-    s.dt2dx = (float)(dt2 / P.dxd);
-    s.dt2dy = (float)(dt2 / P.dyd);
-    s.rr1 = (float)(series_at32(P.rain, P.nrain, P.dtrain, t, P.series_mode) / (P.dtrain * 1000.0));
-    s.rr2 = (float)(series_at32(P.rain, P.nrain, P.dtrain, tm, P.series_mode) / (P.dtrain * 1000.0));
-    if (P.evap) {
-        s.ev1 = (float)(series_at32(P.evap, P.nevap, P.dtrain, t, P.series_mode) / (P.dtrain * 1000.0));
-        s.ev2 = (float)(series_at32(P.evap, P.nevap, P.dtrain, tm, P.series_mode) / (P.dtrain * 1000.0));
-    } else {
-        s.ev1 = s.ev2 = 0.f;
+    Slot32& s = clk->slot;
+    if (lane == 0) {
+        s.active = active;
+        s.dt2 = (float)dt2;
+        clk->dt2 = dt2;
+        if (!active) clk->done = 1;
     }
-    for (int k = 0; k < P.nsrc; k++) {
-        clk->ql1[k] = source_at32(P, k, t);
-        clk->ql2[k] = source_at32(P, k, tm);
+    if (lane < 2) (lane ? &s.dt2dy : &s.dt2dx)[0] = (float)sw2d_div_rn(dt2, lane ? P.dyd : P.dxd);
+    if (lane < 4) { /* rain at t and tm, then evaporation */
+        const bool ev = lane >= 2;
+        const double* v = ev ? P.evap : P.rain;
+        float r = 0.f;
+        if (v)
+            r = (float)sw2d_div_rn(series_at32(v, ev ? P.nevap : P.nrain, P.dtrain, (lane & 1) ? tm : t, P.series_mode),
+                                   P.dtrain * 1000.0);
+        (ev ? ((lane & 1) ? &s.ev2 : &s.ev1) : ((lane & 1) ? &s.rr2 : &s.rr1))[0] = r;
     }
-    clk->dt2 = dt2;
-    if (!active) clk->done = 1;
+    for (int k = lane; k < 2 * P.nsrc; k += 32) {
+        const int i = k >> 1;
+        ((k & 1) ? clk->ql2 : clk->ql1)[i] = source_at32(P, i, (k & 1) ? tm : t);
+    }
 }
 
 /* One scenario's end of iteration, run by the whole CTA: fixed-order sum of
  * its work items' partials (each thread a fixed stride of them, then the
  * warps and the CTA in a fixed order; read past L1: other CTAs wrote them
- * during this launch), then, by thread 0, the ledger, clock, outlet record
- * and the next slot. */
+ * during this launch), then, by the first warp, the ledger, clock, outlet
+ * record and the next slot.  Every CTA waiting for this scenario waits for
+ * it, so its latency counts: the clock is read at once, up front and past
+ * L1 (the CTA that reduced the previous iteration may sit on another SM), the
+ * ledger's entries are updated by one lane each, and sums that the scenario
+ * cannot have are skipped (a binary64 addition takes a warp 71 cycles). */
 __device__ __noinline__ void finalize_scn(const Scn32& P, const Part32* __restrict__ part, double (*red)[4],
-                                          float (*redf)[2]) {
+                                          float (*redf)[6]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    volatile Clock32* clk = P.clk;
-    double clamp = 0, qout = 0, rain = 0, evc = 0;
+    Clock32* clk = P.clk;
+    double v[4] = {0, 0, 0, 0}; /* clamp, outlet, rain, lake cells */
     float sx = 0.f, sy = 0.f;
     for (int k = tid; k < P.nwork; k += NT) {
         const Part32* q = part + P.first_work + k;
-        clamp += __ldcg(&q->clamp);
-        qout += __ldcg(&q->qout);
-        rain += __ldcg(&q->rain);
-        evc += __ldcg(&q->evap);
+        v[0] += __ldcg(&q->clamp);
+        if (P.outflow_south) v[1] += __ldcg(&q->qout);
+        if (P.ledger_cells) {
+            v[2] += __ldcg(&q->rain);
+            v[3] += __ldcg(&q->evap);
+        }
         sx = fmaxf(sx, __ldcg(&q->sx));
         sy = fmaxf(sy, __ldcg(&q->sy));
     }
+    double t = 0, t_end = 0, dt2 = 0, acc = 0;
+    long long iters = 0, outlet_n = 0;
+    float rr2 = 0.f, ev2 = 0.f;
+    int active = 0, cur = 0;
+    if (warp == 0) {
+        t = __ldcg(&clk->t);
+        t_end = __ldcg(&clk->t_end);
+        dt2 = __ldcg(&clk->dt2);
+        iters = __ldcg(&clk->iters);
+        outlet_n = __ldcg(&clk->outlet_n);
+        rr2 = __ldcg(&clk->slot.rr2);
+        ev2 = __ldcg(&clk->slot.ev2);
+        active = __ldcg(&clk->slot.active);
+        cur = __ldcg(&clk->slot.cur);
+        /* rain_in, source_in, evap_out, outflow, clamp_gain */
+        if (lane < 5) acc = __ldcg(&clk->rain_in + lane);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (q == 0 ? __any_sync(0xffffffffu, v[0] != 0.0) : q == 1 ? P.outflow_south != 0 : P.ledger_cells != 0) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+        }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        clamp += __shfl_down_sync(0xffffffffu, clamp, o);
-        qout += __shfl_down_sync(0xffffffffu, qout, o);
-        rain += __shfl_down_sync(0xffffffffu, rain, o);
-        evc += __shfl_down_sync(0xffffffffu, evc, o);
         sx = fmaxf(sx, __shfl_down_sync(0xffffffffu, sx, o));
         sy = fmaxf(sy, __shfl_down_sync(0xffffffffu, sy, o));
     }
     if (lane == 0) {
-        red[warp][0] = clamp;
-        red[warp][1] = qout;
-        red[warp][2] = rain;
-        red[warp][3] = evc;
+#pragma unroll
+        for (int q = 0; q < 4; q++) red[warp][q] = v[q];
         redf[warp][0] = sx;
         redf[warp][1] = sy;
     }
     __syncthreads();
-    if (tid != 0 || !clk->slot.active) return;
+    if (warp != 0 || !active) return;
+    double sum = 0.0;
+    if (lane < 4) {
+        sum = red[0][lane];
+        for (int k = 1; k < NW; k++) sum += red[k][lane];
+    }
+    sx = redf[0][0];
+    sy = redf[0][1];
     for (int k = 1; k < NW; k++) {
-        clamp += red[k][0];
-        qout += red[k][1];
-        rain += red[k][2];
-        evc += red[k][3];
         sx = fmaxf(sx, redf[k][0]);
         sy = fmaxf(sy, redf[k][1]);
     }
-    const float rr2 = clk->slot.rr2, ev2 = clk->slot.ev2;
-    const int cur = clk->slot.cur;
-    const double dt2 = clk->dt2;
-    const double area = P.area;
-    const double rain_sum = P.ledger_cells ? rain : P.rain_static;
-    clk->rain_in = clk->rain_in + dt2 * (double)rr2 * rain_sum * area;
-    clk->evap_out = clk->evap_out + dt2 * (double)ev2 * evc * area;
+    const double clamp = __shfl_sync(0xffffffffu, sum, 0), qout = __shfl_sync(0xffffffffu, sum, 1),
+                 rain = __shfl_sync(0xffffffffu, sum, 2), evc = __shfl_sync(0xffffffffu, sum, 3);
+    const double area = P.area, q_out = qout * P.dyd;
     double qsrc = 0.0;
-    for (int k = 0; k < P.nsrc; k++) qsrc += (double)clk->ql2[k];
-    clk->source_in = clk->source_in + dt2 * qsrc * area;
-    clk->clamp_gain = clk->clamp_gain + clamp * area;
-    const double q_out = qout * P.dyd;
-    clk->q_out = q_out;
-    clk->outflow = clk->outflow + dt2 * q_out;
+    for (int k = 0; k < P.nsrc; k++) qsrc += (double)__ldcg(&clk->ql2[k]);
+    /* lane by lane as acc is: ((a b) c) d */
+    const double fa = lane == 4 ? 1.0 : dt2;
+    const double fb = lane == 0 ? (double)rr2 : lane == 2 ? (double)ev2 : 1.0;
+    const double fc = lane == 0 ? (P.ledger_cells ? rain : P.rain_static) : lane == 1 ? qsrc : lane == 2 ? evc : lane == 3 ? q_out : clamp;
+    acc += fa * fb * fc * (lane == 3 ? 1.0 : area);
     /* the CFL speed of the state this iteration started from */
     const double s_max = (double)sx + (double)sy;
-    clk->s_max = s_max;
-    if (!isfinite(s_max) || !isfinite(qout)) clk->status = clk->status | 1;
-    const double t = (P.dt_mode == 0) ? (clk->t + P.dt_fixed) + P.dt_fixed : clk->t + dt2;
-    clk->t = t;
-    clk->iters = clk->iters + 1;
-    clk->slot.cur = cur ^ 1;
-    if (P.outlet) {
-        const long long k = clk->outlet_n % P.outlet_cap;
-        P.outlet[2 * k] = t;
-        P.outlet[2 * k + 1] = q_out;
-        clk->outlet_n = clk->outlet_n + 1;
+    const double tn = (P.dt_mode == 0) ? (t + P.dt_fixed) + P.dt_fixed : t + dt2;
+    if (lane < 5) (&clk->rain_in)[lane] = acc;
+    if (lane == 0) {
+        clk->q_out = q_out;
+        clk->s_max = s_max;
+        if (!isfinite(s_max) || !isfinite(qout)) atomicOr(&clk->status, 1);
+        clk->t = tn;
+        clk->iters = iters + 1;
+        clk->slot.cur = cur ^ 1;
+        if (P.outlet) {
+            const long long k = outlet_n % P.outlet_cap;
+            P.outlet[2 * k] = tn;
+            P.outlet[2 * k + 1] = q_out;
+            clk->outlet_n = outlet_n + 1;
+        }
     }
-    prepare_slot32(P, clk, t, clk->t_end, s_max);
+    __syncwarp(); /* the rates above are read before they are replaced */
+    prepare_slot32(P, clk, tn, t_end, s_max);
+    __syncwarp();
 }
 
 /* ---------------- the persistent launch ---------------------------------- */
@@ -896,7 +932,8 @@ __device__ __noinline__ unsigned wait_ticket(unsigned q, const Scn32* __restrict
     volatile unsigned* abort_flag = &ctl->abort;
     if (q >= (unsigned)nwork * (unsigned)niter || *abort_flag) return ~0u;
     const int it = (int)(q / (unsigned)nwork);
-    const int sc = work[q % (unsigned)nwork].x;
+    const int4 w = work[q % (unsigned)nwork];
+    const int sc = w.x;
     const long long t0 = clock64();
     while (ld_acquire_gpu(&done[sc]) < it) {
         if (*abort_flag) return ~0u;
@@ -963,7 +1000,7 @@ __global__ void __launch_bounds__(NT, 4) k32_persist(const Scn32* __restrict__ s
         const unsigned q = __shfl_sync(0xffffffffu, S.q, 0);
         if (q == ~0u) break;
         if (threadIdx.x == 0) S.qn = atomicAdd(&ctl->next, 1u); /* the next ticket, drawn while this item runs */
-        const int4 w = work[q % (unsigned)nwork];
+        const int4 w = work[q % (unsigned)nwork]; /* in L1: thread 0 read it while it waited */
         /* the previous iteration's state was written by other CTAs with
          * generic stores; this item reads it with TMA (the async proxy) */
         asm volatile("fence.proxy.async.global;" ::: "memory");
@@ -982,12 +1019,13 @@ __global__ void __launch_bounds__(NT, 4) k32_persist(const Scn32* __restrict__ s
     }
 }
 
-/* first slot of every scenario from its clock (t, s_max, t_end) */
+/* first slot of every scenario from its clock (t, s_max, t_end), one warp each */
 __global__ void k32_prime(const Scn32* __restrict__ scns, int nscn) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (s >= nscn) return;
-    volatile Clock32* clk = scns[s].clk;
-    clk->done = 0;
+    Clock32* clk = scns[s].clk;
+    if ((threadIdx.x & 31) == 0) clk->done = 0;
+    __syncwarp();
     prepare_slot32(scns[s], clk, clk->t, clk->t_end, clk->s_max);
 }
 
@@ -1196,7 +1234,7 @@ cudaError_t fp32_launch_chunk(const Scn32* d_scn, int nscn, const int4* d_work, 
 }
 
 void fp32_launch_prime(const Scn32* d_scn, int nscn, cudaStream_t s) {
-    k32_prime<<<(nscn + 127) / 128, 128, 0, s>>>(d_scn, nscn);
+    k32_prime<<<(nscn + 3) / 4, 128, 0, s>>>(d_scn, nscn);
 }
 
 void fp32_launch_volume(const Scn32* d_scn, int iscn, const Scn32& host_scn, double* d_out, cudaStream_t s) {
