@@ -53,7 +53,8 @@ typedef struct sw2d_scenario {
 typedef struct sw2d_batch_stats {
     int running, queued;
     int work_items;           /* tiles per iteration */
-    int rows_per_item;        /* rows of a work item in use (the autotuner's choice unless set) */
+    int rows_per_item;        /* rows of a work item as set; else the most one may have (the autotuner's choice: a
+                               * work set too small to fill the GPU with such items is cut into shorter ones) */
     double bytes_in_use;
     double device_ms;         /* device time of all iterations so far */
     double cell_updates;      /* sum over scenarios of cells x iterations advanced */

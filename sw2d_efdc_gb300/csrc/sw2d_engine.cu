@@ -402,6 +402,51 @@ int Engine32::remove(int index) {
     return SW2D_OK;
 }
 
+/* Rows per work item of class k: at most seg_, fewer where that leaves the
+ * GPU idle.  An iteration of a class is modelled by what the persistent
+ * kernel measures on a GB300: a CTA marches a row in 1.03 us when it has its
+ * SM to itself, 1.30, 1.52 or 1.85 us beside one, two or three others, over
+ * the item's rows and their six halo rows in whole blocks of M_RB, and about
+ * 9.5 us go by from one iteration's last row to the next one's first.  One
+ * scenario's items run in whole waves over the CTAs; several scenarios fill
+ * one another's gaps.  Against items of 128 rows: 200 x 310 cells 147 -> 21 us
+ * an iteration (2 rows), 1000 x 1000 152 -> 40 (14), 2048 x 2048 172 -> 92
+ * (38); from about 12 M cells on, items of seg_ rows fill the GPU and the
+ * halo rows decide. */
+int Engine32::fill_rows(int k) const {
+    static const double row_us[4] = {1.03, 1.30, 1.52, 1.85};
+    const int per_sm = std::max(1, cps_ > 0 ? std::min(cps_, bps_[k]) : bps_[k]);
+    const int slots = per_sm * nsm_;
+    std::vector<const Scn32*> in;
+    for (auto& s : scn_)
+        if (fp32_feature_class(s->d) == k) in.push_back(&s->d);
+    int best = seg_;
+    double best_us = 0.0;
+    for (int n = 0;; n++) { /* 2, 6, 10, ... rows and the halo make whole blocks; and seg_ itself */
+        const int seg = std::min(seg_, 2 + M_RB * n);
+        long long items = 0, rows = 0;
+        int longest = 0;
+        for (const Scn32* d : in) {
+            const int r = std::min(seg, d->R), ni = d->tiles_x * ((d->R + r - 1) / r);
+            const int marched = (r + 6 + M_RB - 1) / M_RB * M_RB;
+            items += ni;
+            rows += (long long)ni * marched;
+            longest = std::max(longest, marched);
+        }
+        const long long busy = std::min<long long>(items, slots);
+        const double us = row_us[std::min(3, (int)((busy + nsm_ - 1) / nsm_) - 1)];
+        const double waves = in.size() == 1 ? (double)longest * (double)((items + slots - 1) / slots)
+                                            : std::max((double)longest, (double)rows / (double)slots);
+        const double t = waves * us;
+        if (n == 0 || t <= best_us) {
+            best = seg;
+            best_us = t;
+        }
+        if (seg == seg_) break;
+    }
+    return best;
+}
+
 int Engine32::rebuild(std::string* err) {
     if (!dirty_) return SW2D_OK;
     work_.clear();
@@ -410,10 +455,13 @@ int Engine32::rebuild(std::string* err) {
      * .w is the item's slot in the scenario-ordered partials */
     for (int k = 0; k < T32_NCLASS; k++) {
         class_first_[k] = (int)work_.size();
+        bool any = false;
+        for (auto& sp : scn_) any = any || fp32_feature_class(sp->d) == k;
+        const int rows = !any || seg_fixed_ > 0 ? seg_ : fill_rows(k);
         for (size_t i = 0; i < scn_.size(); i++) {
             Scn32& d = scn_[i]->d;
             if (fp32_feature_class(d) != k) continue;
-            d.seg = std::min(seg_, d.R);
+            d.seg = std::min(rows, d.R);
             d.tiles_y = (d.R + d.seg - 1) / d.seg;
             d.first_work = (int)work_.size();
             for (int ty = 0; ty < d.tiles_y; ty++)

@@ -125,7 +125,7 @@ class Engine32 {
         tuned_.clear();
         bucket_ = -1;
     }
-    int segment_rows() const { return seg_; }
+    int segment_rows() const { return seg_; } /* the most a work item has: fill_rows */
     /* CTAs per SM of the persistent launches (the autotuner's second
      * choice; 0 = every CTA the SM holds) */
     int ctas_per_sm() const { return cps_; }
@@ -140,9 +140,10 @@ class Engine32 {
 
   private:
     int rebuild(std::string* err);
+    int fill_rows(int k) const;
     int build_graph(std::string* err);
     int launch(int niter, std::string* err);
-    /* the autotuner: times each candidate pair (rows per item, CTAs per
+    /* the autotuner: times each candidate pair (most rows per item, CTAs per
      * SM) on the scenarios' own iterations -- one untimed, then up to a
      * chunk's worth in one persistent launch, as the chunks run -- and keeps
      * the fastest, cached per size bucket (log2 of the work set's cells).
@@ -170,7 +171,7 @@ class Engine32 {
     cudaEvent_t ev_a_ = nullptr, ev_b_ = nullptr, ev_t0_ = nullptr, ev_t1_ = nullptr;
     double last_ms_ = 0.0;
     long long last_iters_ = 0;
-    int seg_ = 128;            /* rows per work item in use */
+    int seg_ = 128;            /* rows per work item in use; unless fixed, the most (fill_rows) */
     int seg_fixed_ = 0;        /* set by set_segment_rows or SW2D_SEGMENT_ROWS */
     int cps_ = 0;              /* CTAs per SM in use (0: all that fit) */
     int bucket_ = -1;          /* size bucket the setting in use was chosen for */
