@@ -43,15 +43,6 @@ namespace sw2d {
 
 #define H SW2D_HALO
 
-/* a + b that stays inside the branch it is written in: the compiler otherwise
- * computes it ahead for every lane and selects, 71 cycles a warp for a branch
- * that is rarely or never taken */
-__device__ __forceinline__ double add_here(double a, double b) {
-    double r;
-    asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
-    return r;
-}
-
 /* the entry in force at `time`: sw2d_series_index with the division on the integer pipes */
 __device__ __forceinline__ int series_index(double time, double dts, int n) {
     const double f = sw2d_div_rn(time, dts);
@@ -159,7 +150,6 @@ __device__ __forceinline__ double friction(const StepParams& p, double coef, dou
 /* a / dx for the continuity: exact scaling when dx is a power of two (the
  * constant division returns the same bits), else sw2d_div_by */
 __device__ __forceinline__ double div_spacing(double a, const sw2d_divisor& d, int k) {
-    if (sw2d_is0(a)) return 0.0;
     if (k < 0) return sw2d_div_by(a, &d);
     return k == 0 ? a : sw2d_pow2_down(a, k, d.rd);
 }
@@ -314,9 +304,15 @@ __device__ __forceinline__ void block_face_speed_max2(bool okx, double vx, doubl
     *sy = by;
 }
 
-/* raise a running maximum of non-negative doubles kept as bit patterns */
-__device__ __forceinline__ void raise_max(unsigned long long* at, double v) {
-    atomicMax(at, (unsigned long long)__double_as_longlong(v));
+/* Rare binary64 work as calls: inlined, its instructions are computed ahead
+ * of their branch or predicated, and one that is predicated off still takes
+ * its 71 cycles. */
+__device__ __noinline__ bool mean_ge_exact(double ha, double hb, double th) {
+    return sw2d_ge_pos(sw2d_half(ha + hb), th);
+}
+/* raises a running maximum (bits of non-negative doubles) to a face's speed */
+__device__ __noinline__ void raise_speed(unsigned long long* at, double vel, double ha, double hb, double g, double rd) {
+    atomicMax(at, (unsigned long long)__double_as_longlong(face_speed(vel, sw2d_half(ha + hb), g, rd)));
 }
 
 /* mean depth of a face >= th, exactly: decided from the two depths unless
@@ -325,7 +321,7 @@ __device__ __forceinline__ bool mean_ge(double ha, double hb, float est, double 
     const bool a = sw2d_ge_pos(ha, th), b = sw2d_ge_pos(hb, th);
     if (a == b) return a;
     if (fabsf(est - thf) > 1e-5f * thf) return est > thf;
-    return sw2d_ge_pos(sw2d_half(add_here(ha, hb)), th);
+    return mean_ge_exact(ha, hb, th);
 }
 
 /* The new discharges of the faces of a 32 x BY block of cells (north and
@@ -347,16 +343,16 @@ __device__ __forceinline__ bool mean_ge(double ha, double hb, float est, double 
  * not reach the running maximum is done, else its lanes within 1e-5 of the
  * best are evaluated in binary64 and raise the maximum: the result is the
  * exact maximum in any order. */
-template <int BY>
-__global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 5 : 16) k64_flux(StepParams p, int cur) {
-    constexpr int BX = SW2D_BX, NT = BX * BY, SW = BX + 2, NV = (BY + 2) * SW, NH = (BY + 1) * SW;
+template <int BY, int NT, int PER_SM>
+__global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
+    constexpr int BX = SW2D_BX, NF = 2 * BX * BY, SW = BX + 2, NV = (BY + 2) * SW, NH = (BY + 1) * SW;
     static_assert(BX == 32, "one row per warp: its ballot is the row's bit mask");
     __shared__ double sh[NH], sz[NH], se[NH];         /* depth, bed, surface: rows -1 .. BY-1 */
     constexpr int U = 0, V = NV, QX = 2 * NV, QY = 3 * NV;
     __shared__ double sf[4 * NV];                     /* face velocities and discharges: rows -1 .. BY */
     __shared__ double sedge[4 * NH];
     __shared__ uint8_t sact[NH];
-    __shared__ unsigned short flist[2 * NT], elist[4 * NT + 2 * BX + 2 * BY];
+    __shared__ unsigned short flist[NF], elist[2 * NF + 2 * BX + 2 * BY];
     __shared__ unsigned rowx[BY + 1], rowy[BY + 1];
     __shared__ int cnt[3];
     const int tx = threadIdx.x, ty = threadIdx.y, t = ty * BX + tx;
@@ -399,7 +395,7 @@ __global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 5 : 16) k64_flux(StepP
     __syncthreads();
     const int s0 = (ty + 1) * SW + tx + 1;
     const bool doX = r <= R && c < C, doY = r < R && c <= C;
-    {
+    if (ty < BY) {
         const double hc = sh[s0], ec = se[s0], zc = sz[s0];
         const int an = sact[s0 - SW], aw = sact[s0 - 1], ac = sact[s0];
         int kx = 0, ky = 0;
@@ -424,7 +420,7 @@ __global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 5 : 16) k64_flux(StepP
             base = atomicAdd(&cnt[1], __popc(px) + __popc(py));
         }
         int mb = __shfl_sync(all, base, 0) + __popc(mx & lt);
-        int pb = 2 * NT - 1 - (__shfl_sync(all, base, 1) + __popc(px & lt));
+        int pb = NF - 1 - (__shfl_sync(all, base, 1) + __popc(px & lt));
         if (kx == 1) flist[mb] = (unsigned short)(2 * t);
         if (kx > 1) flist[pb] = (unsigned short)(2 * t);
         mb = mb - __popc(mx & lt) + __popc(mx) + __popc(my & lt);
@@ -445,12 +441,12 @@ __global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 5 : 16) k64_flux(StepP
             const float cy = sw2d_f32_est_of_f64(__longlong_as_double((long long)__ldcg(best + 1)));
             const float wx = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ex))), cx) * 0.99999f;
             const float wy = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ey))), cy) * 0.99999f;
-            if (okx && ex >= wx) raise_max(best, face_speed(sf[U + s0], sw2d_half(add_here(hc, sh[s0 - SW])), p.g, p.rdx));
-            if (oky && ey >= wy) raise_max(best + 1, face_speed(sf[V + s0], sw2d_half(add_here(hc, sh[s0 - 1])), p.g, p.rdy));
+            if (okx && ex >= wx) raise_speed(best, sf[U + s0], hc, sh[s0 - SW], p.g, p.rdx);
+            if (oky && ey >= wy) raise_speed(best + 1, sf[V + s0], hc, sh[s0 - 1], p.g, p.rdy);
         }
     }
     __syncthreads();
-    {
+    if (ty < BY) {
         /* edges of the row: south of its cells for x and y faces (types 0,
          * 2), east of them and west of the first (1, 3); warp 0 also the
          * edges north of the block */
@@ -474,7 +470,7 @@ __global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 5 : 16) k64_flux(StepP
         if (tx == 0 && w3) elist[base + n6] = (unsigned short)((s0 - 1) << 2 | 3);
     }
     for (int k = t; k < cnt[1]; k += NT) {
-        const int id = flist[2 * NT - 1 - k], ft = id >> 1, ly = ft / BX, lx = ft % BX;
+        const int id = flist[NF - 1 - k], ft = id >> 1, ly = ft / BX, lx = ft % BX;
         const int sj = (ly + 1) * SW + lx + 1, sa = (id & 1) ? sj - 1 : sj - SW;
         const bool edge = !(id & 1) && r0 + ly == R; /* the open south edge: a weir from the last row */
         const double F = face_special(edge, sh[sa], sh[sj], se[sa], se[sj], sz[sa], sz[sj], th, p.g);
@@ -510,6 +506,7 @@ __global__ void __launch_bounds__(SW2D_BX * BY, BY == 8 ? 5 : 16) k64_flux(StepP
 /* ------------------------------------------------------------------------ */
 /* continuity: SW2D-EFDC.cu:602-664                                          */
 
+template <bool FULL>
 __device__ __forceinline__ double continuity(const StepParams& p, size_t i, uint8_t f, double ho,
                                              double divx, double divy, double dt2, double rr,
                                              double ev, const double* ql, double* raw,
@@ -526,14 +523,14 @@ __device__ __forceinline__ double continuity(const StepParams& p, size_t i, uint
     /* (((dqx/dx + dqy/dy) - q_src) - r pct) + e; subtracting a zero source
      * and adding a zero evaporation change no value, so they are skipped */
     double sum = div_spacing(divx, p.ddx, p.kdx) + div_spacing(divy, p.ddy, p.kdy);
-    if (f & SW2D_F_SOURCE) {
+    if (FULL && (f & SW2D_F_SOURCE)) {
         double qli = 0.0;
         for (int k = 0; k < p.nsrc; k++)
             if (p.src_idx[k] == (int)i) qli = ql[k];
-        sum = add_here(sum, -qli);
+        sum = sum - qli;
     }
     sum = sum - rcell * pct;
-    if (p.evap) sum = add_here(sum, evapo);
+    if (FULL && p.evap) sum = sum + evapo;
     double hn = ho - dt2 * sum;
     *raw = hn;
     *rain_term = rcell * pct;
@@ -586,11 +583,14 @@ __device__ unsigned long long block_max_u64(unsigned long long v, unsigned long 
 
 #define NPART 4 /* prime: volume, CFL bits x, y; update: weighted rain, lake cells, land cells, outlet */
 
-/* Adds the ledger sums of the iteration whose slot is `par` (its tiles'
- * partials were written by the previous k64_update) and its outlet record;
- * by one whole block.  last_row: the tile row that holds the raster's last row. */
+/* Adds the ledger sums of the last iteration of parity `par`, if they are
+ * not added yet (its tiles' partials were written by its k64_update), and its
+ * outlet record; by one whole block.  last_row: the tile row that holds the
+ * raster's last row. */
 __device__ void settle_ledger(const StepParams& p, int par, int gx, int gy, int last_row) {
     __shared__ double smd[NWARP];
+    Flight64::Sums& in = p.flight->sums[par];
+    if (!__ldcg(&in.pending)) return;
     const int nt = blockDim.x, tid = threadIdx.x, tiles = gx * gy;
     const double* part = p.partials + (size_t)par * tiles * NPART;
     double vr = 0.0, ve = 0.0, vd = 0.0, vq = 0.0;
@@ -611,12 +611,9 @@ __device__ void settle_ledger(const StepParams& p, int par, int gx, int gy, int 
     }
     if (tid == 0) {
         DevClock* clk = p.clk;
-        const Slot& s = clk->slot[par];
-        const double dt2 = s.dt2, area = p.area, rr2 = s.rr2, ev2 = s.ev2, tn = s.t_next;
+        const double dt2 = in.dt2, area = p.area, rr2 = in.rr2, ev2 = in.ev2, tn = in.t_next, src = in.src;
         const double l0 = clk->led[LED_RAIN], l1 = clk->led[LED_EVAP], l2 = clk->led[LED_SOURCE], l3 = clk->led[LED_OUTFLOW];
-        double src = 0.0;
-        for (int k = 0; k < p.nsrc; k++) /* a source overridden on its cell adds nothing */
-            if (p.src_idx[k] >= 0) src += s.ql2[k];
+        in.pending = 0;
         const double rain = !p.ledger_cells ? rr2 * p.rain_static
                             : p.rainw       ? vr
                                             : ve * (rr2 * p.pct_lake) + vd * (rr2 * p.pct_land);
@@ -626,7 +623,7 @@ __device__ void settle_ledger(const StepParams& p, int par, int gx, int gy, int 
         clk->led[LED_SOURCE] = l2 + dt2 * src * area;
         clk->led[LED_QOUT] = qo;
         clk->led[LED_OUTFLOW] = l3 + dt2 * qo;
-        if (!isfinite(vq)) clk->status |= 1;
+        if (!isfinite(vq)) atomicOr(&clk->status, 1);
         if (p.outlet) {
             const long long n = clk->outlet_n, k = n % p.outlet_cap;
             p.outlet[2 * k] = tn;
@@ -636,42 +633,47 @@ __device__ void settle_ledger(const StepParams& p, int par, int gx, int gy, int 
     }
 }
 
-/* The clock of the iteration in slot `cur`, by the extra block of its
- * k64_update, beside the tiles: the previous iteration's ledger sums, then
- * the CFL speed k64_flux found and the next iteration's length and forcing. */
-__device__ void advance_clock(const StepParams& p, int cur, int gx, int gy, int last_row) {
+/* The clock of the iteration in slot `cur`, by one warp of an extra block of
+ * its k64_update, beside the tiles: the CFL speed k64_flux found and the next
+ * iteration's length and forcing. */
+__device__ void advance_clock(const StepParams& p, int cur) {
+    if (threadIdx.x >= 32) return;
     DevClock* clk = p.clk;
     Flight64* fl = p.flight;
-    const int pending = __ldcg(&fl->pending);
-    if (pending) settle_ledger(p, pending - 1, gx, gy, last_row);
-    __syncthreads(); /* slot cur^1 is read above and overwritten below */
-    if (threadIdx.x >= 32) return;
     const Slot& s = clk->slot[cur];
     if (!s.active) {
         const unsigned long long* from = reinterpret_cast<const unsigned long long*>(&s);
         unsigned long long* to = reinterpret_cast<unsigned long long*>(&clk->slot[cur ^ 1]);
         for (int k = threadIdx.x; k < (int)(sizeof(Slot) / 8); k += 32) to[k] = from[k];
-        if (threadIdx.x == 0) fl->pending = 0;
         return;
     }
     /* of the state this iteration started from */
     const double smax = __longlong_as_double((long long)__ldcg(&fl->smax[cur][0])) +
                         __longlong_as_double((long long)__ldcg(&fl->smax[cur][1]));
-    const double t = s.t_next, t_end = clk->t_end;
+    const double t = s.t_next, t_end = clk->t_end, dt2 = s.dt2, rr2 = s.rr2, ev2 = s.ev2;
     const long long iters = clk->iters + 1, lim = clk->iter_end;
     __syncwarp();
+    /* past the iteration limit the next slot is inactive: t_end = t */
+    prepare_slot(p, &clk->slot[cur ^ 1], t, smax, iters < lim ? t_end : t);
     if (threadIdx.x == 0) {
         fl->smax[cur][0] = fl->smax[cur][1] = 0ull;
-        fl->pending = cur + 1;
-        clk->led[LED_DTLAST] = s.dt2;
+        Flight64::Sums& o = fl->sums[cur];
+        o.dt2 = dt2;
+        o.rr2 = rr2;
+        o.ev2 = ev2;
+        o.t_next = t;
+        double src = 0.0;
+        for (int k = 0; k < p.nsrc; k++) /* a source overridden on its cell adds nothing */
+            if (p.src_idx[k] >= 0) src += s.ql2[k];
+        o.src = src;
+        o.pending = 1;
+        clk->led[LED_DTLAST] = dt2;
         clk->led[LED_SMAX] = smax;
-        if (!isfinite(smax)) clk->status |= 1;
+        if (!isfinite(smax)) atomicOr(&clk->status, 1);
         clk->t = t;
         clk->s_max = smax;
         clk->iters = iters;
     }
-    /* past the iteration limit the next slot is inactive: t_end = t */
-    prepare_slot(p, &clk->slot[cur ^ 1], t, smax, iters < lim ? t_end : t);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -682,14 +684,16 @@ __device__ void advance_clock(const StepParams& p, int cur, int gx, int gy, int 
  * estimate of the depth, by the exact binary64 continuity only where th lies
  * within the estimate's error (2^-19 of the magnitudes that enter it; the
  * estimate's own rounding stays below 2^-20 of them). */
+template <bool FULL>
 __device__ __noinline__ bool provisional_exact(const StepParams& p, const Slot& s, size_t i, uint8_t f, double ho,
                                                double fN, double fS, double fW, double fE) {
     double raw, rt;
-    return sw2d_lt_pos(continuity(p, i, f, ho, fS - fN, fE - fW, s.dt2, s.rr1, s.ev1, s.ql1, &raw, &rt), p.th);
+    return sw2d_lt_pos(continuity<FULL>(p, i, f, ho, fS - fN, fE - fW, s.dt2, s.rr1, s.ev1, s.ql1, &raw, &rt), p.th);
 }
 struct DryEst {
     float th, ewl, dt2, rdx, rdy, pl, pd, ev;
 };
+template <bool FULL>
 __device__ __forceinline__ bool provisional_dry(const StepParams& p, const Slot& s, const DryEst& q, size_t i,
                                                 uint8_t f, double ho, double fN, double fS, double fW, double fE) {
     const float h = sw2d_f32_est_of_f64(ho), n = sw2d_f32_est_of_f64(fN), so = sw2d_f32_est_of_f64(fS),
@@ -697,38 +701,41 @@ __device__ __forceinline__ bool provisional_dry(const StepParams& p, const Slot&
     const bool lake = sw2d_gt(ho, p.ev_wl_min);
     float rain = lake ? q.pl : q.pd;
     if (p.rainw) rain *= p.rainw[i];
-    const float ev = lake ? q.ev : 0.f;
+    const float ev = FULL && lake ? q.ev : 0.f;
     const float hs = h - q.dt2 * (((so - n) * q.rdx + (e - w) * q.rdy - rain) + ev);
     const float mag = fabsf(h) + q.dt2 * ((fabsf(so) + fabsf(n)) * q.rdx + (fabsf(e) + fabsf(w)) * q.rdy + fabsf(rain) +
                                           fabsf(ev));
     const float d = hs - q.th;
-    if (!(f & SW2D_F_SOURCE) && fabsf(d) > 1.9073486e-6f * (mag + q.th) + 1e-35f) return d < 0.f;
-    return provisional_exact(p, s, i, f, ho, fN, fS, fW, fE);
+    if (!(FULL && (f & SW2D_F_SOURCE)) && fabsf(d) > 1.9073486e-6f * (mag + q.th) + 1e-35f) return d < 0.f;
+    return provisional_exact<FULL>(p, s, i, f, ho, fN, fS, fW, fE);
 }
 
-/* Tile of the update kernel: TW x TH cells (and their north and west faces)
+/* FULL: evaporation, point sources or rain whose ledger is kept per cell.
+ * Tile of the update kernel: TW x TH cells (and their north and west faces)
  * per block.  The dry flags are evaluated on the tile plus two rows north
  * and west and one row south and east, the new depths on the tile plus the
  * row north and the column west: the faces of the tile read both; the halo
- * is recomputed, not exchanged.  Block 0 keeps the clock meanwhile (what it
- * does is a chain of dependent reads and divisions; at the end of the last
- * tile it would be the longest part of a small raster's iteration).
+ * is recomputed, not exchanged.  Block 0 prepares the next iteration
+ * meanwhile and block 1 adds up the previous one's ledger sums (chains of
+ * dependent reads, divisions and sums; at the end of the last tile they would
+ * be the longest part of a small raster's iteration).
  * Bounded by the binary64 additions and products of the final depth and of
  * the face means (71 issue cycles a warp each; the flags take none) and by
  * the latencies between them: six blocks an SM (40 registers, 40 bytes of
  * spills) against four measured 613 against 730 us at 4096 x 4096. */
-template <int TW, int TH, int NT>
+template <int TW, int TH, int NT, bool FULL>
 __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int gx, int gy) {
     constexpr int DW = TW + 3, DH = TH + 3, NW = TW + 1, NH = TH + 1;
-    if (blockIdx.x == 0) {
-        advance_clock(p, cur, gx, gy, (p.R - 1) / TH);
+    if (blockIdx.x < 2) {
+        if (blockIdx.x == 0) advance_clock(p, cur);
+        else settle_ledger(p, cur ^ 1, gx, gy, (p.R - 1) / TH);
         return;
     }
     __shared__ uint8_t sdry[DH][DW];   /* rows r0-2 .. r0+TH, cols c0-2 .. c0+TW */
     __shared__ double shn[NH][NW];     /* rows r0-1 .. r0+TH-1, cols c0-1 .. c0+TW-1 */
     __shared__ double smd[NWARP];
     const int tid = threadIdx.x;
-    const int tile = blockIdx.x - 1, tyi = tile / gx;
+    const int tile = blockIdx.x - 2, tyi = tile / gx;
     const int c0 = (tile - tyi * gx) * TW, r0 = tyi * TH;
     const int nxt = cur ^ 1;
     const Slot& s = p.clk->slot[cur];
@@ -767,7 +774,7 @@ __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int g
             if (r >= 0 && r < R && c >= 0 && c < C) {
                 const size_t i = (size_t)(r + H) * P + (c + H);
                 const uint8_t f = p.flags[i];
-                if (f & SW2D_F_ACTIVE) dflag = provisional_dry(p, s, q, i, f, hc[i], fx[i], fx[i + P], fy[i], fy[i + 1]);
+                if (f & SW2D_F_ACTIVE) dflag = provisional_dry<FULL>(p, s, q, i, f, hc[i], fx[i], fx[i + P], fy[i], fy[i + 1]);
             }
             sdry[rr][cc] = dflag;
         }
@@ -777,7 +784,7 @@ __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int g
      * provisional depth fell below th is closed, :704-719), final depth
      * at t+dt; written for the tile's own cells, kept in shared memory
      * for the faces */
-    double vr = 0.0, vq = 0.0;
+    double vr = 0.0;
     int nlake = 0, nland = 0;
     for (int k = tid; k < NH * NW; k += NT) {
         const int rr = k / NW, cc = k - rr * NW;
@@ -795,17 +802,16 @@ __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int g
             if ((sw2d_gt0(fE) && dC) || (sw2d_lt0(fE) && sdry[dr][dc + 1])) fE = 0;
             const double ho = hc[i];
             double raw, rt;
-            hn = continuity(p, i, f, ho, fS - fN, fE - fW, dt2, rr2, ev2, s.ql2, &raw, &rt);
+            hn = continuity<FULL>(p, i, f, ho, fS - fN, fE - fW, dt2, rr2, ev2, s.ql2, &raw, &rt);
             if (rr >= 1 && cc >= 1) { /* the tile's own cell */
                 p.h[nxt][i] = hn;
                 if (f & SW2D_F_ACTIVE) {
                     if (sw2d_lt0(raw)) atomicAdd(&p.clk->led[LED_CLAMP], -raw * p.area); /* max(h, 0) gain */
-                    if (p.ledger_cells) {
-                        if (p.rainw) vr = add_here(vr, rt);
+                    if (FULL && p.ledger_cells) {
+                        if (p.rainw) vr += rt;
                         if (sw2d_gt(ho, p.ev_wl_min)) nlake++;
                         else nland++;
                     }
-                    if (r == R - 1 && p.outflow_south) vq = add_here(vq, fS);
                 }
             }
         }
@@ -843,9 +849,9 @@ __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int g
             p.vv1[i] = sw2d_ge_pos(hn, th) ? sw2d_div_rn(F, hn) : 0.0;
         }
     }
-    /* ledger sums of the tile, added up by the next iteration's block 0 */
+    /* ledger sums of the tile, added up beside the next iteration's tiles */
     double* pb = p.partials + ((size_t)cur * gx * gy + tile) * NPART;
-    if (p.ledger_cells) {
+    if (FULL && p.ledger_cells) {
         if (p.rainw) vr = block_sum(vr, smd);
         /* counts as binary32-exact integers: at most TW * TH */
         nlake = __reduce_add_sync(0xffffffffu, nlake);
@@ -865,6 +871,15 @@ __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int g
         }
     }
     if (p.outflow_south && r0 <= R - 1 && R - 1 < r0 + TH) {
+        double vq = 0.0;
+        for (int cc = tid; cc < TW; cc += NT) { /* the open faces south of the last row */
+            const int c = c0 + cc, dr = R - 1 - r0 + 2, dc = cc + 2;
+            if (c >= C) continue;
+            const size_t i = (size_t)(R - 1 + H) * P + (c + H);
+            const double F = fx[i + P];
+            const bool shut = (sw2d_gt0(F) && sdry[dr][dc]) || (sw2d_lt0(F) && sdry[dr + 1][dc]);
+            if ((p.flags[i] & SW2D_F_ACTIVE) && !shut) vq += F;
+        }
         vq = block_sum(vq, smd);
         if (tid == 0) pb[3] = vq;
     }
@@ -872,10 +887,8 @@ __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int g
 
 __global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_settle(StepParams p, int gx, int gy,
                                                                      int last_row) {
-    const int pending = __ldcg(&p.flight->pending);
-    if (!pending) return;
-    settle_ledger(p, pending - 1, gx, gy, last_row);
-    if (threadIdx.x == 0) p.flight->pending = 0;
+    settle_ledger(p, 0, gx, gy, last_row); /* the last iteration is of one parity; the other has nothing to add */
+    settle_ledger(p, 1, gx, gy, last_row);
 }
 
 /* Volume (sum of h over active cells) and, with full, the CFL speed of the
@@ -1067,7 +1080,16 @@ static dim3 grid_cells(const StepParams& p) {
 
 int fp64_kernels_per_iteration() { return 2; }
 
-/* How a raster is cut into the update kernel's tiles and the flux kernel's blocks. */
+/* How a raster is cut into the update kernel's tiles and the flux kernel's
+ * blocks: large ones for the smaller share of halo while there are many,
+ * small ones so that a small raster reaches every SM (each block's chain of
+ * dependent binary64 operations then holds fewer of them).  Measured, us an
+ * iteration: update tiles 64 x 16 / 32 x 16 1809 / 1848 at 4096^2, 258.0 /
+ * 258.3 at 1531 x 1207, 151 / 145 at 1024^2; 32 x 16 / 32 x 8 62.9 / 63.9 at
+ * 701 x 556, 41.3 / 38.9 at 400^2; 32 x 8 / 32 x 4 24.1 / 24.1 at 256^2, 17.4
+ * / 15.5 at 33 x 41.  Flux blocks of 8 / 4 rows (256 threads each): 63.9 /
+ * 68.1 at 701 x 556, 38.9 / 37.4 at 400^2, 24.1 / 21.8 at 256^2, 17.4 / 15.7
+ * at 33 x 41. */
 struct Cut64 {
     int kind, tw, th, gx, gy;
     dim3 flux;
@@ -1076,12 +1098,12 @@ struct Cut64 {
 static Cut64 cut_of(int R, int C) {
     Cut64 k;
     const long long cells = (long long)(R + 1) * (C + 1);
-    k.kind = cells >= 64LL * 16 * 152 * 4 ? 0 : cells >= 32LL * 8 * 152 ? 1 : 2;
+    k.kind = cells >= 1800000 ? 0 : cells >= 300000 ? 1 : cells >= 40000 ? 2 : 3;
     k.tw = k.kind == 0 ? 64 : 32;
-    k.th = k.kind == 0 ? 16 : k.kind == 1 ? 8 : 4;
+    k.th = k.kind <= 1 ? 16 : k.kind == 2 ? 8 : 4;
     k.gx = (C + 1 + k.tw - 1) / k.tw;
     k.gy = (R + 1 + k.th - 1) / k.th;
-    k.by = cells >= 32LL * 8 * 152 * 2 ? 8 : 2;
+    k.by = cells >= 320000 ? 8 : 4;
     k.flux = dim3((C + 1 + SW2D_BX - 1) / SW2D_BX, (R + 1 + k.by - 1) / k.by);
     return k;
 }
@@ -1092,16 +1114,26 @@ size_t fp64_partials(int rows, int cols) {
     return NPART * std::max(prime, (size_t)2 * k.gx * k.gy);
 }
 
+template <bool FULL>
+static void launch_update(const Cut64& k, int n, const StepParams& p, int cur, cudaStream_t s) {
+    if (k.kind == 0) k64_update<64, 16, 256, FULL><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
+    else if (k.kind == 1) k64_update<32, 16, 256, FULL><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
+    else if (k.kind == 2) k64_update<32, 8, 256, FULL><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
+    else k64_update<32, 4, 256, FULL><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
+}
+
 void fp64_launch_iteration(const StepParams& p, int cur, cudaStream_t s, cudaEvent_t* ev) {
     const Cut64 k = cut_of(p.R, p.C);
     if (ev) cudaEventRecord(ev[0], s);
-    if (k.by == 8) k64_flux<8><<<k.flux, dim3(SW2D_BX, 8), 0, s>>>(p, cur);
-    else k64_flux<2><<<k.flux, dim3(SW2D_BX, 2), 0, s>>>(p, cur);
+    const dim3 blk(SW2D_BX, 8);
+    if (k.by == 4) k64_flux<4, 256, 5><<<k.flux, blk, 0, s>>>(p, cur);
+    else if (k.kind > 0) k64_flux<8, 256, 5><<<k.flux, blk, 0, s>>>(p, cur);
+    else k64_flux<8, 256, 6><<<k.flux, blk, 0, s>>>(p, cur);
     if (ev) cudaEventRecord(ev[1], s);
-    const int n = k.gx * k.gy + 1;
-    if (k.kind == 0) k64_update<64, 16, 256><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
-    else if (k.kind == 1) k64_update<32, 8, 256><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
-    else k64_update<32, 4, 128><<<n, 128, 0, s>>>(p, cur, k.gx, k.gy);
+    const int n = k.gx * k.gy + 2;
+    const bool full = p.evap || p.nsrc > 0 || p.ledger_cells;
+    if (full) launch_update<true>(k, n, p, cur, s);
+    else launch_update<false>(k, n, p, cur, s);
     if (ev) cudaEventRecord(ev[2], s);
 }
 

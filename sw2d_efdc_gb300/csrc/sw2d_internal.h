@@ -67,12 +67,15 @@ struct DevClock {
     long long iter_end;   /* the slot after iteration iter_end is inactive (a state copy) */
 };
 
-/* Running state between the kernels of consecutive iterations (not part of a
- * snapshot: all zero whenever no iteration is in flight). */
+/* Running state between the kernels of consecutive iterations, by the
+ * iteration's parity (not part of a snapshot: no iteration is in flight when
+ * one is taken). */
 struct Flight64 {
-    unsigned long long smax[2][2]; /* per iteration parity: CFL face-speed maxima (bit patterns), x and y faces */
-    int pending;                   /* 1 + parity of the iteration whose ledger sums are not added yet, 0 none */
-    int pad;
+    unsigned long long smax[2][2]; /* CFL face-speed maxima (bit patterns), x and y faces; 0 before the iteration */
+    struct Sums {
+        double dt2, rr2, ev2, t_next, src;
+        long long pending; /* the iteration's ledger sums are not added yet */
+    } sums[2];
 };
 
 /* Everything a step kernel needs, passed by value. */

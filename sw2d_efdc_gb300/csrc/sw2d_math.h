@@ -73,9 +73,15 @@ SW2D_HD float sw2d_f32_from_bits(uint32_t u) {
 #endif
 }
 
+/* On the device the bits pass through an instruction the optimiser does not
+ * look into: it otherwise recognises integer comparisons and zero tests of
+ * them as binary64 ones (and "zero ? 0 : x" as x + 0) and puts them back on
+ * the FP64 pipe. */
 SW2D_HD uint64_t sw2d_f64_bits(double d) {
 #if defined(__CUDA_ARCH__)
-    return (uint64_t)__double_as_longlong(d);
+    uint64_t u;
+    asm("mov.b64 %0, %1;" : "=l"(u) : "d"(d));
+    return u;
 #else
     uint64_t u;
     memcpy(&u, &d, sizeof u);
@@ -465,8 +471,8 @@ SW2D_HD double sw2d_div_rn(double a, double b) {
 
 /* ------------------------------------------------------------------------
  * sqrt(x) correctly rounded with integer and binary32 operations only (the
- * companion of sw2d_div_rn), for x positive and normal (every other x
- * returns the hardware sqrt).  With x = m 2^E, E even, m in [2^52, 2^54),
+ * companion of sw2d_div_rn), for x positive and normal (a zero returns
+ * itself, every other x the hardware sqrt).  With x = m 2^E, E even, m in [2^52, 2^54),
  * S = floor(sqrt(m 2^54)) (54 bits) is built from its leading 24 bits, a
  * binary32 square root, and two signed digits of 15 bits, each the exact
  * remainder over twice the root so far, estimated with a binary32
@@ -495,7 +501,10 @@ SW2D_HD float sw2d_sqrt_est(float x) {
 SW2D_HD double sw2d_sqrt_rn(double x) {
     const uint64_t ux = sw2d_f64_bits(x);
     const uint32_t ex = (uint32_t)(ux >> 52);
-    if (ex - 1u >= 0x7feu) return sqrt(x); /* negative, zero, subnormal, inf, NaN */
+    if (ex - 1u >= 0x7feu) {
+        if ((ux << 1) == 0) return x;
+        return sqrt(x); /* negative, subnormal, inf, NaN */
+    }
     const uint64_t H = 1ull << 52;
     const uint32_t odd = (ex + 1u) & 1u; /* E = ex - 1075 odd */
     const uint64_t m = ((ux & (H - 1ull)) | H) << odd;
