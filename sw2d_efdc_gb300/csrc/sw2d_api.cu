@@ -164,6 +164,12 @@ struct sw2d_handle {
         };
         p.kdx = pow2_exp(cfg.dx);
         p.kdy = pow2_exp(cfg.dy);
+        p.thf = (float)cfg.th;
+        p.gf = (float)cfg.g;
+        p.rdxf = (float)p.rdx;
+        p.rdyf = (float)p.rdy;
+        p.plf = (float)p.pct_lake;
+        p.pdf = (float)p.pct_land;
         p.ddx = sw2d_divisor_of(cfg.dx);
         p.ddy = sw2d_divisor_of(cfg.dy);
         p.rainw = rainw;

@@ -184,33 +184,29 @@ __device__ __forceinline__ double edge_term(double w1, double w0, double q0, dou
  *   0 closed (an inactive side, or both sides at or below th)
  *   1 momentum (gravity, convection, friction)
  *   2 weir from side a, 3 weir from side b (a side's surface below the
- *     other side's bed), 4 dry-bed front (exactly one side above th).
- * Side a is the north (x faces) / west (y faces) cell, e = h + z its surface.
- * The product (hb - th) (ha - th) < 0 of the reference is decided from the
- * two comparisons with th (the differences keep the comparisons' signs and
- * their product of depths cannot underflow).  A weir from a side at or below
- * th carries nothing: closed. */
-__device__ __forceinline__ int classify(bool act, double ha, double hb, double ea, double eb, double za, double zb,
-                                        double th) {
-    const bool wa = sw2d_gt_pos(ha, th), wb = sw2d_gt_pos(hb, th);
-    if (!act || !(wa || wb)) return 0;
-    if (sw2d_lt(eb, za)) return wa ? 2 : 0;
-    if (sw2d_lt(ea, zb)) return wb ? 3 : 0;
-    return ((wb && sw2d_lt_pos(ha, th)) || (wa && sw2d_lt_pos(hb, th))) ? 4 : 1;
+ *     other side's bed), 4 / 5 dry-bed front with side b / a alone above th.
+ * Side a is the north (x faces) / west (y faces) cell; ea, za its surface
+ * h + z and its bed as ordered integers (sw2d_ord), ca its code.  The product
+ * (hb - th) (ha - th) < 0 of the reference is decided from the two
+ * comparisons with th (the differences keep the comparisons' signs and
+ * their product of depths cannot underflow), and so is the front's sign.  A
+ * weir from a side at or below th carries nothing: closed. */
+constexpr int kActive = 1, kWet = 2, kBelow = 4; /* cell codes: active, h > th, h < th */
+__device__ __forceinline__ int classify(int ca, int cb, int64_t ea, int64_t eb, int64_t za, int64_t zb) {
+    if (!(ca & cb & kActive) || !((ca | cb) & kWet)) return 0;
+    if (eb < za) return (ca & kWet) ? 2 : 0;
+    if (ea < zb) return (cb & kWet) ? 3 : 0;
+    return ((cb & kWet) && (ca & kBelow)) ? 4 : ((ca & kWet) && (cb & kBelow)) ? 5 : 1;
 }
-
-__device__ __forceinline__ double max_ord(double a, double b) { return sw2d_gt(a, b) ? a : b; }
 
 /* Discharge of a weir or dry-bed face, (c d) sqrt(G d): d the depth on the
  * weir's side, or the higher surface above the higher bed (:125-157). */
-__device__ __forceinline__ double face_special(bool from_a, double ha, double hb, double ea, double eb, double za,
-                                               double zb, double th, double gg) {
-    const bool k2 = from_a || sw2d_lt(eb, za), k3 = !k2 && sw2d_lt(ea, zb);
-    const bool wb = sw2d_gt_pos(hb, th);
-    double d = k2 ? ha : hb;
-    if (!(k2 || k3)) d = max_ord(eb, ea) - max_ord(zb, za);
-    const double c = k2 ? 0.5440 : k3 ? -0.544 : wb ? -0.350 : 0.350; /* -sign((hb - th) - (ha - th)) 0.350 */
-    return c * d * sw2d_sqrt_rn(((k2 || k3) ? gg : 2.00 * gg) * d);
+__device__ __forceinline__ double face_special(int kind, double ha, double hb, int64_t ea, int64_t eb, int64_t za,
+                                               int64_t zb, double gg) {
+    double d = kind == 2 ? ha : hb;
+    if (kind > 3) d = sw2d_f64_of_ord(eb > ea ? eb : ea) - sw2d_f64_of_ord(zb > za ? zb : za);
+    const double c = kind == 2 ? 0.5440 : kind == 3 ? -0.544 : kind == 4 ? -0.350 : 0.350;
+    return c * d * sw2d_sqrt_rn((kind <= 3 ? gg : 2.00 * gg) * d);
 }
 
 /* momentum update of a face (SW2D-EFDC.cu:165-202 x, :282-319 y): along /
@@ -312,14 +308,15 @@ __device__ __noinline__ bool mean_ge_exact(double ha, double hb, double th) {
 }
 /* raises a running maximum (bits of non-negative doubles) to a face's speed */
 __device__ __noinline__ void raise_speed(unsigned long long* at, double vel, double ha, double hb, double g, double rd) {
-    atomicMax(at, (unsigned long long)__double_as_longlong(face_speed(vel, sw2d_half(ha + hb), g, rd)));
+    const unsigned long long v = sw2d_f64_bits(face_speed(vel, sw2d_half(ha + hb), g, rd));
+    if (v <= 0x7ff0000000000000ull && v > __ldcg(at)) atomicMax(at, v);
 }
 
-/* mean depth of a face >= th, exactly: decided from the two depths unless
- * th lies between them, then in binary32, in binary64 only within its error */
-__device__ __forceinline__ bool mean_ge(double ha, double hb, float est, double th, float thf) {
-    const bool a = sw2d_ge_pos(ha, th), b = sw2d_ge_pos(hb, th);
-    if (a == b) return a;
+/* mean depth of a face >= th, exactly: decided from the two cells' codes
+ * unless th lies between their depths, then in binary32, in binary64 only
+ * within its error */
+__device__ __forceinline__ bool mean_ge(double ha, double hb, int ca, int cb, float est, double th, float thf) {
+    if (!((ca ^ cb) & kBelow)) return !(ca & kBelow);
     if (fabsf(est - thf) > 1e-5f * thf) return est > thf;
     return mean_ge_exact(ha, hb, th);
 }
@@ -347,11 +344,13 @@ template <int BY, int NT, int PER_SM>
 __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
     constexpr int BX = SW2D_BX, NF = 2 * BX * BY, SW = BX + 2, NV = (BY + 2) * SW, NH = (BY + 1) * SW;
     static_assert(BX == 32, "one row per warp: its ballot is the row's bit mask");
-    __shared__ double sh[NH], sz[NH], se[NH];         /* depth, bed, surface: rows -1 .. BY-1 */
+    __shared__ double sh[NH];                         /* depth: rows -1 .. BY-1 */
+    __shared__ int64_t so[2 * NH];                    /* surface h + z, then bed, as ordered integers */
+    __shared__ float shf[NH];                         /* depth estimate */
     constexpr int U = 0, V = NV, QX = 2 * NV, QY = 3 * NV;
     __shared__ double sf[4 * NV];                     /* face velocities and discharges: rows -1 .. BY */
     __shared__ double sedge[4 * NH];
-    __shared__ uint8_t sact[NH];
+    __shared__ uint8_t scode[NH];
     __shared__ unsigned short flist[NF], elist[2 * NF + 2 * BX + 2 * BY];
     __shared__ unsigned rowx[BY + 1], rowy[BY + 1];
     __shared__ int cnt[3];
@@ -386,9 +385,11 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
             if (k < NH) {
                 const double hh = in ? h[g] : 0.0, zz = in ? z[g] : 0.0;
                 sh[k] = hh;
-                sz[k] = zz;
-                se[k] = hh + zz;
-                sact[k] = in ? (flags[g] & SW2D_F_ACTIVE) : 0;
+                so[k] = sw2d_ord(hh + zz);
+                so[NH + k] = sw2d_ord(zz);
+                shf[k] = sw2d_f32_est_hi(hh);
+                scode[k] = (uint8_t)((in ? (flags[g] & SW2D_F_ACTIVE) : 0) | (sw2d_gt_pos(hh, th) ? kWet : 0) |
+                                     (sw2d_lt_pos(hh, th) ? kBelow : 0));
             }
         }
     }
@@ -396,16 +397,16 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
     const int s0 = (ty + 1) * SW + tx + 1;
     const bool doX = r <= R && c < C, doY = r < R && c <= C;
     if (ty < BY) {
-        const double hc = sh[s0], ec = se[s0], zc = sz[s0];
-        const int an = sact[s0 - SW], aw = sact[s0 - 1], ac = sact[s0];
+        const int cc = scode[s0], cn = scode[s0 - SW], cw = scode[s0 - 1];
+        const int64_t ec = so[s0], zc = so[NH + s0];
         int kx = 0, ky = 0;
         if (doX) {
             if (r == R && p.outflow_south) /* south edge: free overfall when open */
-                kx = (an && sw2d_gt_pos(sh[s0 - SW], th)) ? 2 : 0;
+                kx = (cn & kActive) && (cn & kWet) ? 2 : 0;
             else
-                kx = classify(an & ac, sh[s0 - SW], hc, se[s0 - SW], ec, sz[s0 - SW], zc, th);
+                kx = classify(cn, cc, so[s0 - SW], ec, so[NH + s0 - SW], zc);
         }
-        if (doY) ky = classify(aw & ac, sh[s0 - 1], hc, se[s0 - 1], ec, sz[s0 - 1], zc, th);
+        if (doY) ky = classify(cw, cc, so[s0 - 1], ec, so[NH + s0 - 1], zc);
         if (doX && kx == 0) p.qx[1][i] = 0.0;
         if (doY && ky == 0) p.qy[1][i] = 0.0;
         const unsigned all = 0xffffffffu, lt = (1u << tx) - 1u;
@@ -421,28 +422,23 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
         }
         int mb = __shfl_sync(all, base, 0) + __popc(mx & lt);
         int pb = NF - 1 - (__shfl_sync(all, base, 1) + __popc(px & lt));
-        if (kx == 1) flist[mb] = (unsigned short)(2 * t);
-        if (kx > 1) flist[pb] = (unsigned short)(2 * t);
+        if (kx) flist[kx == 1 ? mb : pb] = (unsigned short)(2 * t | kx << 10);
         mb = mb - __popc(mx & lt) + __popc(mx) + __popc(my & lt);
         pb = pb + __popc(px & lt) - __popc(px) - __popc(py & lt);
-        if (ky == 1) flist[mb] = (unsigned short)(2 * t + 1);
-        if (ky > 1) flist[pb] = (unsigned short)(2 * t + 1);
+        if (ky) flist[ky == 1 ? mb : pb] = (unsigned short)(2 * t + 1 | ky << 10);
         if (p.dt_mode == 1) {
-            const float thf = sw2d_f32_est_of_f64(th), gf = sw2d_f32_est_of_f64(p.g);
-            const float hf = sw2d_f32_est_of_f64(hc);
-            const float hx = 0.5f * (hf + sw2d_f32_est_of_f64(sh[s0 - SW]));
-            const float hy = 0.5f * (hf + sw2d_f32_est_of_f64(sh[s0 - 1]));
-            const bool okx = doX && r > 0 && r < R && (an & ac) && mean_ge(sh[s0 - SW], hc, hx, th, thf);
-            const bool oky = doY && c > 0 && c < C && (aw & ac) && mean_ge(sh[s0 - 1], hc, hy, th, thf);
-            const float ex = okx ? fmaxf((fabsf(sw2d_f32_est_of_f64(sf[U + s0])) + sqrtf(gf * hx)) * sw2d_f32_est_of_f64(p.rdx), 0.f) : 0.f;
-            const float ey = oky ? fmaxf((fabsf(sw2d_f32_est_of_f64(sf[V + s0])) + sqrtf(gf * hy)) * sw2d_f32_est_of_f64(p.rdy), 0.f) : 0.f;
+            const float hx = 0.5f * (shf[s0] + shf[s0 - SW]), hy = 0.5f * (shf[s0] + shf[s0 - 1]);
+            const bool okx = doX && r > 0 && r < R && (cn & cc & kActive) && mean_ge(sh[s0 - SW], sh[s0], cn, cc, hx, th, p.thf);
+            const bool oky = doY && c > 0 && c < C && (cw & cc & kActive) && mean_ge(sh[s0 - 1], sh[s0], cw, cc, hy, th, p.thf);
+            const float ex = okx ? (fabsf(sw2d_f32_est_hi(sf[U + s0])) + sw2d_sqrt_est(p.gf * hx)) * p.rdxf : 0.f;
+            const float ey = oky ? (fabsf(sw2d_f32_est_hi(sf[V + s0])) + sw2d_sqrt_est(p.gf * hy)) * p.rdyf : 0.f;
             unsigned long long* best = p.flight->smax[cur];
-            const float cx = sw2d_f32_est_of_f64(__longlong_as_double((long long)__ldcg(best)));
-            const float cy = sw2d_f32_est_of_f64(__longlong_as_double((long long)__ldcg(best + 1)));
+            const float cx = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best)));
+            const float cy = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best + 1)));
             const float wx = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ex))), cx) * 0.99999f;
             const float wy = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ey))), cy) * 0.99999f;
-            if (okx && ex >= wx) raise_speed(best, sf[U + s0], hc, sh[s0 - SW], p.g, p.rdx);
-            if (oky && ey >= wy) raise_speed(best + 1, sf[V + s0], hc, sh[s0 - 1], p.g, p.rdy);
+            if (okx && ex >= wx) raise_speed(best, sf[U + s0], sh[s0], sh[s0 - SW], p.g, p.rdx);
+            if (oky && ey >= wy) raise_speed(best + 1, sf[V + s0], sh[s0], sh[s0 - 1], p.g, p.rdy);
         }
     }
     __syncthreads();
@@ -470,10 +466,9 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
         if (tx == 0 && w3) elist[base + n6] = (unsigned short)((s0 - 1) << 2 | 3);
     }
     for (int k = t; k < cnt[1]; k += NT) {
-        const int id = flist[NF - 1 - k], ft = id >> 1, ly = ft / BX, lx = ft % BX;
+        const int id = flist[NF - 1 - k], ft = (id & 1023) >> 1, ly = ft / BX, lx = ft % BX;
         const int sj = (ly + 1) * SW + lx + 1, sa = (id & 1) ? sj - 1 : sj - SW;
-        const bool edge = !(id & 1) && r0 + ly == R; /* the open south edge: a weir from the last row */
-        const double F = face_special(edge, sh[sa], sh[sj], se[sa], se[sj], sz[sa], sz[sj], th, p.g);
+        const double F = face_special(id >> 10, sh[sa], sh[sj], so[sa], so[sj], so[NH + sa], so[NH + sj], p.g);
         ((id & 1) ? p.qy[1] : p.qx[1])[(size_t)(r0 + ly + H) * P + (c0 + lx + H)] = F;
     }
     __syncthreads();
@@ -485,9 +480,9 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
     }
     __syncthreads();
     for (int k = t; k < cnt[0]; k += NT) {
-        const int id = flist[k], ft = id >> 1, ly = ft / BX, lx = ft % BX;
+        const int id = flist[k], ft = (id & 1023) >> 1, ly = ft / BX, lx = ft % BX;
         const bool y = (id & 1) != 0; /* the y face west of cell j, else the x face north of it */
-        const int sj = (ly + 1) * SW + lx + 1, da = y ? 1 : SW, so = y ? SW : 1;
+        const int sj = (ly + 1) * SW + lx + 1, da = y ? 1 : SW, st = y ? SW : 1;
         const size_t j = (size_t)(r0 + ly + H) * P + (c0 + lx + H);
         const int ea = (y ? 2 * NH : 0) + sj, eb = ea + NH;
         double along = dt2dx * (sedge[ea] - sedge[ea - SW]), across = dt2dy * (sedge[eb] - sedge[eb - 1]);
@@ -495,8 +490,9 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
         if (!y && c0 + lx == 0) across = 0.0;
         const double hm = sw2d_half(sh[sj] + sh[sj - da]);
         const int T = (y ? U : V) + sj; /* the other direction's face velocities */
-        const double vt = sw2d_quarter(sf[T] + sf[T + so] + sf[T - da] + sf[T - da + so]);
-        const double F = face_momentum(p, friction_coef(p, j, j - (y ? 1 : P)), sh[sj - da], sz[sj - da], se[sj], hm,
+        const double vt = sw2d_quarter(sf[T] + sf[T + st] + sf[T - da] + sf[T - da + st]);
+        const double F = face_momentum(p, friction_coef(p, j, j - (y ? 1 : P)), sh[sj - da],
+                                       sw2d_f64_of_ord(so[NH + sj - da]), sw2d_f64_of_ord(so[sj]), hm,
                                        sf[(y ? QY : QX) + sj], sf[(y ? V : U) + sj], vt, along, across, dt2,
                                        y ? dt2dy : dt2dx);
         (y ? p.qy[1] : p.qx[1])[j] = F;
@@ -680,34 +676,35 @@ __device__ void advance_clock(const StepParams& p, int cur) {
 /* continuity at t, treat_error, continuity at t+dt, hm_hn + uu1_vv1:         */
 /* SW2D-EFDC.cu:602-664, :695-725, :362-452 in one pass                       */
 
-/* "active and provisional depth < th" of a cell: decided from a binary32
- * estimate of the depth, by the exact binary64 continuity only where th lies
- * within the estimate's error (2^-19 of the magnitudes that enter it; the
- * estimate's own rounding stays below 2^-20 of them). */
+/* "active and provisional depth < th" of a cell, decided from a binary32
+ * estimate of the depth: 0 or 1, or 2 where th lies within the estimate's
+ * error (2^-17 of the magnitudes that enter it; their truncation to 21 bits
+ * and the estimate's own rounding stay below 2^-18 of them) and the exact
+ * binary64 continuity has to decide. */
 template <bool FULL>
 __device__ __noinline__ bool provisional_exact(const StepParams& p, const Slot& s, size_t i, uint8_t f, double ho,
                                                double fN, double fS, double fW, double fE) {
     double raw, rt;
     return sw2d_lt_pos(continuity<FULL>(p, i, f, ho, fS - fN, fE - fW, s.dt2, s.rr1, s.ev1, s.ql1, &raw, &rt), p.th);
 }
-struct DryEst {
-    float th, ewl, dt2, rdx, rdy, pl, pd, ev;
-};
 template <bool FULL>
-__device__ __forceinline__ bool provisional_dry(const StepParams& p, const Slot& s, const DryEst& q, size_t i,
-                                                uint8_t f, double ho, double fN, double fS, double fW, double fE) {
-    const float h = sw2d_f32_est_of_f64(ho), n = sw2d_f32_est_of_f64(fN), so = sw2d_f32_est_of_f64(fS),
-                w = sw2d_f32_est_of_f64(fW), e = sw2d_f32_est_of_f64(fE);
+__device__ __forceinline__ uint8_t provisional_dry(const StepParams& p, float dt2, float rl, float rd, float ev, size_t i,
+                                                   uint8_t f, double ho, double fN, double fS, double fW, double fE) {
+    const float h = sw2d_f32_est_hi(ho), n = sw2d_f32_est_hi(fN), so = sw2d_f32_est_hi(fS), w = sw2d_f32_est_hi(fW),
+                e = sw2d_f32_est_hi(fE);
     const bool lake = sw2d_gt(ho, p.ev_wl_min);
-    float rain = lake ? q.pl : q.pd;
-    if (p.rainw) rain *= p.rainw[i];
-    const float ev = FULL && lake ? q.ev : 0.f;
-    const float hs = h - q.dt2 * (((so - n) * q.rdx + (e - w) * q.rdy - rain) + ev);
-    const float mag = fabsf(h) + q.dt2 * ((fabsf(so) + fabsf(n)) * q.rdx + (fabsf(e) + fabsf(w)) * q.rdy + fabsf(rain) +
-                                          fabsf(ev));
-    const float d = hs - q.th;
-    if (!(FULL && (f & SW2D_F_SOURCE)) && fabsf(d) > 1.9073486e-6f * (mag + q.th) + 1e-35f) return d < 0.f;
-    return provisional_exact<FULL>(p, s, i, f, ho, fN, fS, fW, fE);
+    float src = lake ? rl : rd;
+    if (p.rainw) src *= p.rainw[i];
+    float mag = fabsf(src);
+    if (FULL && lake) {
+        src -= ev;
+        mag += fabsf(ev);
+    }
+    const float hs = h - dt2 * ((so - n) * p.rdxf + (e - w) * p.rdyf - src);
+    mag = h + dt2 * ((fabsf(so) + fabsf(n)) * p.rdxf + (fabsf(e) + fabsf(w)) * p.rdyf + mag) + p.thf;
+    const float d = hs - p.thf;
+    if ((FULL && (f & SW2D_F_SOURCE)) || !(fabsf(d) > 7.6293945e-6f * mag + 1e-35f) || !(mag < 1e37f)) return 2;
+    return d < 0.f ? 1 : 0;
 }
 
 /* FULL: evaporation, point sources or rain whose ledger is kept per cell.
@@ -758,15 +755,9 @@ __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int g
     const double dt2 = s.dt2, rr2 = s.rr2, ev2 = s.ev2;
     {
         /* 1: provisional depth at t -> "active and h* < th" (0 outside the raster) */
-        DryEst q;
-        q.th = sw2d_f32_est_of_f64(th);
-        q.dt2 = sw2d_f32_est_of_f64(dt2);
-        q.rdx = sw2d_f32_est_of_f64(p.rdx);
-        q.rdy = sw2d_f32_est_of_f64(p.rdy);
-        const float rr1 = sw2d_f32_est_of_f64(s.rr1);
-        q.pl = rr1 * sw2d_f32_est_of_f64(p.pct_lake);
-        q.pd = rr1 * sw2d_f32_est_of_f64(p.pct_land);
-        q.ev = sw2d_f32_est_of_f64(s.ev1);
+        const float dt2f = sw2d_f32_est_of_f64(dt2), rr1 = sw2d_f32_est_of_f64(s.rr1);
+        const float rl = rr1 * p.plf, rd = rr1 * p.pdf, ev = FULL ? sw2d_f32_est_of_f64(s.ev1) : 0.f;
+        int open = 0;
         for (int k = tid; k < DH * DW; k += NT) {
             const int rr = k / DW, cc = k - rr * DW;
             const int r = r0 - 2 + rr, c = c0 - 2 + cc;
@@ -774,9 +765,19 @@ __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int g
             if (r >= 0 && r < R && c >= 0 && c < C) {
                 const size_t i = (size_t)(r + H) * P + (c + H);
                 const uint8_t f = p.flags[i];
-                if (f & SW2D_F_ACTIVE) dflag = provisional_dry<FULL>(p, s, q, i, f, hc[i], fx[i], fx[i + P], fy[i], fy[i + 1]);
+                if (f & SW2D_F_ACTIVE)
+                    dflag = provisional_dry<FULL>(p, dt2f, rl, rd, ev, i, f, hc[i], fx[i], fx[i + P], fy[i], fy[i + 1]);
             }
             sdry[rr][cc] = dflag;
+            open |= dflag & 2;
+        }
+        if (open) { /* the thread's own undecided cells */
+            for (int k = tid; k < DH * DW; k += NT) {
+                const int rr = k / DW, cc = k - rr * DW;
+                if (sdry[rr][cc] != 2) continue;
+                const size_t i = (size_t)(r0 - 2 + rr + H) * P + (c0 - 2 + cc + H);
+                sdry[rr][cc] = provisional_exact<FULL>(p, s, i, p.flags[i], hc[i], fx[i], fx[i + P], fy[i], fy[i + 1]);
+            }
         }
     }
     __syncthreads();

@@ -111,6 +111,10 @@ SW2D_HD int64_t sw2d_ord(double x) {
     const int64_t s = (int64_t)sw2d_f64_bits(x);
     return s >= 0 ? s : -(s & INT64_MAX);
 }
+/* the double of sw2d_ord's value (+0 for both zeros) */
+SW2D_HD double sw2d_f64_of_ord(int64_t o) {
+    return sw2d_f64_from_bits(o >= 0 ? (uint64_t)o : ((uint64_t)0 - (uint64_t)o) | 0x8000000000000000ULL);
+}
 SW2D_HD int sw2d_lt(double a, double b) { return sw2d_ord(a) < sw2d_ord(b); }
 SW2D_HD int sw2d_gt(double a, double b) { return sw2d_ord(a) > sw2d_ord(b); }
 SW2D_HD int sw2d_le(double a, double b) { return sw2d_ord(a) <= sw2d_ord(b); }
@@ -202,6 +206,18 @@ SW2D_HD float sw2d_f32_est_of_f64(double x) {
     if (e < 897u) r = 0u;
     if (e > 1150u) r = (hi & 0x80000000u) | ((b << 1) > 0xffe0000000000000ULL ? 0x7fc00000u : 0x7f800000u);
     return sw2d_f32_from_bits(r);
+}
+
+/* The same from the high word alone, for the prefilters that run on every
+ * cell: the significand truncated to 21 bits (relative error below 2^-20),
+ * magnitudes below 2^-126 within 2^-126, 2^128 and above (infinities and NaN
+ * too) the largest finite value. */
+SW2D_HD float sw2d_f32_est_hi(double x) {
+    const uint32_t hi = (uint32_t)(sw2d_f64_bits(x) >> 32);
+    uint32_t a = hi & 0x7fffffffu;
+    a = a < 0x47efffffu ? a : 0x47efffffu;
+    a = a > 0x38000000u ? a : 0x38000000u;
+    return sw2d_f32_from_bits((hi & 0x80000000u) | (a - 0x38000000u) << 3);
 }
 
 /* an estimate of (float)v for a 32-bit unsigned v (relative error below
