@@ -312,6 +312,13 @@ __device__ __noinline__ void raise_speed(unsigned long long* at, double vel, dou
     if (v <= 0x7ff0000000000000ull && v > __ldcg(at)) atomicMax(at, v);
 }
 
+/* 8 bytes from global to shared memory past the registers; zeros when !in */
+__device__ __forceinline__ void copy8_async(double* to, const double* from, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
+                 "r"(in ? 8 : 0)
+                 : "memory");
+}
+
 /* mean depth of a face >= th, exactly: decided from the two cells' codes
  * unless th lies between their depths, then in binary32, in binary64 only
  * within its error */
@@ -358,40 +365,46 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
     const int c0 = blockIdx.x * BX, r0 = blockIdx.y * BY;
     const int c = c0 + tx, r = r0 + ty;
     const Slot& s = p.clk->slot[cur];
-    if (!s.active) return;
     const double dt2 = s.dt2, dt2dx = s.dt2dx, dt2dy = s.dt2dy;
+    const int active = s.active;
     const int P = p.P, R = p.R, C = p.C;
     const size_t i = (size_t)(r + H) * P + (c + H);
     const double th = p.th;
     {
-        const double* __restrict__ h = p.h[cur];
-        const double* __restrict__ z = p.z;
-        const double* __restrict__ qx = p.qx[0]; /* the state's discharges */
-        const double* __restrict__ qy = p.qy[0];
-        const double* __restrict__ u = p.uu1;
-        const double* __restrict__ v = p.vv1;
-        const uint8_t* __restrict__ flags = p.flags;
-        if (t < 3) cnt[t] = 0;
-        if (t == 3) rowx[BY] = rowy[BY] = 0u;
+        /* velocities and discharges are first read after the second barrier:
+         * copied past the registers, waited for there */
+        const double* const from[4] = {p.uu1, p.vv1, p.qx[0], p.qy[0]};
         for (int k = t; k < NV; k += NT) {
             const int rr = k / SW, cc = k - rr * SW;
             const int gr = r0 - 1 + rr, gc = c0 - 1 + cc;
             const bool in = gr <= R + 1 && gc <= C + 1; /* the padded raster */
-            const size_t g = (size_t)(gr + H) * P + (gc + H);
-            sf[U + k] = in ? u[g] : 0.0;
-            sf[V + k] = in ? v[g] : 0.0;
-            sf[QX + k] = in ? qx[g] : 0.0;
-            sf[QY + k] = in ? qy[g] : 0.0;
-            if (k < NH) {
-                const double hh = in ? h[g] : 0.0, zz = in ? z[g] : 0.0;
-                sh[k] = hh;
-                so[k] = sw2d_ord(hh + zz);
-                so[NH + k] = sw2d_ord(zz);
-                shf[k] = sw2d_f32_est_hi(hh);
-                scode[k] = (uint8_t)((in ? (flags[g] & SW2D_F_ACTIVE) : 0) | (sw2d_gt_pos(hh, th) ? kWet : 0) |
-                                     (sw2d_lt_pos(hh, th) ? kBelow : 0));
-            }
+            const size_t g = in ? (size_t)(gr + H) * P + (gc + H) : 0;
+#pragma unroll
+            for (int f = 0; f < 4; f++) copy8_async(&sf[f * NV + k], from[f] + g, in);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const double* __restrict__ h = p.h[cur];
+        const double* __restrict__ z = p.z;
+        const uint8_t* __restrict__ flags = p.flags;
+        if (t < 3) cnt[t] = 0;
+        if (t == 3) rowx[BY] = rowy[BY] = 0u;
+        for (int k = t; k < NH; k += NT) {
+            const int rr = k / SW, cc = k - rr * SW;
+            const int gr = r0 - 1 + rr, gc = c0 - 1 + cc;
+            const bool in = gr <= R + 1 && gc <= C + 1;
+            const size_t g = (size_t)(gr + H) * P + (gc + H);
+            const double hh = in ? h[g] : 0.0, zz = in ? z[g] : 0.0;
+            sh[k] = hh;
+            so[k] = sw2d_ord(hh + zz);
+            so[NH + k] = sw2d_ord(zz);
+            shf[k] = sw2d_f32_est_hi(hh);
+            scode[k] = (uint8_t)((in ? (flags[g] & SW2D_F_ACTIVE) : 0) | (sw2d_gt_pos(hh, th) ? kWet : 0) |
+                                 (sw2d_lt_pos(hh, th) ? kBelow : 0));
+        }
+    }
+    if (!active) { /* (the whole block) nothing in flight may outlive it */
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
     }
     __syncthreads();
     const int s0 = (ty + 1) * SW + tx + 1;
@@ -426,21 +439,8 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
         mb = mb - __popc(mx & lt) + __popc(mx) + __popc(my & lt);
         pb = pb + __popc(px & lt) - __popc(px) - __popc(py & lt);
         if (ky) flist[ky == 1 ? mb : pb] = (unsigned short)(2 * t + 1 | ky << 10);
-        if (p.dt_mode == 1) {
-            const float hx = 0.5f * (shf[s0] + shf[s0 - SW]), hy = 0.5f * (shf[s0] + shf[s0 - 1]);
-            const bool okx = doX && r > 0 && r < R && (cn & cc & kActive) && mean_ge(sh[s0 - SW], sh[s0], cn, cc, hx, th, p.thf);
-            const bool oky = doY && c > 0 && c < C && (cw & cc & kActive) && mean_ge(sh[s0 - 1], sh[s0], cw, cc, hy, th, p.thf);
-            const float ex = okx ? (fabsf(sw2d_f32_est_hi(sf[U + s0])) + sw2d_sqrt_est(p.gf * hx)) * p.rdxf : 0.f;
-            const float ey = oky ? (fabsf(sw2d_f32_est_hi(sf[V + s0])) + sw2d_sqrt_est(p.gf * hy)) * p.rdyf : 0.f;
-            unsigned long long* best = p.flight->smax[cur];
-            const float cx = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best)));
-            const float cy = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best + 1)));
-            const float wx = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ex))), cx) * 0.99999f;
-            const float wy = fmaxf(__uint_as_float(__reduce_max_sync(all, __float_as_uint(ey))), cy) * 0.99999f;
-            if (okx && ex >= wx) raise_speed(best, sf[U + s0], sh[s0], sh[s0 - SW], p.g, p.rdx);
-            if (oky && ey >= wy) raise_speed(best + 1, sf[V + s0], sh[s0], sh[s0 - 1], p.g, p.rdy);
-        }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (ty < BY) {
         /* edges of the row: south of its cells for x and y faces (types 0,
@@ -464,6 +464,21 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
         if (u2 & bit) elist[base + n4 + __popc(u2 & lt)] = (unsigned short)((s0 - SW) << 2 | 2);
         if (tx == 0 && w1) elist[base + n5] = (unsigned short)((s0 - 1) << 2 | 1);
         if (tx == 0 && w3) elist[base + n6] = (unsigned short)((s0 - 1) << 2 | 3);
+    }
+    if (p.dt_mode == 1 && ty < BY) {
+        const int cc = scode[s0], cn = scode[s0 - SW], cw = scode[s0 - 1];
+        const float hx = 0.5f * (shf[s0] + shf[s0 - SW]), hy = 0.5f * (shf[s0] + shf[s0 - 1]);
+        const bool okx = doX && r > 0 && r < R && (cn & cc & kActive) && mean_ge(sh[s0 - SW], sh[s0], cn, cc, hx, th, p.thf);
+        const bool oky = doY && c > 0 && c < C && (cw & cc & kActive) && mean_ge(sh[s0 - 1], sh[s0], cw, cc, hy, th, p.thf);
+        const float ex = okx ? (fabsf(sw2d_f32_est_hi(sf[U + s0])) + sw2d_sqrt_est(p.gf * hx)) * p.rdxf : 0.f;
+        const float ey = oky ? (fabsf(sw2d_f32_est_hi(sf[V + s0])) + sw2d_sqrt_est(p.gf * hy)) * p.rdyf : 0.f;
+        unsigned long long* best = p.flight->smax[cur];
+        const float cx = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best)));
+        const float cy = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best + 1)));
+        const float wx = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ex))), cx) * 0.99999f;
+        const float wy = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ey))), cy) * 0.99999f;
+        if (okx && ex >= wx) raise_speed(best, sf[U + s0], sh[s0], sh[s0 - SW], p.g, p.rdx);
+        if (oky && ey >= wy) raise_speed(best + 1, sf[V + s0], sh[s0], sh[s0 - 1], p.g, p.rdy);
     }
     for (int k = t; k < cnt[1]; k += NT) {
         const int id = flist[NF - 1 - k], ft = (id & 1023) >> 1, ly = ft / BX, lx = ft % BX;
