@@ -3,7 +3,7 @@
  *
  * The kernel is the measuring half of the FP64 path's prime kernel (volume
  * of the active cells and the exact CFL face-speed maxima) over the
- * reference-orientation arrays, with the per-tile partial results in a
+ * reference-orientation arrays, with the partial results in a
  * file-scope device array instead of a buffer the handle allocates.  Compiled
  * with --fmad=false like the FP64 step, so the face speeds round exactly as
  * the step's own.
@@ -11,8 +11,11 @@
 #include "sw2d.h"
 #include "sw2d_noalloc.h"
 
+#include "sw2d_math.h"
+
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 
@@ -23,138 +26,173 @@ void set_error_message(const char* msg); /* sw2d_api.cu: the message sw2d_last_e
 namespace {
 
 constexpr int kTile = SW2D_NOALLOC_TILE;              /* 32 x 32 cells per CTA */
-constexpr int kRowsPerThread = kTile / 8;             /* 256 threads = 32 x 8 */
 constexpr int kMaxTiles = SW2D_NOALLOC_MAX_TILES;
-constexpr int kSlots = 3;                             /* volume, x speed bits, y speed bits */
-constexpr int kResult = kSlots * kMaxTiles;           /* volume * area, speed */
-constexpr int kCounter = kResult + 2;                 /* tile-completion counter (low 32 bits) */
+constexpr int kBand = 32;                             /* rows of a warp's task */
+constexpr int kBatch = 4;                             /* of them read at once */
+constexpr int kBlocksPerSm = 3;
+constexpr int kSlots = 3;
+constexpr int kResult = kSlots * kMaxTiles;           /* x and y speed maxima (bits), then volume * area and speed */
+constexpr int kCounter = kResult + 2;                 /* block-completion counter (low 32 bits) */
 constexpr int kScratchDoubles = kCounter + 1;         /* 49,155 doubles = 393,240 bytes */
 
-/* The scratch: kSlots partials per tile, the two results, the counter. */
+/* The scratch: room for kSlots partials per tile (the blocks' volumes take the
+ * first of them), the two results, the counter. */
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
 static_assert(sizeof(double) * kScratchDoubles == 393240, "scratch size stated in sw2d_noalloc.h");
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+/* (|velocity| + sqrt(g hm)) / spacing as the FP64 step evaluates it, raising a
+ * running maximum kept as bits (non-negative doubles order like their bits).
+ * A call: inlined, its binary64 instructions would be predicated, and one
+ * that is predicated off still takes the FP64 pipe's 71 cycles. */
+__device__ __noinline__ void raise_speed(unsigned long long* at, double q, double ha, double hb, double g, double rd) {
+    const double hm = 0.50 * (ha + hb);
+    const double vel = sw2d_div_rn(q, hm);
+    const unsigned long long v = sw2d_f64_bits((fabs(vel) + sw2d_sqrt_rn(g * hm)) * rd);
+    if (v > __ldcg(at)) atomicMax(at, v);
+}
+__device__ __noinline__ bool mean_ge_exact(double ha, double hb, double th) {
+    return sw2d_ge_pos(0.50 * (ha + hb), th);
+}
+/* mean depth of a face >= th, exactly: decided from the two depths unless th
+ * lies between them, then in binary32, in binary64 only within its error */
+__device__ __forceinline__ bool mean_ge(double ha, double hb, float est, double th, float thf) {
+    const bool a = sw2d_ge_pos(ha, th), b = sw2d_ge_pos(hb, th);
+    if (a == b) return a;
+    if (fabsf(est - thf) > 1e-5f * thf) return est > thf;
+    return mean_ge_exact(ha, hb, th);
 }
 
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
+/* sum over the block in a fixed order, valid in thread 0 */
+__device__ __forceinline__ double block_sum256(double v, double* sm) {
+    const int tid = threadIdx.x;
+    sm[tid] = v;
+    __syncthreads();
+    double t = 0.0;
+    if (tid < 32) {
+        for (int k = 0; k < 8; k++) t = __dadd_rn(t, sm[tid + 32 * k]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w > v ? w : v;
-    }
-    return v;
-}
-
-/* (|velocity| + sqrt(g hm)) / spacing as the FP64 step evaluates it; positive
- * binary64 values order like their bit patterns, so maxima are taken on bits */
-__device__ __forceinline__ unsigned long long face_speed_bits(double q, double hm, double g, double rd) {
-    const double vel = (q == 0.0) ? q : __ddiv_rn(q, hm);
-    const double s = __dmul_rn(__dadd_rn(fabs(vel), __dsqrt_rn(__dmul_rn(g, hm))), rd);
-    return (unsigned long long)__double_as_longlong(s);
-}
-
-__global__ void __launch_bounds__(256) k64_measure_noalloc(const double* __restrict__ dem,
-                                                           const double* __restrict__ h,
-                                                           const double* __restrict__ qx,
-                                                           const double* __restrict__ qy, int R, int C,
-                                                           double nodata, double th, double g, double rdx,
-                                                           double rdy, double area, double* scratch) {
-    __shared__ double sv[8];
-    __shared__ unsigned long long sx[8], sy[8];
-    __shared__ bool last;
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
-    const int c = blockIdx.x * kTile + tx;
-    double vol = 0.0;
-    unsigned long long ux = 0ull, uy = 0ull;
-#pragma unroll
-    for (int k = 0; k < kRowsPerThread; k++) {
-        const int r = blockIdx.y * kTile + ty + 8 * k;
-        if (r >= R || c >= C) continue;
-        const size_t i = (size_t)r * C + c;
-        if (dem[i] == nodata) continue;
-        const double hc = h[i];
-        vol = __dadd_rn(vol, hc);
-        if (r > 0 && dem[i - C] != nodata) { /* x face north of (r, c) */
-            const double hm = __dmul_rn(0.50, __dadd_rn(hc, h[i - C]));
-            if (hm >= th) {
-                const unsigned long long b = face_speed_bits(qx[i], hm, g, rdx);
-                ux = b > ux ? b : ux;
-            }
-        }
-        if (c > 0 && dem[i - 1] != nodata) { /* y face west of (r, c) */
-            const double hn = __dmul_rn(0.50, __dadd_rn(hc, h[i - 1]));
-            if (hn >= th) {
-                const unsigned long long b = face_speed_bits(qy[(size_t)r * (C + 1) + c], hn, g, rdy);
-                uy = b > uy ? b : uy;
-            }
-        }
-    }
-    vol = warp_sum(vol);
-    ux = warp_max_u64(ux);
-    uy = warp_max_u64(uy);
-    if (tx == 0) {
-        sv[ty] = vol;
-        sx[ty] = ux;
-        sy[ty] = uy;
+        for (int o = 16; o > 0; o >>= 1) t = __dadd_rn(t, __shfl_down_sync(0xffffffffu, t, o));
     }
     __syncthreads();
-    const int nb = gridDim.x * gridDim.y;
-    const int b = blockIdx.y * gridDim.x + blockIdx.x;
-    if (tid == 0) {
-        double v = 0.0;
-        unsigned long long a = 0ull, w = 0ull;
-        for (int k = 0; k < 8; k++) {
-            v = __dadd_rn(v, sv[k]);
-            a = sx[k] > a ? sx[k] : a;
-            w = sy[k] > w ? sy[k] : w;
+    return t;
+}
+
+struct MeasureIn {
+    const double *dem, *h, *qx, *qy;
+    int R, C;
+    double nodata, th, g, rdx, rdy, area;
+    float thf, gf, rdxf, rdyf;
+};
+
+/* A warp takes tasks of 32 columns x kBand rows and walks down the rows, the
+ * row above in registers, the column left of a lane's from its neighbour, so
+ * each array is read once (plus the row above and the column left of a task);
+ * kBatch rows are in flight at a time.  What it was bound by is the FP64
+ * pipe, a binary64 instruction taking a warp 71 cycles: a division and a
+ * square root on every face.  The face speeds are estimated in binary32
+ * instead (within 2.2e-6), and only lanes within 1e-5 of the running maximum
+ * are evaluated in binary64 and raise it: the exact maximum in any order.
+ * One binary64 addition a cell is left, the volume's.  Bounded by the latency
+ * of HBM reads: 4 rows of 32-row tasks in flight at three blocks an SM
+ * measured 136 us for the whole call at 4096 x 3000 (393 MB), 2 rows at four
+ * or six blocks 159 and 220, 16-row tasks 186; 1320 before. */
+__global__ void __launch_bounds__(256, kBlocksPerSm) k64_measure_noalloc(MeasureIn p, double* scratch) {
+    __shared__ double sm[256];
+    __shared__ bool last;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int R = p.R, C = p.C, sx_n = (C + 31) / 32;
+    const int ntask = sx_n * ((R + kBand - 1) / kBand);
+    const double th = p.th;
+    const int64_t none = sw2d_ord(p.nodata);
+    const bool any_none = p.nodata == p.nodata;
+    unsigned long long* best = reinterpret_cast<unsigned long long*>(scratch + kResult);
+    auto active = [&](double z) { return !(any_none && sw2d_ord(z) == none); }; /* z != nodata */
+    double vol = 0.0;
+    for (int task = (blockIdx.x * 256 + tid) >> 5; task < ntask; task += gridDim.x * 8) {
+        const int band = task / sx_n, c = (task - band * sx_n) * 32 + lane;
+        const int r0 = band * kBand, r1 = min(R, r0 + kBand);
+        const bool in = c < C, left = lane == 0 && c > 0;
+        bool act_n = false;
+        double h_n = 0.0;
+        if (in && r0 > 0) {
+            const size_t i = (size_t)(r0 - 1) * C + c;
+            h_n = p.h[i];
+            act_n = active(p.dem[i]);
         }
-        scratch[(size_t)kSlots * b + 0] = v;
-        scratch[(size_t)kSlots * b + 1] = __longlong_as_double((long long)a);
-        scratch[(size_t)kSlots * b + 2] = __longlong_as_double((long long)w);
+        for (int r = r0; r < r1; r += kBatch) {
+            double z[kBatch], h[kBatch], qx[kBatch], qy[kBatch], zl[kBatch], hl[kBatch];
+#pragma unroll
+            for (int k = 0; k < kBatch; k++) {
+                const bool ok = in && r + k < r1;
+                const size_t i = (size_t)(r + k) * C + c;
+                z[k] = ok ? p.dem[i] : p.nodata;
+                h[k] = ok ? p.h[i] : 0.0;
+                qx[k] = ok ? p.qx[i] : 0.0;
+                qy[k] = ok ? p.qy[i + r + k] : 0.0; /* rows of C + 1 */
+                zl[k] = ok && left ? p.dem[i - 1] : p.nodata;
+                hl[k] = ok && left ? p.h[i - 1] : 0.0;
+            }
+            float ex[kBatch], ey[kBatch], bx = 0.f, by = 0.f;
+            double hw[kBatch], hn[kBatch];
+#pragma unroll
+            for (int k = 0; k < kBatch; k++) {
+                const bool ok = in && r + k < r1;
+                const bool act = ok && active(z[k]);
+                if (act) vol = __dadd_rn(vol, h[k]);
+                int aw = __shfl_up_sync(0xffffffffu, (int)act, 1);
+                hw[k] = __shfl_up_sync(0xffffffffu, h[k], 1);
+                if (lane == 0) {
+                    aw = left && ok && active(zl[k]);
+                    hw[k] = hl[k];
+                }
+                hn[k] = h_n;
+                const float hf = sw2d_f32_est_hi(h[k]);
+                const float mx = 0.5f * (hf + sw2d_f32_est_hi(h_n)), my = 0.5f * (hf + sw2d_f32_est_hi(hw[k]));
+                const bool okx = act && act_n && mean_ge(h_n, h[k], mx, th, p.thf);
+                const bool oky = act && aw && mean_ge(hw[k], h[k], my, th, p.thf);
+                ex[k] = okx ? (fabsf(sw2d_f32_est_hi(qx[k])) * sw2d_rcp_est(mx) + sw2d_sqrt_est(p.gf * mx)) * p.rdxf : -1.f;
+                ey[k] = oky ? (fabsf(sw2d_f32_est_hi(qy[k])) * sw2d_rcp_est(my) + sw2d_sqrt_est(p.gf * my)) * p.rdyf : -1.f;
+                bx = fmaxf(bx, ex[k]);
+                by = fmaxf(by, ey[k]);
+                act_n = act;
+                h_n = h[k];
+            }
+            const float cx = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best)));
+            const float cy = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best + 1)));
+            const float tx = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bx))), cx) * 0.99999f;
+            const float ty = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(by))), cy) * 0.99999f;
+            if (bx >= tx) {
+#pragma unroll
+                for (int k = 0; k < kBatch; k++)
+                    if (ex[k] >= tx) raise_speed(best, qx[k], h[k], hn[k], p.g, p.rdx);
+            }
+            if (by >= ty) {
+#pragma unroll
+                for (int k = 0; k < kBatch; k++)
+                    if (ey[k] >= ty) raise_speed(best + 1, qy[k], h[k], hw[k], p.g, p.rdy);
+            }
+        }
+    }
+    vol = block_sum256(vol, sm);
+    if (tid == 0) {
+        scratch[blockIdx.x] = vol;
         __threadfence();
         unsigned int* counter = reinterpret_cast<unsigned int*>(scratch + kCounter);
-        last = (atomicAdd(counter, 1u) == (unsigned int)nb - 1u);
+        last = (atomicAdd(counter, 1u) == gridDim.x - 1u);
     }
     __syncthreads();
     if (!last) return;
-    /* the last tile to finish combines the partials in a fixed order */
+    /* the last block to finish combines the partials in a fixed order (every
+     * block's raises come before its count) */
     __threadfence();
     double v = 0.0;
-    unsigned long long a = 0ull, w = 0ull;
-    for (int k = tid; k < nb; k += 256) {
-        const volatile double* pk = scratch + (size_t)kSlots * k;
-        v = __dadd_rn(v, pk[0]);
-        const unsigned long long pa = (unsigned long long)__double_as_longlong(pk[1]);
-        const unsigned long long pw = (unsigned long long)__double_as_longlong(pk[2]);
-        a = pa > a ? pa : a;
-        w = pw > w ? pw : w;
-    }
-    v = warp_sum(v);
-    a = warp_max_u64(a);
-    w = warp_max_u64(w);
-    __syncthreads();
-    if (tx == 0) {
-        sv[ty] = v;
-        sx[ty] = a;
-        sy[ty] = w;
-    }
-    __syncthreads();
+    for (unsigned k = tid; k < gridDim.x; k += 256) v = __dadd_rn(v, __ldcg(scratch + k));
+    v = block_sum256(v, sm);
     if (tid == 0) {
-        double vt = 0.0;
-        unsigned long long at = 0ull, wt = 0ull;
-        for (int k = 0; k < 8; k++) {
-            vt = __dadd_rn(vt, sv[k]);
-            at = sx[k] > at ? sx[k] : at;
-            wt = sy[k] > wt ? sy[k] : wt;
-        }
-        scratch[kResult + 0] = __dmul_rn(vt, area);
-        scratch[kResult + 1] =
-            __dadd_rn(__longlong_as_double((long long)at), __longlong_as_double((long long)wt));
+        const double a = __longlong_as_double((long long)__ldcg(best)), w = __longlong_as_double((long long)__ldcg(best + 1));
+        scratch[kResult + 0] = __dmul_rn(v, p.area);
+        scratch[kResult + 1] = __dadd_rn(a, w);
     }
 }
 
@@ -204,12 +242,33 @@ extern "C" int sw2d_measure_state_noalloc(const double* d_dem, const double* d_d
     if (e != cudaSuccess) return cuda_fail("cudaGetSymbolAddress", e);
     double* scratch = static_cast<double*>(addr);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    /* the counter must be zero when the kernel starts */
-    e = cudaMemsetAsync(scratch + kCounter, 0, sizeof(double), s);
+    /* the running maxima and the counter must be zero when the kernel starts */
+    e = cudaMemsetAsync(scratch + kResult, 0, 3 * sizeof(double), s);
     if (e != cudaSuccess) return cuda_fail("cudaMemsetAsync", e);
-    const dim3 grid((unsigned)tiles_x, (unsigned)tiles_y), block(32, 8);
-    k64_measure_noalloc<<<grid, block, 0, s>>>(d_dem, d_depth, d_qx, d_qy, rows, cols, nodata, th, g, 1.0 / dx,
-                                                1.0 / dy, dx * dy, scratch);
+    MeasureIn in;
+    in.dem = d_dem;
+    in.h = d_depth;
+    in.qx = d_qx;
+    in.qy = d_qy;
+    in.R = rows;
+    in.C = cols;
+    in.nodata = nodata;
+    in.th = th;
+    in.g = g;
+    in.rdx = 1.0 / dx;
+    in.rdy = 1.0 / dy;
+    in.area = dx * dy;
+    in.thf = (float)th;
+    in.gf = (float)g;
+    in.rdxf = (float)in.rdx;
+    in.rdyf = (float)in.rdy;
+    int dev = 0, nsm = 0;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return cuda_fail("cudaDeviceGetAttribute", e);
+    const long long tasks = (cols + 31LL) / 32 * ((rows + kBand - 1LL) / kBand);
+    const int blocks = (int)std::min<long long>((tasks + 7) / 8, (long long)kBlocksPerSm * nsm);
+    k64_measure_noalloc<<<blocks, 256, 0, s>>>(in, scratch);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail("k64_measure_noalloc launch", e);
     double res[2];
