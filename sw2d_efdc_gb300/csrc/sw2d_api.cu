@@ -410,9 +410,9 @@ int launch_iterations(sw2d_handle* h, long long n) {
         fp64_launch_settle(p, h->stream);
         return sync_check(h);
     }
-    int rc = build_graph(h);
-    if (rc) return rc;
-    long long full = n / kChunk, rem = n % kChunk;
+    const long long full = n / kChunk, rem = n % kChunk;
+    int rc;
+    if (full > 0 && (rc = build_graph(h))) return rc;
     for (long long k = 0; k < full; k++) CK(cudaGraphLaunch(h->graph, h->stream));
     StepParams p = h->params();
     for (long long k = 0; k < rem; k++) fp64_launch_iteration(p, (int)(k & 1), h->stream, nullptr);
@@ -512,74 +512,62 @@ int run_until_fp32(sw2d_handle* h, double t_end, long long max_iters, int64_t* d
     return SW2D_OK;
 }
 
+int read_report(sw2d_handle* h, Flight64::Report* out) {
+    CK(cudaMemcpyAsync(out, &h->flight->report, sizeof *out, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    return SW2D_OK;
+}
+
 int run_until(sw2d_handle* h, double t_end, long long max_iters, int64_t* done_out) {
     int rc = check_ready(h);
     if (rc) return rc;
     if (h->fp32()) return run_until_fp32(h, t_end, max_iters, done_out);
-    if ((rc = put(h, &h->clk->t_end, &t_end, sizeof(double)))) return rc;
-    if ((rc = prime(h, 0))) return rc;
-    DevClock c0;
-    if ((rc = read_clock(h, &c0))) return rc;
-    const long long it0 = c0.iters;
-    CK(cudaEventRecord(h->ev_a, h->stream));
-    long long launched = 0;
-    if (h->cfg.dt_mode == SW2D_DT_FIXED) {
+    /* iterations are launched in pairs (the state ends in buffer 0); of an odd
+     * bounded count, the extra one is left inactive (a state copy) by the
+     * device's iteration limit */
+    const long long limit = max_iters >= 0 && (max_iters & 1) ? max_iters : -1;
+    fp64_launch_begin(h->params(), t_end, limit, h->stream);
+    Flight64::Report st;
+    if (h->cfg.dt_mode == SW2D_DT_CFL && max_iters >= 0) {
+        CK(cudaEventRecord(h->ev_a, h->stream));
+        if ((rc = launch_iterations(h, max_iters + (max_iters & 1)))) return rc;
+        CK(cudaEventRecord(h->ev_b, h->stream));
+        if ((rc = read_report(h, &st))) return rc;
+    } else if (h->cfg.dt_mode == SW2D_DT_FIXED) {
         /* the reference's loop condition, replayed on the host to size the launch */
-        double t = c0.t, dt = h->cfg.dt;
+        if ((rc = read_report(h, &st))) return rc;
+        double t = st.t, dt = h->cfg.dt;
         long long n = 0;
         while (t + dt <= t_end && (max_iters < 0 || n < max_iters)) {
             t = (t + dt) + dt;
             n++;
         }
-        long long ne = n + (n & 1);
-        if (max_iters >= 0 && (n & 1)) {
-            /* an odd bounded count: the extra iteration must not advance */
-            double te = t;
-            if ((rc = put(h, &h->clk->t_end, &te, sizeof(double)))) return rc;
-            if ((rc = prime(h, 0))) return rc;
-        }
-        if ((rc = launch_iterations(h, ne))) return rc;
-        launched = ne;
-    } else if (max_iters >= 0) {
-        /* a bounded CFL run: an odd count launches one iteration more, which
-         * the device's iteration limit leaves inactive (a state copy), so the
-         * state ends in buffer 0 as the captured pairs need */
-        const long long ne = max_iters + (max_iters & 1);
-        if (max_iters & 1) {
-            const long long lim = it0 + max_iters;
-            if ((rc = put(h, &h->clk->iter_end, &lim, sizeof lim))) return rc;
-            if ((rc = prime(h, 0))) return rc;
-        }
-        rc = launch_iterations(h, ne);
-        if (max_iters & 1) {
-            const long long none = LLONG_MAX;
-            const int rc2 = put(h, &h->clk->iter_end, &none, sizeof none);
-            if (!rc) rc = rc2;
-        }
-        if (rc) return rc;
-        launched = ne;
+        CK(cudaEventRecord(h->ev_a, h->stream));
+        if ((rc = launch_iterations(h, n + (n & 1)))) return rc;
+        CK(cudaEventRecord(h->ev_b, h->stream));
+        if ((rc = read_report(h, &st))) return rc;
     } else {
-        for (;;) {
-            if ((rc = launch_iterations(h, kChunk))) return rc;
-            launched += kChunk;
-            DevClock c;
-            if ((rc = read_clock(h, &c))) return rc;
-            if (!c.slot[0].active) break;
-            if (c.status & 1) return fail(SW2D_ERR_NUMERIC, "non-finite depth");
+        /* CFL to an end time: as many iterations at a time as the current
+         * length leaves (it changes slowly), at most 1024 */
+        if ((rc = read_report(h, &st))) return rc;
+        CK(cudaEventRecord(h->ev_a, h->stream));
+        while (st.active) {
+            const double left = (t_end - st.t) / st.dt2;
+            const long long n = left < 1022.0 ? (long long)left + 1 : 1024;
+            if ((rc = launch_iterations(h, n + (n & 1)))) return rc;
+            CK(cudaEventRecord(h->ev_b, h->stream));
+            if ((rc = read_report(h, &st))) return rc;
+            if (st.status & 1) return fail(SW2D_ERR_NUMERIC, "non-finite depth");
         }
+        CK(cudaEventRecord(h->ev_b, h->stream));
+        CK(cudaEventSynchronize(h->ev_b));
     }
-    CK(cudaEventRecord(h->ev_b, h->stream));
-    CK(cudaEventSynchronize(h->ev_b));
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, h->ev_a, h->ev_b));
-    DevClock c1;
-    if ((rc = read_clock(h, &c1))) return rc;
-    long long done = c1.iters - it0;
+    const long long done = st.iters - st.iters0;
     h->last_ms_per_iter = done > 0 ? ms / (double)done : 0.0;
     if (done_out) *done_out = done;
-    if (c1.status & 1) return fail(SW2D_ERR_NUMERIC, "non-finite depth");
-    (void)launched;
-    /* restore the open-ended t_end in the clock slot for later queries */
+    if (st.status & 1) return fail(SW2D_ERR_NUMERIC, "non-finite depth");
     return SW2D_OK;
 }
 

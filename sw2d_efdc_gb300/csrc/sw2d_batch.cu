@@ -7,8 +7,8 @@
  * A request is queued on submit with a host copy of its inputs.  Every
  * sw2d_batch_step() admits queued requests (first fit, in arrival order)
  * while the HBM budget and the running-slot limit allow, advances all
- * running scenarios by a chunk of iterations (replayed from a captured CUDA
- * graph), and retires the ones that reached their end time: their final
+ * running scenarios by a chunk of iterations (one persistent launch per
+ * feature class), and retires the ones that reached their end time: their final
  * depth and discharges are copied to host memory and their device memory is
  * released for the next admissions.  Running state stays on the device
  * between steps.
@@ -280,20 +280,18 @@ int sw2d_batch_step(sw2d_batch* b, int iterations, int* n_running_out, int* n_qu
     admit(b);
     if (!b->running.empty() && iterations > 0) {
         double cells = 0;
-        std::vector<sw2d::Clock32> before(b->running.size());
-        for (size_t k = 0; k < b->running.size(); k++) {
-            int rc = b->eng->get_clock((int)k, &before[k], &err);
-            if (rc) return bfail(rc, err);
-        }
-        int rc = b->eng->run(iterations, &err);
+        std::vector<sw2d::Status32> before, after;
+        int rc = b->eng->get_status(&before, &err);
+        if (rc) return bfail(rc, err);
+        rc = b->eng->run(iterations, &err);
         if (rc) return bfail(rc, err);
         b->device_ms += b->eng->last_ms();
         b->launches += (long long)((iterations + sw2d::Engine32::kChunk - 1) / sw2d::Engine32::kChunk) *
                        b->eng->launches_per_chunk();
         /* retire finished scenarios (highest index first keeps indices valid) */
+        if ((rc = b->eng->get_status(&after, &err))) return bfail(rc, err);
         for (size_t k = b->running.size(); k-- > 0;) {
-            sw2d::Clock32 c;
-            if ((rc = b->eng->get_clock((int)k, &c, &err))) return bfail(rc, err);
+            const sw2d::Status32& c = after[k];
             Request& r = *b->reqs[b->running[k]];
             const double cu = (double)(c.iters - before[k].iters) * r.desc.rows * r.desc.cols;
             r.cell_updates += cu;
@@ -369,9 +367,10 @@ int sw2d_batch_tune(sw2d_batch* b, int max_iterations, int* iterations_out) {
     if (!b->running.empty()) {
         int rc = b->eng->tune_now(max_iterations, &err, &done);
         if (rc) return bfail(rc, err);
+        std::vector<sw2d::Status32> st;
+        if ((rc = b->eng->get_status(&st, &err))) return bfail(rc, err);
         for (size_t k = b->running.size(); k-- > 0;) {
-            sw2d::Clock32 c;
-            if ((rc = b->eng->get_clock((int)k, &c, &err))) return bfail(rc, err);
+            const sw2d::Status32& c = st[k];
             if (c.done || (c.status & 3)) {
                 if ((rc = retire(b, k))) return rc;
             }

@@ -4,6 +4,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -45,6 +46,34 @@ bool make_map(CUtensorMap* tm, void* base, CUtensorMapDataType dt, size_t esize,
 
 int pitch_of(int cols) { return ((cols + 12 + 31) / 32) * 32; }
 
+/* f(first, last) over [0, n) on host threads, one per `grain` elements of
+ * work at most (a thread costs tens of microseconds to start) */
+template <typename F>
+void on_threads(size_t n, size_t work, size_t grain, F f) {
+    const size_t nt = std::max<size_t>(1, std::min<size_t>({16, std::thread::hardware_concurrency(), n, work / grain}));
+    if (nt == 1) {
+        f((size_t)0, n);
+        return;
+    }
+    std::vector<std::thread> th;
+    const size_t per = (n + nt - 1) / nt;
+    for (size_t a = 0; a < n; a += per) th.emplace_back([=] { f(a, std::min(n, a + per)); });
+    for (auto& x : th) x.join();
+}
+
+/* device arrays of a scenario in one allocation, each 256-byte aligned */
+struct Carver {
+    size_t at = 0, bytes = 0; /* the end of the last one; the arrays' own bytes */
+    size_t take(size_t n) {
+        const size_t o = at;
+        bytes += n;
+        at = (at + std::max<size_t>(n, 16) + 255) & ~(size_t)255;
+        return o;
+    }
+};
+constexpr size_t kNone = ~(size_t)0;
+constexpr size_t kPinInputs = (size_t)8 << 20; /* inputs up to here pay for pinned staging (larger ones use it if it is there) */
+
 #define ECK(call)                                                                   \
     do {                                                                            \
         cudaError_t e_ = (call);                                                    \
@@ -61,14 +90,13 @@ Engine32::Engine32(int device) : device_(device) {}
 Engine32::~Engine32() {
     cudaSetDevice(device_);
     if (stream_) cudaStreamSynchronize(stream_);
-    for (auto& s : scn_)
-        for (void* p : s->allocs) cudaFree(p);
-    if (graph_) cudaGraphExecDestroy(graph_);
+    for (auto& s : scn_) cudaFree(s->slab);
     cudaFree(d_scn_);
     cudaFree(d_work_);
     cudaFree(d_part_);
     cudaFree(d_ctl_);
     cudaFree(d_tmp_);
+    cudaFree(d_stat_);
     if (ev_a_) cudaEventDestroy(ev_a_);
     if (ev_b_) cudaEventDestroy(ev_b_);
     if (ev_t0_) cudaEventDestroy(ev_t0_);
@@ -147,172 +175,202 @@ int Engine32::add(const ScenarioInput& in, long long id, std::string* err, int* 
     S.NR = NR;
     const size_t cells = (size_t)P * NR;
     const int tx = (C + M_CW - 1) / M_CW, nb = (R + M_DR - 1) / M_DR; /* datum tiles: strips x bands */
-    auto alloc = [&](size_t bytes, void** p) -> int {
-        cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
-        if (e != cudaSuccess) {
-            if (err) *err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
-            return SW2D_ERR_NOMEM;
-        }
-        S.allocs.push_back(*p);
-        S.bytes += bytes;
-        cudaMemsetAsync(*p, 0, std::max<size_t>(bytes, 16), stream_);
-        return SW2D_OK;
-    };
-    auto fail_free = [&](int rc) {
-        cudaStreamSynchronize(stream_);
-        for (void* p : S.allocs) cudaFree(p);
-        return rc;
-    };
-    Scn32& d = S.d;
-    void* p;
-    int rc;
-    for (int k = 0; k < 2; k++) {
-        if ((rc = alloc(cells * 4, &p))) return fail_free(rc);
-        d.h[k] = (float*)p;
-        if ((rc = alloc(cells * 4, &p))) return fail_free(rc);
-        d.qx[k] = (float*)p;
-        if ((rc = alloc(cells * 4, &p))) return fail_free(rc);
-        d.qy[k] = (float*)p;
-    }
-    if ((rc = alloc(cells * 4, &p))) return fail_free(rc);
-    d.kc = (float*)p;
-    float* dz;
-    if ((rc = alloc(cells * 4, &p))) return fail_free(rc);
-    dz = (float*)p;
-    d.z = dz;
-    uint8_t* dcls = nullptr;
-    if (in.mclass) {
-        if ((rc = alloc(cells, &p))) return fail_free(rc);
-        dcls = (uint8_t*)p;
-    }
-    d.cls = dcls;
-    float* ddatum;
-    if ((rc = alloc((size_t)tx * nb * 4, &p))) return fail_free(rc);
-    ddatum = (float*)p;
-    d.datum = ddatum;
-    float* drw = nullptr;
-    if (in.rain_weight) {
-        if ((rc = alloc(cells * 4, &p))) return fail_free(rc);
-        drw = (float*)p;
-    }
-    d.rainw = drw;
-    const int nrain = std::max(in.nrain, 1);
-    double* drain;
-    if ((rc = alloc((size_t)(nrain + 2) * 8, &p))) return fail_free(rc);
-    drain = (double*)p;
-    d.rain = drain;
-    /* evaporation series and point sources (a later source on a cell
-     * replaces an earlier one, as the reference's stream_flow writes them) */
-    double* devap = nullptr;
-    if (in.evap && in.nevap > 0) {
-        if ((rc = alloc((size_t)(in.nevap + 2) * 8, &p))) return fail_free(rc);
-        devap = (double*)p;
-    }
+    /* point sources (a later source on a cell replaces an earlier one, as the
+     * reference's stream_flow writes them) */
     std::vector<int> src_keep;
     if (in.nsrc > 0) {
         if (in.nsrc > T32_MAXSRC || !in.src_cells || !in.src_q || in.nq <= 0 || !(in.dtoq > 0)) {
             if (err) *err = "point sources";
-            return fail_free(SW2D_ERR_INVALID);
+            return SW2D_ERR_INVALID;
         }
         for (int k = 0; k < in.nsrc; k++) {
             if (in.src_cells[k] < 0 || in.src_cells[k] >= R * C) {
                 if (err) *err = "source cell out of range";
-                return fail_free(SW2D_ERR_INVALID);
+                return SW2D_ERR_INVALID;
             }
             bool later = false;
             for (int j = k + 1; j < in.nsrc; j++) later |= in.src_cells[j] == in.src_cells[k];
             if (!later) src_keep.push_back(k);
         }
     }
-    const int nu = (int)src_keep.size();
-    int* dsrc_cell = nullptr;
-    double* dsrcq = nullptr;
-    if (nu > 0) {
-        if ((rc = alloc((size_t)nu * 4, &p))) return fail_free(rc);
-        dsrc_cell = (int*)p;
-        if ((rc = alloc((size_t)(in.nq + 2) * nu * 8, &p))) return fail_free(rc);
-        dsrcq = (double*)p;
-    }
-    d.evap = devap;
-    d.srcq = dsrcq;
-    d.src_cell = dsrc_cell;
-    d.outlet = nullptr;
-    if (in.outlet_cap > 0) {
-        if ((rc = alloc((size_t)in.outlet_cap * 16, &p))) return fail_free(rc);
-        d.outlet = (double*)p;
-    }
-    Clock32* dclk;
-    if ((rc = alloc(sizeof(Clock32), &p))) return fail_free(rc);
-    dclk = (Clock32*)p;
-    d.clk = dclk;
+    const int nu = (int)src_keep.size(), nrain = std::max(in.nrain, 1);
+    const bool has_evap = in.evap && in.nevap > 0;
 
-    /* host staging: per datum tile (a strip of 224 columns x a band of 64
-     * rows) the mean active elevation rounded to 1/16 m, bed offsets from it
-     * with NaN for inactive cells */
-    std::vector<float> datum((size_t)tx * nb, 0.f);
-    std::vector<float> zoff(cells, std::numeric_limits<float>::quiet_NaN()), hbuf(cells, 0.f), rw;
-    std::vector<uint8_t> cls;
-    if (in.mclass) cls.assign(cells, 0);
-    double active_weight = 0.0;
-    for (int j = 0; j < nb; j++)
-        for (int i = 0; i < tx; i++) {
-            double sum = 0;
-            long n = 0;
-            for (int r = j * M_DR; r < std::min(R, (j + 1) * M_DR); r++)
-                for (int c = i * M_CW; c < std::min(C, (i + 1) * M_CW); c++) {
-                    double z = in.dem[(size_t)r * C + c];
-                    if (z != in.nodata) {
-                        sum += z;
-                        n++;
+    /* what the host fills (contiguous in the slab and in its staging copy),
+     * then what starts as zeros */
+    Carver cv;
+    const size_t o_z = cv.take(cells * 4), o_h = cv.take(cells * 4);
+    const size_t o_cls = in.mclass ? cv.take(cells) : kNone;
+    const size_t o_rw = in.rain_weight ? cv.take(cells * 4) : kNone;
+    const size_t o_datum = cv.take((size_t)tx * nb * 4);
+    const size_t o_rain = cv.take((size_t)(nrain + 2) * 8);
+    const size_t o_evap = has_evap ? cv.take((size_t)(in.nevap + 2) * 8) : kNone;
+    const size_t o_srcc = nu > 0 ? cv.take((size_t)nu * 4) : kNone;
+    const size_t o_srcq = nu > 0 ? cv.take((size_t)(in.nq + 2) * nu * 8) : kNone;
+    const size_t o_clk = cv.take(sizeof(Clock32));
+    const size_t staged = cv.at;
+    const size_t o_h1 = cv.take(cells * 4);
+    const size_t o_qx[2] = {cv.take(cells * 4), cv.take(cells * 4)}, o_qy[2] = {cv.take(cells * 4), cv.take(cells * 4)};
+    const size_t o_kc = cv.take(cells * 4);
+    const size_t o_out = in.outlet_cap > 0 ? cv.take((size_t)in.outlet_cap * 16) : kNone;
+
+    char* slab = nullptr;
+    {
+        cudaError_t e = cudaMalloc((void**)&slab, cv.at);
+        if (e != cudaSuccess) {
+            if (err) *err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+            return SW2D_ERR_NOMEM;
+        }
+    }
+    S.slab = slab;
+    S.bytes = cv.bytes;
+    auto fail_free = [&](int rc) {
+        cudaStreamSynchronize(stream_);
+        cudaFree(slab);
+        return rc;
+    };
+    int rc;
+#define ACK(call)                                                               \
+    do {                                                                        \
+        cudaError_t e_ = (call);                                                \
+        if (e_ != cudaSuccess) {                                                \
+            if (err) *err = std::string(#call) + ": " + cudaGetErrorString(e_); \
+            return fail_free(SW2D_ERR_CUDA);                                    \
+        }                                                                       \
+    } while (0)
+    ACK(cudaMemsetAsync(slab + staged, 0, cv.at - staged, stream_));
+    Scn32& d = S.d;
+    auto dev = [&](size_t o) -> void* { return o == kNone ? nullptr : slab + o; };
+    d.h[0] = (float*)dev(o_h);
+    d.h[1] = (float*)dev(o_h1);
+    for (int k = 0; k < 2; k++) {
+        d.qx[k] = (float*)dev(o_qx[k]);
+        d.qy[k] = (float*)dev(o_qy[k]);
+    }
+    d.kc = (float*)dev(o_kc);
+    float* const dz = (float*)dev(o_z);
+    d.z = dz;
+    uint8_t* const dcls = (uint8_t*)dev(o_cls);
+    d.cls = dcls;
+    d.datum = (float*)dev(o_datum);
+    float* const drw = (float*)dev(o_rw);
+    d.rainw = drw;
+    d.rain = (double*)dev(o_rain);
+    d.evap = (double*)dev(o_evap);
+    d.srcq = (double*)dev(o_srcq);
+    d.src_cell = (int*)dev(o_srcc);
+    d.outlet = (double*)dev(o_out);
+    d.clk = (Clock32*)dev(o_clk);
+
+    /* host staging: per datum tile (a
+     * strip of 224 columns x a band of 64 rows) the mean active elevation
+     * rounded to 1/16 m, bed offsets from it with NaN for inactive cells */
+    std::vector<char> pageable;
+    char* stage;
+    if (staged <= std::max(kPinInputs, pin_bytes_)) {
+        if ((rc = reserve_pin(staged, err))) return fail_free(rc);
+        stage = static_cast<char*>(pin_);
+    } else {
+        pageable.resize(staged);
+        stage = pageable.data();
+    }
+    float* const zoff = (float*)(stage + o_z);
+    float* const hbuf = (float*)(stage + o_h);
+    uint8_t* const cls = in.mclass ? (uint8_t*)(stage + o_cls) : nullptr;
+    float* const rw = in.rain_weight ? (float*)(stage + o_rw) : nullptr;
+    float* const datum = (float*)(stage + o_datum);
+    const float nan = std::numeric_limits<float>::quiet_NaN();
+    for (int r = 0; r < NR; r++) { /* the halo: inactive, dry, class 0, weight 1 */
+        const bool in_rows = r >= M_H && r < M_H + R;
+        const size_t row = (size_t)r * P;
+        auto blank = [&](size_t a, size_t b) {
+            std::fill(zoff + row + a, zoff + row + b, nan);
+            std::fill(hbuf + row + a, hbuf + row + b, 0.f);
+            if (cls) std::fill(cls + row + a, cls + row + b, (uint8_t)0);
+            if (rw) std::fill(rw + row + a, rw + row + b, 1.f);
+        };
+        if (in_rows) {
+            blank(0, M_H);
+            blank((size_t)(M_H + C), (size_t)P);
+        } else {
+            blank(0, (size_t)P);
+        }
+    }
+    std::vector<double> band_weight((size_t)nb, 0.0); /* active cells' rain weight, band by band */
+    std::atomic<bool> bad_class(false);
+    on_threads((size_t)nb, (size_t)R * C, (size_t)1 << 19, [&](size_t j0, size_t j1) {
+        for (size_t j = j0; j < j1; j++) {
+            const int ra = (int)j * M_DR, rb = std::min(R, ra + M_DR);
+            double aw = 0.0;
+            for (int i = 0; i < tx; i++) {
+                const int ca = i * M_CW, cb = std::min(C, ca + M_CW);
+                double sum = 0;
+                long n = 0;
+                for (int r = ra; r < rb; r++)
+                    for (int c = ca; c < cb; c++) {
+                        const double z = in.dem[(size_t)r * C + c];
+                        if (z != in.nodata) {
+                            sum += z;
+                            n++;
+                        }
                     }
+                const float dt = n ? (float)(std::round(sum / n * 16.0) / 16.0) : 0.f;
+                datum[j * tx + i] = dt;
+                const double dat = dt;
+                for (int r = ra; r < rb; r++) {
+                    const size_t k = (size_t)r * C, g = (size_t)(r + M_H) * P + M_H;
+                    for (int c = ca; c < cb; c++) {
+                        const double z = in.dem[k + c];
+                        const bool act = z != in.nodata;
+                        zoff[g + c] = act ? (float)(z - dat) : nan;
+                        hbuf[g + c] = act && in.depth ? (float)in.depth[k + c] : 0.f;
+                        if (!rw && act) aw += 1.0;
+                    }
+                    if (cls)
+                        for (int c = ca; c < cb; c++) {
+                            const uint8_t cl = in.mclass[k + c];
+                            if (cl >= in.ntable) bad_class = true;
+                            cls[g + c] = cl;
+                        }
+                    if (rw)
+                        for (int c = ca; c < cb; c++) {
+                            rw[g + c] = in.rain_weight[k + c];
+                            if (in.dem[k + c] != in.nodata) aw += (double)in.rain_weight[k + c];
+                        }
                 }
-            datum[(size_t)j * tx + i] = n ? (float)(std::round(sum / n * 16.0) / 16.0) : 0.f;
-        }
-    if (in.rain_weight) rw.assign(cells, 1.f);
-    for (int r = 0; r < R; r++)
-        for (int c = 0; c < C; c++) {
-            const size_t k = (size_t)r * C + c;
-            const size_t g = (size_t)(r + M_H) * P + (c + M_H);
-            const double z = in.dem[k];
-            const bool act = z != in.nodata;
-            const double dat = datum[(size_t)(r / M_DR) * tx + (c / M_CW)];
-            if (act) zoff[g] = (float)(z - dat);
-            if (in.mclass) {
-                const uint8_t cl = in.mclass[k];
-                if (cl >= in.ntable) {
-                    if (err) *err = "Manning class out of table range";
-                    return fail_free(SW2D_ERR_INVALID);
-                }
-                cls[g] = cl;
             }
-            hbuf[g] = (act && in.depth) ? (float)in.depth[k] : 0.f;
-            if (in.rain_weight) rw[g] = in.rain_weight[k];
-            if (act) active_weight += in.rain_weight ? (double)in.rain_weight[k] : 1.0;
+            band_weight[j] = aw;
         }
-    ECK(cudaMemcpyAsync(dz, zoff.data(), cells * 4, cudaMemcpyHostToDevice, stream_));
-    if (dcls) ECK(cudaMemcpyAsync(dcls, cls.data(), cells, cudaMemcpyHostToDevice, stream_));
-    ECK(cudaMemcpyAsync(d.h[0], hbuf.data(), cells * 4, cudaMemcpyHostToDevice, stream_));
-    ECK(cudaMemcpyAsync(ddatum, datum.data(), datum.size() * 4, cudaMemcpyHostToDevice, stream_));
-    if (drw) ECK(cudaMemcpyAsync(drw, rw.data(), cells * 4, cudaMemcpyHostToDevice, stream_));
-    std::vector<double> rain(nrain + 2, 0.0);
-    for (int k = 0; k < in.nrain; k++) rain[k] = in.rain[k];
-    ECK(cudaMemcpyAsync(drain, rain.data(), rain.size() * 8, cudaMemcpyHostToDevice, stream_));
-    std::vector<double> evap, srcq;
-    std::vector<int> srcc;
-    if (devap) {
-        evap.assign((size_t)in.nevap + 2, 0.0);
-        for (int k = 0; k < in.nevap; k++) evap[k] = in.evap[k];
-        ECK(cudaMemcpyAsync(devap, evap.data(), evap.size() * 8, cudaMemcpyHostToDevice, stream_));
+    });
+    if (bad_class) {
+        if (err) *err = "Manning class out of table range";
+        return fail_free(SW2D_ERR_INVALID);
     }
+    double active_weight = 0.0;
+    for (double w : band_weight) active_weight += w;
+    auto series = [&](size_t o, const double* v, int n, size_t total) {
+        double* t = (double*)(stage + o);
+        std::fill(t, t + total, 0.0);
+        for (int k = 0; k < n; k++) t[k] = v[k];
+    };
+    series(o_rain, in.rain, in.nrain, (size_t)nrain + 2);
+    if (has_evap) series(o_evap, in.evap, in.nevap, (size_t)in.nevap + 2);
     if (nu > 0) {
-        srcq.assign((size_t)(in.nq + 2) * nu, 0.0);
+        int* cellv = (int*)(stage + o_srcc);
+        double* q = (double*)(stage + o_srcq);
+        std::fill(q, q + (size_t)(in.nq + 2) * nu, 0.0);
         for (int u = 0; u < nu; u++) {
-            srcc.push_back(in.src_cells[src_keep[u]]);
-            for (int t = 0; t < in.nq; t++) srcq[(size_t)t * nu + u] = in.src_q[(size_t)t * in.nsrc + src_keep[u]];
+            cellv[u] = in.src_cells[src_keep[u]];
+            for (int t = 0; t < in.nq; t++) q[(size_t)t * nu + u] = in.src_q[(size_t)t * in.nsrc + src_keep[u]];
         }
-        ECK(cudaMemcpyAsync(dsrc_cell, srcc.data(), srcc.size() * 4, cudaMemcpyHostToDevice, stream_));
-        ECK(cudaMemcpyAsync(dsrcq, srcq.data(), srcq.size() * 8, cudaMemcpyHostToDevice, stream_));
     }
+    {
+        Clock32 c{};
+        c.t = in.t0;
+        c.t_end = in.t_end;
+        std::memcpy(stage + o_clk, &c, sizeof c);
+    }
+    ACK(cudaMemcpyAsync(slab, stage, staged, cudaMemcpyHostToDevice, stream_));
 
     /* tensor maps: rows of 232 columns, four rows per staged block; the bed
      * reads NaN (inactive) outside the array */
@@ -341,7 +399,7 @@ int Engine32::add(const ScenarioInput& in, long long id, std::string* err, int* 
     d.series_mode = in.series_mode;
     d.dt_mode = in.dt_mode;
     d.nrain = nrain;
-    d.nevap = devap ? in.nevap : 0;
+    d.nevap = has_evap ? in.nevap : 0;
     d.nsrc = nu;
     d.nq = nu > 0 ? in.nq : 0;
     d.dtoq = nu > 0 ? in.dtoq : 3600.0;
@@ -356,7 +414,7 @@ int Engine32::add(const ScenarioInput& in, long long id, std::string* err, int* 
     d.pct_lake = (float)pct_lake;
     d.pct_land = (float)pct_land;
     d.ev_wl_min = (float)in.ev_wl_min;
-    d.ledger_cells = pct_lake != pct_land || devap != nullptr; /* evaporation acts on lake cells only */
+    d.ledger_cells = pct_lake != pct_land || has_evap; /* evaporation acts on lake cells only */
     d.rain_static = active_weight * pct_land;
     d.dxd = in.dx;
     d.dyd = in.dy;
@@ -367,28 +425,47 @@ int Engine32::add(const ScenarioInput& in, long long id, std::string* err, int* 
     d.area = in.dx * in.dy;
     for (int k = 0; k < T32_MAXCLASS; k++)
         d.ntab[k] = (float)(in.mclass ? (k < in.ntable ? in.mtable[k] : 0.0) : in.manning);
-    Clock32 c{};
-    c.t = in.t0;
-    c.t_end = in.t_end;
-    ECK(cudaMemcpyAsync(dclk, &c, sizeof c, cudaMemcpyHostToDevice, stream_));
-    ECK(cudaStreamSynchronize(stream_));
     S.t_end_default = in.t_end;
+    /* initial volume and CFL speed into the clock, then the first slot, from
+     * the scenario's own descriptor (the work lists are built when it runs) */
+    const size_t idx = scn_.size();
+    if ((rc = reserve_scn(idx + 1, err))) return fail_free(rc);
+    ACK(cudaMemcpyAsync(d_scn_ + idx, &d, sizeof d, cudaMemcpyHostToDevice, stream_));
+    fp32_launch_volume(d_scn_, (int)idx, d, d_tmp_, true, stream_);
+    fp32_launch_prime(d_scn_ + idx, 1, nullptr, stream_);
+    ACK(cudaStreamSynchronize(stream_)); /* the staging copy is the next scenario's */
+    ACK(cudaGetLastError());
+#undef ACK
     scn_.push_back(std::move(sp));
-    const int idx = (int)scn_.size() - 1;
     dirty_ = true;
-    if ((rc = rebuild(err))) return rc;
-    /* initial volume and CFL speed, then the first slot */
-    fp32_launch_volume(d_scn_, idx, scn_[idx]->d, d_tmp_, stream_);
-    double vs[2];
-    ECK(cudaMemcpyAsync(vs, d_tmp_, 2 * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-    ECK(cudaStreamSynchronize(stream_));
-    c.volume0 = vs[0];
-    c.s_max = vs[1];
-    ECK(cudaMemcpyAsync(dclk, &c, sizeof c, cudaMemcpyHostToDevice, stream_));
-    fp32_launch_prime(d_scn_ + idx, 1, stream_);
-    ECK(cudaStreamSynchronize(stream_));
-    ECK(cudaGetLastError());
-    if (index_out) *index_out = idx;
+    if (index_out) *index_out = (int)idx;
+    return SW2D_OK;
+}
+
+int Engine32::reserve_pin(size_t bytes, std::string* err) {
+    if (pin_bytes_ >= bytes) return SW2D_OK;
+    if (pin_) cudaFreeHost(pin_);
+    pin_ = nullptr;
+    pin_bytes_ = 0;
+    ECK(cudaMallocHost(&pin_, bytes));
+    pin_bytes_ = bytes;
+    return SW2D_OK;
+}
+
+/* room for n descriptors; those on the device are lost when it grows (the
+ * next rebuild uploads them all) */
+int Engine32::reserve_scn(size_t n, std::string* err) {
+    if (n <= d_scn_cap_) return SW2D_OK;
+    const size_t cap = std::max(n, 2 * d_scn_cap_);
+    cudaFree(d_scn_);
+    cudaFree(d_stat_);
+    d_scn_ = nullptr;
+    d_stat_ = nullptr;
+    d_scn_cap_ = 0;
+    dirty_ = true;
+    ECK(cudaMalloc(&d_scn_, cap * sizeof(Scn32)));
+    ECK(cudaMalloc(&d_stat_, cap * sizeof(Status32)));
+    d_scn_cap_ = cap;
     return SW2D_OK;
 }
 
@@ -396,7 +473,7 @@ int Engine32::remove(int index) {
     if (index < 0 || index >= (int)scn_.size()) return SW2D_ERR_INVALID;
     cudaSetDevice(device_);
     cudaStreamSynchronize(stream_);
-    for (void* p : scn_[index]->allocs) cudaFree(p);
+    cudaFree(scn_[index]->slab);
     scn_.erase(scn_.begin() + index);
     dirty_ = true;
     return SW2D_OK;
@@ -482,12 +559,8 @@ int Engine32::rebuild(std::string* err) {
         std::stable_sort(work_.begin() + class_first_[k], work_.end(),
                          [&](const int4& a, const int4& b) { return rows_of(a) > rows_of(b); });
     }
-    if (host.size() > d_scn_cap_) {
-        cudaFree(d_scn_);
-        d_scn_ = nullptr;
-        d_scn_cap_ = std::max<size_t>(host.size(), 2 * d_scn_cap_);
-        ECK(cudaMalloc(&d_scn_, d_scn_cap_ * sizeof(Scn32)));
-    }
+    int rc = reserve_scn(host.size(), err);
+    if (rc) return rc;
     if (work_.size() > d_work_cap_) {
         cudaFree(d_work_);
         cudaFree(d_part_);
@@ -508,10 +581,6 @@ int Engine32::rebuild(std::string* err) {
     if (!work_.empty())
         ECK(cudaMemcpyAsync(d_work_, work_.data(), work_.size() * sizeof(int4), cudaMemcpyHostToDevice, stream_));
     ECK(cudaStreamSynchronize(stream_));
-    if (graph_) {
-        cudaGraphExecDestroy(graph_);
-        graph_ = nullptr;
-    }
     dirty_ = false;
     return SW2D_OK;
 }
@@ -534,28 +603,6 @@ int Engine32::launch(int niter, std::string* err) {
     return SW2D_OK;
 }
 
-int Engine32::build_graph(std::string* err) {
-    if (graph_ || graph_failed_) return SW2D_OK;
-    cudaGraph_t g = nullptr;
-    ECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    int grid[T32_NCLASS];
-    for (int k = 0; k < T32_NCLASS; k++) grid[k] = grid_of(k);
-    cudaError_t el = fp32_launch_chunk(d_scn_, (int)scn_.size(), d_work_, class_first_, class_n_, d_part_, d_ctl_, kChunk,
-                                       grid, stream_);
-    cudaError_t ec = cudaStreamEndCapture(stream_, &g);
-    cudaError_t ei = cudaErrorUnknown;
-    if (el == cudaSuccess && ec == cudaSuccess && g) ei = cudaGraphInstantiate(&graph_, g, 0);
-    if (g) cudaGraphDestroy(g);
-    if (ei != cudaSuccess) {
-        /* a cooperative launch the capture could not take: the chunks are
-         * launched directly (one launch per 32 iterations either way) */
-        graph_ = nullptr;
-        graph_failed_ = true;
-        cudaGetLastError();
-    }
-    return SW2D_OK;
-}
-
 int Engine32::tune(long long budget, std::string* err, long long* advanced) {
     *advanced = 0;
     double cells = 0;
@@ -568,7 +615,7 @@ int Engine32::tune(long long budget, std::string* err, long long* advanced) {
         if (seg != seg_ || cps != cps_) {
             seg_ = seg;
             cps_ = cps;
-            dirty_ = true; /* new work items, and the chunk graph holds the grid */
+            dirty_ = true; /* new work items */
             return rebuild(err);
         }
         return (int)SW2D_OK;
@@ -628,18 +675,13 @@ int Engine32::tune_now(long long budget, std::string* err, long long* advanced) 
 
 int Engine32::set_t_end(int index, double t_end, std::string* err) {
     ECK(cudaSetDevice(device_));
-    for (int i = 0; i < (int)scn_.size(); i++) {
-        if (index >= 0 && i != index) continue;
-        ECK(cudaMemcpyAsync(&scn_[i]->d.clk->t_end, &t_end, sizeof(double), cudaMemcpyHostToDevice, stream_));
-        ECK(cudaStreamSynchronize(stream_));
-    }
     int rc = rebuild(err);
     if (rc) return rc;
     if (index >= 0)
-        fp32_launch_prime(d_scn_ + index, 1, stream_);
+        fp32_launch_prime(d_scn_ + index, 1, &t_end, stream_);
     else if (!scn_.empty())
-        fp32_launch_prime(d_scn_, (int)scn_.size(), stream_);
-    ECK(cudaStreamSynchronize(stream_));
+        fp32_launch_prime(d_scn_, (int)scn_.size(), &t_end, stream_);
+    ECK(cudaGetLastError());
     return SW2D_OK;
 }
 
@@ -651,13 +693,8 @@ int Engine32::run(long long n, std::string* err) {
     ECK(cudaEventRecord(ev_a_, stream_));
     long long done = 0;
     if ((rc = tune(n, err, &done))) return rc;
-    if ((rc = build_graph(err))) return rc;
-    for (; n - done >= kChunk; done += kChunk) {
-        if (graph_)
-            ECK(cudaGraphLaunch(graph_, stream_));
-        else if ((rc = launch(kChunk, err)))
-            return rc;
-    }
+    for (; n - done >= kChunk; done += kChunk)
+        if ((rc = launch(kChunk, err))) return rc;
     if (n > done && (rc = launch((int)(n - done), err))) return rc;
     ECK(cudaGetLastError());
     ECK(cudaEventRecord(ev_b_, stream_));
@@ -680,6 +717,17 @@ int Engine32::get_clock(int index, Clock32* out, std::string* err) {
     return SW2D_OK;
 }
 
+int Engine32::get_status(std::vector<Status32>* out, std::string* err) {
+    out->resize(scn_.size());
+    if (scn_.empty()) return SW2D_OK;
+    int rc = rebuild(err);
+    if (rc) return rc;
+    fp32_launch_status(d_scn_, (int)scn_.size(), d_stat_, stream_);
+    ECK(cudaMemcpyAsync(out->data(), d_stat_, scn_.size() * sizeof(Status32), cudaMemcpyDeviceToHost, stream_));
+    ECK(cudaStreamSynchronize(stream_));
+    return SW2D_OK;
+}
+
 int Engine32::get_state(int index, double* depth, double* qx, double* qy, std::string* err) {
     Scenario32& S = *scn_[index];
     Clock32 c;
@@ -687,39 +735,41 @@ int Engine32::get_state(int index, double* depth, double* qx, double* qy, std::s
     if (rc) return rc;
     const int cur = c.slot.cur;
     const int R = S.R, C = S.C, P = S.P;
+    struct Field {
+        const float* src;
+        int rows, cols;
+        double* dst;
+    } f[3] = {{S.d.h[cur], R, C, depth}, {S.d.qx[cur], R + 1, C, qx}, {S.d.qy[cur], R, C + 1, qy}};
     /* whole padded rows into pinned staging (a copy into pageable memory runs
-     * at a few GB/s), then the interior widened to binary64 on host threads */
-    const size_t need = (size_t)(R + 1) * P * sizeof(float);
-    if (pin_bytes_ < need) {
-        if (pin_) cudaFreeHost(pin_);
-        pin_ = nullptr;
-        pin_bytes_ = 0;
-        ECK(cudaMallocHost(&pin_, need));
-        pin_bytes_ = need;
-    }
-    auto fetch = [&](const float* src, int rows, int cols, double* dst) -> int {
-        ECK(cudaMemcpyAsync(pin_, src + (size_t)M_H * P, (size_t)rows * P * sizeof(float), cudaMemcpyDeviceToHost,
-                            stream_));
-        ECK(cudaStreamSynchronize(stream_));
-        const float* s = static_cast<const float*>(pin_) + M_H;
-        const size_t nt = std::max<size_t>(1, std::min<size_t>({16, std::thread::hardware_concurrency(),
-                                                                (size_t)rows / 64 + 1}));
-        std::vector<std::thread> th;
-        const size_t per = ((size_t)rows + nt - 1) / nt;
-        for (size_t t = 0; t < nt; t++) {
-            const size_t a = t * per, b = std::min((size_t)rows, a + per);
-            if (a >= b) continue;
-            th.emplace_back([=] {
-                for (size_t r = a; r < b; r++)
-                    for (int k = 0; k < cols; k++) dst[r * cols + k] = s[r * P + k];
-            });
-        }
-        for (auto& x : th) x.join();
-        return SW2D_OK;
+     * at a few GB/s), all fields of a small raster at once, then the interior
+     * widened to binary64 on host threads */
+    const size_t one = (size_t)(R + 1) * P * sizeof(float);
+    const bool together = 3 * one <= ((size_t)16 << 20);
+    if ((rc = reserve_pin(together ? 3 * one : one, err))) return rc;
+    auto fetch = [&](const Field& x, char* to) {
+        return cudaMemcpyAsync(to, x.src + (size_t)M_H * P, (size_t)x.rows * P * sizeof(float), cudaMemcpyDeviceToHost,
+                               stream_);
     };
-    if (depth && (rc = fetch(S.d.h[cur], R, C, depth))) return rc;
-    if (qx && (rc = fetch(S.d.qx[cur], R + 1, C, qx))) return rc;
-    if (qy && (rc = fetch(S.d.qy[cur], R, C + 1, qy))) return rc;
+    auto widen = [&](const Field& x, const char* from) {
+        const float* s = reinterpret_cast<const float*>(from) + M_H;
+        on_threads((size_t)x.rows, (size_t)x.rows * x.cols, (size_t)1 << 18, [=](size_t a, size_t b) {
+            for (size_t r = a; r < b; r++)
+                for (int k = 0; k < x.cols; k++) x.dst[r * x.cols + k] = s[r * P + k];
+        });
+    };
+    char* const base = static_cast<char*>(pin_);
+    for (int k = 0; k < 3; k++) {
+        if (!f[k].dst) continue;
+        ECK(fetch(f[k], together ? base + k * one : base));
+        if (together) continue;
+        ECK(cudaStreamSynchronize(stream_));
+        widen(f[k], base);
+    }
+    if (together) {
+        ECK(cudaStreamSynchronize(stream_));
+        for (int k = 0; k < 3; k++)
+            if (f[k].dst) widen(f[k], base + k * one);
+    }
     return SW2D_OK;
 }
 
@@ -770,7 +820,7 @@ int Engine32::restore(int index, const void* buf, std::string* err) {
 int Engine32::get_volume(int index, double* vol, double* smax, std::string* err) {
     int rc = rebuild(err);
     if (rc) return rc;
-    fp32_launch_volume(d_scn_, index, scn_[index]->d, d_tmp_, stream_);
+    fp32_launch_volume(d_scn_, index, scn_[index]->d, d_tmp_, false, stream_);
     double vs[2];
     ECK(cudaMemcpyAsync(vs, d_tmp_, 2 * sizeof(double), cudaMemcpyDeviceToHost, stream_));
     ECK(cudaStreamSynchronize(stream_));

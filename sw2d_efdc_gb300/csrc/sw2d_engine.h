@@ -56,7 +56,7 @@ struct Scenario32 {
     Scn32 d{};                 /* host copy of the device descriptor */
     int R = 0, C = 0, P = 0, NR = 0;
     size_t bytes = 0;          /* device bytes held */
-    std::vector<void*> allocs;
+    void* slab = nullptr;      /* all its device arrays */
     double t_end_default = 0.0;
     long long id = -1;
     bool finished = false;
@@ -73,13 +73,15 @@ class Engine32 {
     int remove(int index);
     int count() const { return (int)scn_.size(); }
     Scenario32& at(int i) { return *scn_[i]; }
-    /* set every scenario's t_end (or one) and recompute first slots */
+    /* set every scenario's t_end (or one) and recompute first slots (in stream order) */
     int set_t_end(int index, double t_end, std::string* err);
     /* run n iterations of every scenario (finished ones idle) */
     int run(long long n, std::string* err);
     /* state of one scenario, reference orientation */
     int get_state(int index, double* depth, double* qx, double* qy, std::string* err);
     int get_clock(int index, Clock32* out, std::string* err);
+    /* iterations, done and status of every scenario */
+    int get_status(std::vector<Status32>* out, std::string* err);
     int get_volume(int index, double* vol, double* smax, std::string* err);
     int get_outlet(int index, double* t, double* q, int cap, int* count, std::string* err);
     /* the scenario's device state (clock, then depth, x and y discharges and
@@ -141,7 +143,8 @@ class Engine32 {
   private:
     int rebuild(std::string* err);
     int fill_rows(int k) const;
-    int build_graph(std::string* err);
+    int reserve_pin(size_t bytes, std::string* err);
+    int reserve_scn(size_t n, std::string* err);
     int launch(int niter, std::string* err);
     /* the autotuner: times each candidate pair (most rows per item, CTAs per
      * SM) on the scenarios' own iterations -- one untimed, then up to a
@@ -158,7 +161,8 @@ class Engine32 {
     std::vector<int4> work_;
     int class_first_[T32_NCLASS] = {}, class_n_[T32_NCLASS] = {}; /* work ranges per feature class */
     Scn32* d_scn_ = nullptr;
-    size_t d_scn_cap_ = 0;
+    Status32* d_stat_ = nullptr;
+    size_t d_scn_cap_ = 0;     /* descriptors (and status entries) there is room for */
     int4* d_work_ = nullptr;
     size_t d_work_cap_ = 0;
     Part32* d_part_ = nullptr;
@@ -166,8 +170,6 @@ class Engine32 {
     size_t d_ctl_cap_ = 0;
     double* d_tmp_ = nullptr;
     bool dirty_ = true;
-    cudaGraphExec_t graph_ = nullptr;
-    bool graph_failed_ = false; /* capture of the cooperative launch refused: launch directly */
     cudaEvent_t ev_a_ = nullptr, ev_b_ = nullptr, ev_t0_ = nullptr, ev_t1_ = nullptr;
     double last_ms_ = 0.0;
     long long last_iters_ = 0;
@@ -178,7 +180,7 @@ class Engine32 {
     std::map<int, std::pair<int, int>> tuned_; /* size bucket -> (rows per item, CTAs per SM) */
     double tuning_ms_ = 0.0;
     int tunings_ = 0;
-    void* pin_ = nullptr;      /* pinned staging of state downloads */
+    void* pin_ = nullptr;      /* pinned staging of inputs and state downloads */
     size_t pin_bytes_ = 0;
 };
 

@@ -1020,13 +1020,24 @@ __global__ void __launch_bounds__(NT, 4) k32_persist(const Scn32* __restrict__ s
 }
 
 /* first slot of every scenario from its clock (t, s_max, t_end), one warp each */
-__global__ void k32_prime(const Scn32* __restrict__ scns, int nscn) {
+__global__ void k32_prime(const Scn32* __restrict__ scns, int nscn, int set_end, double t_end) {
     const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (s >= nscn) return;
     Clock32* clk = scns[s].clk;
-    if ((threadIdx.x & 31) == 0) clk->done = 0;
+    const double te = set_end ? t_end : clk->t_end;
+    if ((threadIdx.x & 31) == 0) {
+        clk->done = 0;
+        clk->t_end = te;
+    }
     __syncwarp();
-    prepare_slot32(scns[s], clk, clk->t, clk->t_end, clk->s_max);
+    prepare_slot32(scns[s], clk, clk->t, te, clk->s_max);
+}
+
+__global__ void k32_status(const Scn32* __restrict__ scns, int nscn, Status32* __restrict__ out) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nscn) return;
+    const Clock32* clk = scns[s].clk;
+    out[s] = Status32{clk->iters, clk->done, clk->status};
 }
 
 /* volume = sum of (h - kc) over active cells, and the CFL face speed of the
@@ -1097,7 +1108,7 @@ __global__ void __launch_bounds__(256) k32_volume_part(const Scn32* __restrict__
 }
 
 __global__ void __launch_bounds__(1024) k32_volume_fin(const Scn32* __restrict__ scns, int iscn,
-                                                       const VolPart* __restrict__ part, int n, double* out) {
+                                                       const VolPart* __restrict__ part, int n, int init, double* out) {
     const Scn32& P = scns[iscn];
     double vol = 0.0;
     float sx = 0.f, sy = 0.f;
@@ -1110,6 +1121,10 @@ __global__ void __launch_bounds__(1024) k32_volume_fin(const Scn32* __restrict__
     if (threadIdx.x == 0) {
         out[0] = vol * P.area;
         out[1] = (double)sx + (double)sy;
+        if (init) {
+            P.clk->volume0 = out[0];
+            P.clk->s_max = out[1];
+        }
     }
 }
 
@@ -1233,15 +1248,19 @@ cudaError_t fp32_launch_chunk(const Scn32* d_scn, int nscn, const int4* d_work, 
     return cudaSuccess;
 }
 
-void fp32_launch_prime(const Scn32* d_scn, int nscn, cudaStream_t s) {
-    k32_prime<<<(nscn + 3) / 4, 128, 0, s>>>(d_scn, nscn);
+void fp32_launch_prime(const Scn32* d_scn, int nscn, const double* t_end, cudaStream_t s) {
+    k32_prime<<<(nscn + 3) / 4, 128, 0, s>>>(d_scn, nscn, t_end ? 1 : 0, t_end ? *t_end : 0.0);
 }
 
-void fp32_launch_volume(const Scn32* d_scn, int iscn, const Scn32& host_scn, double* d_out, cudaStream_t s) {
+void fp32_launch_status(const Scn32* d_scn, int nscn, Status32* out, cudaStream_t s) {
+    k32_status<<<(nscn + 127) / 128, 128, 0, s>>>(d_scn, nscn, out);
+}
+
+void fp32_launch_volume(const Scn32* d_scn, int iscn, const Scn32& host_scn, double* d_out, bool init, cudaStream_t s) {
     const int nb = std::max(1, std::min(host_scn.R, kVolBlocks));
     VolPart* part = reinterpret_cast<VolPart*>(reinterpret_cast<char*>(d_out) + 32);
     k32_volume_part<<<nb, 256, 0, s>>>(d_scn, iscn, part);
-    k32_volume_fin<<<1, 1024, 0, s>>>(d_scn, iscn, part, nb, d_out);
+    k32_volume_fin<<<1, 1024, 0, s>>>(d_scn, iscn, part, nb, init ? 1 : 0, d_out);
 }
 
 } // namespace sw2d

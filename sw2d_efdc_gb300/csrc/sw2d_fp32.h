@@ -137,10 +137,18 @@ cudaError_t fp32_launch_chunk(const Scn32* d_scn, int nscn, const int4* d_work, 
                               cudaStream_t s);
 /* CTAs of class k's persistent kernel one SM holds */
 int fp32_blocks_per_sm(int k);
-void fp32_launch_prime(const Scn32* d_scn, int nscn, cudaStream_t s);
-/* volume and CFL speed of one scenario into d_out[0..1]; d_out holds
- * fp32_volume_scratch_bytes() (the partials follow the two results) */
-void fp32_launch_volume(const Scn32* d_scn, int iscn, const Scn32& host_scn, double* d_out, cudaStream_t s);
+/* first slots from the scenarios' clocks, whose end time *t_end replaces first (unless NULL) */
+void fp32_launch_prime(const Scn32* d_scn, int nscn, const double* t_end, cudaStream_t s);
+/* volume and CFL speed of one scenario into d_out[0..1] and, with init, into
+ * its clock as those it starts from; d_out holds fp32_volume_scratch_bytes()
+ * (the partials follow the two results) */
+void fp32_launch_volume(const Scn32* d_scn, int iscn, const Scn32& host_scn, double* d_out, bool init, cudaStream_t s);
+/* what the host asks of a running scenario between steps */
+struct Status32 {
+    long long iters;
+    int done, status;
+};
+void fp32_launch_status(const Scn32* d_scn, int nscn, Status32* out, cudaStream_t s);
 size_t fp32_volume_scratch_bytes();
 /* boundary-discharge sample of one scenario (device descriptor d_scn_one):
  * faces holds (raster cell r*cols+c, side) pairs; q and vel_prev nfaces

@@ -38,6 +38,7 @@
 #include "sw2d_math.h"
 
 #include <algorithm>
+#include <climits>
 
 namespace sw2d {
 
@@ -901,10 +902,37 @@ __global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int g
     }
 }
 
+__device__ __forceinline__ void report(const StepParams& p) {
+    const DevClock* clk = p.clk;
+    Flight64::Report& o = p.flight->report;
+    o.iters = clk->iters;
+    o.t = clk->t;
+    o.dt2 = clk->slot[0].dt2;
+    o.active = clk->slot[0].active;
+    o.status = clk->status;
+}
+
 __global__ void __launch_bounds__(SW2D_BX * SW2D_BY) k64_settle(StepParams p, int gx, int gy,
                                                                      int last_row) {
     settle_ledger(p, 0, gx, gy, last_row); /* the last iteration is of one parity; the other has nothing to add */
     settle_ledger(p, 1, gx, gy, last_row);
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        p.clk->iter_end = LLONG_MAX;
+        report(p);
+    }
+}
+
+__global__ void __launch_bounds__(32) k64_begin(StepParams p, double t_end, long long limit) {
+    DevClock* clk = p.clk;
+    const long long iters = clk->iters, end = limit < 0 ? LLONG_MAX : iters + limit;
+    prepare_slot(p, &clk->slot[0], clk->t, clk->s_max, iters < end ? t_end : clk->t);
+    __syncwarp();
+    if (threadIdx.x == 0) {
+        clk->t_end = t_end;
+        clk->iter_end = end;
+        p.flight->report.iters0 = iters;
+        report(p);
+    }
 }
 
 /* Volume (sum of h over active cells) and, with full, the CFL speed of the
@@ -1156,6 +1184,10 @@ void fp64_launch_iteration(const StepParams& p, int cur, cudaStream_t s, cudaEve
 void fp64_launch_settle(const StepParams& p, cudaStream_t s) {
     const Cut64 k = cut_of(p.R, p.C);
     k64_settle<<<1, SW2D_BX * SW2D_BY, 0, s>>>(p, k.gx, k.gy, (p.R - 1) / k.th);
+}
+
+void fp64_launch_begin(const StepParams& p, double t_end, long long limit, cudaStream_t s) {
+    k64_begin<<<1, 32, 0, s>>>(p, t_end, limit);
 }
 
 void fp64_launch_prime(const StepParams& p, int cur, int full, cudaStream_t s) {

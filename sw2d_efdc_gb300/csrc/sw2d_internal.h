@@ -76,6 +76,12 @@ struct Flight64 {
         double dt2, rr2, ev2, t_next, src;
         long long pending; /* the iteration's ledger sums are not added yet */
     } sums[2];
+    /* what the host asks between launches, written by k64_begin and k64_settle */
+    struct Report {
+        long long iters0, iters; /* at the run's start, now */
+        double t, dt2;           /* now, and the next iteration's length */
+        int active, status;      /* of the next iteration, so far */
+    } report;
 };
 
 /* Everything a step kernel needs, passed by value. */
@@ -119,8 +125,12 @@ struct StepParams {
 /* FP64 step kernels (sw2d_fp64.cu) */
 size_t fp64_partials(int rows, int cols); /* doubles the partials of a raster of this size take */
 void fp64_launch_iteration(const StepParams& p, int cur, cudaStream_t s, cudaEvent_t* ev);
-/* after the last iteration of a run: its ledger sums */
+/* before the first iteration of a run: its end time, its iteration limit
+ * (< 0: none) and the first slot */
+void fp64_launch_begin(const StepParams& p, double t_end, long long limit, cudaStream_t s);
+/* after the last iteration of a launch: its ledger sums; lifts the limit */
 void fp64_launch_settle(const StepParams& p, cudaStream_t s);
+/* full = 0: recompute the next iteration's slot; 1: volume; 2: initial state */
 void fp64_launch_prime(const StepParams& p, int cur, int full, cudaStream_t s);
 void fp64_launch_face_velocity(const StepParams& p, int cur, cudaStream_t s);
 void fp64_launch_cell_velocity(const StepParams& p, int cur, double* uu, double* vv, double* uua,
