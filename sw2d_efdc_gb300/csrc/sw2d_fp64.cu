@@ -329,6 +329,14 @@ __device__ __forceinline__ bool mean_ge(double ha, double hb, int ca, int cb, fl
     return mean_ge_exact(ha, hb, th);
 }
 
+/* Every kernel of an iteration is launched with programmatic serialisation:
+ * its blocks may be set up while the one before drains, and wait here for it
+ * to be complete and its writes visible.  (Letting them come earlier, by an
+ * explicit trigger, measured 11.1 against 11.6 us an iteration at 33 x 41 but
+ * 21.1 against 19.5 at 256 x 256, where they take the place of running blocks;
+ * plain launches 12.1 and 20.0.) */
+__device__ __forceinline__ void after_previous() { cudaGridDependencySynchronize(); }
+
 /* The new discharges of the faces of a 32 x BY block of cells (north and
  * west face of each), four block barriers:
  *   1  the block and a ring around it staged in shared memory; the surface
@@ -366,6 +374,7 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
     const int c0 = blockIdx.x * BX, r0 = blockIdx.y * BY;
     const int c = c0 + tx, r = r0 + ty;
     const Slot& s = p.clk->slot[cur];
+    after_previous();
     const double dt2 = s.dt2, dt2dx = s.dt2dx, dt2dy = s.dt2dy;
     const int active = s.active;
     const int P = p.P, R = p.R, C = p.C;
@@ -734,11 +743,13 @@ __device__ __forceinline__ uint8_t provisional_dry(const StepParams& p, float dt
  * be the longest part of a small raster's iteration).
  * Bounded by the binary64 additions and products of the final depth and of
  * the face means (71 issue cycles a warp each; the flags take none) and by
- * the latencies between them: six blocks an SM (40 registers, 40 bytes of
- * spills) against four measured 613 against 730 us at 4096 x 4096. */
+ * the latencies between them: large tiles run eight blocks an SM (32
+ * registers, up to 80 bytes of spills), 438 us at 4096 x 4096 against 472 and
+ * 511 with six and five. */
 template <int TW, int TH, int NT, bool FULL>
-__global__ void __launch_bounds__(NT, 6) k64_update(StepParams p, int cur, int gx, int gy) {
+__global__ void __launch_bounds__(NT, TH >= 16 && !FULL ? 8 : 6) k64_update(StepParams p, int cur, int gx, int gy) {
     constexpr int DW = TW + 3, DH = TH + 3, NW = TW + 1, NH = TH + 1;
+    after_previous();
     if (blockIdx.x < 2) {
         if (blockIdx.x == 0) advance_clock(p, cur);
         else settle_ledger(p, cur ^ 1, gx, gy, (p.R - 1) / TH);
@@ -1158,21 +1169,35 @@ size_t fp64_partials(int rows, int cols) {
     return NPART * std::max(prime, (size_t)2 * k.gx * k.gy);
 }
 
+template <typename... A>
+static void chain_launch(void (*k)(A...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, args...); /* an error stays for the caller's cudaGetLastError */
+}
+
 template <bool FULL>
 static void launch_update(const Cut64& k, int n, const StepParams& p, int cur, cudaStream_t s) {
-    if (k.kind == 0) k64_update<64, 16, 256, FULL><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
-    else if (k.kind == 1) k64_update<32, 16, 256, FULL><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
-    else if (k.kind == 2) k64_update<32, 8, 256, FULL><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
-    else k64_update<32, 4, 256, FULL><<<n, 256, 0, s>>>(p, cur, k.gx, k.gy);
+    if (k.kind == 0) chain_launch(k64_update<64, 16, 256, FULL>, dim3(n), dim3(256), s, p, cur, k.gx, k.gy);
+    else if (k.kind == 1) chain_launch(k64_update<32, 16, 256, FULL>, dim3(n), dim3(256), s, p, cur, k.gx, k.gy);
+    else if (k.kind == 2) chain_launch(k64_update<32, 8, 256, FULL>, dim3(n), dim3(256), s, p, cur, k.gx, k.gy);
+    else chain_launch(k64_update<32, 4, 256, FULL>, dim3(n), dim3(256), s, p, cur, k.gx, k.gy);
 }
 
 void fp64_launch_iteration(const StepParams& p, int cur, cudaStream_t s, cudaEvent_t* ev) {
     const Cut64 k = cut_of(p.R, p.C);
     if (ev) cudaEventRecord(ev[0], s);
     const dim3 blk(SW2D_BX, 8);
-    if (k.by == 4) k64_flux<4, 256, 5><<<k.flux, blk, 0, s>>>(p, cur);
-    else if (k.kind > 0) k64_flux<8, 256, 5><<<k.flux, blk, 0, s>>>(p, cur);
-    else k64_flux<8, 256, 6><<<k.flux, blk, 0, s>>>(p, cur);
+    if (k.by == 4) chain_launch(k64_flux<4, 256, 5>, k.flux, blk, s, p, cur);
+    else if (k.kind > 0) chain_launch(k64_flux<8, 256, 5>, k.flux, blk, s, p, cur);
+    else chain_launch(k64_flux<8, 256, 7>, k.flux, blk, s, p, cur);
     if (ev) cudaEventRecord(ev[1], s);
     const int n = k.gx * k.gy + 2;
     const bool full = p.evap || p.nsrc > 0 || p.ledger_cells;
