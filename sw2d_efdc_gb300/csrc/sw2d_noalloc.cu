@@ -27,7 +27,7 @@ namespace {
 
 constexpr int kTile = SW2D_NOALLOC_TILE;              /* 32 x 32 cells per CTA */
 constexpr int kMaxTiles = SW2D_NOALLOC_MAX_TILES;
-constexpr int kBand = 32;                             /* rows of a warp's task */
+constexpr int kBand = 32;                             /* most rows of a warp's task */
 constexpr int kBatch = 4;                             /* of them read at once */
 constexpr int kBlocksPerSm = 3;
 constexpr int kSlots = 3;
@@ -83,9 +83,10 @@ struct MeasureIn {
     int R, C;
     double nodata, th, g, rdx, rdy, area;
     float thf, gf, rdxf, rdyf;
+    int band; /* rows of a warp's task */
 };
 
-/* A warp takes tasks of 32 columns x kBand rows and walks down the rows, the
+/* A warp takes tasks of 32 columns x `band` rows and walks down the rows, the
  * row above in registers, the column left of a lane's from its neighbour, so
  * each array is read once (plus the row above and the column left of a task);
  * kBatch rows are in flight at a time.  What it was bound by is the FP64
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(256, kBlocksPerSm) k64_measure_noalloc(Measure
     __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31;
     const int R = p.R, C = p.C, sx_n = (C + 31) / 32;
-    const int ntask = sx_n * ((R + kBand - 1) / kBand);
+    const int ntask = sx_n * ((R + p.band - 1) / p.band);
     const double th = p.th;
     const int64_t none = sw2d_ord(p.nodata);
     const bool any_none = p.nodata == p.nodata;
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(256, kBlocksPerSm) k64_measure_noalloc(Measure
     double vol = 0.0;
     for (int task = (blockIdx.x * 256 + tid) >> 5; task < ntask; task += gridDim.x * 8) {
         const int band = task / sx_n, c = (task - band * sx_n) * 32 + lane;
-        const int r0 = band * kBand, r1 = min(R, r0 + kBand);
+        const int r0 = band * p.band, r1 = min(R, r0 + p.band);
         const bool in = c < C, left = lane == 0 && c > 0;
         bool act_n = false;
         double h_n = 0.0;
@@ -262,12 +263,13 @@ extern "C" int sw2d_measure_state_noalloc(const double* d_dem, const double* d_d
     in.gf = (float)g;
     in.rdxf = (float)in.rdx;
     in.rdyf = (float)in.rdy;
-    int dev = 0, nsm = 0;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return cuda_fail("cudaDeviceGetAttribute", e);
-    const long long tasks = (cols + 31LL) / 32 * ((rows + kBand - 1LL) / kBand);
-    const int blocks = (int)std::min<long long>((tasks + 7) / 8, (long long)kBlocksPerSm * nsm);
+    /* fewer rows a task while the tasks would not reach every warp */
+    const int most = kBlocksPerSm * 152; /* GB300's SMs */
+    const long long strips = (cols + 31LL) / 32;
+    in.band = kBand;
+    while (in.band > kBatch && strips * ((rows + in.band - 1) / in.band) < 8LL * most) in.band /= 2;
+    const long long tasks = strips * ((rows + in.band - 1LL) / in.band);
+    const int blocks = (int)std::min<long long>((tasks + 7) / 8, most);
     k64_measure_noalloc<<<blocks, 256, 0, s>>>(in, scratch);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail("k64_measure_noalloc launch", e);
