@@ -209,11 +209,10 @@ __device__ __forceinline__ float2 edge2(float2 w, float2 q0, float2 q1) {
 
 struct Face2 {
     float2 hw, he;         /* the two cells' depths (w: north / west, e: south / east) */
-    float2 dz;             /* bed step z_e - z_w */
+    float2 dz;             /* bed step z_e - z_w, NaN unless both cells are active */
     float2 q0, u0, vt;     /* old discharge, face velocity, cross velocity at the face */
     float2 conv;           /* along + across convection, already scaled */
     float2 fr;             /* -dt2/2 * g * n_face^2 */
-    int act;               /* both cells active, per column */
 };
 
 /* Weir and dry-bed discharges of a face pair (SW2D-EFDC.cu:125-157), for the
@@ -253,7 +252,7 @@ __device__ __forceinline__ float2 face_flux2(const Face2& f, float th, float g, 
     const B2 d1a = lt2(se, 0.f);
     const B2 d1b = lt2(sub2(f.hw, f.dz), 0.f);
     const B2 d2 = lt2(mul2(sub2(f.he, f2(th)), sub2(f.hw, f2(th))), 0.f);
-    const B2 open = bits2(f.act) & wet;
+    const B2 open = act2(f.dz) & wet; /* the bed step is NaN beside an inactive cell */
     const B2 special = open & (d1a | d1b | d2);
     float2 F = sel2(andnot(open, special), fm, f2(0.f));
     if (__any_sync(0xffffffffu, any2(special))) F = sel2(special, face_special2(f, se, d1a, d1b, th, g), F);
@@ -405,14 +404,15 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
     /* register windows, slot = (row - Ls) & 3 */
     float2 H[4], DZX[4], QX[4], QY[4], U[4], UU[4], V[4], VV[4], VR[4];
     float2 HL[4], DZY[4], EX[4], GY[4], FX[4], FY[4], FYR[4];
-    int ACT[4], ACTL[4], DRY[4];
+    int ACT[4], DRY[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         H[k] = DZX[k] = QX[k] = QY[k] = U[k] = UU[k] = V[k] = VV[k] = VR[k] = f2(0.f);
         HL[k] = DZY[k] = EX[k] = GY[k] = FX[k] = FY[k] = FYR[k] = f2(0.f);
-        ACT[k] = ACTL[k] = DRY[k] = 0;
+        ACT[k] = DRY[k] = 0;
     }
     float2 Zp = f2(0.f); /* bed offsets of the row above */
+    const float nan0 = __int_as_float(0x7fffffff);
     /* datum band of the row in hand, counted from the band of the first staged
      * row; it grows by one at each band edge (rows past the last band are
      * the halo, whose bed is NaN whatever its datum) */
@@ -487,7 +487,6 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
             ACT[s0] = mask2(act2(z0));
             const float2 hl = left2(h0);
             HL[s0] = hl;
-            ACTL[s0] = leftbits(ACT[s0]);
             /* bed steps of the x face north of row L and the y faces west of
              * its cells, plus the datum step where the face crosses a datum
              * tile's edge (a band edge above row L, a strip edge west) */
@@ -501,6 +500,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
             Zp = z0;
             float2 dzy = sub2(z0, left2(z0));
             if (yedge) dzy.x += S.dband[bj][creg] - S.dband[bj][creg - 1];
+            if (lane == 0) dzy.x = nan0; /* the warp's first column has no western neighbour: no y face */
             DZY[s0] = dzy;
             /* ---- face velocities of row L (uu1 at the x face north, vv1 at the y face west) ---- */
             const float2 hm = (L == R) ? H[s1] : mul2(add2(h0, H[s1]), f2(0.5f));
@@ -514,10 +514,12 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
             UU[s0] = add2(u, ul);
             VV[s0] = add2(v, vr);
             VR[s0] = vr;
-            /* CFL face speeds (|velocity| + sqrt(g h)) of the owned faces */
+            /* CFL face speeds (|velocity| + sqrt(g h)) of the item's rows (the
+             * halo columns' faces are other items' own: the maximum over all
+             * items is the same with them) */
             if (L >= rs && L < re) {
-                const float2 cx = sel2(okm & bits2(ownm & ACT[s0] & ACT[s1]), absadd2(u, sqrt2(mul2(f2(gg), hm))), f2(0.f));
-                const float2 cy = sel2(okn & bits2(ownm & ACT[s0] & ACTL[s0]), absadd2(v, sqrt2(mul2(f2(gg), hn))), f2(0.f));
+                const float2 cx = sel2(okm & act2(dzx), absadd2(u, sqrt2(mul2(f2(gg), hm))), f2(0.f));
+                const float2 cy = sel2(okn & act2(dzy), absadd2(v, sqrt2(mul2(f2(gg), hn))), f2(0.f));
                 sxm = fmaxf(sxm, fmaxf(cx.x, cx.y));
                 sym = fmaxf(sym, fmaxf(cy.x, cy.y));
             }
@@ -533,7 +535,6 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
                 f.hw = H[s2];
                 f.he = H[s1];
                 f.dz = DZX[s1];
-                f.act = ACT[s2] & ACT[s1];
                 f.q0 = QX[s1];
                 f.u0 = U[s1];
                 f.vt = mul2(add2(VV[s1], VV[s2]), f2(0.25f));
@@ -561,7 +562,6 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
                 f.hw = HL[s1];
                 f.he = H[s1];
                 f.dz = DZY[s1];
-                f.act = ACTL[s1] & ACT[s1];
                 f.q0 = QY[s1];
                 f.u0 = V[s1];
                 f.vt = mul2(add2(UU[s1], UU[s0]), f2(0.25f));
