@@ -412,6 +412,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
         ACT[k] = DRY[k] = 0;
     }
     float2 Zp = f2(0.f); /* bed offsets of the row above */
+    float2 NC = f2(0.f); /* Manning n of row L-1 */
     const float nan0 = __int_as_float(0x7fffffff);
     /* datum band of the row in hand, counted from the band of the first staged
      * row; it grows by one at each band edge (rows past the last band are
@@ -539,13 +540,12 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
                 f.u0 = U[s1];
                 f.vt = mul2(add2(VV[s1], VV[s2]), f2(0.25f));
                 f.conv = fma2(sub2(EX[s1], EX[s2]), f2(dt2dx), mul2(mul2(sub2(GX, left2(GX)), f2(dt2dy)), colm));
-                if (has_cls) { /* face n = mean of the two cells' n; class rows L-2, L-1 at j, j+1 */
+                if (has_cls) { /* face n = mean of the two cells' n (the row above's from the last row) */
                     const unsigned char* c1 = scl + (j + 1) * M_CLSW + sc;
-                    const unsigned char* c2 = scl + j * M_CLSW + sc;
-                    const float2 nf = mul2(add2(make_float2(S.ntab[c1[0] & 63], S.ntab[c1[1] & 63]),
-                                                make_float2(S.ntab[c2[0] & 63], S.ntab[c2[1] & 63])),
-                                           f2(0.5f));
+                    const float2 n1 = make_float2(S.ntab[c1[0] & 63], S.ntab[c1[1] & 63]);
+                    const float2 nf = mul2(add2(n1, NC), f2(0.5f));
                     f.fr = mul2(mul2(nf, nf), f2(fr_scale));
+                    NC = n1;
                 } else {
                     f.fr = f2(fr_uni);
                 }
@@ -567,10 +567,8 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
                 f.vt = mul2(add2(UU[s1], UU[s0]), f2(0.25f));
                 const float2 along = mul2(sub2(EY, left2(EY)), f2(dt2dy));
                 f.conv = (rf == 0) ? along : fma2(sub2(GY[s1], GY[s2]), f2(dt2dx), along);
-                if (has_cls) { /* row L-1, columns c-1, c, c+1 (sc >= 0 and row j+1 >= 1 keep c-1 inside) */
-                    const unsigned char* c1 = scl + (j + 1) * M_CLSW + sc;
-                    const float nl = S.ntab[c1[-1] & 63], n0 = S.ntab[c1[0] & 63], n1 = S.ntab[c1[1] & 63];
-                    const float2 nf = mul2(add2(make_float2(n0, n1), make_float2(nl, n0)), f2(0.5f));
+                if (has_cls) { /* n of row L-1 and of the columns to the west */
+                    const float2 nf = mul2(add2(NC, left2(NC)), f2(0.5f));
                     f.fr = mul2(mul2(nf, nf), f2(fr_scale));
                 } else {
                     f.fr = f2(fr_uni);
