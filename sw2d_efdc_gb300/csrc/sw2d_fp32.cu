@@ -651,26 +651,23 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
                     if (r == R - 1) P.qx[nxt][g + Pp] = fS.x;
                 }
             };
-            if (r >= rs && r < re) {
-                const int dc = DRY[s3], dN = DRY[s0], dS = DRY[s2];
-                float2 fN = FX[s3], fS = FX[s2], fW = FY[s3], fE = FYR[s3];
-                if (__any_sync(0xffffffffu, (dc | dN | dS) != 0)) {
-                    /* treat_error (SW2D-EFDC.cu:695-725): no outflow from a
-                     * dry cell; a warp-uniform branch taken only near dry
-                     * cells, the finish below shared by both paths (one
-                     * copy of it per row keeps the unrolled loop small) */
-                    const int dW = leftbits(dc), dE = rightbits(dc);
-                    const B2 bc = bits2(dc), bN = bits2(dN), bS = bits2(dS), bW = bits2(dW), bE = bits2(dE);
-                    const B2 zN = (gt2(fN, 0.f) & bN) | (lt2(fN, 0.f) & bc);
-                    const B2 zS = (gt2(fS, 0.f) & bc) | (lt2(fS, 0.f) & bS);
-                    const B2 zW = (gt2(fW, 0.f) & bW) | (lt2(fW, 0.f) & bc);
-                    const B2 zE = (gt2(fE, 0.f) & bc) | (lt2(fE, 0.f) & bE);
-                    fN = sel2(zN, f2(0.f), fN);
-                    fS = sel2(zS, f2(0.f), fS);
-                    fW = sel2(zW, f2(0.f), fW);
-                    fE = sel2(zE, f2(0.f), fE);
+            if (r >= rs - 1 && r < re) {
+                /* treat_error (SW2D-EFDC.cu:695-725): no outflow from a dry
+                 * cell; a warp-uniform branch taken only near dry cells.  Each
+                 * face is closed once: the one south of row r here (it is the
+                 * north one of the next row; row rs-1 closes the item's first),
+                 * the west one by its own lane, the east one is the next
+                 * lane's west. */
+                const int dc = DRY[s3], dS = DRY[s2];
+                float2 fW = FY[s3], fE = FYR[s3];
+                if (__any_sync(0xffffffffu, (dc | dS) != 0)) {
+                    const B2 bc = bits2(dc), bS = bits2(dS), bW = bits2(leftbits(dc));
+                    const float2 fS = FX[s2];
+                    FX[s2] = sel2((gt2(fS, 0.f) & bc) | (lt2(fS, 0.f) & bS), f2(0.f), fS);
+                    fW = sel2((gt2(fW, 0.f) & bW) | (lt2(fW, 0.f) & bc), f2(0.f), fW);
+                    fE = right2(fW);
                 }
-                finish(fN, fS, fW, fE);
+                if (r >= rs) finish(FX[s3], FX[s2], fW, fE);
             }
         }
         __syncthreads(); /* every warp is done with block b */
