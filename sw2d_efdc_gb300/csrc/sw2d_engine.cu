@@ -481,17 +481,17 @@ int Engine32::remove(int index) {
 
 /* Rows per work item of class k: at most seg_, fewer where that leaves the
  * GPU idle.  An iteration of a class is modelled by what the persistent
- * kernel measures on a GB300: a CTA marches a row in 1.03 us when it has its
- * SM to itself, 1.30, 1.52 or 1.85 us beside one, two or three others, over
- * the item's rows and their six halo rows in whole blocks of M_RB, and about
- * 9.5 us go by from one iteration's last row to the next one's first.  One
- * scenario's items run in whole waves over the CTAs; several scenarios fill
- * one another's gaps.  Against items of 128 rows: 200 x 310 cells 147 -> 21 us
- * an iteration (2 rows), 1000 x 1000 152 -> 40 (14), 2048 x 2048 172 -> 92
- * (38); from about 12 M cells on, items of seg_ rows fill the GPU and the
- * halo rows decide. */
+ * kernel measures on a GB300: a CTA marches a row in 0.70 us when it has its
+ * SM to itself, 0.95, 1.19 or 1.49 us beside one, two or three others, over
+ * the item's rows and their six halo rows in whole blocks of M_RB (what goes
+ * by between iterations does not depend on the choice).  One scenario's items
+ * run in whole waves over the CTAs; several scenarios fill one another's
+ * gaps.  Measured, us an iteration: 200 x 310 cells 105 with items of 128
+ * rows, 19 with 2; 1000^2 62 with 64, 34 with 18; 2048^2 130 with 128, 76 with
+ * 38; from about 12 M cells on, items of seg_ rows fill the GPU and the halo
+ * rows decide. */
 int Engine32::fill_rows(int k) const {
-    static const double row_us[4] = {1.03, 1.30, 1.52, 1.85};
+    static const double row_us[4] = {0.70, 0.95, 1.19, 1.49};
     const int per_sm = std::max(1, cps_ > 0 ? std::min(cps_, bps_[k]) : bps_[k]);
     const int slots = per_sm * nsm_;
     std::vector<const Scn32*> in;

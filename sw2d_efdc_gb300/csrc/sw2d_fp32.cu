@@ -401,6 +401,16 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
     /* the cross convection of x faces vanishes on column 0 (SW2D-EFDC.cu:164) */
     const float2 colm = make_float2(cg == 0 ? 0.f : 1.f, cg + 1 == 0 ? 0.f : 1.f);
 
+    /* what the rows read of the descriptor, in registers: behind the rows'
+     * stores the compiler has to read it again from memory for every row
+     * (measured: 776 against 725 us an iteration at 8192 x 8192) */
+    float* const oh = P.h[nxt];
+    float* const okc = P.kc;
+    float* const oqx = P.qx[nxt];
+    float* const oqy = P.qy[nxt];
+    const bool open_south = P.outflow_south != 0;
+    const float pct_lake = P.pct_lake, pct_land = P.pct_land;
+
     /* register windows, slot = (row - Ls) & 3 */
     float2 H[4], DZX[4], QX[4], QY[4], U[4], UU[4], V[4], VV[4], VR[4];
     float2 HL[4], DZY[4], EX[4], GY[4], FX[4], FY[4], FYR[4];
@@ -552,7 +562,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
                 float2 F = face_flux2(f, th, gg, gdx);
                 if (rf == R) { /* south edge: free overfall when open (SW2D-EFDC.cu:131 law) */
                     const float2 hw = f.hw;
-                    const B2 m = bits2(P.outflow_south ? ACT[s2] : 0) & gt2(hw, th);
+                    const B2 m = bits2(open_south ? ACT[s2] : 0) & gt2(hw, th);
                     F = sel2(m, mul2(mul2(f2(0.5440f), hw), sqrt2(mul2(f2(gg), hw))), f2(0.f));
                 }
                 FX[s1] = F;
@@ -623,7 +633,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
                     clamp -= ng.x + ng.y;
                 }
                 if (LAKE) {
-                    float2 pw = sel2(lake, f2(P.pct_lake), f2(P.pct_land));
+                    float2 pw = sel2(lake, f2(pct_lake), f2(pct_land));
                     if (RW) pw = mul2(pw, wgt);
                     pw = sel2(oa, pw, f2(0.f));
                     rainacc += pw.x + pw.y;
@@ -638,17 +648,17 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
                 const float2 hout = sel2(act, make_float2(fmaxf(t.x, 0.f), fmaxf(t.y, 0.f)), f2(0.f));
                 const size_t g = (size_t)(r + M_H) * Pp + (cg + M_H);
                 if (own1) {
-                    *reinterpret_cast<float2*>(P.h[nxt] + g) = hout;
-                    *reinterpret_cast<float2*>(P.kc + g) = kc;
-                    *reinterpret_cast<float2*>(P.qx[nxt] + g) = fN;
-                    *reinterpret_cast<float2*>(P.qy[nxt] + g) = fW;
-                    if (r == R - 1) *reinterpret_cast<float2*>(P.qx[nxt] + g + Pp) = fS;
+                    *reinterpret_cast<float2*>(oh + g) = hout;
+                    *reinterpret_cast<float2*>(okc + g) = kc;
+                    *reinterpret_cast<float2*>(oqx + g) = fN;
+                    *reinterpret_cast<float2*>(oqy + g) = fW;
+                    if (r == R - 1) *reinterpret_cast<float2*>(oqx + g + Pp) = fS;
                 } else if (own0) {
-                    P.h[nxt][g] = hout.x;
-                    P.kc[g] = kc.x;
-                    P.qx[nxt][g] = fN.x;
-                    P.qy[nxt][g] = fW.x;
-                    if (r == R - 1) P.qx[nxt][g + Pp] = fS.x;
+                    oh[g] = hout.x;
+                    okc[g] = kc.x;
+                    oqx[g] = fN.x;
+                    oqy[g] = fW.x;
+                    if (r == R - 1) oqx[g + Pp] = fS.x;
                 }
             };
             if (r >= rs - 1 && r < re) {
