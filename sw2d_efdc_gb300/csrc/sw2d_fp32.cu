@@ -950,25 +950,29 @@ __device__ __noinline__ unsigned wait_ticket(unsigned q, const Scn32* __restrict
             *abort_flag = 1u;
             return ~0u;
         }
-        __nanosleep(64);
+        __nanosleep(20);
     }
     return q;
 }
 
 /* thread 0 after an item of scenario sc: count it; true when it was the
- * scenario's last of the iteration */
+ * scenario's last of the iteration.  The one atomic releases the item's state
+ * and partial (its CTA's writes, ordered before it by the barriers above) and
+ * acquires the others'; fences around a relaxed one are sequentially
+ * consistent ones and cost a round trip each. */
 __device__ __noinline__ bool count_item(const Scn32* __restrict__ scns, int nscn, int sc, Ctl32* ctl) {
     unsigned* cnt = reinterpret_cast<unsigned*>(reinterpret_cast<int*>(ctl + 1) + nscn);
-    __threadfence(); /* the item's state and partial before its count */
-    return atomicAdd(&cnt[sc], 1u) == (unsigned)scns[sc].nwork - 1u;
+    unsigned before;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(&cnt[sc]) : "memory");
+    return before == (unsigned)scns[sc].nwork - 1u;
 }
 
-/* thread 0 after the scenario's reduction: release its next iteration */
+/* thread 0 after the scenario's reduction (by its own warp): release its
+ * next iteration */
 __device__ __noinline__ void release_scenario(int nscn, int sc, int iterations_done, Ctl32* ctl) {
     int* done = reinterpret_cast<int*>(ctl + 1);
     unsigned* cnt = reinterpret_cast<unsigned*>(done + nscn);
     cnt[sc] = 0u;
-    __threadfence();
     st_release_gpu(&done[sc], iterations_done);
 }
 
@@ -1019,7 +1023,6 @@ __global__ void __launch_bounds__(NT, 4) k32_persist(const Scn32* __restrict__ s
         if (threadIdx.x == 0) S.last = count_item(scns, nscn, w.x, ctl);
         __syncthreads();
         if (__shfl_sync(0xffffffffu, S.last, 0)) {
-            __threadfence();
             finalize_scn(scns[w.x], part, S.red, S.redf);
             if (threadIdx.x == 0) release_scenario(nscn, w.x, (int)(q / (unsigned)nwork) + 1, ctl);
         }
