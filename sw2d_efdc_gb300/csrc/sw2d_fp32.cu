@@ -57,6 +57,7 @@ struct alignas(128) RwStage {
  * them launch with less shared memory (fp32_smem_bytes_variant) */
 struct SmemM {
     alignas(128) float stage[NS][NF][RB][BW];
+    ScnBody32 scn;              /* the scenario of the item in hand */
     unsigned long long bar[NS];
     float ntab[T32_MAXCLASS];
     float dband[M_MAXBANDS][3]; /* datums of the bands the item spans, strips west / own / east */
@@ -68,6 +69,8 @@ struct SmemM {
     unsigned q;                 /* queue ticket of the item in hand (~0u: leave) */
     unsigned qn;                /* the ticket drawn ahead for the next item */
     int last;                   /* this CTA finished its scenario's iteration */
+    int4 w;                     /* the item in hand */
+    int have;                   /* the scenario whose descriptor scn is (-1: none) */
     ClsStage cls[NS];
     RwStage rw[NS];
 };
@@ -289,8 +292,9 @@ template <bool CLS, bool RW, bool LAKE, bool SRC>
 __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 w, Part32* __restrict__ part,
                                            unsigned& gb) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    Clock32* clk = P.clk;
+    Clock32* const clk = reinterpret_cast<Clock32*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(S.scn.clk), 0));
     const Slot32 sl = load_slot(clk);
+    const int R = P.R, C = P.C, Pp = P.P, stall = P.stall_staging;
     if (!sl.active) {
         if (tid == 0) {
             Part32 zp = {};
@@ -299,7 +303,6 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
         return true;
     }
     const int cur = sl.cur, nxt = cur ^ 1;
-    const int R = P.R, C = P.C, Pp = P.P;
     const int strip = w.y, seg = w.z;
     const int c0 = strip * M_CW;             /* first output column of the strip */
     const int rs = seg * P.seg, re = min(rs + P.seg, R);
@@ -332,7 +335,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
         if (has_cls) tma_load_2d(&S.cls[st].v[0][0], &P.tm_cls, c0, y - 2, &S.bar[st]);
         if (has_rw) tma_load_2d(&S.rw[st].v[0][0], &P.tm_rw, c0, y - 3, &S.bar[st]);
     };
-    if (tid == 0 && !P.stall_staging) {
+    if (tid == 0 && !stall) {
         /* the staging buffers were last read by the generic proxy */
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         for (int b = 0; b < NS && b < nblk; b++) issue(b, (int)((gb + b) % NS));
@@ -735,9 +738,9 @@ __device__ __forceinline__ int series_index32(double time, double dts, int n) {
     return f >= (double)n ? n : (int)f;
 }
 
-__device__ __forceinline__ double series_at32(const double* v, int n, double dts, double time, int mode) {
+/* the series' value at `time`, whose entry in force is `it` */
+__device__ __forceinline__ double series_at32(const double* v, int it, double dts, double time, int mode) {
     if (mode == 0 && time <= 1.00) return v[0] * time;
-    const int it = series_index32(time, dts, n);
     const double a = v[it];
     if (mode == 2) return a;
     const double b = v[it + 1], d = time - dts * (it);
@@ -746,7 +749,7 @@ __device__ __forceinline__ double series_at32(const double* v, int n, double dts
 
 /* point-source rate (m/s) of source i at time t: the reference's stream_flow
  * interpolation (SW2D-EFDC.cu:531-538) in REFERENCE mode, else LINEAR / STEP */
-__device__ __forceinline__ float source_at32(const Scn32& P, int i, double time) {
+__device__ __forceinline__ float source_at32(const ScnBody32& P, int i, double time) {
     const double* Q = P.srcq;
     const int ns = P.nsrc;
     double q;
@@ -765,97 +768,133 @@ __device__ __forceinline__ float source_at32(const Scn32& P, int i, double time)
     return (float)sw2d_div_rn(q, P.dxd * P.dyd);
 }
 
-/* Length and forcing of the iteration starting at time t, by one whole warp:
- * every lane computes the length, lane k the k-th of the quotients and series
- * values that follow from it (independent chains of divisions and reads that
- * one thread would walk one after another). */
-__device__ __forceinline__ void prepare_slot32(const Scn32& P, Clock32* clk, double t, double t_end, double s_max) {
-    const int lane = threadIdx.x & 31;
-    double dt2, tm;
+/* The iteration that starts at time t: whether there is one, its length and
+ * the time of its second forcing values. */
+struct Times32 {
+    double t, dt2, tm;
     int active;
+};
+__device__ __forceinline__ Times32 times32(const ScnBody32& P, double t, double t_end, double s_max) {
+    Times32 n;
+    n.t = t;
     if (P.dt_mode == 0) {
         /* the reference's time grid: the clock advances by dt twice, as the
          * FP64 path's; only the state update uses dt2 rounded to binary32 */
         const double dt = P.dt_fixed;
-        active = (t + dt <= t_end);
-        dt2 = 2.0 * dt;
-        tm = t + dt;
+        n.active = (t + dt <= t_end);
+        n.dt2 = 2.0 * dt;
+        n.tm = t + dt;
     } else {
-        active = (t < t_end);
-        dt2 = s_max > 0 ? fmin(P.dt_max, sw2d_div_rn(P.cfl, s_max)) : P.dt_max;
+        n.active = (t < t_end);
+        double dt2 = s_max > 0 ? fmin(P.dt_max, sw2d_div_rn(P.cfl, s_max)) : P.dt_max;
         dt2 = (double)(float)dt2;
         if (t + dt2 > t_end) dt2 = t_end - t;
-        tm = t + 0.5 * dt2;
+        n.dt2 = dt2;
+        n.tm = t + 0.5 * dt2;
     }
+    return n;
+}
+
+/* Its slot, in three parts that a warp each can write: the length, the rates
+ * and quotients, and the point sources (lane k the k-th of the values: chains
+ * of divisions and reads that one thread would walk one after another). */
+__device__ __forceinline__ void put_length32(Clock32* clk, const Times32& n) {
+    if ((threadIdx.x & 31) == 0) {
+        clk->slot.active = n.active;
+        clk->slot.dt2 = (float)n.dt2;
+        clk->dt2 = n.dt2;
+        if (!n.active) clk->done = 1;
+    }
+}
+__device__ __forceinline__ void put_rates32(const ScnBody32& P, Clock32* clk, const Times32& n) {
+    /* lanes 0..3: rain at t and tm, then evaporation; lanes 4 and 5: the
+     * quotients by the spacings.  One division serves the lookups and them. */
+    const int lane = threadIdx.x & 31;
     Slot32& s = clk->slot;
-    if (lane == 0) {
-        s.active = active;
-        s.dt2 = (float)dt2;
-        clk->dt2 = dt2;
-        if (!active) clk->done = 1;
+    if (lane >= 6) return;
+    const bool ev = lane >= 2, spacing = lane >= 4;
+    const double time = (lane & 1) ? n.tm : n.t;
+    const double f = sw2d_div_rn(spacing ? n.dt2 : time, lane == 4 ? P.dxd : lane == 5 ? P.dyd : P.dtrain);
+    float r = 0.f;
+    const double* v = ev ? P.evap : P.rain;
+    if (spacing) {
+        r = (float)f;
+    } else if (v) {
+        const int nv = ev ? P.nevap : P.nrain, it = f >= (double)nv ? nv : (int)f;
+        r = (float)sw2d_div_rn(series_at32(v, it, P.dtrain, time, P.series_mode), P.dtrain * 1000.0);
     }
-    if (lane < 2) (lane ? &s.dt2dy : &s.dt2dx)[0] = (float)sw2d_div_rn(dt2, lane ? P.dyd : P.dxd);
-    if (lane < 4) { /* rain at t and tm, then evaporation */
-        const bool ev = lane >= 2;
-        const double* v = ev ? P.evap : P.rain;
-        float r = 0.f;
-        if (v)
-            r = (float)sw2d_div_rn(series_at32(v, ev ? P.nevap : P.nrain, P.dtrain, (lane & 1) ? tm : t, P.series_mode),
-                                   P.dtrain * 1000.0);
-        (ev ? ((lane & 1) ? &s.ev2 : &s.ev1) : ((lane & 1) ? &s.rr2 : &s.rr1))[0] = r;
-    }
-    for (int k = lane; k < 2 * P.nsrc; k += 32) {
+    float* const out = lane == 0 ? &s.rr1 : lane == 1 ? &s.rr2 : lane == 2 ? &s.ev1 : lane == 3 ? &s.ev2 : lane == 4 ? &s.dt2dx : &s.dt2dy;
+    *out = r;
+}
+__device__ __forceinline__ void put_sources32(const ScnBody32& P, Clock32* clk, const Times32& n) {
+    for (int k = threadIdx.x & 31; k < 2 * P.nsrc; k += 32) {
         const int i = k >> 1;
-        ((k & 1) ? clk->ql2 : clk->ql1)[i] = source_at32(P, i, (k & 1) ? tm : t);
+        ((k & 1) ? clk->ql2 : clk->ql1)[i] = source_at32(P, i, (k & 1) ? n.tm : n.t);
     }
 }
 
 /* One scenario's end of iteration, run by the whole CTA: fixed-order sum of
  * its work items' partials (each thread a fixed stride of them, then the
  * warps and the CTA in a fixed order; read past L1: other CTAs wrote them
- * during this launch), then, by the first warp, the ledger, clock, outlet
- * record and the next slot.  Every CTA waiting for this scenario waits for
- * it, so its latency counts: the clock is read at once, up front and past
- * L1 (the CTA that reduced the previous iteration may sit on another SM), the
- * ledger's entries are updated by one lane each, and sums that the scenario
- * cannot have are skipped (a binary64 addition takes a warp 71 cycles). */
-__device__ __noinline__ void finalize_scn(const Scn32& P, const Part32* __restrict__ part, double (*red)[4],
+ * during this launch), then, a warp each, the clock with the next length, the
+ * ledger with the outlet record, the next rates and the next point sources.
+ * Every CTA waiting for this scenario waits for it, and its time is round
+ * trips to memory (about 1000 cycles each, the acquire having emptied the L1) and
+ * binary64 latency (71 cycles an operation).  So the descriptor comes from
+ * shared memory, the clock is read up front and the partials four at a time, both
+ * past L1 (other SMs wrote them); the length is computed by every warp; the
+ * ledger's entries are updated by one lane each; and sums that the scenario
+ * cannot have, or whose terms are zero, are skipped.  11 to 16 thousand cycles
+ * an iteration before, of 38 thousand at 200 x 310; an iteration there 19.0
+ * us, now 14.7. */
+__device__ __noinline__ void finalize_scn(const ScnBody32& P, const Part32* __restrict__ part, double (*red)[4],
                                           float (*redf)[6]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     Clock32* clk = P.clk;
-    double v[4] = {0, 0, 0, 0}; /* clamp, outlet, rain, lake cells */
-    float sx = 0.f, sy = 0.f;
-    for (int k = tid; k < P.nwork; k += NT) {
-        const Part32* q = part + P.first_work + k;
-        v[0] += __ldcg(&q->clamp);
-        if (P.outflow_south) v[1] += __ldcg(&q->qout);
-        if (P.ledger_cells) {
-            v[2] += __ldcg(&q->rain);
-            v[3] += __ldcg(&q->evap);
-        }
-        sx = fmaxf(sx, __ldcg(&q->sx));
-        sy = fmaxf(sy, __ldcg(&q->sy));
-    }
-    double t = 0, t_end = 0, dt2 = 0, acc = 0;
-    long long iters = 0, outlet_n = 0;
-    float rr2 = 0.f, ev2 = 0.f;
-    int active = 0, cur = 0;
-    if (warp == 0) {
-        t = __ldcg(&clk->t);
-        t_end = __ldcg(&clk->t_end);
-        dt2 = __ldcg(&clk->dt2);
-        iters = __ldcg(&clk->iters);
-        outlet_n = __ldcg(&clk->outlet_n);
-        rr2 = __ldcg(&clk->slot.rr2);
-        ev2 = __ldcg(&clk->slot.ev2);
-        active = __ldcg(&clk->slot.active);
-        cur = __ldcg(&clk->slot.cur);
+    const double t = __ldcg(&clk->t), t_end = __ldcg(&clk->t_end), dt2 = __ldcg(&clk->dt2);
+    const int active = __ldcg(&clk->slot.active), cur = __ldcg(&clk->slot.cur);
+    const long long iters = __ldcg(&clk->iters), outlet_n = __ldcg(&clk->outlet_n);
+    const float rr2 = __ldcg(&clk->slot.rr2), ev2 = __ldcg(&clk->slot.ev2);
+    double acc = 0.0, qsrc = 0.0;
+    if (warp == 1) {
         /* rain_in, source_in, evap_out, outflow, clamp_gain */
         if (lane < 5) acc = __ldcg(&clk->rain_in + lane);
+        for (int k = 0; k < P.nsrc; k++) qsrc += (double)__ldcg(&clk->ql2[k]);
+    }
+    double v[4] = {0, 0, 0, 0}; /* clamp, outlet, rain, lake cells */
+    float sx = 0.f, sy = 0.f;
+    const bool per_cell = P.ledger_cells != 0, south = P.outflow_south != 0;
+    const int nw = P.nwork;
+    const Part32* const mine = part + P.first_work + tid;
+    for (int k0 = 0; k0 < nw; k0 += 4 * NT) {
+        double2 a[4], b[4]; /* rain, clamp; qout, evap */
+        float2 m[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            a[u] = b[u] = make_double2(0.0, 0.0);
+            m[u] = make_float2(0.f, 0.f);
+            if (k0 + u * NT + tid < nw) {
+                const Part32* q = mine + k0 + u * NT;
+                a[u] = __ldcg(reinterpret_cast<const double2*>(&q->rain));
+                if (south || per_cell) b[u] = __ldcg(reinterpret_cast<const double2*>(&q->qout));
+                m[u] = __ldcg(reinterpret_cast<const float2*>(&q->sx));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (__any_sync(0xffffffffu, sw2d_f64_bits(a[u].y) != 0)) v[0] += a[u].y;
+            if (south) v[1] += b[u].x;
+            if (per_cell) {
+                v[2] += a[u].x;
+                v[3] += b[u].y;
+            }
+            sx = fmaxf(sx, m[u].x);
+            sy = fmaxf(sy, m[u].y);
+        }
     }
 #pragma unroll
     for (int q = 0; q < 4; q++)
-        if (q == 0 ? __any_sync(0xffffffffu, v[0] != 0.0) : q == 1 ? P.outflow_south != 0 : P.ledger_cells != 0) {
+        if (q == 0 ? __any_sync(0xffffffffu, sw2d_f64_bits(v[0]) != 0) : q == 1 ? south : per_cell) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
         }
@@ -870,12 +909,36 @@ __device__ __noinline__ void finalize_scn(const Scn32& P, const Part32* __restri
         redf[warp][0] = sx;
         redf[warp][1] = sy;
     }
-    __syncthreads();
-    if (warp != 0 || !active) return;
-    double sum = 0.0;
-    if (lane < 4) {
-        sum = red[0][lane];
-        for (int k = 1; k < NW; k++) sum += red[k][lane];
+    __syncthreads(); /* the old clock and rates are read, too, before they are replaced */
+    if (!active) return;
+    const double tn = (P.dt_mode == 0) ? (t + P.dt_fixed) + P.dt_fixed : t + dt2;
+    if (warp == 1) { /* ledger and outlet */
+        double sum = 0.0;
+        if (lane < 4) {
+            sum = red[0][lane];
+            for (int k = 1; k < NW; k++) sum += red[k][lane];
+        }
+        const double clamp = __shfl_sync(0xffffffffu, sum, 0), qout = __shfl_sync(0xffffffffu, sum, 1),
+                     rain = __shfl_sync(0xffffffffu, sum, 2), evc = __shfl_sync(0xffffffffu, sum, 3);
+        const double area = P.area, q_out = qout * P.dyd;
+        /* lane by lane as acc is: ((a b) c) d */
+        const double fa = lane == 4 ? 1.0 : dt2;
+        const double fb = lane == 0 ? (double)rr2 : lane == 2 ? (double)ev2 : 1.0;
+        const double fc = lane == 0 ? (per_cell ? rain : P.rain_static) : lane == 1 ? qsrc : lane == 2 ? evc : lane == 3 ? q_out : clamp;
+        acc += fa * fb * fc * (lane == 3 ? 1.0 : area);
+        if (lane < 5) (&clk->rain_in)[lane] = acc;
+        if (lane == 0) {
+            clk->q_out = q_out;
+            if (!isfinite(qout)) atomicOr(&clk->status, 1);
+            clk->iters = iters + 1;
+            if (P.outlet) {
+                const long long k = outlet_n % P.outlet_cap;
+                P.outlet[2 * k] = tn;
+                P.outlet[2 * k + 1] = q_out;
+                clk->outlet_n = outlet_n + 1;
+            }
+        }
+        return;
     }
     sx = redf[0][0];
     sy = redf[0][1];
@@ -883,38 +946,27 @@ __device__ __noinline__ void finalize_scn(const Scn32& P, const Part32* __restri
         sx = fmaxf(sx, redf[k][0]);
         sy = fmaxf(sy, redf[k][1]);
     }
-    const double clamp = __shfl_sync(0xffffffffu, sum, 0), qout = __shfl_sync(0xffffffffu, sum, 1),
-                 rain = __shfl_sync(0xffffffffu, sum, 2), evc = __shfl_sync(0xffffffffu, sum, 3);
-    const double area = P.area, q_out = qout * P.dyd;
-    double qsrc = 0.0;
-    for (int k = 0; k < P.nsrc; k++) qsrc += (double)__ldcg(&clk->ql2[k]);
-    /* lane by lane as acc is: ((a b) c) d */
-    const double fa = lane == 4 ? 1.0 : dt2;
-    const double fb = lane == 0 ? (double)rr2 : lane == 2 ? (double)ev2 : 1.0;
-    const double fc = lane == 0 ? (P.ledger_cells ? rain : P.rain_static) : lane == 1 ? qsrc : lane == 2 ? evc : lane == 3 ? q_out : clamp;
-    acc += fa * fb * fc * (lane == 3 ? 1.0 : area);
     /* the CFL speed of the state this iteration started from */
     const double s_max = (double)sx + (double)sy;
-    const double tn = (P.dt_mode == 0) ? (t + P.dt_fixed) + P.dt_fixed : t + dt2;
-    if (lane < 5) (&clk->rain_in)[lane] = acc;
-    if (lane == 0) {
-        clk->q_out = q_out;
-        clk->s_max = s_max;
-        if (!isfinite(s_max) || !isfinite(qout)) atomicOr(&clk->status, 1);
-        clk->t = tn;
-        clk->iters = iters + 1;
-        clk->slot.cur = cur ^ 1;
-        if (P.outlet) {
-            const long long k = outlet_n % P.outlet_cap;
-            P.outlet[2 * k] = tn;
-            P.outlet[2 * k + 1] = q_out;
-            clk->outlet_n = outlet_n + 1;
+    const Times32 next = times32(P, tn, t_end, s_max);
+    if (warp == 0) {
+        put_length32(clk, next);
+        if (lane == 0) {
+            clk->s_max = s_max;
+            if (!isfinite(s_max)) atomicOr(&clk->status, 1);
+            clk->t = tn;
+            clk->slot.cur = cur ^ 1;
         }
+    } else if (warp == 2) {
+        put_rates32(P, clk, next);
+    } else {
+        put_sources32(P, clk, next);
     }
-    __syncwarp(); /* the rates above are read before they are replaced */
-    prepare_slot32(P, clk, tn, t_end, s_max);
-    __syncwarp();
 }
+static_assert(NW == 4, "the end of an iteration is split over four warps");
+static_assert(offsetof(Part32, rain) == 0 && offsetof(Part32, clamp) == 8 && offsetof(Part32, qout) == 16 &&
+                  offsetof(Part32, evap) == 24 && offsetof(Part32, sx) == 32 && sizeof(Part32) % 16 == 0,
+              "partials read in pairs");
 
 /* ---------------- the persistent launch ---------------------------------- */
 
@@ -955,20 +1007,31 @@ __device__ __noinline__ unsigned wait_ticket(unsigned q, const Scn32* __restrict
     return q;
 }
 
+/* What the CTA's next item needs besides the previous iteration's results,
+ * into shared memory before the wait for those (which empties the L1). */
+__device__ __noinline__ void prepare_item(SmemM& S, const Scn32* __restrict__ scns, const int4* __restrict__ work, int nwork) {
+    const int4 w = work[S.qn % (unsigned)nwork];
+    if (w.x != S.have) {
+        const int4* src = reinterpret_cast<const int4*>(static_cast<const ScnBody32*>(scns + w.x));
+        if (threadIdx.x < sizeof(ScnBody32) / 16) reinterpret_cast<int4*>(&S.scn)[threadIdx.x] = src[threadIdx.x];
+    }
+    if (threadIdx.x == 0) S.w = w;
+}
+
 /* thread 0 after an item of scenario sc: count it; true when it was the
  * scenario's last of the iteration.  The one atomic releases the item's state
  * and partial (its CTA's writes, ordered before it by the barriers above) and
  * acquires the others'; fences around a relaxed one are sequentially
  * consistent ones and cost a round trip each. */
-__device__ __noinline__ bool count_item(const Scn32* __restrict__ scns, int nscn, int sc, Ctl32* ctl) {
+__device__ __noinline__ bool count_item(int nwork, int nscn, int sc, Ctl32* ctl) {
     unsigned* cnt = reinterpret_cast<unsigned*>(reinterpret_cast<int*>(ctl + 1) + nscn);
     unsigned before;
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(&cnt[sc]) : "memory");
-    return before == (unsigned)scns[sc].nwork - 1u;
+    return before == (unsigned)nwork - 1u;
 }
 
-/* thread 0 after the scenario's reduction (by its own warp): release its
- * next iteration */
+/* thread 0 after the scenario's reduction and a barrier: release its next
+ * iteration */
 __device__ __noinline__ void release_scenario(int nscn, int sc, int iterations_done, Ctl32* ctl) {
     int* done = reinterpret_cast<int*>(ctl + 1);
     unsigned* cnt = reinterpret_cast<unsigned*>(done + nscn);
@@ -999,10 +1062,14 @@ __global__ void __launch_bounds__(NT, 4) k32_persist(const Scn32* __restrict__ s
         for (int k = 0; k < NS; k++) mbar_init(&S.bar[k], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncthreads();
     unsigned gb = 0; /* staged blocks used so far by this CTA */
-    if (threadIdx.x == 0) S.qn = atomicAdd(&ctl->next, 1u);
+    if (threadIdx.x == 0) {
+        S.qn = atomicAdd(&ctl->next, 1u);
+        S.have = -1;
+    }
+    __syncthreads();
     for (;;) {
+        prepare_item(S, scns, work, nwork);
         if (threadIdx.x == 0) S.q = wait_ticket(S.qn, scns, work, nwork, niter, ctl);
         __syncthreads();
         /* read through a shuffle from lane 0: the compiler then knows the
@@ -1011,8 +1078,10 @@ __global__ void __launch_bounds__(NT, 4) k32_persist(const Scn32* __restrict__ s
          * thread to the marching windows */
         const unsigned q = __shfl_sync(0xffffffffu, S.q, 0);
         if (q == ~0u) break;
+        const int4 sw = S.w;
+        const int4 w = make_int4(__shfl_sync(0xffffffffu, sw.x, 0), __shfl_sync(0xffffffffu, sw.y, 0),
+                                 __shfl_sync(0xffffffffu, sw.z, 0), __shfl_sync(0xffffffffu, sw.w, 0));
         if (threadIdx.x == 0) S.qn = atomicAdd(&ctl->next, 1u); /* the next ticket, drawn while this item runs */
-        const int4 w = work[q % (unsigned)nwork]; /* in L1: thread 0 read it while it waited */
         /* the previous iteration's state was written by other CTAs with
          * generic stores; this item reads it with TMA (the async proxy) */
         asm volatile("fence.proxy.async.global;" ::: "memory");
@@ -1020,12 +1089,14 @@ __global__ void __launch_bounds__(NT, 4) k32_persist(const Scn32* __restrict__ s
             if (threadIdx.x == 0) ctl->abort = 1u;
             break;
         }
-        if (threadIdx.x == 0) S.last = count_item(scns, nscn, w.x, ctl);
+        if (threadIdx.x == 0) S.last = count_item(S.scn.nwork, nscn, S.w.x, ctl);
         __syncthreads();
         if (__shfl_sync(0xffffffffu, S.last, 0)) {
-            finalize_scn(scns[w.x], part, S.red, S.redf);
-            if (threadIdx.x == 0) release_scenario(nscn, w.x, (int)(q / (unsigned)nwork) + 1, ctl);
+            finalize_scn(S.scn, part, S.red, S.redf);
+            __syncthreads();
+            if (threadIdx.x == 0) release_scenario(nscn, S.w.x, (int)(S.q / (unsigned)nwork) + 1, ctl);
         }
+        if (threadIdx.x == 0) S.have = S.w.x;
         __syncthreads();
     }
 }
@@ -1041,7 +1112,10 @@ __global__ void k32_prime(const Scn32* __restrict__ scns, int nscn, int set_end,
         clk->t_end = te;
     }
     __syncwarp();
-    prepare_slot32(scns[s], clk, clk->t, te, clk->s_max);
+    const Times32 n = times32(scns[s], clk->t, te, clk->s_max);
+    put_length32(clk, n);
+    put_rates32(scns[s], clk, n);
+    put_sources32(scns[s], clk, n);
 }
 
 __global__ void k32_status(const Scn32* __restrict__ scns, int nscn, Status32* __restrict__ out) {

@@ -81,9 +81,14 @@ struct Part32 {
     int pad[6];
 };
 
-struct Scn32 {
+struct ScnMaps32 {
     CUtensorMap tm_h[2], tm_qx[2], tm_qy[2], tm_z, tm_kc;
     CUtensorMap tm_cls, tm_rw;   /* set when the scenario has a class raster / a rain-weight field */
+};
+
+/* what the end of an iteration reads; constant over a launch, so a CTA keeps
+ * its scenario's in shared memory */
+struct alignas(16) ScnBody32 {
     float* h[2];
     float* qx[2];
     float* qy[2];
@@ -109,6 +114,9 @@ struct Scn32 {
     float pct_lake, pct_land, ev_wl_min;
     double rain_static;    /* sum over active cells of weight * runoff fraction */
     double dxd, dyd, dtrain, dt_fixed, cfl, dt_max, area;
+};
+
+struct Scn32 : ScnMaps32, ScnBody32 {
     float ntab[T32_MAXCLASS];
 };
 
