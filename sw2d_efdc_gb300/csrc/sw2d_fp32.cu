@@ -53,11 +53,18 @@ struct alignas(128) RwStage {
     float v[M_RWR][BW]; /* rows L-3 .. L+RB-2 */
 };
 
+/* a work item and its scenario's descriptor */
+struct ItemM {
+    int4 w;   /* scenario, column strip, row segment, place of its partial */
+    int have; /* the scenario whose descriptor scn is (-1: none) */
+    ScnBody32 scn;
+};
+
 /* the class and rain-weight rings come last, so that the variants without
  * them launch with less shared memory (fp32_smem_bytes_variant) */
 struct SmemM {
     alignas(128) float stage[NS][NF][RB][BW];
-    ScnBody32 scn;              /* the scenario of the item in hand */
+    ItemM item[2];              /* the item in hand and the next one */
     unsigned long long bar[NS];
     float ntab[T32_MAXCLASS];
     float dband[M_MAXBANDS][3]; /* datums of the bands the item spans, strips west / own / east */
@@ -69,8 +76,6 @@ struct SmemM {
     unsigned q;                 /* queue ticket of the item in hand (~0u: leave) */
     unsigned qn;                /* the ticket drawn ahead for the next item */
     int last;                   /* this CTA finished its scenario's iteration */
-    int4 w;                     /* the item in hand */
-    int have;                   /* the scenario whose descriptor scn is (-1: none) */
     ClsStage cls[NS];
     RwStage rw[NS];
 };
@@ -289,10 +294,10 @@ static_assert(sizeof(Slot32) % 16 == 0 && offsetof(Clock32, slot) == 0, "slot re
  * load did not arrive in time (the status bit is set; the launch's results
  * are void). */
 template <bool CLS, bool RW, bool LAKE, bool SRC>
-__device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 w, Part32* __restrict__ part,
+__device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, int slot, const int4 w, Part32* __restrict__ part,
                                            unsigned& gb) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    Clock32* const clk = reinterpret_cast<Clock32*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(S.scn.clk), 0));
+    Clock32* const clk = reinterpret_cast<Clock32*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(S.item[slot].scn.clk), 0));
     const Slot32 sl = load_slot(clk);
     const int R = P.R, C = P.C, Pp = P.P, stall = P.stall_staging;
     if (!sl.active) {
@@ -300,6 +305,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
             Part32 zp = {};
             part[w.w] = zp;
         }
+        __syncthreads(); /* as at the end */
         return true;
     }
     const int cur = sl.cur, nxt = cur ^ 1;
@@ -315,6 +321,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
             Part32 zp = {};
             part[w.w] = zp;
         }
+        __syncthreads();
         return true; /* tile skipped, status bit 2 */
     }
     constexpr bool has_cls = CLS, has_rw = RW;
@@ -341,7 +348,6 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
         for (int b = 0; b < NS && b < nblk; b++) issue(b, (int)((gb + b) % NS));
     }
     /* while the first blocks are on their way */
-    if (tid < T32_MAXCLASS) S.ntab[tid] = P.ntab[tid];
     if (SRC && warp == 0) {
         /* the point sources inside the staged window (rows rs-3 .. re+2,
          * the strip's staged columns), in source order */
@@ -368,14 +374,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
         }
         if (lane == 0) S.nls = n;
     }
-    /* datums of the bands the staged rows span, for the strips west, own
-     * and east (0 outside the raster) */
-    if (tid < 3 * M_MAXBANDS) {
-        const int b0 = max(Ls, 0) / M_DR;
-        const int j = tid / 3, cr = tid - 3 * j, nx = strip + cr - 1;
-        S.dband[j][cr] = (nx >= 0 && nx < P.tiles_x && b0 + j < P.bands) ? P.datum[(b0 + j) * P.tiles_x + nx] : 0.f;
-    }
-    __syncthreads();
+    if (SRC) __syncthreads();
 
     /* lane geometry: staged columns sc, sc+1; global columns cg, cg+1 */
     const int sc = warp * M_SW + 2 * lane;
@@ -691,16 +690,21 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
     }
     gb += (unsigned)nblk;
 
-    /* block reductions: warp sums in binary32, across warps in binary64 */
+    /* block reductions: warp sums in binary32, across warps in binary64.  Sums
+     * that are not kept or whose terms are zero are left at zero; speeds are
+     * not negative, so their bits order them. */
+    sxm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(sxm)));
+    sym = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(sym)));
+    auto warp_sum = [](float x) {
+        if (!__any_sync(0xffffffffu, x != 0.f)) return 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sxm = fmaxf(sxm, __shfl_xor_sync(0xffffffffu, sxm, o));
-        sym = fmaxf(sym, __shfl_xor_sync(0xffffffffu, sym, o));
-        clamp += __shfl_xor_sync(0xffffffffu, clamp, o);
-        qout += __shfl_xor_sync(0xffffffffu, qout, o);
-        rainacc += __shfl_xor_sync(0xffffffffu, rainacc, o);
-        evc += __shfl_xor_sync(0xffffffffu, evc, o);
-    }
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    };
+    clamp = warp_sum(clamp);
+    qout = warp_sum(qout);
+    rainacc = warp_sum(rainacc);
+    evc = warp_sum(evc);
     if (lane == 0) {
         float* f = S.redf[warp];
         f[0] = clamp;
@@ -715,13 +719,18 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, const int4 
      * takes 71 cycles whether one lane or six take part) */
     if (tid < 6) {
         Part32* o = part + w.w; /* the partials stay in scenario order whatever the launch order */
+        float f[NW];
+#pragma unroll
+        for (int k = 0; k < NW; k++) f[k] = S.redf[k][tid];
         if (tid < 4) {
             double v = 0.0;
-            for (int k = 0; k < NW; k++) v += sw2d_f64_of_f32(S.redf[k][tid]);
+            if (__any_sync(0xfu, f[0] != 0.f || f[1] != 0.f || f[2] != 0.f || f[3] != 0.f))
+                for (int k = 0; k < NW; k++) v += sw2d_f64_of_f32(f[k]);
             (tid == 0 ? &o->clamp : tid == 1 ? &o->qout : tid == 2 ? &o->rain : &o->evap)[0] = v;
         } else {
             float v = 0.f;
-            for (int k = 0; k < NW; k++) v = fmaxf(v, S.redf[k][tid]);
+#pragma unroll
+            for (int k = 0; k < NW; k++) v = fmaxf(v, f[k]);
             /* rdx > 0: the maximum commutes with the scaling */
             (tid == 4 ? &o->sx : &o->sy)[0] = v * (tid == 4 ? rdxy.x : rdxy.y);
         }
@@ -738,12 +747,12 @@ __device__ __forceinline__ int series_index32(double time, double dts, int n) {
     return f >= (double)n ? n : (int)f;
 }
 
-/* the series' value at `time`, whose entry in force is `it` */
-__device__ __forceinline__ double series_at32(const double* v, int it, double dts, double time, int mode) {
+/* the series' value at `time`, with a its entry in force (the it-th) and b the next */
+__device__ __forceinline__ double series_at32(const double* v, double a, double b, int it, double dts, double time,
+                                              int mode) {
     if (mode == 0 && time <= 1.00) return v[0] * time;
-    const double a = v[it];
     if (mode == 2) return a;
-    const double b = v[it + 1], d = time - dts * (it);
+    const double d = time - dts * (it);
     return mode == 0 ? a + sw2d_div_rn(b - a, dts * d) : a + (b - a) * sw2d_div_rn(d, dts);
 }
 
@@ -806,7 +815,27 @@ __device__ __forceinline__ void put_length32(Clock32* clk, const Times32& n) {
         if (!n.active) clk->done = 1;
     }
 }
-__device__ __forceinline__ void put_rates32(const ScnBody32& P, Clock32* clk, const Times32& n) {
+/* Series entries read ahead of the length they depend on: those from the
+ * entry in force at the iteration's start (lanes 0..3 as put_rates32). */
+struct Ahead32 {
+    int it;
+    double v[3];
+};
+__device__ __forceinline__ Ahead32 series_ahead32(const ScnBody32& P, double t) {
+    Ahead32 a;
+    a.it = -8;
+    const int lane = threadIdx.x & 31;
+    const double* v = lane >= 2 ? P.evap : P.rain;
+    if (lane < 4 && v) {
+        const int n = lane >= 2 ? P.nevap : P.nrain;
+        a.it = series_index32(t, P.dtrain, n);
+        a.v[0] = v[a.it];
+        a.v[1] = v[a.it + 1];
+        a.v[2] = v[min(a.it + 2, n + 1)];
+    }
+    return a;
+}
+__device__ __forceinline__ void put_rates32(const ScnBody32& P, Clock32* clk, const Times32& n, const Ahead32& ahead) {
     /* lanes 0..3: rain at t and tm, then evaporation; lanes 4 and 5: the
      * quotients by the spacings.  One division serves the lookups and them. */
     const int lane = threadIdx.x & 31;
@@ -821,7 +850,10 @@ __device__ __forceinline__ void put_rates32(const ScnBody32& P, Clock32* clk, co
         r = (float)f;
     } else if (v) {
         const int nv = ev ? P.nevap : P.nrain, it = f >= (double)nv ? nv : (int)f;
-        r = (float)sw2d_div_rn(series_at32(v, it, P.dtrain, time, P.series_mode), P.dtrain * 1000.0);
+        const int from = it - ahead.it; /* 0 or 1 unless the iteration is long */
+        const double a = from == 0 ? ahead.v[0] : from == 1 ? ahead.v[1] : v[it];
+        const double b = from == 0 ? ahead.v[1] : from == 1 ? ahead.v[2] : v[it + 1];
+        r = (float)sw2d_div_rn(series_at32(v, a, b, it, P.dtrain, time, P.series_mode), P.dtrain * 1000.0);
     }
     float* const out = lane == 0 ? &s.rr1 : lane == 1 ? &s.rr2 : lane == 2 ? &s.ev1 : lane == 3 ? &s.ev2 : lane == 4 ? &s.dt2dx : &s.dt2dy;
     *out = r;
@@ -892,17 +924,17 @@ __device__ __noinline__ void finalize_scn(const ScnBody32& P, const Part32* __re
             sy = fmaxf(sy, m[u].y);
         }
     }
+    const double tn = (P.dt_mode == 0) ? (t + P.dt_fixed) + P.dt_fixed : t + dt2;
+    Ahead32 ahead;
+    if (warp == 2) ahead = series_ahead32(P, tn);
 #pragma unroll
     for (int q = 0; q < 4; q++)
         if (q == 0 ? __any_sync(0xffffffffu, sw2d_f64_bits(v[0]) != 0) : q == 1 ? south : per_cell) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
         }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sx = fmaxf(sx, __shfl_down_sync(0xffffffffu, sx, o));
-        sy = fmaxf(sy, __shfl_down_sync(0xffffffffu, sy, o));
-    }
+    sx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(sx)));
+    sy = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(sy)));
     if (lane == 0) {
 #pragma unroll
         for (int q = 0; q < 4; q++) red[warp][q] = v[q];
@@ -911,7 +943,6 @@ __device__ __noinline__ void finalize_scn(const ScnBody32& P, const Part32* __re
     }
     __syncthreads(); /* the old clock and rates are read, too, before they are replaced */
     if (!active) return;
-    const double tn = (P.dt_mode == 0) ? (t + P.dt_fixed) + P.dt_fixed : t + dt2;
     if (warp == 1) { /* ledger and outlet */
         double sum = 0.0;
         if (lane < 4) {
@@ -958,7 +989,7 @@ __device__ __noinline__ void finalize_scn(const ScnBody32& P, const Part32* __re
             clk->slot.cur = cur ^ 1;
         }
     } else if (warp == 2) {
-        put_rates32(P, clk, next);
+        put_rates32(P, clk, next, ahead);
     } else {
         put_sources32(P, clk, next);
     }
@@ -981,19 +1012,17 @@ __device__ __forceinline__ void st_release_gpu(int* p, int v) {
 
 /* The queue side of the persistent loop, run by thread 0: the bounded wait
  * of ticket q (drawn ahead, while the CTA worked on its previous item) for
- * its scenario's previous iteration.  Returns the ticket, or ~0u when the
+ * the previous iteration of its scenario sc.  Returns the ticket, or ~0u when the
  * CTA is to leave (the queue is empty, or a wait ran out: then the
  * scenario's timeout bit and the abort flag are set).  A waiting ticket only
  * ever waits for smaller tickets, so holding one ticket ahead cannot close a
  * cycle of waits. */
-__device__ __noinline__ unsigned wait_ticket(unsigned q, const Scn32* __restrict__ scns,
-                                             const int4* __restrict__ work, int nwork, int niter, Ctl32* ctl) {
+__device__ __noinline__ unsigned wait_ticket(unsigned q, const Scn32* __restrict__ scns, int sc, int nwork, int niter,
+                                             Ctl32* ctl) {
     const int* done = reinterpret_cast<const int*>(ctl + 1);
     volatile unsigned* abort_flag = &ctl->abort;
     if (q >= (unsigned)nwork * (unsigned)niter || *abort_flag) return ~0u;
     const int it = (int)(q / (unsigned)nwork);
-    const int4 w = work[q % (unsigned)nwork];
-    const int sc = w.x;
     const long long t0 = clock64();
     while (ld_acquire_gpu(&done[sc]) < it) {
         if (*abort_flag) return ~0u;
@@ -1008,14 +1037,27 @@ __device__ __noinline__ unsigned wait_ticket(unsigned q, const Scn32* __restrict
 }
 
 /* What the CTA's next item needs besides the previous iteration's results,
- * into shared memory before the wait for those (which empties the L1). */
-__device__ __noinline__ void prepare_item(SmemM& S, const Scn32* __restrict__ scns, const int4* __restrict__ work, int nwork) {
+ * into shared memory before the wait for those (which empties the L1), by all
+ * warps but the first: that one counts the item before meanwhile. */
+__device__ __noinline__ void prepare_item(SmemM& S, int slot, const Scn32* __restrict__ scns,
+                                          const int4* __restrict__ work, int nwork) {
+    const int k = (int)threadIdx.x - 32;
+    if (k < 0) return;
+    ItemM& it = S.item[slot];
+    const ItemM& old = S.item[slot ^ 1];
     const int4 w = work[S.qn % (unsigned)nwork];
-    if (w.x != S.have) {
-        const int4* src = reinterpret_cast<const int4*>(static_cast<const ScnBody32*>(scns + w.x));
-        if (threadIdx.x < sizeof(ScnBody32) / 16) reinterpret_cast<int4*>(&S.scn)[threadIdx.x] = src[threadIdx.x];
+    const Scn32& P = scns[w.x];
+    const ScnBody32& B = w.x == old.have ? old.scn : P;
+    if (w.x != it.have && k < (int)(sizeof(ScnBody32) / 16))
+        reinterpret_cast<int4*>(&it.scn)[k] = reinterpret_cast<const int4*>(&B)[k];
+    if (w.x != old.have && k < T32_MAXCLASS) S.ntab[k] = P.ntab[k];
+    /* datums of the bands the staged rows span, for the strips west, own
+     * and east (0 outside the raster) */
+    for (int e = k; e < 3 * M_MAXBANDS; e += NT - 32) {
+        const int j = e / 3, cr = e - 3 * j, nx = w.y + cr - 1, band = max(w.z * B.seg - 3, 0) / M_DR + j;
+        S.dband[j][cr] = (nx >= 0 && nx < B.tiles_x && band < B.bands) ? B.datum[band * B.tiles_x + nx] : 0.f;
     }
-    if (threadIdx.x == 0) S.w = w;
+    if (k == 0) it.w = w;
 }
 
 /* thread 0 after an item of scenario sc: count it; true when it was the
@@ -1065,12 +1107,16 @@ __global__ void __launch_bounds__(NT, 4) k32_persist(const Scn32* __restrict__ s
     unsigned gb = 0; /* staged blocks used so far by this CTA */
     if (threadIdx.x == 0) {
         S.qn = atomicAdd(&ctl->next, 1u);
-        S.have = -1;
+        S.item[0].have = S.item[1].have = -1;
     }
     __syncthreads();
-    for (;;) {
-        prepare_item(S, scns, work, nwork);
-        if (threadIdx.x == 0) S.q = wait_ticket(S.qn, scns, work, nwork, niter, ctl);
+    prepare_item(S, 0, scns, work, nwork);
+    __syncthreads();
+    for (int slot = 0;; slot ^= 1) {
+        if (threadIdx.x == 0) {
+            S.item[slot].have = S.item[slot].w.x;
+            S.q = wait_ticket(S.qn, scns, S.item[slot].w.x, nwork, niter, ctl);
+        }
         __syncthreads();
         /* read through a shuffle from lane 0: the compiler then knows the
          * ticket, the item and the scenario's fields are uniform across the
@@ -1078,26 +1124,28 @@ __global__ void __launch_bounds__(NT, 4) k32_persist(const Scn32* __restrict__ s
          * thread to the marching windows */
         const unsigned q = __shfl_sync(0xffffffffu, S.q, 0);
         if (q == ~0u) break;
-        const int4 sw = S.w;
+        const int4 sw = S.item[slot].w;
         const int4 w = make_int4(__shfl_sync(0xffffffffu, sw.x, 0), __shfl_sync(0xffffffffu, sw.y, 0),
                                  __shfl_sync(0xffffffffu, sw.z, 0), __shfl_sync(0xffffffffu, sw.w, 0));
         if (threadIdx.x == 0) S.qn = atomicAdd(&ctl->next, 1u); /* the next ticket, drawn while this item runs */
         /* the previous iteration's state was written by other CTAs with
          * generic stores; this item reads it with TMA (the async proxy) */
         asm volatile("fence.proxy.async.global;" ::: "memory");
-        if (!march_item<CLS, RW, LAKE, SRC>(S, scns[w.x], w, part, gb)) {
+        if (!march_item<CLS, RW, LAKE, SRC>(S, scns[w.x], slot, w, part, gb)) {
             if (threadIdx.x == 0) ctl->abort = 1u;
             break;
         }
-        if (threadIdx.x == 0) S.last = count_item(S.scn.nwork, nscn, S.w.x, ctl);
+        /* the march is over (its last barrier): ntab, dband and the other
+         * slot are free for the next item */
+        if (threadIdx.x == 0) S.last = count_item(S.item[slot].scn.nwork, nscn, S.item[slot].w.x, ctl);
+        prepare_item(S, slot ^ 1, scns, work, nwork);
         __syncthreads();
         if (__shfl_sync(0xffffffffu, S.last, 0)) {
-            finalize_scn(S.scn, part, S.red, S.redf);
+            finalize_scn(S.item[slot].scn, part, S.red, S.redf);
             __syncthreads();
-            if (threadIdx.x == 0) release_scenario(nscn, S.w.x, (int)(S.q / (unsigned)nwork) + 1, ctl);
+            if (threadIdx.x == 0)
+                release_scenario(nscn, S.item[slot].w.x, (int)(S.q / (unsigned)nwork) + 1, ctl);
         }
-        if (threadIdx.x == 0) S.have = S.w.x;
-        __syncthreads();
     }
 }
 
@@ -1114,7 +1162,7 @@ __global__ void k32_prime(const Scn32* __restrict__ scns, int nscn, int set_end,
     __syncwarp();
     const Times32 n = times32(scns[s], clk->t, te, clk->s_max);
     put_length32(clk, n);
-    put_rates32(scns[s], clk, n);
+    put_rates32(scns[s], clk, n, series_ahead32(scns[s], clk->t));
     put_sources32(scns[s], clk, n);
 }
 
