@@ -331,21 +331,34 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, int slot, c
      * compensation of the rows three above (the rows finished during b) and,
      * when present, the class rows from two above and the rain weights from
      * three above */
-    auto issue = [&](int b, int st) {
-        mbar_arrive_expect_tx(&S.bar[st], blk_bytes);
+    auto issue = [&](int b, int st, int part) { /* part: 0..3 for one of four issuers, 4 for all of it */
         const int y = Ls + b * RB + M_H; /* padded row of the block's first row */
-        tma_load_2d(&S.stage[st][0][0][0], &P.tm_h[cur], c0, y, &S.bar[st]);
-        tma_load_2d(&S.stage[st][1][0][0], &P.tm_z, c0, y, &S.bar[st]);
-        tma_load_2d(&S.stage[st][2][0][0], &P.tm_qx[cur], c0, y, &S.bar[st]);
-        tma_load_2d(&S.stage[st][3][0][0], &P.tm_qy[cur], c0, y, &S.bar[st]);
-        tma_load_2d(&S.stage[st][4][0][0], &P.tm_kc, c0, y - 3, &S.bar[st]);
-        if (has_cls) tma_load_2d(&S.cls[st].v[0][0], &P.tm_cls, c0, y - 2, &S.bar[st]);
-        if (has_rw) tma_load_2d(&S.rw[st].v[0][0], &P.tm_rw, c0, y - 3, &S.bar[st]);
+        if (part == 0 || part == 4) {
+            mbar_arrive_expect_tx(&S.bar[st], blk_bytes);
+            tma_load_2d(&S.stage[st][0][0][0], &P.tm_h[cur], c0, y, &S.bar[st]);
+        }
+        if (part == 1 || part == 4) {
+            tma_load_2d(&S.stage[st][1][0][0], &P.tm_z, c0, y, &S.bar[st]);
+            if (has_cls) tma_load_2d(&S.cls[st].v[0][0], &P.tm_cls, c0, y - 2, &S.bar[st]);
+        }
+        if (part == 2 || part == 4) {
+            tma_load_2d(&S.stage[st][2][0][0], &P.tm_qx[cur], c0, y, &S.bar[st]);
+            if (has_rw) tma_load_2d(&S.rw[st].v[0][0], &P.tm_rw, c0, y - 3, &S.bar[st]);
+        }
+        if (part == 3 || part == 4) {
+            tma_load_2d(&S.stage[st][3][0][0], &P.tm_qy[cur], c0, y, &S.bar[st]);
+            tma_load_2d(&S.stage[st][4][0][0], &P.tm_kc, c0, y - 3, &S.bar[st]);
+        }
     };
-    if (tid == 0 && !stall) {
+    /* The first blocks, a share by each warp: at an item's start the ten copies
+     * of one thread are what all warps wait for (4096^2 194 -> 191 us an
+     * iteration).  A copy may complete before the first warp's share has told
+     * the barrier how many bytes to expect: the phase stays open until that
+     * share's arrival, and the byte count may be negative meanwhile. */
+    if (lane == 0 && !stall) {
         /* the staging buffers were last read by the generic proxy */
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        for (int b = 0; b < NS && b < nblk; b++) issue(b, (int)((gb + b) % NS));
+        for (int b = 0; b < NS && b < nblk; b++) issue(b, (int)((gb + b) % NS), warp);
     }
     /* while the first blocks are on their way */
     if (SRC && warp == 0) {
@@ -685,7 +698,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, int slot, c
         __syncthreads(); /* every warp is done with block b */
         if (tid == 0 && b + NS < nblk) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            issue(b + NS, st);
+            issue(b + NS, st, 4);
         }
     }
     gb += (unsigned)nblk;
