@@ -21,10 +21,11 @@
  *                extra block adds up the previous iteration's partials in a
  *                fixed order and prepares the next iteration's length and
  *                forcing beside the tiles.
- * At 4096 x 4096 (pond break) an iteration takes 1.92 ms against 5.17 ms
- * with part-empty warps, a binary64 provisional depth and conversions and
- * sums predicated off beside the path taken; at 256 x 256 24 us against 62 us,
- * most of it the clock's work at the end of the last tile's block before.
+ * At 4096 x 4096 (pond break) an iteration takes 1.28 ms (flux 0.87, update
+ * 0.44) against 5.17 ms with part-empty warps, a binary64 provisional depth
+ * and conversions and sums predicated off beside the path taken; at 256 x 256
+ * 19.5 us against 62 us, most of it the clock's work at the end of the last
+ * tile's block before.
  * forward (:670-693) is a buffer swap for the depth (h[cur] -> h[nxt]); the
  * discharges keep fixed roles: qx[0]/qy[0] hold the state, k64_flux writes
  * its new faces into qx[1]/qy[1], and k64_update writes every face, closed
