@@ -837,20 +837,22 @@ __device__ __forceinline__ void put_length32(Clock32* clk, const Times32& n) {
         if (!n.active) clk->done = 1;
     }
 }
-/* Series entries read ahead of the length they depend on: those from the
- * entry in force at the iteration's start (lanes 0..3 as put_rates32). */
+/* Series entries read ahead of the length they depend on (lanes 0..3 as
+ * put_rates32): those from the entry of the iteration before, which the slot
+ * keeps as a hint: 27.5 us an iteration at 1000^2 against 27.8 with the entry
+ * looked up by its division first, 16 mixed scenarios 18.5 ms against 18.9. */
 struct Ahead32 {
     int it;
     double v[3];
 };
-__device__ __forceinline__ Ahead32 series_ahead32(const ScnBody32& P, double t) {
+__device__ __forceinline__ Ahead32 series_ahead32(const ScnBody32& P, const int* entry) {
     Ahead32 a;
     a.it = -8;
-    const int lane = threadIdx.x & 31;
-    const double* v = lane >= 2 ? P.evap : P.rain;
+    const int lane = threadIdx.x & 31, ev = lane >> 1;
+    const double* v = ev ? P.evap : P.rain;
     if (lane < 4 && v) {
-        const int n = lane >= 2 ? P.nevap : P.nrain;
-        a.it = series_index32(t, P.dtrain, n);
+        const int n = ev ? P.nevap : P.nrain;
+        a.it = min(max(__ldcg(entry + ev), 0), n);
         a.v[0] = v[a.it];
         a.v[1] = v[a.it + 1];
         a.v[2] = v[min(a.it + 2, n + 1)];
@@ -872,6 +874,7 @@ __device__ __forceinline__ void put_rates32(const ScnBody32& P, Clock32* clk, co
         r = (float)f;
     } else if (v) {
         const int nv = ev ? P.nevap : P.nrain, it = f >= (double)nv ? nv : (int)f;
+        if (lane & 1) s.entry[ev] = it;
         const int from = it - ahead.it; /* 0 or 1 unless the iteration is long */
         const double a = from == 0 ? ahead.v[0] : from == 1 ? ahead.v[1] : v[it];
         const double b = from == 0 ? ahead.v[1] : from == 1 ? ahead.v[2] : v[it + 1];
@@ -909,6 +912,8 @@ __device__ __noinline__ void finalize_scn(const ScnBody32& P, const Part32* __re
     const int active = __ldcg(&clk->slot.active), cur = __ldcg(&clk->slot.cur);
     const long long iters = __ldcg(&clk->iters), outlet_n = __ldcg(&clk->outlet_n);
     const float rr2 = __ldcg(&clk->slot.rr2), ev2 = __ldcg(&clk->slot.ev2);
+    Ahead32 ahead;
+    if (warp == 2) ahead = series_ahead32(P, clk->slot.entry);
     double acc = 0.0, qsrc = 0.0;
     if (warp == 1) {
         /* rain_in, source_in, evap_out, outflow, clamp_gain */
@@ -947,8 +952,6 @@ __device__ __noinline__ void finalize_scn(const ScnBody32& P, const Part32* __re
         }
     }
     const double tn = (P.dt_mode == 0) ? (t + P.dt_fixed) + P.dt_fixed : t + dt2;
-    Ahead32 ahead;
-    if (warp == 2) ahead = series_ahead32(P, tn);
 #pragma unroll
     for (int q = 0; q < 4; q++)
         if (q == 0 ? __any_sync(0xffffffffu, sw2d_f64_bits(v[0]) != 0) : q == 1 ? south : per_cell) {
@@ -1184,7 +1187,7 @@ __global__ void k32_prime(const Scn32* __restrict__ scns, int nscn, int set_end,
     __syncwarp();
     const Times32 n = times32(scns[s], clk->t, te, clk->s_max);
     put_length32(clk, n);
-    put_rates32(scns[s], clk, n, series_ahead32(scns[s], clk->t));
+    put_rates32(scns[s], clk, n, series_ahead32(scns[s], clk->slot.entry));
     put_sources32(scns[s], clk, n);
 }
 

@@ -55,7 +55,8 @@ struct Slot32 {
     float ev1, ev2;     /* evaporation rate, m/s */
     int active;
     int cur;            /* which of the two state buffers is current */
-    int pad[7];
+    int entry[2];       /* series entries in force at its second time: rain, evaporation (a hint) */
+    int pad[5];
 };
 
 struct Clock32 {
