@@ -38,13 +38,13 @@ BYTES_PER_CELL_FP64_CFG2 = 62  # h,qx,qy r+w 48 + z 8 + flag 1 + Manning class 1
 # k64_flux per cell: reads h, z, qx, qy, uu1, vv1 (6 x 8) + flag + Manning class, writes qx, qy (2 x 8)
 BYTES_PER_CELL_K64_FLUX = 66
 # DRAM bytes per cell of one k64_flux launch, 4096 x 4096 pond-break at t = 600 s: ncu
-# dram__bytes_read.sum + dram__bytes_write.sum = 821.7 + 250.3 MB over 16.78 M cells
-TRAFFIC_PER_CELL_K64_FLUX = 63.90
+# dram__bytes_read.sum + dram__bytes_write.sum = 845.4 + 259.5 MB over 16.78 M cells
+TRAFFIC_PER_CELL_K64_FLUX = 65.86
 BYTES_PER_CELL_FP32_CFG3 = 37  # h,qx,qy r+w 24 + z offset 4 + info byte 1 + Kahan compensation r+w 8
 # DRAM bytes per cell-update of the FP32 step (k32_persist), 4096 x 4096 precision form at t = 1200 s,
-# one launch of four iterations: ncu dram__bytes_read.sum + dram__bytes_write.sum = 1419.1 + 1031.9 MB
+# one launch of four iterations: ncu dram__bytes_read.sum + dram__bytes_write.sum = 1454.3 + 1037.8 MB
 # over 4 x 16.78 M cell-updates; every field is streamed once per iteration, so the figure scales with cells
-TRAFFIC_PER_CELL_K32 = 36.52
+TRAFFIC_PER_CELL_K32 = 37.13
 
 
 class TimedRegion:
@@ -504,8 +504,8 @@ def make_batch_specs(n, lo, hi, seed, t_scale=1.0):
 
 def run_batched_leg(args, peak, fp64_value):
     """The batched form: 256 scenarios of uneven size advanced together, one
-    row-marching launch per feature class and a finalize per iteration
-    (graph-captured chunks), each scenario with its own CFL length."""
+    persistent launch per feature class and chunk of iterations, each scenario
+    with its own CFL length."""
     from sw2d_efdc_gb300 import api
     t0 = time.time()
     specs = make_batch_specs(args.batch_n, 128, 2048, 4)
@@ -732,8 +732,8 @@ def run_ours(args):
     roof.update({"peak_source": peak_kind,
                  "iteration": {"achieved": round(achieved_it, 2), "bytes_per_cell_update": BYTES_PER_CELL_FP64_CFG2,
                                "frac": round(achieved_it / peak, 5)},
-                 "note": "binary64 arithmetic bounds the FP64 step on GB300 (FP64 pipe 80-84% busy in k64_flux and "
-                         "k64_update, ncu), not HBM; the FP32 precision form is the HBM-bound path"})
+                 "note": "binary64 arithmetic bounds the FP64 step on GB300 (FP64 pipe 68-69% busy in k64_flux and "
+                         "k64_update beside the integer work that replaced binary64, ncu), not HBM; the FP32 precision form is the HBM-bound path"})
     out = {
         "metric": METRIC, "value": round(value, 4), "unit": UNIT, "n_gpus": world, "steps": K,
         "warmup": W, "ms_per_step": round(ms_iter, 4), "higher_is_better": True, "scaling": "weak",

@@ -1061,6 +1061,7 @@ __device__ __noinline__ unsigned wait_ticket(unsigned q, const Scn32* __restrict
     return q;
 }
 
+static_assert(sizeof(ScnBody32) / 16 <= NT - 32 && T32_MAXCLASS <= NT - 32, "prepare_item copies with three warps");
 /* What the CTA's next item needs besides the previous iteration's results,
  * into shared memory before the wait for those (which empties the L1), by all
  * warps but the first: that one counts the item before meanwhile. */
