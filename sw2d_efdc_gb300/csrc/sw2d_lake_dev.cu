@@ -27,8 +27,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
-#include <mutex>
 
 namespace sw2d {
 void set_error_message(const char* msg); /* sw2d_api.cu */
@@ -116,11 +116,42 @@ constexpr int kHash = 32768;    /* slots of its table */
 constexpr int kSolveThreads = 1024;
 constexpr int kPer = kListMax / kSolveThreads;
 
-/* The list of a call in flight: its length, then the cells.  One per device
- * and context; calls take turns (list_mutex), each synchronises its stream
- * before it returns. */
-__device__ int g_lake_list[1 + kListMax];
-std::mutex list_mutex;
+/* The lists of the calls in flight: a list's length, then the cells.  A call
+ * takes a free one for as long as it runs (it synchronises its stream before
+ * it returns), so calls of several threads, streams and devices run side by
+ * side; one that finds none free allocates its own.  The array is per device
+ * and context; a number is taken in all of them at once. */
+constexpr int kLists = 8;
+__device__ int g_lake_list[kLists][1 + kListMax];
+std::atomic<unsigned> lists_taken{0u};
+
+class ListOfCall {
+  public:
+    ~ListOfCall() {
+        if (number_ >= 0) lists_taken.fetch_and(~(1u << number_));
+        if (own_) cudaFree(own_);
+    }
+    /* the call's list on the current device */
+    cudaError_t take(int** list) {
+        unsigned t = lists_taken.load();
+        while (t != (1u << kLists) - 1u) {
+            const unsigned free_bit = ~t & (t + 1u);
+            if (!lists_taken.compare_exchange_weak(t, t | free_bit)) continue;
+            while (free_bit >> ++number_ != 1u) {}
+            void* base = nullptr;
+            const cudaError_t e = cudaGetSymbolAddress(&base, g_lake_list);
+            *list = static_cast<int*>(base) + (size_t)number_ * (1 + kListMax);
+            return e;
+        }
+        const cudaError_t e = cudaMalloc(&own_, sizeof(int) * (1 + kListMax));
+        *list = own_;
+        return e;
+    }
+
+  private:
+    int number_ = -1;
+    int* own_ = nullptr;
+};
 
 /* edge cells in any order; count[0] their number, also past the list's end */
 __global__ void k_lake_list(const int* __restrict__ m, int R, int C, int* __restrict__ count, int* __restrict__ list) {
@@ -256,9 +287,10 @@ extern "C" int sw2d_lake_catchment_smooth_device(int rows, int cols, const int* 
     const int grid = (int)std::min<long long>((n + 255) / 256, 152 * 16);
     int total = 0;
     {
-        std::lock_guard<std::mutex> turn(list_mutex);
+        ListOfCall mine;
         int* d_list = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(reinterpret_cast<void**>(&d_list), g_lake_list);
+        cudaError_t e = mine.take(&d_list);
+        if (e == cudaErrorMemoryAllocation) return fail(SW2D_ERR_NOMEM, "cudaMalloc", e);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_lake_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LakeSolve));
         if (e == cudaSuccess) e = cudaMemsetAsync(d_list, 0, sizeof(int), s);
@@ -268,7 +300,7 @@ extern "C" int sw2d_lake_catchment_smooth_device(int rows, int cols, const int* 
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(&total, d_list, sizeof(int), cudaMemcpyDeviceToHost, s);
-        const cudaError_t es = cudaStreamSynchronize(s); /* also after an error: the next call may use the list */
+        const cudaError_t es = cudaStreamSynchronize(s); /* also after an error: another call may take the list next */
         if (e == cudaSuccess) e = es;
         if (e != cudaSuccess) return fail(SW2D_ERR_CUDA, "lake-edge device pass", e);
         if (total <= kListMax) return SW2D_OK;
