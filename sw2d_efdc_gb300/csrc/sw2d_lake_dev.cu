@@ -312,22 +312,16 @@ extern "C" int sw2d_lake_catchment_smooth_device(int rows, int cols, const int* 
     cudaError_t e = cudaMalloc(&d_cnt, sizeof(int) * (size_t)(2 * nd + 2));
     if (e != cudaSuccess) return fail(SW2D_ERR_NOMEM, "cudaMalloc", e);
     int* d_fill = d_cnt + nd + 1;
-    e = cudaMemsetAsync(d_cnt, 0, sizeof(int) * (size_t)(2 * nd + 2), s);
+    e = cudaMalloc(&d_list, sizeof(int) * (size_t)total);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, sizeof(int) * (size_t)(2 * nd + 2), s);
     if (e == cudaSuccess) {
         k_lake_count<<<grid, 256, 0, s>>>(d_mask, rows, cols, d_cnt);
         k_lake_scan<<<1, 1024, 0, s>>>(d_cnt, nd);
-        e = cudaMemcpyAsync(&total, d_cnt + nd, sizeof(int), cudaMemcpyDeviceToHost, s);
+        k_lake_fill<<<grid, 256, 0, s>>>(d_mask, rows, cols, d_cnt, d_fill, d_list);
+        k_lake_sweep<<<1, 1024, 0, s>>>(d_mask, cols, d_cnt, d_list, nd, d_dem);
+        e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess && total > 0) {
-        e = cudaMalloc(&d_list, sizeof(int) * (size_t)total);
-        if (e == cudaSuccess) {
-            k_lake_fill<<<grid, 256, 0, s>>>(d_mask, rows, cols, d_cnt, d_fill, d_list);
-            k_lake_sweep<<<1, 1024, 0, s>>>(d_mask, cols, d_cnt, d_list, nd, d_dem);
-            e = cudaGetLastError();
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        }
-    }
     cudaFree(d_list);
     cudaFree(d_cnt);
     if (e != cudaSuccess) return fail(SW2D_ERR_CUDA, "lake-edge device pass", e);
