@@ -313,6 +313,11 @@ __device__ __noinline__ void raise_speed(unsigned long long* at, double vel, dou
     const unsigned long long v = sw2d_f64_bits(face_speed(vel, sw2d_half(ha + hb), g, rd));
     if (v <= 0x7ff0000000000000ull && v > __ldcg(at)) atomicMax(at, v);
 }
+/* the same for a face whose mean depth is known by estimate only */
+__device__ __noinline__ void raise_speed_exact(unsigned long long* at, double vel, double ha, double hb, double g, double rd,
+                                               double th) {
+    if (mean_ge_exact(ha, hb, th)) raise_speed(at, vel, ha, hb, g, rd);
+}
 
 /* 8 bytes from global to shared memory past the registers; zeros when !in */
 __device__ __forceinline__ void copy8_async(double* to, const double* from, bool in) {
@@ -486,10 +491,15 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
         unsigned long long* best = p.flight->smax[cur];
         const float cx = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best)));
         const float cy = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best + 1)));
-        const float wx = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ex))), cx) * 0.99999f;
-        const float wy = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ey))), cy) * 0.99999f;
-        if (okx && ex >= wx) raise_speed(best, sf[U + s0], sh[s0], sh[s0 - SW], p.g, p.rdx);
-        if (oky && ey >= wy) raise_speed(best + 1, sf[V + s0], sh[s0], sh[s0 - 1], p.g, p.rdy);
+        const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ex)));
+        const float my = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ey)));
+        if (mx < 1e30f && my < 1e30f) {
+            if (okx && ex >= fmaxf(mx, cx) * 0.99999f) raise_speed(best, sf[U + s0], sh[s0], sh[s0 - SW], p.g, p.rdx);
+            if (oky && ey >= fmaxf(my, cy) * 0.99999f) raise_speed(best + 1, sf[V + s0], sh[s0], sh[s0 - 1], p.g, p.rdy);
+        } else { /* an infinite or NaN velocity would hide the warp's other faces: all of them */
+            if (okx) raise_speed_exact(best, sf[U + s0], sh[s0], sh[s0 - SW], p.g, p.rdx, th);
+            if (oky) raise_speed_exact(best + 1, sf[V + s0], sh[s0], sh[s0 - 1], p.g, p.rdy, th);
+        }
     }
     for (int k = t; k < cnt[1]; k += NT) {
         const int id = flist[NF - 1 - k], ft = (id & 1023) >> 1, ly = ft / BX, lx = ft % BX;

@@ -1,0 +1,56 @@
+"""CFL speed of states with depths that are NaN in the FP64 step.  The speed is the maximum over faces between two active cells whose
+mean depth is >= th, in binary64; a face whose mean depth is NaN has none.
+Tolerance: bit-identical to numpy's binary64 evaluation of that rule (|q| / hm,
+the square root and the sum are single IEEE operations on both sides)."""
+import numpy as np
+import pytest
+
+from sw2d_efdc_gb300 import api
+
+pytestmark = pytest.mark.gpu
+
+G, ND = 9.80, -9999.0
+
+
+def _speed(h, qx, qy, dx, th):
+    """The rule above; a NaN speed (of a NaN discharge) counts."""
+    s = 0.0
+    with np.errstate(all="ignore"):
+        for a, b, q in ((h[:-1], h[1:], qx[1:-1]), (h[:, :-1], h[:, 1:], qy[:, 1:-1])):
+            hm = 0.5 * (a + b)
+            v = (np.abs(np.where(q == 0, 0.0, q / hm)) + np.sqrt(G * hm)) * (1.0 / dx)
+            v = v[hm >= th]
+            s += np.max(v) if v.size else 0.0
+    return s
+
+
+def _stepped(h, dx, th):
+    """The step's own speed of the entering state h (discharges zero), as its ledger has it."""
+    R, C = h.shape
+    m = api.Model(api.default_config(rows=R, cols=C, dx=dx, dy=dx, dt_mode=api.DT_CFL, series_mode=api.SERIES_STEP,
+                                     manning=0.03, cfl=0.1, dt_max=0.01, th=th, g=G, nodata=ND))
+    m.set_dem(np.zeros((R, C)))
+    m.set_rain_series(np.zeros(4), 3600.0)
+    m.set_depth(h)
+    m.step(1)
+    s = m.ledger()["s_max"]
+    m.close()
+    return s
+
+
+def _zero_q(h):
+    R, C = h.shape
+    return np.zeros((R + 1, C)), np.zeros((R, C + 1))
+
+
+def _nan_beside_deep_water():
+    h = np.full((40, 70), 0.01)
+    h[10, 20] = 2.0     # the fastest faces, in the same rows of 32 cells as the NaN's
+    h[10, 5] = np.nan
+    return h
+
+
+def test_step_nan_hides_no_other_face():
+    h = _nan_beside_deep_water()
+    got, want = _stepped(h, 10.0, 1e-4), _speed(h, *_zero_q(h), 10.0, 1e-4)
+    assert got == want
