@@ -360,8 +360,9 @@ __device__ __forceinline__ void after_previous() { cudaGridDependencySynchronize
  * stream each (they differ in shared-memory offsets and selected operands).
  * CFL: face speeds estimated in binary32; a warp whose best estimate does
  * not reach the running maximum is done, else its lanes within 1e-5 of the
- * best are evaluated in binary64 and raise the maximum: the result is the
- * exact maximum in any order. */
+ * best are evaluated in binary64 and raise the maximum, all of its lanes where
+ * an estimate says nothing (1e30 and above): the result is the exact maximum
+ * in any order. */
 template <int BY, int NT, int PER_SM>
 __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
     constexpr int BX = SW2D_BX, NF = 2 * BX * BY, SW = BX + 2, NV = (BY + 2) * SW, NH = (BY + 1) * SW;
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
             sh[k] = hh;
             so[k] = sw2d_ord(hh + zz);
             so[NH + k] = sw2d_ord(zz);
-            shf[k] = sw2d_f32_est_hi(hh);
+            shf[k] = sw2d_f32_est_depth(hh);
             scode[k] = (uint8_t)((in ? (flags[g] & SW2D_F_ACTIVE) : 0) | (sw2d_gt_pos(hh, th) ? kWet : 0) |
                                  (sw2d_lt_pos(hh, th) ? kBelow : 0));
         }
@@ -496,7 +497,7 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
         if (mx < 1e30f && my < 1e30f) {
             if (okx && ex >= fmaxf(mx, cx) * 0.99999f) raise_speed(best, sf[U + s0], sh[s0], sh[s0 - SW], p.g, p.rdx);
             if (oky && ey >= fmaxf(my, cy) * 0.99999f) raise_speed(best + 1, sf[V + s0], sh[s0], sh[s0 - 1], p.g, p.rdy);
-        } else { /* an infinite or NaN velocity would hide the warp's other faces: all of them */
+        } else { /* a negative, infinite or NaN depth or velocity, which would hide the warp's other faces: all of them */
             if (okx) raise_speed_exact(best, sf[U + s0], sh[s0], sh[s0 - SW], p.g, p.rdx, th);
             if (oky) raise_speed_exact(best + 1, sf[V + s0], sh[s0], sh[s0 - 1], p.g, p.rdy, th);
         }

@@ -220,6 +220,17 @@ SW2D_HD float sw2d_f32_est_hi(double x) {
     return sw2d_f32_from_bits((hi & 0x80000000u) | (a - 0x38000000u) << 3);
 }
 
+/* A depth's estimate for a sum with another's: as above for depths that are
+ * not negative, infinity for all others (an estimate of the mean of two depths
+ * of opposite sign would have no relative error; NaN counts with them) and
+ * from 2^128. */
+SW2D_HD float sw2d_f32_est_depth(double x) {
+    uint32_t a = (uint32_t)(sw2d_f64_bits(x) >> 32);
+    a = a < 0x47f00000u ? a : 0x47f00000u;
+    a = a > 0x38000000u ? a : 0x38000000u;
+    return sw2d_f32_from_bits((a - 0x38000000u) << 3);
+}
+
 /* an estimate of (float)v for a 32-bit unsigned v (relative error below
  * 2^-22): v = hi 2^16 + lo, each half exact in binary32 by the 2^23
  * magic-number construction */

@@ -1,5 +1,6 @@
-"""CFL speed of states with depths that are NaN in the FP64 step.  The speed is the maximum over faces between two active cells whose
-mean depth is >= th, in binary64; a face whose mean depth is NaN has none.
+"""CFL speed of states with depths that are NaN or negative in the FP64 step.
+The speed is the maximum over faces between two active cells whose mean depth
+is >= th, in binary64; a face whose mean depth is NaN has none.
 Tolerance: bit-identical to numpy's binary64 evaluation of that rule (|q| / hm,
 the square root and the sum are single IEEE operations on both sides)."""
 import numpy as np
@@ -53,4 +54,33 @@ def _nan_beside_deep_water():
 def test_step_nan_hides_no_other_face():
     h = _nan_beside_deep_water()
     got, want = _stepped(h, 10.0, 1e-4), _speed(h, *_zero_q(h), 10.0, 1e-4)
+    assert got == want
+
+
+def _cancelling(rng, th, off):
+    """Cells of 1 to 1000 m, each beside one negative cell that leaves a mean
+    depth of th + off; every other mean is negative."""
+    h = np.full((34, 66), -4000.0)
+    for r in range(2, 32, 4):
+        for c in range(2, 62, 4):
+            a = float(rng.uniform(1.0, 1000.0))
+            h[r, c] = a
+            h[r, c + 1] = 2.0 * (th + off) - a
+    return h
+
+
+@pytest.mark.parametrize("off", [1e-10, -1e-10, 1e-5, -3e-5])
+@pytest.mark.parametrize("run", [_stepped], ids=["step"])
+def test_depths_of_opposite_sign(run, off):
+    h = _cancelling(np.random.default_rng(7), 1e-4, off)
+    got, want = run(h, 10.0, 1e-4), _speed(h, *_zero_q(h), 10.0, 1e-4)
+    assert got == want
+
+
+@pytest.mark.parametrize("run", [_stepped], ids=["step"])
+def test_the_fastest_face_between_depths_of_opposite_sign(run):
+    h = np.full((34, 66), -4000.0)
+    h[4, 4], h[4, 5] = 0.5001, 0.5001
+    h[4, 12], h[4, 13] = 1000.0 + 4.8e-4, -999.0  # mean 0.50024; truncated to 21 bits 0.5
+    got, want = run(h, 10.0, 1e-4), _speed(h, *_zero_q(h), 10.0, 1e-4)
     assert got == want
