@@ -51,6 +51,12 @@ __device__ __noinline__ void raise_speed(unsigned long long* at, double q, doubl
     const unsigned long long v = sw2d_f64_bits((fabs(vel) + sw2d_sqrt_rn(g * hm)) * rd);
     if (v > __ldcg(at)) atomicMax(at, v);
 }
+/* the same for a face whose mean depth is known by estimate only; one whose
+ * mean depth is NaN has no speed */
+__device__ __noinline__ void raise_speed_exact(unsigned long long* at, double q, double ha, double hb, double g, double rd,
+                                               double th) {
+    if (0.50 * (ha + hb) >= th) raise_speed(at, q, ha, hb, g, rd);
+}
 __device__ __noinline__ bool mean_ge_exact(double ha, double hb, double th) {
     return sw2d_ge_pos(0.50 * (ha + hb), th);
 }
@@ -161,8 +167,18 @@ __global__ void __launch_bounds__(256, kBlocksPerSm) k64_measure_noalloc(Measure
             }
             const float cx = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best)));
             const float cy = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best + 1)));
-            const float tx = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bx))), cx) * 0.99999f;
-            const float ty = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(by))), cy) * 0.99999f;
+            const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bx)));
+            const float my = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(by)));
+            const float tx = fmaxf(mx, cx) * 0.99999f, ty = fmaxf(my, cy) * 0.99999f;
+            if (!(mx < 1e30f && my < 1e30f)) {
+                /* an infinite or NaN depth or discharge would hide the warp's other faces: all of them */
+#pragma unroll
+                for (int k = 0; k < kBatch; k++) {
+                    if (ex[k] >= 0.f) raise_speed_exact(best, qx[k], h[k], hn[k], p.g, p.rdx, th);
+                    if (ey[k] >= 0.f) raise_speed_exact(best + 1, qy[k], h[k], hw[k], p.g, p.rdy, th);
+                }
+                continue;
+            }
             if (bx >= tx) {
 #pragma unroll
                 for (int k = 0; k < kBatch; k++)

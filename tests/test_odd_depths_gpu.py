@@ -1,6 +1,6 @@
-"""CFL speed of states with depths that are NaN or negative in the FP64 step.
-The speed is the maximum over faces between two active cells whose mean depth
-is >= th, in binary64; a face whose mean depth is NaN has none.
+"""CFL speed of states with depths that are infinite, NaN or negative in the
+FP64 step and in the no-allocation measure.  The speed is the maximum over
+faces between two active cells whose mean depth is >= th, in binary64; a face whose mean depth is NaN has none.
 Tolerance: bit-identical to numpy's binary64 evaluation of that rule (|q| / hm,
 the square root and the sum are single IEEE operations on both sides)."""
 import numpy as np
@@ -9,6 +9,8 @@ import pytest
 from sw2d_efdc_gb300 import api
 
 pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
 
 G, ND = 9.80, -9999.0
 
@@ -39,6 +41,15 @@ def _stepped(h, dx, th):
     return s
 
 
+def _measured(h, dx, th, qx=None, qy=None):
+    R, C = h.shape
+    qx = np.zeros((R + 1, C)) if qx is None else qx
+    qy = np.zeros((R, C + 1)) if qy is None else qy
+    a = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (np.zeros((R, C)), h, qx, qy)]
+    torch.cuda.synchronize()
+    return api.measure_state_noalloc(*[x.data_ptr() for x in a], R, C, dx, dx, ND, th, G)[1]
+
+
 def _zero_q(h):
     R, C = h.shape
     return np.zeros((R + 1, C)), np.zeros((R, C + 1))
@@ -55,6 +66,27 @@ def test_step_nan_hides_no_other_face():
     h = _nan_beside_deep_water()
     got, want = _stepped(h, 10.0, 1e-4), _speed(h, *_zero_q(h), 10.0, 1e-4)
     assert got == want
+
+
+def test_measure_nan_depth_has_no_speed():
+    h = _nan_beside_deep_water()
+    got, want = _measured(h, 10.0, 1e-4), _speed(h, *_zero_q(h), 10.0, 1e-4)
+    assert got == want
+
+
+def test_measure_nan_discharge_shows_in_the_speed():
+    h = np.full((40, 70), 0.5)
+    qx, qy = _zero_q(h)
+    qx[7, 9] = np.nan
+    assert np.isnan(_measured(h, 10.0, 1e-4, qx, qy))
+    qx[7, 9] = np.inf
+    assert _measured(h, 10.0, 1e-4, qx, qy) == np.inf
+
+
+def test_measure_infinite_depth():
+    h = np.full((40, 70), 0.5)
+    h[3, 4] = np.inf
+    assert _measured(h, 10.0, 1e-4) == np.inf
 
 
 def _cancelling(rng, th, off):
