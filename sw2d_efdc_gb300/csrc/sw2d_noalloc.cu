@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(256, kBlocksPerSm) k64_measure_noalloc(Measure
                     hw[k] = hl[k];
                 }
                 hn[k] = h_n;
-                const float hf = sw2d_f32_est_hi(h[k]);
-                const float mx = 0.5f * (hf + sw2d_f32_est_hi(h_n)), my = 0.5f * (hf + sw2d_f32_est_hi(hw[k]));
+                const float hf = sw2d_f32_est_depth(h[k]);
+                const float mx = 0.5f * (hf + sw2d_f32_est_depth(h_n)), my = 0.5f * (hf + sw2d_f32_est_depth(hw[k]));
                 const bool okx = act && act_n && mean_ge(h_n, h[k], mx, th, p.thf);
                 const bool oky = act && aw && mean_ge(hw[k], h[k], my, th, p.thf);
                 ex[k] = okx ? (fabsf(sw2d_f32_est_hi(qx[k])) * sw2d_rcp_est(mx) + sw2d_sqrt_est(p.gf * mx)) * p.rdxf : -1.f;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256, kBlocksPerSm) k64_measure_noalloc(Measure
             const float my = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(by)));
             const float tx = fmaxf(mx, cx) * 0.99999f, ty = fmaxf(my, cy) * 0.99999f;
             if (!(mx < 1e30f && my < 1e30f)) {
-                /* an infinite or NaN depth or discharge would hide the warp's other faces: all of them */
+                /* a negative, infinite or NaN depth or discharge, which would hide the warp's other faces: all of them */
 #pragma unroll
                 for (int k = 0; k < kBatch; k++) {
                     if (ex[k] >= 0.f) raise_speed_exact(best, qx[k], h[k], hn[k], p.g, p.rdx, th);

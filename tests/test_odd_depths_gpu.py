@@ -102,14 +102,14 @@ def _cancelling(rng, th, off):
 
 
 @pytest.mark.parametrize("off", [1e-10, -1e-10, 1e-5, -3e-5])
-@pytest.mark.parametrize("run", [_stepped], ids=["step"])
+@pytest.mark.parametrize("run", [_stepped, _measured], ids=["step", "measure"])
 def test_depths_of_opposite_sign(run, off):
     h = _cancelling(np.random.default_rng(7), 1e-4, off)
     got, want = run(h, 10.0, 1e-4), _speed(h, *_zero_q(h), 10.0, 1e-4)
     assert got == want
 
 
-@pytest.mark.parametrize("run", [_stepped], ids=["step"])
+@pytest.mark.parametrize("run", [_stepped, _measured], ids=["step", "measure"])
 def test_the_fastest_face_between_depths_of_opposite_sign(run):
     h = np.full((34, 66), -4000.0)
     h[4, 4], h[4, 5] = 0.5001, 0.5001
