@@ -714,10 +714,8 @@ __device__ void advance_clock(const StepParams& p, int cur) {
 /* SW2D-EFDC.cu:602-664, :695-725, :362-452 in one pass                       */
 
 /* "active and provisional depth < th" of a cell, decided from a binary32
- * estimate of the depth: 0 or 1, or 2 where th lies within the estimate's
- * error (2^-17 of the magnitudes that enter it; their truncation to 21 bits
- * and the estimate's own rounding stay below 2^-18 of them) and the exact
- * binary64 continuity has to decide. */
+ * estimate of the depth (sw2d_dry_est): 0 or 1, or 2 where the exact binary64
+ * continuity has to decide. */
 template <bool FULL>
 __device__ __noinline__ bool provisional_exact(const StepParams& p, const Slot& s, size_t i, uint8_t f, double ho,
                                                double fN, double fS, double fW, double fE) {
@@ -727,8 +725,6 @@ __device__ __noinline__ bool provisional_exact(const StepParams& p, const Slot& 
 template <bool FULL>
 __device__ __forceinline__ uint8_t provisional_dry(const StepParams& p, float dt2, float rl, float rd, float ev, size_t i,
                                                    uint8_t f, double ho, double fN, double fS, double fW, double fE) {
-    const float h = sw2d_f32_est_hi(ho), n = sw2d_f32_est_hi(fN), so = sw2d_f32_est_hi(fS), w = sw2d_f32_est_hi(fW),
-                e = sw2d_f32_est_hi(fE);
     const bool lake = sw2d_gt(ho, p.ev_wl_min);
     float src = lake ? rl : rd;
     if (p.rainw) src *= p.rainw[i];
@@ -737,11 +733,9 @@ __device__ __forceinline__ uint8_t provisional_dry(const StepParams& p, float dt
         src -= ev;
         mag += fabsf(ev);
     }
-    const float hs = h - dt2 * ((so - n) * p.rdxf + (e - w) * p.rdyf - src);
-    mag = h + dt2 * ((fabsf(so) + fabsf(n)) * p.rdxf + (fabsf(e) + fabsf(w)) * p.rdyf + mag) + p.thf;
-    const float d = hs - p.thf;
-    if ((FULL && (f & SW2D_F_SOURCE)) || !(fabsf(d) > 7.6293945e-6f * mag + 1e-35f) || !(mag < 1e37f)) return 2;
-    return d < 0.f ? 1 : 0;
+    const int dry = sw2d_dry_est(sw2d_f32_est_hi(ho), sw2d_f32_est_hi(fN), sw2d_f32_est_hi(fS), sw2d_f32_est_hi(fW),
+                                 sw2d_f32_est_hi(fE), src, mag, dt2, p.rdxf, p.rdyf, p.thf);
+    return (uint8_t)(FULL && (f & SW2D_F_SOURCE) ? 2 : dry);
 }
 
 /* FULL: evaporation, point sources or rain whose ledger is kept per cell.

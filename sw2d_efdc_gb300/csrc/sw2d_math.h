@@ -211,13 +211,30 @@ SW2D_HD float sw2d_f32_est_of_f64(double x) {
 /* The same from the high word alone, for the prefilters that run on every
  * cell: the significand truncated to 21 bits (relative error below 2^-20),
  * magnitudes below 2^-126 within 2^-126, 2^128 and above (infinities and NaN
- * too) the largest finite value. */
+ * too) infinity. */
 SW2D_HD float sw2d_f32_est_hi(double x) {
     const uint32_t hi = (uint32_t)(sw2d_f64_bits(x) >> 32);
     uint32_t a = hi & 0x7fffffffu;
-    a = a < 0x47efffffu ? a : 0x47efffffu;
+    a = a < 0x47f00000u ? a : 0x47f00000u;
     a = a > 0x38000000u ? a : 0x38000000u;
     return sw2d_f32_from_bits((hi & 0x80000000u) | (a - 0x38000000u) << 3);
+}
+
+/* "depth h - dt2 ((qs - qn) rdx + (qe - qw) rdy - src), or 0 if that is
+ * negative, < th" from sw2d_f32_est_hi of the binary64 values (src, dt2 and
+ * the spacings truncated or rounded to binary32; srcmag: the magnitudes that
+ * src is the sum of): 0 or 1, or 2 where th lies within the estimate's error
+ * (2^-17 of the magnitudes that enter it; their truncation to 21 bits and the
+ * estimate's own rounding stay below 2^-18 of them) or an infinity or NaN
+ * takes part. */
+SW2D_HD int sw2d_dry_est(float h, float qn, float qs, float qw, float qe, float src, float srcmag, float dt2, float rdx,
+                         float rdy, float th) {
+    const float hs = h - dt2 * ((qs - qn) * rdx + (qe - qw) * rdy - src);
+    const float mag =
+        fabsf(h) + dt2 * ((fabsf(qs) + fabsf(qn)) * rdx + (fabsf(qe) + fabsf(qw)) * rdy + srcmag) + th;
+    const float d = hs - th;
+    if (!(fabsf(d) > 7.6293945e-6f * mag + 1e-35f) || !(mag < 1e37f)) return 2;
+    return d < 0.f ? 1 : 0;
 }
 
 /* A depth's estimate for a sum with another's: as above for depths that are
