@@ -164,7 +164,9 @@ struct sw2d_handle {
         };
         p.kdx = pow2_exp(cfg.dx);
         p.kdy = pow2_exp(cfg.dy);
-        p.thf = (float)cfg.th;
+        const bool est = sw2d_est_range(cfg.th) && sw2d_est_range(cfg.g) && sw2d_est_range(cfg.dx) && sw2d_est_range(cfg.dy);
+        p.thf = est ? (float)cfg.th : std::numeric_limits<float>::quiet_NaN();
+        p.est_most = est ? SW2D_EST_MOST : 0.f;
         p.gf = (float)cfg.g;
         p.rdxf = (float)p.rdx;
         p.rdyf = (float)p.rdy;

@@ -331,7 +331,7 @@ __device__ __forceinline__ void copy8_async(double* to, const double* from, bool
  * within its error */
 __device__ __forceinline__ bool mean_ge(double ha, double hb, int ca, int cb, float est, double th, float thf) {
     if (!((ca ^ cb) & kBelow)) return !(ca & kBelow);
-    if (fabsf(est - thf) > 1e-5f * thf) return est > thf;
+    if (fabsf(est - thf) > 1e-5f * thf) return est > thf; /* not with thf NaN */
     return mean_ge_exact(ha, hb, th);
 }
 
@@ -361,8 +361,8 @@ __device__ __forceinline__ void after_previous() { cudaGridDependencySynchronize
  * CFL: face speeds estimated in binary32; a warp whose best estimate does
  * not reach the running maximum is done, else its lanes within 1e-5 of the
  * best are evaluated in binary64 and raise the maximum, all of its lanes where
- * an estimate says nothing (1e30 and above): the result is the exact maximum
- * in any order. */
+ * an estimate says nothing (est_most and above): the result is the exact
+ * maximum in any order. */
 template <int BY, int NT, int PER_SM>
 __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
     constexpr int BX = SW2D_BX, NF = 2 * BX * BY, SW = BX + 2, NV = (BY + 2) * SW, NH = (BY + 1) * SW;
@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(NT, PER_SM) k64_flux(StepParams p, int cur) {
         const float cy = sw2d_f32_est_hi(__longlong_as_double((long long)__ldcg(best + 1)));
         const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ex)));
         const float my = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ey)));
-        if (mx < 1e30f && my < 1e30f) {
+        if (mx < p.est_most && my < p.est_most) {
             if (okx && ex >= fmaxf(mx, cx) * 0.99999f) raise_speed(best, sf[U + s0], sh[s0], sh[s0 - SW], p.g, p.rdx);
             if (oky && ey >= fmaxf(my, cy) * 0.99999f) raise_speed(best + 1, sf[V + s0], sh[s0], sh[s0 - 1], p.g, p.rdy);
         } else { /* a negative, infinite or NaN depth or velocity, which would hide the warp's other faces: all of them */

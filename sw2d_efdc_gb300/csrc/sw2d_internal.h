@@ -105,7 +105,9 @@ struct StepParams {
     double gnn_uni;        /* (g n) n of the uniform n */
     int kdx, kdy;          /* dx = 2^kdx (dy = 2^kdy) when a power of two >= 1, else -1 */
     sw2d_divisor ddx, ddy;
-    float thf, gf, rdxf, rdyf, plf, pdf; /* th, g, 1/dx, 1/dy and the runoff fractions in binary32, for the prefilters */
+    /* th, g, 1/dx, 1/dy and the runoff fractions in binary32, for the prefilters; where one of them is outside
+     * sw2d_est_range thf is NaN and est_most 0, which leave everything to binary64 */
+    float thf, gf, rdxf, rdyf, plf, pdf, est_most;
     const float* rainw;    /* rain weight per cell or NULL */
     const int* src_idx;    /* padded cell index per source */
     const double* rain;    /* nrain + 2 */

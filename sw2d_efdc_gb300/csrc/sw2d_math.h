@@ -220,13 +220,18 @@ SW2D_HD float sw2d_f32_est_hi(double x) {
     return sw2d_f32_from_bits((hi & 0x80000000u) | (a - 0x38000000u) << 3);
 }
 
+/* The estimates hold for parameters of a run (threshold, gravity,
+ * spacings) in this range; with others every value is evaluated in binary64. */
+SW2D_HD int sw2d_est_range(double x) { return x >= 1e-30 && x <= 1e30; }
+#define SW2D_EST_MOST 1e30f /* speeds up to here are compared by their estimates */
+
 /* "depth h - dt2 ((qs - qn) rdx + (qe - qw) rdy - src), or 0 if that is
  * negative, < th" from sw2d_f32_est_hi of the binary64 values (src, dt2 and
  * the spacings truncated or rounded to binary32; srcmag: the magnitudes that
  * src is the sum of): 0 or 1, or 2 where th lies within the estimate's error
  * (2^-17 of the magnitudes that enter it; their truncation to 21 bits and the
  * estimate's own rounding stay below 2^-18 of them) or an infinity or NaN
- * takes part. */
+ * takes part.  For values of sw2d_est_range's parameters; with others pass a NaN th. */
 SW2D_HD int sw2d_dry_est(float h, float qn, float qs, float qw, float qe, float src, float srcmag, float dt2, float rdx,
                          float rdy, float th) {
     const float hs = h - dt2 * ((qs - qn) * rdx + (qe - qw) * rdy - src);

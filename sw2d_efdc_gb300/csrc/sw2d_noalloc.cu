@@ -88,7 +88,7 @@ struct MeasureIn {
     const double *dem, *h, *qx, *qy;
     int R, C;
     double nodata, th, g, rdx, rdy, area;
-    float thf, gf, rdxf, rdyf;
+    float thf, gf, rdxf, rdyf, est_most; /* StepParams' */
     int band; /* rows of a warp's task */
 };
 
@@ -170,12 +170,12 @@ __global__ void __launch_bounds__(256, kBlocksPerSm) k64_measure_noalloc(Measure
             const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bx)));
             const float my = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(by)));
             const float tx = fmaxf(mx, cx) * 0.99999f, ty = fmaxf(my, cy) * 0.99999f;
-            if (!(mx < 1e30f && my < 1e30f)) {
+            if (!(mx < p.est_most && my < p.est_most)) {
                 /* a negative, infinite or NaN depth or discharge, which would hide the warp's other faces: all of them */
 #pragma unroll
                 for (int k = 0; k < kBatch; k++) {
-                    if (ex[k] >= 0.f) raise_speed_exact(best, qx[k], h[k], hn[k], p.g, p.rdx, th);
-                    if (ey[k] >= 0.f) raise_speed_exact(best + 1, qy[k], h[k], hw[k], p.g, p.rdy, th);
+                    if (!(ex[k] < 0.f)) raise_speed_exact(best, qx[k], h[k], hn[k], p.g, p.rdx, th);
+                    if (!(ey[k] < 0.f)) raise_speed_exact(best + 1, qy[k], h[k], hw[k], p.g, p.rdy, th);
                 }
                 continue;
             }
@@ -275,7 +275,9 @@ extern "C" int sw2d_measure_state_noalloc(const double* d_dem, const double* d_d
     in.rdx = 1.0 / dx;
     in.rdy = 1.0 / dy;
     in.area = dx * dy;
-    in.thf = (float)th;
+    const bool est = sw2d_est_range(th) && sw2d_est_range(g) && sw2d_est_range(dx) && sw2d_est_range(dy);
+    in.thf = est ? (float)th : std::nanf("");
+    in.est_most = est ? SW2D_EST_MOST : 0.f;
     in.gf = (float)g;
     in.rdxf = (float)in.rdx;
     in.rdyf = (float)in.rdy;

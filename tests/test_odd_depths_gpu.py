@@ -1,6 +1,7 @@
-"""CFL speed of states with depths that are infinite, NaN or negative in the
-FP64 step and in the no-allocation measure.  The speed is the maximum over
-faces between two active cells whose mean depth is >= th, in binary64; a face whose mean depth is NaN has none.
+"""CFL speed of states with depths that are infinite, NaN or negative, and with
+thresholds below the binary32 range, in the FP64 step and in the no-allocation
+measure.  The speed is the maximum over faces between two active cells whose
+mean depth is >= th, in binary64; a face whose mean depth is NaN has none.
 Tolerance: bit-identical to numpy's binary64 evaluation of that rule (|q| / hm,
 the square root and the sum are single IEEE operations on both sides)."""
 import numpy as np
@@ -115,4 +116,14 @@ def test_the_fastest_face_between_depths_of_opposite_sign(run):
     h[4, 4], h[4, 5] = 0.5001, 0.5001
     h[4, 12], h[4, 13] = 1000.0 + 4.8e-4, -999.0  # mean 0.50024; truncated to 21 bits 0.5
     got, want = run(h, 10.0, 1e-4), _speed(h, *_zero_q(h), 10.0, 1e-4)
+    assert got == want
+
+
+@pytest.mark.parametrize("th", [1e-40, 3e-39, 1e-310])
+@pytest.mark.parametrize("run", [_stepped, _measured], ids=["step", "measure"])
+def test_thresholds_below_binary32(run, th):
+    h = np.zeros((20, 40))
+    h[5, 6] = 2.5 * th     # mean 1.25 th beside a dry cell
+    h[9, 30] = 1.5 * th    # mean 0.75 th
+    got, want = run(h, 10.0, th), _speed(h, *_zero_q(h), 10.0, th)
     assert got == want
