@@ -125,7 +125,7 @@ SW2D_HD int sw2d_is0(double x) { return (sw2d_f64_bits(x) << 1) == 0; }         
 /* max(x, 0) with +0 for every x <= 0 */
 SW2D_HD double sw2d_max0(double x) { return (int64_t)sw2d_f64_bits(x) > 0 ? x : 0.0; }
 
-/* x * 2^-k for k = 1, 2, correctly rounded: an exponent decrement while the
+/* x * 2^-k for 1 <= k <= 31, correctly rounded: an exponent decrement while the
  * result stays normal, else the magnitude shifted right with
  * round-half-to-even (the subnormal result of the IEEE product). */
 SW2D_HD double sw2d_scale_down(double x, int k) {
@@ -134,10 +134,11 @@ SW2D_HD double sw2d_scale_down(double x, int k) {
     const uint64_t e = mag >> 52;
     if (e == 0x7ff) return x;                                   /* inf, NaN */
     if (e > (uint64_t)k) return sw2d_f64_from_bits(b - ((uint64_t)k << 52));
-    /* result subnormal (or zero): mag counts units of 2^-1074 including the
-     * implicit bit for e >= 1, so the result is mag / 2^k rounded */
-    const uint64_t m = (e == 0) ? mag : ((mag & 0x000fffffffffffffULL) | 0x0010000000000000ULL) << (e - 1);
-    const uint64_t q = m >> k, rem = m & ((1ULL << k) - 1), halfw = 1ULL << (k - 1);
+    /* result subnormal (or zero): the significand m counts units of 2^-1074
+     * (of 2^(e - 1 - 1074) for e >= 1), so the result is m / 2^s rounded */
+    const uint64_t m = (e == 0) ? mag : (mag & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
+    const uint32_t s = e == 0 ? (uint32_t)k : (uint32_t)k + 1u - (uint32_t)e;
+    const uint64_t q = m >> s, rem = m & ((1ULL << s) - 1), halfw = 1ULL << (s - 1);
     const uint64_t r = q + ((rem > halfw || (rem == halfw && (q & 1))) ? 1 : 0);
     return sw2d_f64_from_bits(sign | r);
 }
