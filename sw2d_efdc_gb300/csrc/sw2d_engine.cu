@@ -267,10 +267,11 @@ int Engine32::add(const ScenarioInput& in, long long id, std::string* err, int* 
      * rounded to 1/16 m, bed offsets from it with NaN for inactive cells */
     std::vector<char> pageable;
     char* stage;
-    if (staged <= std::max(kPinInputs, pin_bytes_)) {
-        if ((rc = reserve_pin(staged, err))) return fail_free(rc);
+    std::string refused;
+    if (staged <= std::max(kPinInputs, pin_bytes_) && reserve_pin(staged, &refused) == SW2D_OK) {
         stage = static_cast<char*>(pin_);
-    } else {
+    } else { /* large inputs, or no pinned memory to be had */
+        cudaGetLastError();
         pageable.resize(staged);
         stage = pageable.data();
     }
