@@ -74,10 +74,13 @@ struct Carver {
 constexpr size_t kNone = ~(size_t)0;
 constexpr size_t kPinInputs = (size_t)8 << 20; /* inputs up to here pay for pinned staging (larger ones use it if it is there) */
 
+/* An error is returned once: the runtime's own record of it is cleared, which
+ * the next call would report as its own (what broke the context stays). */
 #define ECK(call)                                                                   \
     do {                                                                            \
         cudaError_t e_ = (call);                                                    \
         if (e_ != cudaSuccess) {                                                    \
+            cudaGetLastError();                                                     \
             if (err) *err = std::string(#call) + ": " + cudaGetErrorString(e_);     \
             return e_ == cudaErrorMemoryAllocation ? SW2D_ERR_NOMEM : SW2D_ERR_CUDA; \
         }                                                                           \
@@ -218,6 +221,7 @@ int Engine32::add(const ScenarioInput& in, long long id, std::string* err, int* 
     {
         cudaError_t e = cudaMalloc((void**)&slab, cv.at);
         if (e != cudaSuccess) {
+            cudaGetLastError();
             if (err) *err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
             return SW2D_ERR_NOMEM;
         }
@@ -234,6 +238,7 @@ int Engine32::add(const ScenarioInput& in, long long id, std::string* err, int* 
     do {                                                                        \
         cudaError_t e_ = (call);                                                \
         if (e_ != cudaSuccess) {                                                \
+            cudaGetLastError();                                                 \
             if (err) *err = std::string(#call) + ": " + cudaGetErrorString(e_); \
             return fail_free(SW2D_ERR_CUDA);                                    \
         }                                                                       \
@@ -271,7 +276,6 @@ int Engine32::add(const ScenarioInput& in, long long id, std::string* err, int* 
     if (staged <= std::max(kPinInputs, pin_bytes_) && reserve_pin(staged, &refused) == SW2D_OK) {
         stage = static_cast<char*>(pin_);
     } else { /* large inputs, or no pinned memory to be had */
-        cudaGetLastError();
         pageable.resize(staged);
         stage = pageable.data();
     }

@@ -1,6 +1,8 @@
-"""Failed allocations, made by a fake of the failing call (the library's own
-objects linked with it wrapped): without pinned staging a raster's inputs go
-through pageable memory.  Results: the same bits as without the failure."""
+"""Failed allocations, made by fakes of the failing calls (the library's own
+objects linked with them wrapped): without pinned staging a raster's inputs go
+through pageable memory, and a scenario that finds no device memory waits
+without spoiling the ones that run.  Results: the same bits as without the
+failure."""
 import glob
 import os
 import subprocess
@@ -18,13 +20,19 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 FAKES = r"""
 #include <cuda_runtime.h>
 extern "C" {
-int fail_pinned = 0; /* how many calls to refuse */
+int fail_pinned = 0, fail_device = 0; /* how many calls to refuse, of cudaMalloc those of 800 kB and more */
+cudaError_t __real_cudaMalloc(void** p, size_t n);
+cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
+    if (fail_device <= 0 || n < 800000) return __real_cudaMalloc(p, n);
+    fail_device--;
+    return __real_cudaMalloc(p, (size_t)1 << 60); /* refused by the runtime, which keeps it as its last error, too */
+}
 cudaError_t __real_cudaMallocHost(void** p, size_t n);
 cudaError_t __wrap_cudaMallocHost(void** p, size_t n) {
     if (fail_pinned <= 0) return __real_cudaMallocHost(p, n);
     fail_pinned--;
     void* q = nullptr;
-    return cudaMalloc(&q, (size_t)1 << 60); /* refused by the runtime, which keeps it as its last error, too */
+    return __real_cudaMalloc(&q, (size_t)1 << 60);
 }
 }
 """
@@ -48,6 +56,36 @@ assert n.value == 0
 m.step(20)
 np.savez(sys.argv[4], **dict(zip(("h", "qx", "qy"), m.state())))
 """
+BATCH = r"""
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+from sw2d_efdc_gb300 import api
+lib = api.load(sys.argv[2])
+rng = np.random.default_rng(5)
+b = api.Batch()
+ids = []
+def submit(side):
+    dem = 0.01 * np.arange(side)[::-1, None] + 0.02 * rng.standard_normal((side, side))
+    ids.append(b.submit(dem=dem, depth=np.full((side, side), 0.02), rain_mm=np.full(4, 5.0), dtrain=300.0, dx=2.0,
+                        t_end=20.0, outflow=api.OUTFLOW_SOUTH, manning=0.03))
+submit(210)
+assert b.step(4) == (1, 0)
+submit(230)
+n = ctypes.c_int.in_dll(lib, "fail_device")
+n.value = int(sys.argv[3])
+steps = [b.step(2)]
+assert n.value == 0
+while steps[-1] != (0, 0):
+    steps.append(b.step(16))
+out = {"first": np.array(steps[0])}
+for k, i in enumerate(ids):
+    out["status%d" % k] = np.array(b.poll(i, ledger=False)[0])
+    for f, v in zip(("h", "qx", "qy"), b.result(i)):
+        out["%s%d" % (f, k)] = v
+np.savez(sys.argv[4], **out)
+"""
+
 
 @pytest.fixture(scope="module")
 def variant(tmp_path_factory):
@@ -57,7 +95,7 @@ def variant(tmp_path_factory):
     so = d / "libsw2d_fakes.so"
     subprocess.check_call([build.nvcc()] + build.ARCH + ["-shared", "-Xcompiler", "-fPIC", str(d / "fakes.cu")] +
                           sorted(glob.glob(os.path.join(build.OBJ_DIR, "*.o"))) +
-                          ["-Xlinker", "--wrap=cudaMallocHost", "-o", str(so)])
+                          ["-Xlinker", "--wrap=cudaMalloc", "-Xlinker", "--wrap=cudaMallocHost", "-o", str(so)])
     return d, so
 
 
@@ -77,3 +115,9 @@ def _same(a, b):
 
 def test_no_pinned_staging(variant):
     assert _same(_run(variant, RASTER, "pinned", 1), _run(variant, RASTER, "plain", 0))
+
+
+def test_no_device_memory_waits(variant):
+    late, plain = _run(variant, BATCH, "device", 1), _run(variant, BATCH, "plain", 0)
+    assert tuple(late.pop("first")) == (1, 1) and tuple(plain.pop("first")) == (2, 0)
+    assert _same(late, plain)
