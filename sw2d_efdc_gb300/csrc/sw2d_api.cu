@@ -35,10 +35,13 @@ int fail(int code, const std::string& msg) {
     return code;
 }
 
+/* an error is returned once: the runtime's own record of it, which another
+ * handle's next call would report as its own, is cleared */
 #define CK(call)                                                                           \
     do {                                                                                   \
         cudaError_t e_ = (call);                                                           \
         if (e_ != cudaSuccess) {                                                           \
+            cudaGetLastError();                                                            \
             return fail(e_ == cudaErrorMemoryAllocation ? SW2D_ERR_NOMEM : SW2D_ERR_CUDA,  \
                         std::string(#call) + ": " + cudaGetErrorString(e_));               \
         }                                                                                  \

@@ -1,8 +1,8 @@
 """Failed allocations, made by fakes of the failing calls (the library's own
 objects linked with them wrapped): without pinned staging a raster's inputs go
-through pageable memory, and a scenario that finds no device memory waits
-without spoiling the ones that run.  Results: the same bits as without the
-failure."""
+through pageable memory, and a scenario or a raster that finds no device
+memory does not spoil the ones that run.  Results: the same bits as without
+the failure."""
 import glob
 import os
 import subprocess
@@ -86,6 +86,31 @@ for k, i in enumerate(ids):
 np.savez(sys.argv[4], **out)
 """
 
+CREATE = r"""
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+from sw2d_efdc_gb300 import api
+lib = api.load(sys.argv[2])
+def config(side):
+    return api.default_config(rows=side, cols=side, dx=2.0, dy=2.0, dt_mode=api.DT_CFL, series_mode=api.SERIES_STEP,
+                              outflow=api.OUTFLOW_SOUTH, manning=0.03)
+m = api.Model(config(100))
+m.set_dem(0.01 * np.arange(100)[::-1, None] + np.zeros((100, 100)))
+m.set_rain_series(np.full(4, 5.0), 300.0)
+m.set_depth(np.full((100, 100), 0.02))
+n = ctypes.c_int.in_dll(lib, "fail_device")
+n.value = int(sys.argv[3])
+refused = False
+try:
+    api.Model(config(1000))
+except api.Sw2dError as e:
+    refused = e.code == -3
+assert refused == bool(int(sys.argv[3])) and n.value == 0
+m.step(20)
+np.savez(sys.argv[4], **dict(zip(("h", "qx", "qy"), m.state())))
+"""
+
 
 @pytest.fixture(scope="module")
 def variant(tmp_path_factory):
@@ -121,3 +146,7 @@ def test_no_device_memory_waits(variant):
     late, plain = _run(variant, BATCH, "device", 1), _run(variant, BATCH, "plain", 0)
     assert tuple(late.pop("first")) == (1, 1) and tuple(plain.pop("first")) == (2, 0)
     assert _same(late, plain)
+
+
+def test_a_raster_that_finds_no_device_memory(variant):
+    assert _same(_run(variant, CREATE, "refused", 1), _run(variant, CREATE, "plain", 0))
