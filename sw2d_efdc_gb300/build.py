@@ -37,7 +37,7 @@ UNITS = {
     "sw2d_case_prep.cu": ["-Xcompiler", "-ffp-contract=off"],
     "sw2d_lake_dev.cu": ["--fmad=false"],
 }
-HEADERS = ["sw2d_internal.h", "sw2d_math.h", "sw2d_fp32.h", "sw2d_engine.h"]
+HEADERS = ["sw2d_internal.h", "sw2d_math.h", "sw2d_fp32.h", "sw2d_engine.h", "sw2d_threads.h"]
 
 
 def nvcc() -> str:

@@ -11,12 +11,14 @@
 #include "sw2d_engine.h"
 #include "sw2d_test.h"
 #include "sw2d_internal.h"
+#include "sw2d_threads.h"
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <limits>
 #include <memory>
 #include <thread>
 #include <cstdio>
@@ -249,18 +251,7 @@ int stage_reserve(sw2d_handle* h, size_t bytes) {
 /* f(first, last) over [0, n) split across up to 16 host threads */
 template <typename F>
 void parallel_ranges(size_t n, F f) {
-    const size_t nt = std::max<size_t>(1, std::min<size_t>({16, std::thread::hardware_concurrency(), n / 8 + 1}));
-    if (nt == 1) {
-        f((size_t)0, n);
-        return;
-    }
-    std::vector<std::thread> th;
-    const size_t per = (n + nt - 1) / nt;
-    for (size_t t = 0; t < nt; t++) {
-        const size_t a = t * per, b = std::min(n, a + per);
-        if (a < b) th.emplace_back([=] { f(a, b); });
-    }
-    for (auto& x : th) x.join();
+    sw2d::split_over_threads(n, std::min<size_t>({16, std::thread::hardware_concurrency(), n / 8 + 1}), f);
 }
 
 int d2h(sw2d_handle* h, void* dst, const void* src, size_t bytes) {

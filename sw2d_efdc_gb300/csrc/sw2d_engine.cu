@@ -1,5 +1,6 @@
 /* Host engine of the FP32 precision form (see sw2d_engine.h). */
 #include "sw2d_engine.h"
+#include "sw2d_threads.h"
 
 #include <cudaTypedefs.h>
 
@@ -50,15 +51,7 @@ int pitch_of(int cols) { return ((cols + 12 + 31) / 32) * 32; }
  * work at most (a thread costs tens of microseconds to start) */
 template <typename F>
 void on_threads(size_t n, size_t work, size_t grain, F f) {
-    const size_t nt = std::max<size_t>(1, std::min<size_t>({16, std::thread::hardware_concurrency(), n, work / grain}));
-    if (nt == 1) {
-        f((size_t)0, n);
-        return;
-    }
-    std::vector<std::thread> th;
-    const size_t per = (n + nt - 1) / nt;
-    for (size_t a = 0; a < n; a += per) th.emplace_back([=] { f(a, std::min(n, a + per)); });
-    for (auto& x : th) x.join();
+    split_over_threads(n, std::min<size_t>({16, std::thread::hardware_concurrency(), n, work / grain}), f);
 }
 
 /* device arrays of a scenario in one allocation, each 256-byte aligned */
