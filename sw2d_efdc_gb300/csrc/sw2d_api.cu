@@ -553,7 +553,7 @@ int run_until(sw2d_handle* h, double t_end, long long max_iters, int64_t* done_o
             if ((rc = launch_iterations(h, n + (n & 1)))) return rc;
             CK(cudaEventRecord(h->ev_b, h->stream));
             if ((rc = read_report(h, &st))) return rc;
-            if (st.status & 1) return fail(SW2D_ERR_NUMERIC, "non-finite depth");
+            if (st.status & 1) break; /* reported below, with the iterations that ran */
         }
         CK(cudaEventRecord(h->ev_b, h->stream));
         CK(cudaEventSynchronize(h->ev_b));
