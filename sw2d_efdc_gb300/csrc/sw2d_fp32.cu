@@ -210,10 +210,6 @@ __device__ __forceinline__ int leftbits(int v) { /* bit k = column k; returns th
     const int up = __shfl_up_sync(0xffffffffu, v, 1);
     return ((up >> 1) & 1) | ((v & 1) << 1);
 }
-__device__ __forceinline__ int rightbits(int v) {
-    const int dn = __shfl_down_sync(0xffffffffu, v, 1);
-    return ((v >> 1) & 1) | ((dn & 1) << 1);
-}
 
 /* Upwind donor-cell transport across the edge between two faces of the same
  * orientation (the reference's umr/uml, umu/umd, vnr/vnl, vnu/vnd terms,
