@@ -1144,27 +1144,39 @@ int fp64_kernels_per_iteration() { return 2; }
 /* How a raster is cut into the update kernel's tiles and the flux kernel's
  * blocks: large ones for the smaller share of halo while there are many,
  * small ones so that a small raster reaches every SM (each block's chain of
- * dependent binary64 operations then holds fewer of them).  Measured, us an
- * iteration: update tiles 64 x 16 / 32 x 16 1809 / 1848 at 4096^2, 258.0 /
- * 258.3 at 1531 x 1207, 151 / 145 at 1024^2; 32 x 16 / 32 x 8 62.9 / 63.9 at
- * 701 x 556, 41.3 / 38.9 at 400^2; 32 x 8 / 32 x 4 24.1 / 24.1 at 256^2, 17.4
- * / 15.5 at 33 x 41.  Flux blocks of 8 / 4 rows (256 threads each): 63.9 /
- * 68.1 at 701 x 556, 38.9 / 37.4 at 400^2, 24.1 / 21.8 at 256^2, 17.4 / 15.7
- * at 33 x 41. */
+ * dependent binary64 operations then holds fewer of them).  Each line lies
+ * between the sizes where one side and the other is faster; measured, us an
+ * iteration, plain slopes / fractal terrain with lake terms and sources:
+ *   update tiles 64 x 16 against 32 x 16: 1482 / 1364 and 1510 / 1400 at
+ *     4096^2, 213.6 / 204.8 and 214.5 / 205.5 at 1450^2, 192.6 / 175.9 and
+ *     191.3 / 174.0 at 1361^2;
+ *   32 x 16 against 32 x 8: 56.4 / 49.1 and 57.7 / 50.8 at 600^2, 48.4 / 48.0
+ *     and 48.4 / 48.7 at 548^2, 35.7 / 33.9 and 34.0 / 32.4 at 400^2;
+ *   32 x 8 against 32 x 4: 27.5 / 28.6 and 28.6 / 28.5 at 330^2, 23.8 / 26.1
+ *     and 23.9 / 24.5 at 310^2, 21.2 / 21.7 and 20.3 / 20.1 at 256^2, 13.5 /
+ *     17.8 and 12.6 / 16.4 at 33^2;
+ *   flux blocks of 8 rows against 4 (256 threads each): 67.4 / 64.3 and 67.6
+ *     / 68.5 at 700^2, 52.4 / 46.8 and 50.7 / 48.9 at 566^2, 47.3 / 43.6 and
+ *     43.2 / 41.8 at 480^2;
+ *   flux blocks with 32 registers against 48: 1482 / 1364 and 1525 / 1422 at
+ *     4096^2, 118.9 / 108.2 and 119.7 / 110.2 at 1024^2, 86.5 / 80.2 and 86.6
+ *     / 81.5 at 836^2, 74.9 / 69.8 and 74.6 / 69.6 at 767^2. */
 struct Cut64 {
     int kind, tw, th, gx, gy;
     dim3 flux;
     int by;
+    bool lean; /* the flux kernel with 32 registers */
 };
 static Cut64 cut_of(int R, int C) {
     Cut64 k;
     const long long cells = (long long)(R + 1) * (C + 1);
-    k.kind = cells >= 1800000 ? 0 : cells >= 300000 ? 1 : cells >= 40000 ? 2 : 3;
+    k.kind = cells >= 2000000 ? 0 : cells >= 300000 ? 1 : cells >= 100000 ? 2 : 3;
     k.tw = k.kind == 0 ? 64 : 32;
     k.th = k.kind <= 1 ? 16 : k.kind == 2 ? 8 : 4;
     k.gx = (C + 1 + k.tw - 1) / k.tw;
     k.gy = (R + 1 + k.th - 1) / k.th;
     k.by = cells >= 320000 ? 8 : 4;
+    k.lean = cells >= 700000;
     k.flux = dim3((C + 1 + SW2D_BX - 1) / SW2D_BX, (R + 1 + k.by - 1) / k.by);
     return k;
 }
@@ -1202,7 +1214,7 @@ void fp64_launch_iteration(const StepParams& p, int cur, cudaStream_t s, cudaEve
     if (ev) cudaEventRecord(ev[0], s);
     const dim3 blk(SW2D_BX, 8);
     if (k.by == 4) chain_launch(k64_flux<4, 256, 5>, k.flux, blk, s, p, cur);
-    else if (k.kind > 0) chain_launch(k64_flux<8, 256, 5>, k.flux, blk, s, p, cur);
+    else if (!k.lean) chain_launch(k64_flux<8, 256, 5>, k.flux, blk, s, p, cur);
     else chain_launch(k64_flux<8, 256, 7>, k.flux, blk, s, p, cur);
     if (ev) cudaEventRecord(ev[1], s);
     const int n = k.gx * k.gy + 2;

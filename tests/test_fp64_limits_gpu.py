@@ -1,6 +1,6 @@
 """The FP64 step on both sides of every raster size at which its kernels are
-cut differently ((rows + 1)(cols + 1) = 40,000, 300,000, 320,000 and
-1,800,000) and above the largest, with the last row first and last in a row
+cut differently ((rows + 1)(cols + 1) = 100,000, 300,000, 320,000, 700,000 and
+2,000,000) and above the largest, with the last row first and last in a row
 of tiles, plain and with the terms whose sums go tile by tile.  Bit-identical
 to the oracle's device-math flavour (as every FP64 case); ledger sums, which
 are added in another order, within 1e-12."""
@@ -13,8 +13,8 @@ from tests.helpers import bumpy_case, model_from_case
 pytestmark = pytest.mark.gpu
 
 # below and at each limit; then 16-row tiles with the last row first (1344 = 84 x 16) and last in its tile
-SIZES = [(198, 200), (199, 199), (498, 600), (499, 599), (498, 640), (499, 639), (1198, 1500), (1199, 1499),
-         (1345, 1345), (1344, 1409)]
+SIZES = [(248, 400), (249, 399), (498, 600), (499, 599), (498, 640), (499, 639), (698, 1000), (699, 999), (1248, 1600),
+         (1249, 1599), (1345, 1500), (1344, 1499)]
 
 
 @pytest.mark.parametrize("R,C", SIZES)
