@@ -136,8 +136,12 @@ SW2D_HD double sw2d_scale_down(double x, int k) {
     if (e > (uint64_t)k) return sw2d_f64_from_bits(b - ((uint64_t)k << 52));
     /* result subnormal (or zero): the significand m counts units of 2^-1074
      * (of 2^(e - 1 - 1074) for e >= 1), so the result is m / 2^s rounded */
-    const uint64_t m = (e == 0) ? mag : (mag & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
-    const uint32_t s = e == 0 ? (uint32_t)k : (uint32_t)k + 1u - (uint32_t)e;
+    uint64_t m = (e == 0) ? mag : (mag & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
+    uint32_t s = (uint32_t)k;
+    if (e != 0) {
+        if (k <= 2) m <<= e - 1; /* shorter where k is known (a step at 33 x 41 10.0 us, 10.2 without) */
+        else s = (uint32_t)k + 1u - (uint32_t)e;
+    }
     const uint64_t q = m >> s, rem = m & ((1ULL << s) - 1), halfw = 1ULL << (s - 1);
     const uint64_t r = q + ((rem > halfw || (rem == halfw && (q & 1))) ? 1 : 0);
     return sw2d_f64_from_bits(sign | r);
