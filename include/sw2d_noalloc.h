@@ -15,14 +15,16 @@
  * the whole device, stalling the kernels the caller keeps in flight on other
  * streams.  This call makes no cudaMalloc, cudaFree or other allocating call.
  *
- * Scratch.  The per-tile partial results live in one file-scope device array
- * of the library, 393,240 bytes, so the raster may span at most
- * SW2D_NOALLOC_MAX_TILES tiles of 32 x 32 cells (4096 x 4096 cells, or any
- * rows x cols with ceil(rows/32) * ceil(cols/32) <= 16384); larger rasters are
- * rejected with SW2D_ERR_INVALID before anything is launched.  The partial
- * slots need no initial value (each is written before it is read); the
- * tile-completion counter must be zero when the kernel starts, and each call
- * clears it on `stream` before its launch.
+ * Scratch.  One file-scope device array of the library, 393,240 bytes: a
+ * volume per thread block (at most 456, each written before it is read), the
+ * running maxima of the x and y face speeds, which become the two results,
+ * and the count of finished blocks.  The maxima and the count must be zero
+ * when the kernel starts; each call clears them on `stream` before its launch.
+ * The array's size, and with it the limit of SW2D_NOALLOC_MAX_TILES tiles of
+ * 32 x 32 cells (4096 x 4096 cells, or any rows x cols with ceil(rows/32) *
+ * ceil(cols/32) <= 16384; larger rasters are rejected with SW2D_ERR_INVALID
+ * before anything is launched), are those of a version that kept three values
+ * a tile; callers may rely on both, so they stay.
  *
  * Rules for the caller.
  *  - Calls share the one scratch array per device: two calls in flight at the

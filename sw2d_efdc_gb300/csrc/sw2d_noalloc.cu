@@ -25,21 +25,23 @@ void set_error_message(const char* msg); /* sw2d_api.cu: the message sw2d_last_e
 
 namespace {
 
-constexpr int kTile = SW2D_NOALLOC_TILE;              /* 32 x 32 cells per CTA */
+constexpr int kTile = SW2D_NOALLOC_TILE;              /* of the raster limit (sw2d_noalloc.h) */
 constexpr int kMaxTiles = SW2D_NOALLOC_MAX_TILES;
 constexpr int kBand = 32;                             /* most rows of a warp's task */
 constexpr int kBatch = 4;                             /* of them read at once */
 constexpr int kBlocksPerSm = 3;
-constexpr int kSlots = 3;
+constexpr int kBlocks = kBlocksPerSm * 152;           /* the most: GB300's SMs */
+constexpr int kSlots = 3;                             /* a tile's share of the array, once its partials */
 constexpr int kResult = kSlots * kMaxTiles;           /* x and y speed maxima (bits), then volume * area and speed */
 constexpr int kCounter = kResult + 2;                 /* block-completion counter (low 32 bits) */
 constexpr int kScratchDoubles = kCounter + 1;         /* 49,155 doubles = 393,240 bytes */
 
-/* The scratch: room for kSlots partials per tile (the blocks' volumes take the
- * first of them), the two results, the counter. */
+/* The scratch: the blocks' volumes (the array's size is the interface's), the
+ * two maxima and then results, the counter. */
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
 static_assert(sizeof(double) * kScratchDoubles == 393240, "scratch size stated in sw2d_noalloc.h");
+static_assert(kBlocks <= kResult && kBlocks == 456, "the blocks' volumes, as sw2d_noalloc.h states them");
 
 /* (|velocity| + sqrt(g hm)) / spacing as the FP64 step evaluates it, raising a
  * running maximum kept as bits (non-negative doubles order like their bits).
@@ -99,7 +101,8 @@ struct MeasureIn {
  * pipe, a binary64 instruction taking a warp 71 cycles: a division and a
  * square root on every face.  The face speeds are estimated in binary32
  * instead (within 2.2e-6), and only lanes within 1e-5 of the running maximum
- * are evaluated in binary64 and raise it: the exact maximum in any order.
+ * are evaluated in binary64 and raise it, all lanes of a warp where an
+ * estimate says nothing (est_most and above): the exact maximum in any order.
  * One binary64 addition a cell is left, the volume's.  Bounded by the latency
  * of HBM reads: 4 rows of 32-row tasks in flight at three blocks an SM
  * measured 136 us for the whole call at 4096 x 3000 (393 MB), 2 rows at four
@@ -282,12 +285,11 @@ extern "C" int sw2d_measure_state_noalloc(const double* d_dem, const double* d_d
     in.rdxf = (float)in.rdx;
     in.rdyf = (float)in.rdy;
     /* fewer rows a task while the tasks would not reach every warp */
-    const int most = kBlocksPerSm * 152; /* GB300's SMs */
     const long long strips = (cols + 31LL) / 32;
     in.band = kBand;
-    while (in.band > kBatch && strips * ((rows + in.band - 1) / in.band) < 8LL * most) in.band /= 2;
+    while (in.band > kBatch && strips * ((rows + in.band - 1) / in.band) < 8LL * kBlocks) in.band /= 2;
     const long long tasks = strips * ((rows + in.band - 1LL) / in.band);
-    const int blocks = (int)std::min<long long>((tasks + 7) / 8, most);
+    const int blocks = (int)std::min<long long>((tasks + 7) / 8, kBlocks);
     k64_measure_noalloc<<<blocks, 256, 0, s>>>(in, scratch);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail("k64_measure_noalloc launch", e);
