@@ -484,10 +484,10 @@ int Engine32::remove(int index) {
  * the item's rows and their six halo rows in whole blocks of M_RB (what goes
  * by between iterations does not depend on the choice).  One scenario's items
  * run in whole waves over the CTAs; several scenarios fill one another's
- * gaps.  Measured, us an iteration: 200 x 310 cells 105 with items of 128
- * rows, 19 with 2; 1000^2 62 with 64, 34 with 18; 2048^2 130 with 128, 76 with
- * 38; from about 12 M cells on, items of seg_ rows fill the GPU and the halo
- * rows decide. */
+ * gaps.  Measured, us an iteration, with items of 128, 64 and 16 rows and with
+ * this rule's: 200 x 310 cells 101, 56, 24 and 13.7 (2 rows); 1000^2 103, 58,
+ * 32 and 28.3 (18); 2048^2 124, 85, 88 and 66.2 (46); from about 12 M cells on,
+ * items of seg_ rows fill the GPU and the halo rows decide. */
 int Engine32::fill_rows(int k) const {
     static const double row_us[4] = {0.70, 0.95, 1.19, 1.49};
     const int per_sm = std::max(1, cps_ > 0 ? std::min(cps_, bps_[k]) : bps_[k]);

@@ -898,8 +898,8 @@ __device__ __forceinline__ void put_sources32(const ScnBody32& P, Clock32* clk, 
  * past L1 (other SMs wrote them); the length is computed by every warp; the
  * ledger's entries are updated by one lane each; and sums that the scenario
  * cannot have, or whose terms are zero, are skipped.  11 to 16 thousand cycles
- * an iteration before, of 38 thousand at 200 x 310; an iteration there 19.0
- * us, now 14.7. */
+ * an iteration before, of 38 thousand at 200 x 310; an iteration there went
+ * from 19.0 to 14.7 us (13.7 with the steps after this one). */
 __device__ __noinline__ void finalize_scn(const ScnBody32& P, const Part32* __restrict__ part, double (*red)[4],
                                           float (*redf)[6]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -21,11 +21,11 @@
  *                extra block adds up the previous iteration's partials in a
  *                fixed order and prepares the next iteration's length and
  *                forcing beside the tiles.
- * At 4096 x 4096 (pond break) an iteration takes 1.28 ms (flux 0.87, update
- * 0.44) against 5.17 ms with part-empty warps, a binary64 provisional depth
- * and conversions and sums predicated off beside the path taken; at 256 x 256
- * 19.5 us against 62 us, most of it the clock's work at the end of the last
- * tile's block before.
+ * At 4096 x 4096 (pond break) an iteration takes 1.24 ms early in the run
+ * (flux 0.82, update 0.44) and 1.32 ms at t = 600 s (0.89, 0.44), against 5.17
+ * ms with part-empty warps, a binary64 provisional depth and conversions and
+ * sums predicated off beside the path taken; at 256 x 256 18.5 us against 62
+ * us, most of it the clock's work at the end of the last tile's block before.
  * forward (:670-693) is a buffer swap for the depth (h[cur] -> h[nxt]); the
  * discharges keep fixed roles: qx[0]/qy[0] hold the state, k64_flux writes
  * its new faces into qx[1]/qy[1], and k64_update writes every face, closed
@@ -326,9 +326,10 @@ __device__ __forceinline__ void copy8_async(double* to, const double* from, bool
                  : "memory");
 }
 
-/* mean depth of a face >= th, exactly: decided from the two cells' codes
- * unless th lies between their depths, then in binary32, in binary64 only
- * within its error */
+/* mean depth of a face >= th, exactly (true where the estimate is infinite,
+ * which sends the face to raise_speed_exact): decided from the two cells'
+ * codes unless th lies between their depths, then in binary32, in binary64
+ * only within its error */
 __device__ __forceinline__ bool mean_ge(double ha, double hb, int ca, int cb, float est, double th, float thf) {
     if (!((ca ^ cb) & kBelow)) return !(ca & kBelow);
     if (fabsf(est - thf) > 1e-5f * thf) return est > thf; /* not with thf NaN */
