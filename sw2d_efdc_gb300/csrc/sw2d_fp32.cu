@@ -761,8 +761,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, int slot, c
 
 /* the entry in force at `time`: sw2d_series_index with the division on the integer pipes */
 __device__ __forceinline__ int series_index32(double time, double dts, int n) {
-    const double f = sw2d_div_rn(time, dts);
-    return f >= (double)n ? n : (int)f;
+    return sw2d_series_entry(sw2d_div_rn(time, dts), n);
 }
 
 /* the series' value at `time`, with a its entry in force (the it-th) and b the next */
@@ -869,7 +868,7 @@ __device__ __forceinline__ void put_rates32(const ScnBody32& P, Clock32* clk, co
     if (spacing) {
         r = (float)f;
     } else if (v) {
-        const int nv = ev ? P.nevap : P.nrain, it = f >= (double)nv ? nv : (int)f;
+        const int it = sw2d_series_entry(f, ev ? P.nevap : P.nrain);
         if (lane & 1) s.entry[ev] = it;
         const int from = it - ahead.it; /* 0 or 1 unless the iteration is long */
         const double a = from == 0 ? ahead.v[0] : from == 1 ? ahead.v[1] : v[it];

@@ -47,8 +47,7 @@ namespace sw2d {
 
 /* the entry in force at `time`: sw2d_series_index with the division on the integer pipes */
 __device__ __forceinline__ int series_index(double time, double dts, int n) {
-    const double f = sw2d_div_rn(time, dts);
-    return f >= (double)n ? n : (int)f;
+    return sw2d_series_entry(sw2d_div_rn(time, dts), n);
 }
 
 __device__ __forceinline__ double series_at(const double* v, int n, double dts, double time, int mode) {

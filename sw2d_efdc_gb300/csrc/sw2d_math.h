@@ -39,15 +39,22 @@
 #endif
 
 /* Index of the series entry in force at `time` (one entry every dts
- * seconds), clamped to n, the first entry of the series' zero tail: the
- * reference's int(time / dts) (SW2D-EFDC.cu:537, :550) without reading past
- * the series.  The clamp is decided in binary64, so a quotient beyond the
- * int range (a long run with a short series interval) clamps instead of
- * converting out of range. */
-SW2D_HD int sw2d_series_index(double time, double dts, int n) {
-    const double f = time / dts;
-    return f >= (double)n ? n : (int)f;
+ * seconds), clamped to n, the first entry of the series' zero tail, and to
+ * the first entry (a clock that starts before time 0): the reference's
+ * int(time / dts) (SW2D-EFDC.cu:537, :550) without reading outside the
+ * series.  The clamps are decided on the quotient f = time / dts, so one
+ * beyond the int range (a long run with a short series interval) clamps
+ * instead of converting out of range. */
+SW2D_HD int sw2d_series_entry(double f, int n) {
+#if defined(__CUDA_ARCH__)
+    /* the conversion saturates, and of NaN gives 0 or the least int */
+    const int it = f >= (double)n ? n : (int)f;
+    return it > 0 ? it : 0;
+#else
+    return f >= (double)n ? n : f > 0.0 ? (int)f : 0;
+#endif
 }
+SW2D_HD int sw2d_series_index(double time, double dts, int n) { return sw2d_series_entry(time / dts, n); }
 
 /* 1.3333330 - 4/3 evaluated exactly (binary64 value of 1.3333330 minus the
  * real 4/3), then rounded to binary64. */
