@@ -56,7 +56,7 @@ namespace sw2d {
 #define NF 5 /* staged fields: h, z, qx, qy, Kahan compensation (three rows behind) */
 
 struct alignas(128) ClsStage {
-    unsigned char v[M_CLSR][M_CLSW]; /* rows L-1 .. L+RB-2 of the block's first row L */
+    unsigned char v[M_CLSR][M_CLSW]; /* rows L-2 .. L+RB-1 of the block's first row L */
 };
 struct alignas(128) RwStage {
     float v[M_RWR][BW]; /* rows L-3 .. L+RB-2 */
@@ -334,7 +334,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, int slot, c
                                (has_rw ? (unsigned)(M_RWR * BW * 4) : 0u);
     /* block b holds rows Ls + b*RB .. +RB-1 of h, z, qx, qy, the Kahan
      * compensation of the rows three above (the rows finished during b) and,
-     * when present, the class rows from one above and the rain weights from
+     * when present, the class rows from two above and the rain weights from
      * three above */
     auto issue = [&](int b, int st, int part) { /* part: 0..3 for one of four issuers, 4 for all of it */
         const int y = Ls + b * RB + M_H; /* padded row of the block's first row */
@@ -344,7 +344,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, int slot, c
         }
         if (part == 1 || part == 4) {
             tma_load_2d(&S.stage[st][1][0][0], &P.tm_z, c0, y, &S.bar[st]);
-            if (has_cls) tma_load_2d(&S.cls[st].v[0][0], &P.tm_cls, c0, y - 1, &S.bar[st]);
+            if (has_cls) tma_load_2d(&S.cls[st].v[0][0], &P.tm_cls, c0, y - 2, &S.bar[st]);
         }
         if (part == 2 || part == 4) {
             tma_load_2d(&S.stage[st][2][0][0], &P.tm_qx[cur], c0, y, &S.bar[st]);
@@ -571,7 +571,7 @@ __device__ __forceinline__ bool march_item(SmemM& S, const Scn32& P, int slot, c
                 f.vt = mul2(add2(VV[s1], VV[s2]), f2(0.25f));
                 f.conv = fma2(sub2(EX[s1], EX[s2]), f2(dt2dx), mul2(mul2(sub2(GX, left2(GX)), f2(dt2dy)), colm));
                 if (has_cls) { /* face n = mean of the two cells' n (the row above's from the last row) */
-                    const unsigned char* c1 = scl + j * M_CLSW + sc;
+                    const unsigned char* c1 = scl + (j + 1) * M_CLSW + sc;
                     const float2 n1 = make_float2(S.ntab[c1[0] & 63], S.ntab[c1[1] & 63]);
                     const float2 nf = mul2(add2(n1, NC), f2(0.5f));
                     f.fr = mul2(mul2(nf, nf), f2(fr_scale));
