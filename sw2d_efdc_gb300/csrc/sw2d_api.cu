@@ -409,10 +409,13 @@ int launch_iterations(sw2d_handle* h, long long n) {
     const long long full = n / kChunk, rem = n % kChunk;
     int rc;
     if (full > 0 && (rc = build_graph(h))) return rc;
-    for (long long k = 0; k < full; k++) CK(cudaGraphLaunch(h->graph, h->stream));
+    cudaError_t refused = cudaSuccess;
+    for (long long k = 0; k < full && refused == cudaSuccess; k++) refused = cudaGraphLaunch(h->graph, h->stream);
     StepParams p = h->params();
-    for (long long k = 0; k < rem; k++) fp64_launch_iteration(p, (int)(k & 1), h->stream, nullptr);
-    fp64_launch_settle(p, h->stream);
+    if (refused == cudaSuccess)
+        for (long long k = 0; k < rem; k++) fp64_launch_iteration(p, (int)(k & 1), h->stream, nullptr);
+    fp64_launch_settle(p, h->stream); /* of the iterations that were launched */
+    CK(refused);
     CK(cudaGetLastError());
     return SW2D_OK;
 }

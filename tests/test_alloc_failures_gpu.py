@@ -1,8 +1,9 @@
-"""Failed allocations, made by fakes of the failing calls (the library's own
-objects linked with them wrapped): without pinned staging a raster's inputs go
-through pageable memory, and a scenario or a raster that finds no device
-memory does not spoil the ones that run.  Results: the same bits as without
-the failure."""
+"""Failed allocations and launches, made by fakes of the failing calls (the
+library's own objects linked with them wrapped): without pinned staging a
+raster's inputs go through pageable memory, a scenario or a raster that finds
+no device memory does not spoil the ones that run, and after a launch that was
+refused state and ledger are those of the iterations that ran.  Results: the
+same bits as without the failure."""
 import glob
 import os
 import subprocess
@@ -21,6 +22,13 @@ FAKES = r"""
 #include <cuda_runtime.h>
 extern "C" {
 int fail_pinned = 0, fail_device = 0; /* how many calls to refuse, of cudaMalloc those of 800 kB and more */
+int graphs_left = -1;                 /* graph launches until all are refused (-1: never) */
+cudaError_t __real_cudaGraphLaunch(cudaGraphExec_t g, cudaStream_t s);
+cudaError_t __wrap_cudaGraphLaunch(cudaGraphExec_t g, cudaStream_t s) {
+    if (graphs_left == 0) return cudaErrorMemoryAllocation;
+    if (graphs_left > 0) graphs_left--;
+    return __real_cudaGraphLaunch(g, s);
+}
 cudaError_t __real_cudaMalloc(void** p, size_t n);
 cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
     if (fail_device <= 0 || n < 800000) return __real_cudaMalloc(p, n);
@@ -111,6 +119,36 @@ m.step(20)
 np.savez(sys.argv[4], **dict(zip(("h", "qx", "qy"), m.state())))
 """
 
+LAUNCH = r"""
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+from sw2d_efdc_gb300 import api
+lib = api.load(sys.argv[2])
+m = api.Model(api.default_config(rows=100, cols=90, dx=2.0, dy=2.0, dt_mode=api.DT_CFL, series_mode=api.SERIES_STEP,
+                                 outflow=api.OUTFLOW_SOUTH, manning=0.03))
+m.set_dem(0.01 * np.arange(100)[::-1, None] + np.zeros((100, 90)))
+m.set_rain_series(np.full(4, 5.0), 300.0)
+m.set_depth(np.full((100, 90), 0.02))
+n = ctypes.c_int.in_dll(lib, "graphs_left")
+if int(sys.argv[3]):
+    n.value = 2
+    try:
+        m.step(160)
+        assert False
+    except api.Sw2dError as e:
+        assert e.code == -3
+    n.value = -1
+else:
+    m.step(64)
+led = m.ledger()
+out = dict(zip(("h", "qx", "qy"), m.state()), ledger=np.array([led[k] for k in sorted(led)]))
+m.step(64)
+led = m.ledger()
+out["later"] = np.array([led[k] for k in sorted(led)])
+np.savez(sys.argv[4], **out)
+"""
+
 
 @pytest.fixture(scope="module")
 def variant(tmp_path_factory):
@@ -120,7 +158,8 @@ def variant(tmp_path_factory):
     so = d / "libsw2d_fakes.so"
     subprocess.check_call([build.nvcc()] + build.ARCH + ["-shared", "-Xcompiler", "-fPIC", str(d / "fakes.cu")] +
                           sorted(glob.glob(os.path.join(build.OBJ_DIR, "*.o"))) +
-                          ["-Xlinker", "--wrap=cudaMalloc", "-Xlinker", "--wrap=cudaMallocHost", "-o", str(so)])
+                          ["-Xlinker", "--wrap=cudaMalloc", "-Xlinker", "--wrap=cudaMallocHost",
+                           "-Xlinker", "--wrap=cudaGraphLaunch", "-o", str(so)])
     return d, so
 
 
@@ -150,3 +189,7 @@ def test_no_device_memory_waits(variant):
 
 def test_a_raster_that_finds_no_device_memory(variant):
     assert _same(_run(variant, CREATE, "refused", 1), _run(variant, CREATE, "plain", 0))
+
+
+def test_a_refused_launch_leaves_the_iterations_that_ran(variant):
+    assert _same(_run(variant, LAUNCH, "refused", 1), _run(variant, LAUNCH, "plain", 0))
