@@ -22,8 +22,8 @@
  *                fixed order and prepares the next iteration's length and
  *                forcing beside the tiles.
  * At 4096 x 4096 (pond break) an iteration takes 1.24 ms early in the run
- * (flux 0.82, update 0.44) and 1.32 ms at t = 600 s (0.89, 0.44), against 5.17
- * ms with part-empty warps, a binary64 provisional depth and conversions and
+ * (timed apart: flux 0.82, update 0.44) and 1.32 ms at t = 600 s (0.89, 0.44),
+ * against 5.17 ms with part-empty warps, a binary64 provisional depth and conversions and
  * sums predicated off beside the path taken; at 256 x 256 18.5 us against 62
  * us, most of it the clock's work at the end of the last tile's block before.
  * forward (:670-693) is a buffer swap for the depth (h[cur] -> h[nxt]); the
